@@ -15,13 +15,13 @@
 // regions with its running value/error sums, its Gladwell batch (pop the largest
 // errors until the rest is within tolerance), its cut and its push order, so the
 // refinement follows the reference's; the block's half-warps evaluate the 15-point
-// Gauss-Kronrod rule of one region each, and lane 0 of each half-warp forms the
-// rule's value and QUADPACK error in the reference's operation order
-// (src/hcubature.cpp:620-765, 772-1021).  The heap and the batch live in shared memory.
+// Gauss-Kronrod rule of one region each and form its value and QUADPACK error across
+// their lanes (src/hcubature.cpp:620-765, 772-1021).  The heap and the batch live in shared memory.
 // Integral parameters (radii, growth factors, grids) are computed on the host with
 // the reference's expressions; the integrands and the tables are evaluated here.
-// Compiled with -fmad=false, so results differ from the reference only by the
-// device libm's last-ulp differences in sin, cos, exp, log and pow.
+// Compiled with -fmad=false; results differ from the reference by the device libm's
+// last-ulp differences, the order of the rule's sums and the divisions merged in the
+// sigma^2 integrands (~1e-16 relative per operation; tables within 1e-13).
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -105,12 +105,6 @@ __device__ __forceinline__ double tophat(double k, double R)
     double x = k * R;
     return 3 / x / x / x * (sin(x) - x * cos(x));
 }
-__device__ __forceinline__ double d_tophat(double k, double R)
-{   // src/Powerspectrum.cpp:110-114
-    double x = k * R;
-    return ((x * x - 3.) * sin(x) + 3. * x * cos(x)) * 3 * k / x / x / x / x;
-}
-
 // The Eisenstein & Hu (1998, ApJ 496, 605) transfer function with baryon acoustic
 // terms: eqs. 17-21 (CDM part T_c with the ln/C fitting forms), eqs. 21-24 (baryon part
 // T_b with the node shift s_tilde and Silk damping), weighted by the baryon fraction.
@@ -146,6 +140,85 @@ __device__ __forceinline__ double spectrum(const PkDev &P, double k, double gz)
     return P.amplitude * trans * trans * gz * gz * pow(k, P.ns);
 }
 
+// The k-dependent factors of the sigma^2 integrands, amplitude T(k)^2 and k^ns, do not
+// depend on the radius or redshift, and every sigma^2 and dsigma^2/dm integral bisects the
+// same interval [0, 1e12], so its regions are nodes of one tree: ~2.4M regions of a 64-bin
+// call visit a few thousand distinct nodes.  The factors are nearly all of a point's FP64
+// work (two logarithms, seven pow and an exp in the transfer function), so each node's 15
+// pairs are kept in a hash table in device memory for the length of the call, keyed by the
+// region's centre and half-width.  A slot is claimed by compare-and-swap and published
+// with a release store; a reader that meets a slot being filled, a full table or a probe
+// run of PC_PROBES evaluates its node itself, so nothing waits and every value is that of
+// the same expressions either way.  Measured on the 64-bin tables: 98.7 -> 12.3 ms.
+struct PcNode {
+    double c, hw;            // key
+    double at[15], pk[15];   // amplitude T^2 and k^ns at the 15 abscissae
+};
+constexpr int PC_CACHE_LOG2 = 15;  // 32768 nodes, 8.4 MB (L2-resident)
+constexpr int PC_PROBES = 16;
+
+struct PcCache {
+    PcNode *node;     // null: no cache (the integrals before the amplitude is known)
+    unsigned *state;  // 0 free, 1 being filled, 2 ready
+};
+
+__device__ __forceinline__ unsigned ld_acquire(const unsigned *p)
+{
+    unsigned v;
+    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+    return v;
+}
+__device__ __forceinline__ void st_release(unsigned *p, unsigned v)
+{
+    asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+}
+
+// Find node (c, hw): mode 2 = ready at the returned slot, 1 = claimed by this caller (to
+// be filled and published), 0 = evaluate without the table.
+__device__ int pc_find(const PcCache &C, double c, double hw, int &mode)
+{
+    const unsigned long long k0 = (unsigned long long)__double_as_longlong(c);
+    const unsigned long long k1 = (unsigned long long)__double_as_longlong(hw);
+    unsigned ix = (unsigned)(((k0 * 0x9E3779B97F4A7C15ull) ^ (k1 * 0xC2B2AE3D27D4EB4Full)) >>
+                             (64 - PC_CACHE_LOG2));
+    for (int p = 0; p < PC_PROBES; ++p, ix = (ix + 1) & ((1u << PC_CACHE_LOG2) - 1)) {
+        unsigned st = ld_acquire(C.state + ix);
+        if (st == 0) {
+            st = atomicCAS(C.state + ix, 0u, 1u);
+            if (st == 0) {
+                mode = 1;
+                return (int)ix;
+            }
+        }
+        if (st == 1) break;  // being filled, perhaps by this node's first visitor
+        const double nc = __ldcg(&C.node[ix].c), nh = __ldcg(&C.node[ix].hw);
+        if (st == 2 && __double_as_longlong(nc) == (long long)k0 &&
+            __double_as_longlong(nh) == (long long)k1) {
+            mode = 2;
+            return (int)ix;
+        }
+    }
+    mode = 0;
+    return -1;
+}
+
+// sigma^2 and dsigma^2/dm integrands from at = amplitude T^2 and pk = k^ns at k = x, in
+// the operation order of spectrum()
+__device__ __forceinline__ double sigma_integrand(const PcTask &t, double x, double at, double pk)
+{
+    const double y = x * t.R;
+    double sy, cy;
+    sincos(y, &sy, &cy);
+    // the top-hat's W = 3 (sin y - y cos y) / y^3 and its derivative with one division each
+    const double q = 3 / (y * y * y);
+    const double W = q * (sy - y * cy);
+    const double ps = at * t.gz * t.gz * pk;
+    if (t.type == PC_SIGMA2) return x * x * W * W * ps;  // src/Powerspectrum.cpp:219-243
+    // src/Powerspectrum.cpp:110-114, 267-293
+    const double Wprime = ((y * y - 3.) * sy + 3. * y * cy) * x * q / y;
+    return x * x * W * Wprime * t.dR * ps;
+}
+
 __device__ double integrand(const PkDev &P, const PcTask &t, double x)
 {
     switch (t.type) {
@@ -155,64 +228,53 @@ __device__ double integrand(const PkDev &P, const PcTask &t, double x)
         double T = transfer(P, x);
         return W * W * T * T * pow(x, P.ns + 2);
     }
-    case PC_SIGMA2: {  // src/Powerspectrum.cpp:219-243
-        double W = tophat(x, t.R);
-        return x * x * W * W * spectrum(P, x, t.gz);
-    }
-    case PC_DSIGMA2: {  // src/Powerspectrum.cpp:267-293
-        double W = tophat(x, t.R);
-        double Wprime = d_tophat(x, t.R);
-        return x * x * W * Wprime * t.dR * spectrum(P, x, t.gz);
-    }
-    default:  // comoving distance integrand c/H0/sqrt(E(z)) (src/Cosmology.cpp:101-122)
+    default:  // comoving distance integrand c/H0/sqrt(E(z)) (src/Cosmology.cpp:101-122);
+              // PC_SIGMA2 and PC_DSIGMA2 are evaluated by sigma_integrand
         return kC / P.H0 / sqrt(E_of(P, x));
     }
 }
 
-// 15-point Gauss-Kronrod value and QUADPACK error of one region from its point values
-// in the reference's order (centre, then the Gauss pairs, then the Kronrod pairs)
-__device__ void rule_gk15(const double *vk, double hw, double &val, double &err)
+// 15-point Gauss-Kronrod value and QUADPACK error of one region (src/hcubature.cpp:
+// 675-740), formed across the 16 lanes of a half-warp (lane i holds the value at abscissa i
+// of gk_point's order; lane 15 holds nothing): the reference's sums in another order.  An
+// FP64 instruction occupies the pipe for 64 cycles however few lanes take part, so one lane
+// per region summing 15 values three times cost more than the integrand; the power 3/2 is
+// x sqrt(x) (an FP64 pow is ~75 instructions).  Valid in lane 0 of the half-warp.
+__device__ __forceinline__ void rule_gk15_hw(double f, int hl, double hw, double &val, double &err)
 {
-    double rg = vk[0] * cWg[3], rk = vk[0] * cWgk[7];
-    double rabs = fabs(rk);
-    int n = 1;
-    for (int j = 0; j < 3; ++j) {
-        int j2 = 2 * j + 1;
-        double v = vk[n] + vk[n + 1];
-        rg += cWg[j] * v;
-        rk += cWgk[j2] * v;
-        rabs += cWgk[j2] * (fabs(vk[n]) + fabs(vk[n + 1]));
-        n += 2;
+    // abscissa i: 0 centre, then pairs (2j+1, 2j+2): Gauss-Kronrod pair j (Kronrod-only
+    // nodes for j = 0, 2, 4, 6 of cXgk; Gauss nodes for odd j)
+    double wk = 0, wg = 0;
+    if (hl == 0) {
+        wk = cWgk[7];
+        wg = cWg[3];
+    } else if (hl < 7) {  // pairs j = 0..2: Gauss nodes cXgk[2j+1]
+        const int j = (hl - 1) >> 1;
+        wk = cWgk[2 * j + 1];
+        wg = cWg[j];
+    } else if (hl < 15) {  // pairs j = 3..6: Kronrod nodes cXgk[2(j-3)]
+        const int j = (hl - 1) >> 1;
+        wk = cWgk[2 * (j - 3)];
     }
-    for (int j = 0; j < 4; ++j) {
-        int j2 = 2 * j;
-        rk += cWgk[j2] * (vk[n] + vk[n + 1]);
-        rabs += cWgk[j2] * (fabs(vk[n]) + fabs(vk[n + 1]));
-        n += 2;
+    double rk = wk * f, rg = wg * f, ra = wk * fabs(f);
+    for (int o = 8; o > 0; o >>= 1) {
+        rk += __shfl_xor_sync(0xffffffffu, rk, o, 16);
+        rg += __shfl_xor_sync(0xffffffffu, rg, o, 16);
+        ra += __shfl_xor_sync(0xffffffffu, ra, o, 16);
     }
+    const double mean = rk * 0.5;
+    double rs = wk * fabs(f - mean);
+    for (int o = 8; o > 0; o >>= 1) rs += __shfl_xor_sync(0xffffffffu, rs, o, 16);
     val = rk * hw;
-    double mean = rk * 0.5;
-    double rasc = cWgk[7] * fabs(vk[0] - mean);
-    n = 1;
-    for (int j = 0; j < 3; ++j) {
-        int j2 = 2 * j + 1;
-        rasc += cWgk[j2] * (fabs(vk[n] - mean) + fabs(vk[n + 1] - mean));
-        n += 2;
-    }
-    for (int j = 0; j < 4; ++j) {
-        int j2 = 2 * j;
-        rasc += cWgk[j2] * (fabs(vk[n] - mean) + fabs(vk[n + 1] - mean));
-        n += 2;
-    }
     double e = fabs(rk - rg) * hw;
-    rabs *= hw;
-    rasc *= hw;
+    const double rabs = ra * hw, rasc = rs * hw;
     if (rasc != 0 && e != 0) {
-        double scale = pow((200 * e / rasc), 1.5);
+        const double q = 200 * e / rasc;
+        const double scale = q * sqrt(q);
         e = (scale < 1) ? rasc * scale : rasc;
     }
     if (rabs > DBL_MIN / (50 * DBL_EPSILON)) {
-        double min_err = 50 * DBL_EPSILON * rabs;
+        const double min_err = 50 * DBL_EPSILON * rabs;
         if (min_err > e) e = min_err;
     }
     err = e;
@@ -236,7 +298,12 @@ __device__ __forceinline__ bool converged(double err, double val)
     return !(err > 0 && err > fabs(val) * 1e-4);
 }
 
-// the reference's heap discipline (src/hcubature.cpp:772-890), on shared arrays
+// the reference's heap discipline (src/hcubature.cpp:772-890), on shared arrays.  Errors
+// are >= 0, so they are compared by bit pattern (an FP64 compare occupies the FP64 pipe for
+// 64 cycles), and the sifted entry is moved once, into the hole its path leaves, instead of
+// being swapped down level by level.
+__device__ __forceinline__ long long ebits(double e) { return __double_as_longlong(e); }
+
 __device__ void heap_push(Heap H, int &n, double &hv, double &he, double c, double hw, double v,
                           double e)
 {
@@ -245,7 +312,7 @@ __device__ void heap_push(Heap H, int &n, double &hv, double &he, double c, doub
     int ins = n++;
     while (ins) {
         int parent = (ins - 1) / 2;
-        if (e <= H.err[parent]) break;
+        if (ebits(e) <= ebits(H.err[parent])) break;
         H.c[ins] = H.c[parent];
         H.hw[ins] = H.hw[parent];
         H.val[ins] = H.val[parent];
@@ -266,23 +333,26 @@ __device__ void heap_pop(Heap H, int &nn, double &hv, double &he, double &c, dou
     v = H.val[0];
     e = H.err[0];
     const int n = nn - 1;
-    H.c[0] = H.c[n];
-    H.hw[0] = H.hw[n];
-    H.val[0] = H.val[n];
-    H.err[0] = H.err[n];
+    const double lc = H.c[n], lh = H.hw[n], lv = H.val[n], le = H.err[n];
+    const long long lb = ebits(le);
     nn = n;
     int i = 0, child;
     while ((child = i * 2 + 1) < n) {
-        int largest = (H.err[child] <= H.err[i]) ? i : child;
-        if (++child < n && H.err[largest] < H.err[child]) largest = child;
+        long long cb = ebits(H.err[child]);
+        int largest = cb <= lb ? i : child;
+        long long gb = cb <= lb ? lb : cb;
+        if (++child < n && gb < ebits(H.err[child])) largest = child;
         if (largest == i) break;
-        double t;
-        t = H.c[i]; H.c[i] = H.c[largest]; H.c[largest] = t;
-        t = H.hw[i]; H.hw[i] = H.hw[largest]; H.hw[largest] = t;
-        t = H.val[i]; H.val[i] = H.val[largest]; H.val[largest] = t;
-        t = H.err[i]; H.err[i] = H.err[largest]; H.err[largest] = t;
+        H.c[i] = H.c[largest];
+        H.hw[i] = H.hw[largest];
+        H.val[i] = H.val[largest];
+        H.err[i] = H.err[largest];
         i = largest;
     }
+    H.c[i] = lc;
+    H.hw[i] = lh;
+    H.val[i] = lv;
+    H.err[i] = le;
     hv -= v;
     he -= e;
 }
@@ -528,6 +598,7 @@ __device__ PcOut gk_integrate_sorted(double lo, double hi, double *sm, const Eva
 struct PcEval {
     const PkDev &P;
     const PcTask &t;
+    const PcCache &C;
     __device__ void operator()(int nb, const double *bc, const double *bh, double *bv,
                                double *be) const
     {
@@ -536,11 +607,44 @@ struct PcEval {
         for (int r0 = 2 * warp; r0 < nb; r0 += 2 * nwarps) {
             const int r = r0 + half;
             double f = 0;
-            if (r < nb && hl < 15) f = integrand(P, t, gk_point(bc[r], bh[r], hl));
-            double vk[15];
-#pragma unroll
-            for (int k = 0; k < 15; ++k) vk[k] = __shfl_sync(0xffffffffu, f, k, 16);
-            if (r < nb && hl == 0) rule_gk15(vk, bh[r], bv[r], be[r]);
+            if (t.type == PC_SIGMA2 || t.type == PC_DSIGMA2) {  // block-uniform
+                int mode = 0, ix = -1;
+                if (r < nb && hl == 0) ix = pc_find(C, bc[r], bh[r], mode);
+                mode = __shfl_sync(0xffffffffu, mode, 0, 16);
+                ix = __shfl_sync(0xffffffffu, ix, 0, 16);
+                if (r < nb && hl < 15) {
+                    const double x = gk_point(bc[r], bh[r], hl);
+                    double at, pk;
+                    if (mode == 2) {
+                        at = __ldcg(&C.node[ix].at[hl]);
+                        pk = __ldcg(&C.node[ix].pk[hl]);
+                    } else {
+                        const double trans = transfer(P, x);
+                        at = P.amplitude * trans * trans;
+                        pk = pow(x, P.ns);
+                        if (mode == 1) {
+                            C.node[ix].at[hl] = at;
+                            C.node[ix].pk[hl] = pk;
+                            if (hl == 0) {
+                                C.node[ix].c = bc[r];
+                                C.node[ix].hw = bh[r];
+                            }
+                            __threadfence();  // before lane 0's release below
+                        }
+                    }
+                    f = sigma_integrand(t, x, at, pk);
+                }
+                __syncwarp();
+                if (hl == 0 && mode == 1) st_release(C.state + ix, 2u);
+            } else if (r < nb && hl < 15) {
+                f = integrand(P, t, gk_point(bc[r], bh[r], hl));
+            }
+            double v, e;
+            rule_gk15_hw(f, hl, r < nb ? bh[r] : 1.0, v, e);
+            if (r < nb && hl == 0) {
+                bv[r] = v;
+                be[r] = e;
+            }
         }
     }
 };
@@ -551,14 +655,15 @@ template <int CAP>
 __global__ void __launch_bounds__(PC_THREADS) k_pc_integrate(const PkDev *__restrict__ Pp,
                                                              const PcTask *__restrict__ tasks,
                                                              const int *__restrict__ idx,
-                                                             int ntask, PcOut *__restrict__ out)
+                                                             int ntask, PcOut *__restrict__ out,
+                                                             PcCache C)
 {
     extern __shared__ double sm[];
     const PkDev P = *Pp;
     for (int tj = blockIdx.x; tj < ntask; tj += gridDim.x) {
         const int ti = idx ? idx[tj] : tj;
         const PcTask t = tasks[ti];
-        const PcOut o = gk_integrate<CAP>(t.lo, t.hi, sm, PcEval{P, t});
+        const PcOut o = gk_integrate<CAP>(t.lo, t.hi, sm, PcEval{P, t, C});
         if (threadIdx.x == 0) out[ti] = o;
     }
 }
@@ -662,49 +767,6 @@ __global__ void __launch_bounds__(256) k_nbar_factors(NbarArgs A, int nh)
         A.fS[t] = S;
         A.fmix[t] = mix;
     }
-}
-
-// The 15-point Gauss-Kronrod value and QUADPACK error of rule_gk15, formed across the
-// 16 lanes of a half-warp (lane i holds the value at abscissa i of gk_point's order;
-// lane 15 holds nothing) instead of by one lane: the same sums in another order.
-// Valid in lane 0 of the half-warp.
-__device__ __forceinline__ void rule_gk15_hw(double f, int hl, double hw, double &val, double &err)
-{
-    // abscissa i: 0 centre, then pairs (2j+1, 2j+2): Gauss-Kronrod pair j (Kronrod-only
-    // nodes for j = 0, 2, 4, 6 of cXgk; Gauss nodes for odd j)
-    double wk = 0, wg = 0;
-    if (hl == 0) {
-        wk = cWgk[7];
-        wg = cWg[3];
-    } else if (hl < 7) {  // pairs j = 0..2: Gauss nodes cXgk[2j+1]
-        const int j = (hl - 1) >> 1;
-        wk = cWgk[2 * j + 1];
-        wg = cWg[j];
-    } else if (hl < 15) {  // pairs j = 3..6: Kronrod nodes cXgk[2(j-3)]
-        const int j = (hl - 1) >> 1;
-        wk = cWgk[2 * (j - 3)];
-    }
-    double rk = wk * f, rg = wg * f, ra = wk * fabs(f);
-    for (int o = 8; o > 0; o >>= 1) {
-        rk += __shfl_xor_sync(0xffffffffu, rk, o, 16);
-        rg += __shfl_xor_sync(0xffffffffu, rg, o, 16);
-        ra += __shfl_xor_sync(0xffffffffu, ra, o, 16);
-    }
-    const double mean = rk * 0.5;
-    double rs = wk * fabs(f - mean);
-    for (int o = 8; o > 0; o >>= 1) rs += __shfl_xor_sync(0xffffffffu, rs, o, 16);
-    val = rk * hw;
-    double e = fabs(rk - rg) * hw;
-    const double rabs = ra * hw, rasc = rs * hw;
-    if (rasc != 0 && e != 0) {
-        const double scale = pow((200 * e / rasc), 1.5);
-        e = (scale < 1) ? rasc * scale : rasc;
-    }
-    if (rabs > DBL_MIN / (50 * DBL_EPSILON)) {
-        const double min_err = 50 * DBL_EPSILON * rabs;
-        if (min_err > e) e = min_err;
-    }
-    err = e;
 }
 
 // one thread per (HOD, edge, depth, side, abscissa): walk from the root towards the edge
@@ -840,37 +902,60 @@ struct TableArgs {
     int *mstar_ix;                      // [N]
 };
 
-__global__ void k_pc_zrow(const PkDev *__restrict__ Pp, TableArgs A)
+// one warp per redshift
+__global__ void __launch_bounds__(128) k_pc_zrow(const PkDev *__restrict__ Pp, TableArgs A)
 {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
     if (i >= A.N) return;
     const PkDev P = *Pp;
     const double z = A.zs[i];
-    // lensing efficiency (src/Cosmology.cpp:132-150)
+    // lensing efficiency (src/Cosmology.cpp:132-150): the lanes form the terms, summed in
+    // the reference's order
     const double wz = A.chi_z[i].val;
     double r = 0;
-    for (int j = 0; j < A.Ns; ++j) {
-        const double zp = A.zsrc[j];
-        const double wp = A.chi_src[j].val;
-        if (zp >= z) r += A.nzsrc[j] * (wp - wz) / wp;
+    for (int j0 = 0; j0 < A.Ns; j0 += 32) {
+        const int j = j0 + lane;
+        double q = 0;
+        bool on = false;
+        if (j < A.Ns && A.zsrc[j] >= z) {
+            const double wp = A.chi_src[j].val;
+            q = A.nzsrc[j] * (wp - wz) / wp;
+            on = true;
+        }
+        unsigned m = __ballot_sync(0xffffffffu, on);
+        for (; m; m &= m - 1) r += __shfl_sync(0xffffffffu, q, __ffs(m) - 1);
     }
-    A.g[i] = r * A.deltaZ;
-    A.w[i] = wz;
-    A.dwdz[i] = kC / P.H0 / sqrt(E_of(P, z));  // src/Cosmology.cpp:101-104
     // M*(z): the first of the masses closest to sigma = delta_c (src/Powerspectrum.cpp:117-140)
     const double dc = delta_c(P, z);
     int best = 0;
     double bd = 0;
-    for (int j = 0; j < A.Nstar; ++j) {
+    bool have = false;
+    for (int j = lane; j < A.Nstar; j += 32) {
         const double s2 = A.sig_star[(size_t)i * A.Nstar + j].val / 2 / kPi / kPi;
         const double diff = dc - sqrt(s2);
         const double d = sqrt(diff * diff);
-        if (j == 0 || d < bd) {
+        if (!have || d < bd) {
             bd = d;
             best = j;
+            have = true;
         }
     }
-    A.mstar_ix[i] = best;
+    for (int o = 16; o > 0; o >>= 1) {
+        const double od = __shfl_xor_sync(0xffffffffu, bd, o);
+        const int oj = __shfl_xor_sync(0xffffffffu, best, o);
+        const bool oh = __shfl_xor_sync(0xffffffffu, (int)have, o) != 0;
+        if (oh && (!have || od < bd || (od == bd && oj < best))) {
+            bd = od;
+            best = oj;
+            have = true;
+        }
+    }
+    if (lane == 0) {
+        A.g[i] = r * A.deltaZ;
+        A.w[i] = wz;
+        A.dwdz[i] = kC / P.H0 / sqrt(E_of(P, z));  // src/Cosmology.cpp:101-104
+        A.mstar_ix[i] = best;
+    }
 }
 
 __global__ void k_pc_table(const PkDev *__restrict__ Pp, TableArgs A)
@@ -976,7 +1061,7 @@ cudaError_t upload(DevBuf<T> &b, const std::vector<T> &v, cudaStream_t s)
 }
 
 int run_tasks(const PkDev *dP, const std::vector<PcTask> &tasks, std::vector<PcOut> &res,
-              DevBuf<PcOut> &dres, cudaStream_t s, int nsm)
+              DevBuf<PcOut> &dres, cudaStream_t s, int nsm, PcCache C)
 {
     DevBuf<PcTask> dt;
     PC_CK(upload(dt, tasks, s));
@@ -985,10 +1070,10 @@ int run_tasks(const PkDev *dP, const std::vector<PcTask> &tasks, std::vector<PcO
     const char *fc = std::getenv("G3L_PC_FIRST_CAP");
     if (fc && std::atoi(fc) == PC_CAP_TINY)
         k_pc_integrate<PC_CAP_TINY><<<std::min(n, nsm * 8), PC_THREADS, pc_smem(PC_CAP_TINY), s>>>(
-            dP, dt.p, nullptr, n, dres.p);
+            dP, dt.p, nullptr, n, dres.p, C);
     else
         k_pc_integrate<PC_CAP_SMALL><<<std::min(n, nsm * 4), PC_THREADS, pc_smem(PC_CAP_SMALL),
-                                       s>>>(dP, dt.p, nullptr, n, dres.p);
+                                       s>>>(dP, dt.p, nullptr, n, dres.p, C);
     PC_CK(cudaGetLastError());
     res.resize(n);
     PC_CK(cudaMemcpyAsync(res.data(), dres.p, n * sizeof(PcOut), cudaMemcpyDeviceToHost, s));
@@ -1001,7 +1086,7 @@ int run_tasks(const PkDev *dP, const std::vector<PcTask> &tasks, std::vector<PcO
         PC_CK(upload(di, big, s));
         const int nb = (int)big.size();
         k_pc_integrate<PC_CAP_LARGE><<<std::min(nb, nsm), PC_THREADS, pc_smem(PC_CAP_LARGE), s>>>(
-            dP, dt.p, di.p, nb, dres.p);
+            dP, dt.p, di.p, nb, dres.p, C);
         PC_CK(cudaGetLastError());
         PC_CK(cudaMemcpyAsync(res.data(), dres.p, n * sizeof(PcOut), cudaMemcpyDeviceToHost, s));
         PC_CK(cudaStreamSynchronize(s));
@@ -1245,7 +1330,7 @@ int precompute_impl(const g3l_precompute_in *in, int device, g3l_precompute_out 
     PC_CK(cudaMemcpyAsync(dP.p, &P, sizeof P, cudaMemcpyHostToDevice, s));
     std::vector<PcOut> r1;
     DevBuf<PcOut> dr1;
-    int st = run_tasks(dP.p, t1, r1, dr1, s, nsm);
+    int st = run_tasks(dP.p, t1, r1, dr1, s, nsm, PcCache{});
     if (st) return st;
     const double factor = kPi * in->cosmo[3];
     P.amplitude = 2 * factor * factor / r1[0].val;
@@ -1276,7 +1361,12 @@ int precompute_impl(const g3l_precompute_in *in, int device, g3l_precompute_out 
         }
     std::vector<PcOut> r2;
     DevBuf<PcOut> dr2;
-    st = run_tasks(dP.p, t2, r2, dr2, s, nsm);
+    DevBuf<PcNode> cnode;
+    DevBuf<unsigned> cstate;
+    PC_CK(cnode.alloc((size_t)1 << PC_CACHE_LOG2));
+    PC_CK(cstate.alloc((size_t)1 << PC_CACHE_LOG2));
+    PC_CK(cudaMemsetAsync(cstate.p, 0, sizeof(unsigned) << PC_CACHE_LOG2, s));
+    st = run_tasks(dP.p, t2, r2, dr2, s, nsm, PcCache{cnode.p, cstate.p});
     if (st) return st;
 
     // the tables
@@ -1323,7 +1413,7 @@ int precompute_impl(const g3l_precompute_in *in, int device, g3l_precompute_out 
     A.hmf = dhm.p;
     A.b_h = dbh.p;
     A.mstar_ix = dmix.p;
-    k_pc_zrow<<<(N + 127) / 128, 128, 0, s>>>(dP.p, A);
+    k_pc_zrow<<<(N + 3) / 4, 128, 0, s>>>(dP.p, A);
     PC_CK(cudaGetLastError());
     k_pc_table<<<(int)((NN + 127) / 128), 128, 0, s>>>(dP.p, A);
     PC_CK(cudaGetLastError());
