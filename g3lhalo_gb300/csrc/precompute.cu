@@ -10,8 +10,7 @@
 // dsigma^2/dm at every (z, m), sigma^2 at 256 masses per z for M*), each one run by
 // the reference's hcubature_v on the host.
 //
-// Here every integral runs on the device.  One block integrates one integral at a
-// time (grid-stride over the integrals): thread 0 keeps the reference's max-heap of
+// Here every integral runs on the device.  One block integrates one integral: thread 0 keeps the reference's max-heap of
 // regions with its running value/error sums, its Gladwell batch (pop the largest
 // errors until the rest is within tolerance), its cut and its push order, so the
 // refinement follows the reference's; the block's half-warps evaluate the 15-point
@@ -38,18 +37,22 @@
 namespace g3l {
 namespace {
 
-constexpr int PC_THREADS = 128;
-// live regions of one integral (the heap) and regions of one round (the batch, at most
-// twice the heap): a first pass with 512 (48 KB of shared memory, 4 blocks per SM)
-// integrates almost everything; integrals that need more run again with 2048.
-constexpr int PC_CAP_SMALL = 512, PC_CAP_LARGE = 2048;
+// Live regions of one integral (the heap).  The first pass runs one integral per warp with
+// room for 256 regions (12 KB of shared memory, 18 integrals per SM): an integral is ~45
+// dependent rounds of mostly one bisection each (the descent from [0, 1e12] to the scales
+// that matter), so one warp evaluates a round's two regions at once and the other
+// integrals of the SM cover its latency (measured on the 64-bin tables: 18.3 ms with four
+// warps and 512 regions per integral, 4 integrals per SM).  Integrals that need more
+// regions run again with 2048.
+constexpr int PC_CAP_SMALL = 256, PC_CAP_LARGE = 2048;
+constexpr int PC_THREADS_SMALL = 32, PC_THREADS_LARGE = 128;
 // G3L_PC_FIRST_CAP=64 makes the first pass hold only 64 regions, so that most
 // integrals take the 2048-region pass (its results are the same: an integral that
 // overflows starts again from its root region); used to test that pass.
 constexpr int PC_CAP_TINY = 64;
 constexpr int PC_MAX_ROUNDS = 4096;
-constexpr size_t pc_smem(int cap) { return sizeof(double) * 4 * (cap + 2 * cap); }
-constexpr size_t nbar_smem(int cap) { return pc_smem(cap) + sizeof(int) * cap; }
+constexpr size_t pc_smem(int cap) { return sizeof(double) * 6 * cap; }  // heap, popped regions
+constexpr size_t nbar_smem(int cap) { return sizeof(double) * 12 * cap + sizeof(int) * cap; }
 
 // QUADPACK qk15 nodes and weights (the reference's rule15gauss, src/hcubature.cpp:626-660)
 __constant__ double cXgk[8] = {0.991455371120812639206854697526329, 0.949107912342758524526189684047851,
@@ -100,11 +103,6 @@ __device__ __forceinline__ double delta_c(const PkDev &P, double z)
 {   // src/Cosmology.cpp:74-77
     return 1.686 * (1 + 0.0123 * log10(Om_of(P, z)));
 }
-__device__ __forceinline__ double tophat(double k, double R)
-{   // src/Powerspectrum.cpp:104-108
-    double x = k * R;
-    return 3 / x / x / x * (sin(x) - x * cos(x));
-}
 // The Eisenstein & Hu (1998, ApJ 496, 605) transfer function with baryon acoustic
 // terms: eqs. 17-21 (CDM part T_c with the ln/C fitting forms), eqs. 21-24 (baryon part
 // T_b with the node shift s_tilde and Silk damping), weighted by the baryon fraction.
@@ -140,25 +138,25 @@ __device__ __forceinline__ double spectrum(const PkDev &P, double k, double gz)
     return P.amplitude * trans * trans * gz * gz * pow(k, P.ns);
 }
 
-// The k-dependent factors of the sigma^2 integrands, amplitude T(k)^2 and k^ns, do not
-// depend on the radius or redshift, and every sigma^2 and dsigma^2/dm integral bisects the
-// same interval [0, 1e12], so its regions are nodes of one tree: ~2.4M regions of a 64-bin
-// call visit a few thousand distinct nodes.  The factors are nearly all of a point's FP64
+// The k-dependent factor of the integrands over k, k^2 T(k)^2 k^ns, does not depend on the
+// radius or redshift, and the amplitude's, every sigma^2 and every dsigma^2/dm integral
+// bisect the same interval [0, 1e12], so their regions are nodes of one tree: ~2.4M regions
+// of a 64-bin call visit a few thousand distinct nodes.  The factor is nearly all of a point's FP64
 // work (two logarithms, seven pow and an exp in the transfer function), so each node's 15
-// pairs are kept in a hash table in device memory for the length of the call, keyed by the
+// abscissae and factors are kept in a hash table in device memory for the length of the call, keyed by the
 // region's centre and half-width.  A slot is claimed by compare-and-swap and published
 // with a release store; a reader that meets a slot being filled, a full table or a probe
 // run of PC_PROBES evaluates its node itself, so nothing waits and every value is that of
-// the same expressions either way.  Measured on the 64-bin tables: 98.7 -> 12.3 ms.
+// the same expressions either way.  Measured on the 64-bin tables: 99.5 -> 32.7 ms.
 struct PcNode {
     double c, hw;            // key
-    double at[15], pk[15];   // amplitude T^2 and k^ns at the 15 abscissae
+    double x[15], g[15];     // abscissae and k^2 T^2 k^ns there
 };
 constexpr int PC_CACHE_LOG2 = 15;  // 32768 nodes, 8.4 MB (L2-resident)
 constexpr int PC_PROBES = 16;
 
 struct PcCache {
-    PcNode *node;     // null: no cache (the integrals before the amplitude is known)
+    PcNode *node;
     unsigned *state;  // 0 free, 1 being filled, 2 ready
 };
 
@@ -202,36 +200,43 @@ __device__ int pc_find(const PcCache &C, double c, double hw, int &mode)
     return -1;
 }
 
-// sigma^2 and dsigma^2/dm integrands from at = amplitude T^2 and pk = k^ns at k = x, in
-// the operation order of spectrum()
-__device__ __forceinline__ double sigma_integrand(const PcTask &t, double x, double at, double pk)
+// lane hl < 15 stores its abscissa and factor of claimed slot ix; the caller publishes the
+// slot (st_release) after a __syncwarp
+__device__ __forceinline__ void pc_store(const PcCache &C, int ix, double c, double hw, int hl,
+                                         double x, double g)
+{
+    C.node[ix].x[hl] = x;
+    C.node[ix].g[hl] = g;
+    if (hl == 0) {
+        C.node[ix].c = c;
+        C.node[ix].hw = hw;
+    }
+    __threadfence();  // before lane 0's release
+}
+
+// k^2 T(k)^2 k^ns
+__device__ __forceinline__ double k_factor(const PkDev &P, double x)
+{
+    const double T = transfer(P, x);
+    return x * x * T * T * pow(x, P.ns);
+}
+
+// The integrands over k = x from g = k_factor(x); amp: amplitude x (growth(z)/growth(0))^2
+// of the spectrum, 1 for the amplitude's own integral
+__device__ __forceinline__ double k_integrand(const PcTask &t, double x, double g, double amp)
 {
     const double y = x * t.R;
     double sy, cy;
     sincos(y, &sy, &cy);
     // the top-hat's W = 3 (sin y - y cos y) / y^3 and its derivative with one division each
-    const double q = 3 / (y * y * y);
+    // (src/Powerspectrum.cpp:104-114)
+    const double y2 = y * y;
+    const double q = 3 / (y2 * y);
     const double W = q * (sy - y * cy);
-    const double ps = at * t.gz * t.gz * pk;
-    if (t.type == PC_SIGMA2) return x * x * W * W * ps;  // src/Powerspectrum.cpp:219-243
-    // src/Powerspectrum.cpp:110-114, 267-293
-    const double Wprime = ((y * y - 3.) * sy + 3. * y * cy) * x * q / y;
-    return x * x * W * Wprime * t.dR * ps;
-}
-
-__device__ double integrand(const PkDev &P, const PcTask &t, double x)
-{
-    switch (t.type) {
-    case PC_AMP: {  // src/Powerspectrum.cpp:79-102
-        double R = 8. / P.H0 * 100;
-        double W = tophat(x, R);
-        double T = transfer(P, x);
-        return W * W * T * T * pow(x, P.ns + 2);
-    }
-    default:  // comoving distance integrand c/H0/sqrt(E(z)) (src/Cosmology.cpp:101-122);
-              // PC_SIGMA2 and PC_DSIGMA2 are evaluated by sigma_integrand
-        return kC / P.H0 / sqrt(E_of(P, x));
-    }
+    if (t.type != PC_DSIGMA2) return W * W * g * amp;  // src/Powerspectrum.cpp:79-102, 219-243
+    // src/Powerspectrum.cpp:267-293
+    const double Wprime = ((y2 - 3.) * sy + 3. * y * cy) * x * q / y;
+    return W * Wprime * g * (t.dR * amp);
 }
 
 // 15-point Gauss-Kronrod value and QUADPACK error of one region (src/hcubature.cpp:
@@ -256,18 +261,34 @@ __device__ __forceinline__ void rule_gk15_hw(double f, int hl, double hw, double
         const int j = (hl - 1) >> 1;
         wk = cWgk[2 * (j - 3)];
     }
-    double rk = wk * f, rg = wg * f, ra = wk * fabs(f);
-    for (int o = 8; o > 0; o >>= 1) {
-        rk += __shfl_xor_sync(0xffffffffu, rk, o, 16);
-        rg += __shfl_xor_sync(0xffffffffu, rg, o, 16);
-        ra += __shfl_xor_sync(0xffffffffu, ra, o, 16);
+    // rk, rg and ra are summed side by side: after the first step each lane carries two of
+    // them, after the second one (lane bits 3 and 2 say which: 00 rk, 01 rg, 1x ra), so the
+    // 12 additions of three butterflies take 5
+    const bool up = hl & 8, odd = hl & 4;
+    const double k0 = wk * f, g0 = wg * f, a0 = wk * fabs(f);
+    double s0, s1;  // lanes 0-7: rk and rg; lanes 8-15: ra
+    {
+        const double o0 = __shfl_xor_sync(0xffffffffu, up ? k0 : a0, 8, 16);
+        const double o1 = __shfl_xor_sync(0xffffffffu, g0, 8, 16);
+        s0 = (up ? a0 : k0) + o0;
+        s1 = up ? 0.0 : g0 + o1;
     }
+    {
+        const double o0 = __shfl_xor_sync(0xffffffffu, up ? s0 : (odd ? s0 : s1), 4, 16);
+        s0 = (up ? s0 : (odd ? s1 : s0)) + o0;
+    }
+    s0 += __shfl_xor_sync(0xffffffffu, s0, 2, 16);
+    s0 += __shfl_xor_sync(0xffffffffu, s0, 1, 16);
+    const double rk = __shfl_sync(0xffffffffu, s0, 0, 16);
     const double mean = rk * 0.5;
     double rs = wk * fabs(f - mean);
     for (int o = 8; o > 0; o >>= 1) rs += __shfl_xor_sync(0xffffffffu, rs, o, 16);
-    val = rk * hw;
-    double e = fabs(rk - rg) * hw;
-    const double rabs = ra * hw, rasc = rs * hw;
+    // times the half-width, one lane each: value, |rk - rg|, rabs, rasc
+    const double rg = __shfl_sync(0xffffffffu, s0, 4, 16), ra = __shfl_sync(0xffffffffu, s0, 8, 16);
+    const double t = (hl == 0 ? rk : hl == 1 ? fabs(rk - rg) : hl == 2 ? ra : rs) * hw;
+    val = t;
+    double e = __shfl_sync(0xffffffffu, t, 1, 16);
+    const double rabs = __shfl_sync(0xffffffffu, t, 2, 16), rasc = __shfl_sync(0xffffffffu, t, 3, 16);
     if (rasc != 0 && e != 0) {
         const double q = 200 * e / rasc;
         const double scale = q * sqrt(q);
@@ -289,6 +310,31 @@ __device__ __forceinline__ double gk_point(double c, double hw, int i)
     return (i & 1) ? c - w : c + w;
 }
 
+// Fill the table with the nodes every integral descends through: the PC_WARM leftmost of
+// each depth (one half-warp per node).  The amplitude's integral would otherwise evaluate
+// them one round after another, and the first wave of the others all at once, each for
+// itself (tables of 16 bins 4.5 -> 2.9 ms).  Centres by the cut's arithmetic; they are exact
+// multiples of the half-width.
+constexpr int PC_WARM = 32, PC_WARM_DEPTH = 60;
+__global__ void __launch_bounds__(64) k_pc_warm(const PkDev *__restrict__ Pp, double hi, PcCache C)
+{
+    const int q = (blockIdx.x * blockDim.x + threadIdx.x) >> 4, hl = threadIdx.x & 15;
+    const int d = q / PC_WARM, k = q % PC_WARM;
+    const PkDev P = *Pp;
+    const bool live = d <= PC_WARM_DEPTH && (d >= 6 || k < (1 << d));
+    const double hw = ldexp(0.5 * hi, -d), c = (2 * k + 1) * hw;
+    int mode = 0, ix = -1;
+    if (live && hl == 0) ix = pc_find(C, c, hw, mode);
+    mode = __shfl_sync(0xffffffffu, mode, 0, 16);
+    ix = __shfl_sync(0xffffffffu, ix, 0, 16);
+    if (mode == 1 && hl < 15) {
+        const double x = gk_point(c, hw, hl);
+        pc_store(C, ix, c, hw, hl, x, k_factor(P, x));
+    }
+    __syncwarp();
+    if (mode == 1 && hl == 0) st_release(C.state + ix, 2u);
+}
+
 struct Heap {
     double *c, *hw, *val, *err;
 };
@@ -304,12 +350,14 @@ __device__ __forceinline__ bool converged(double err, double val)
 // being swapped down level by level.
 __device__ __forceinline__ long long ebits(double e) { return __double_as_longlong(e); }
 
-__device__ void heap_push(Heap H, int &n, double &hv, double &he, double c, double hw, double v,
-                          double e)
+// entry n, appended behind the heap's n entries, joins it
+__device__ void heap_push(Heap H, int &n, double &hv, double &he)
 {
+    int ins = n++;
+    const double c = H.c[ins], hw = H.hw[ins], v = H.val[ins], e = H.err[ins];
     hv += v;
     he += e;
-    int ins = n++;
+    const int ins0 = ins;
     while (ins) {
         int parent = (ins - 1) / 2;
         if (ebits(e) <= ebits(H.err[parent])) break;
@@ -319,6 +367,7 @@ __device__ void heap_push(Heap H, int &n, double &hv, double &he, double c, doub
         H.err[ins] = H.err[parent];
         ins = parent;
     }
+    if (ins == ins0) return;
     H.c[ins] = c;
     H.hw[ins] = hw;
     H.val[ins] = v;
@@ -359,35 +408,36 @@ __device__ void heap_pop(Heap H, int &nn, double &hv, double &he, double &c, dou
 
 // One adaptive 15-point Gauss-Kronrod integral over [lo, hi] by the whole block, with
 // the reference's refinement: thread 0 keeps the heap, the Gladwell batch and the cut;
-// ev(nb, bc, bh, bv, be) is called by every thread and evaluates the batch's regions
-// (centres bc, half-widths bh) into their values bv and errors be.  Status: 0 ok,
+// ev(nb, H, n, pc, ph) is called by every thread and evaluates the batch's nb regions into
+// the heap's entries n .. n + nb - 1 (centre, half-width, value, error): the children of the
+// popped regions (centres pc, half-widths ph), or the root in entry 0.  Status: 0 ok,
 // G3L_ERR_POOL (more than CAP live regions), G3L_ERR_ROUNDS (more than PC_MAX_ROUNDS
 // rounds).  The result is valid in thread 0; the block is synchronised on return.
 template <int CAP, class Eval>
 __device__ PcOut gk_integrate(double lo, double hi, double *sm, const Eval &ev)
 {
-    constexpr int PC_CAP = CAP, PC_BATCH = 2 * CAP;
-    Heap H{sm, sm + PC_CAP, sm + 2 * PC_CAP, sm + 3 * PC_CAP};
-    double *bc = sm + 4 * PC_CAP, *bh = bc + PC_BATCH, *bv = bh + PC_BATCH, *be = bv + PC_BATCH;
-    __shared__ int s_nb, s_done;
+    Heap H{sm, sm + CAP, sm + 2 * CAP, sm + 3 * CAP};
+    double *pc = sm + 4 * CAP, *ph = sm + 5 * CAP;
+    __shared__ int s_nb, s_n, s_done;
     // thread 0's state: heap size, running sums, counters
     int n = 0, status = 0, rounds = 0;
     double hv = 0, he = 0;
     unsigned long long neval = 15;
     if (threadIdx.x == 0) {
-        bc[0] = 0.5 * (lo + hi);
-        bh[0] = 0.5 * (hi - lo);
+        H.c[0] = 0.5 * (lo + hi);
+        H.hw[0] = 0.5 * (hi - lo);
         s_nb = 1;
+        s_n = 0;
         s_done = 0;
     }
     __syncthreads();
     while (true) {
-        ev(s_nb, bc, bh, bv, be);
+        ev(s_nb, H, s_n, pc, ph);
         __syncthreads();
         if (threadIdx.x == 0) {
             const int nb = s_nb;
-            for (int b = 0; b < nb; ++b) heap_push(H, n, hv, he, bc[b], bh[b], bv[b], be[b]);
-            int nbn = 0;
+            for (int b = 0; b < nb; ++b) heap_push(H, n, hv, he);
+            int K = 0;
             if (converged(he, hv)) {
                 s_done = 1;
             } else if (++rounds > PC_MAX_ROUNDS) {
@@ -398,8 +448,8 @@ __device__ PcOut gk_integrate(double lo, double hi, double *sm, const Eval &ev)
                 double eErr = he;
                 const double eVal = hv;
                 do {
-                    // after this pop and the pushes the heap holds n + nbn + 1 regions
-                    if (n + nbn + 1 > PC_CAP) {
+                    // after this pop and the pushes the heap holds n + 2 K + 1 regions
+                    if (n + 2 * K + 1 > CAP) {
                         status = G3L_ERR_POOL;
                         s_done = 1;
                         break;
@@ -407,17 +457,15 @@ __device__ PcOut gk_integrate(double lo, double hi, double *sm, const Eval &ev)
                     double c, hw, v, e;
                     heap_pop(H, n, hv, he, c, hw, v, e);
                     eErr -= e;
-                    const double h2 = hw * 0.5;  // cut (src/hcubature.cpp:206-218)
-                    bc[nbn] = c - h2;
-                    bh[nbn] = h2;
-                    bc[nbn + 1] = c + h2;
-                    bh[nbn + 1] = h2;
-                    nbn += 2;
+                    pc[K] = c;
+                    ph[K] = hw;
+                    ++K;
                     neval += 30;
                     if (converged(eErr, eVal)) break;
                 } while (n > 0);
             }
-            s_nb = nbn;
+            s_nb = 2 * K;
+            s_n = n;
         }
         __syncthreads();
         if (s_done) break;
@@ -599,60 +647,63 @@ struct PcEval {
     const PkDev &P;
     const PcTask &t;
     const PcCache &C;
-    __device__ void operator()(int nb, const double *bc, const double *bh, double *bv,
-                               double *be) const
+    __device__ void operator()(int nb, Heap H, int n, const double *pc, const double *ph) const
     {
         const int lane = threadIdx.x & 31, half = lane >> 4, hl = lane & 15;
         const int warp = threadIdx.x >> 5, nwarps = blockDim.x / 32;
+        const double amp = t.type == PC_AMP ? 1.0 : P.amplitude * t.gz * t.gz;
         for (int r0 = 2 * warp; r0 < nb; r0 += 2 * nwarps) {
             const int r = r0 + half;
-            double f = 0;
-            if (t.type == PC_SIGMA2 || t.type == PC_DSIGMA2) {  // block-uniform
+            const bool live = r < nb;
+            double c = 0, hw = 1, f = 0;
+            if (live) {
+                if (nb == 1) {  // the root
+                    c = H.c[0];
+                    hw = H.hw[0];
+                } else {  // cut (src/hcubature.cpp:206-218)
+                    hw = ph[r >> 1] * 0.5;
+                    c = (r & 1) ? pc[r >> 1] + hw : pc[r >> 1] - hw;
+                }
+            }
+            const bool on = live && hl < 15;
+            if (t.type == PC_CHI) {  // block-uniform
+                if (on) f = kC / P.H0 / sqrt(E_of(P, gk_point(c, hw, hl)));  // src/Cosmology.cpp:101-122
+            } else {
                 int mode = 0, ix = -1;
-                if (r < nb && hl == 0) ix = pc_find(C, bc[r], bh[r], mode);
+                if (live && hl == 0) ix = pc_find(C, c, hw, mode);
                 mode = __shfl_sync(0xffffffffu, mode, 0, 16);
                 ix = __shfl_sync(0xffffffffu, ix, 0, 16);
-                if (r < nb && hl < 15) {
-                    const double x = gk_point(bc[r], bh[r], hl);
-                    double at, pk;
+                if (on) {
+                    double x, g;
                     if (mode == 2) {
-                        at = __ldcg(&C.node[ix].at[hl]);
-                        pk = __ldcg(&C.node[ix].pk[hl]);
+                        x = __ldcg(&C.node[ix].x[hl]);
+                        g = __ldcg(&C.node[ix].g[hl]);
                     } else {
-                        const double trans = transfer(P, x);
-                        at = P.amplitude * trans * trans;
-                        pk = pow(x, P.ns);
-                        if (mode == 1) {
-                            C.node[ix].at[hl] = at;
-                            C.node[ix].pk[hl] = pk;
-                            if (hl == 0) {
-                                C.node[ix].c = bc[r];
-                                C.node[ix].hw = bh[r];
-                            }
-                            __threadfence();  // before lane 0's release below
-                        }
+                        x = gk_point(c, hw, hl);
+                        g = k_factor(P, x);
+                        if (mode == 1) pc_store(C, ix, c, hw, hl, x, g);
                     }
-                    f = sigma_integrand(t, x, at, pk);
+                    f = k_integrand(t, x, g, amp);
                 }
                 __syncwarp();
                 if (hl == 0 && mode == 1) st_release(C.state + ix, 2u);
-            } else if (r < nb && hl < 15) {
-                f = integrand(P, t, gk_point(bc[r], bh[r], hl));
             }
             double v, e;
-            rule_gk15_hw(f, hl, r < nb ? bh[r] : 1.0, v, e);
-            if (r < nb && hl == 0) {
-                bv[r] = v;
-                be[r] = e;
+            rule_gk15_hw(f, hl, hw, v, e);
+            if (live && hl == 0) {
+                H.c[n + r] = c;
+                H.hw[n + r] = hw;
+                H.val[n + r] = v;
+                H.err[n + r] = e;
             }
         }
     }
 };
 
-// One block per integral at a time (grid-stride).  idx: the integrals to run (null:
-// all ntask).
-template <int CAP>
-__global__ void __launch_bounds__(PC_THREADS) k_pc_integrate(const PkDev *__restrict__ Pp,
+// One block per integral (the block scheduler balances their uneven lengths).  idx: the
+// integrals to run (null: all ntask).
+template <int CAP, int THREADS>
+__global__ void __launch_bounds__(THREADS) k_pc_integrate(const PkDev *__restrict__ Pp,
                                                              const PcTask *__restrict__ tasks,
                                                              const int *__restrict__ idx,
                                                              int ntask, PcOut *__restrict__ out,
@@ -660,12 +711,12 @@ __global__ void __launch_bounds__(PC_THREADS) k_pc_integrate(const PkDev *__rest
 {
     extern __shared__ double sm[];
     const PkDev P = *Pp;
-    for (int tj = blockIdx.x; tj < ntask; tj += gridDim.x) {
-        const int ti = idx ? idx[tj] : tj;
-        const PcTask t = tasks[ti];
-        const PcOut o = gk_integrate<CAP>(t.lo, t.hi, sm, PcEval{P, t, C});
-        if (threadIdx.x == 0) out[ti] = o;
-    }
+    const int tj = blockIdx.x;
+    if (tj >= ntask) return;
+    const int ti = idx ? idx[tj] : tj;
+    const PcTask t = tasks[ti];
+    const PcOut o = gk_integrate<CAP>(t.lo, t.hi, sm, PcEval{P, t, C});
+    if (threadIdx.x == 0) out[ti] = o;
 }
 
 // ------------------------------------------------------------------ n_bar(z) per HOD
@@ -1061,7 +1112,7 @@ cudaError_t upload(DevBuf<T> &b, const std::vector<T> &v, cudaStream_t s)
 }
 
 int run_tasks(const PkDev *dP, const std::vector<PcTask> &tasks, std::vector<PcOut> &res,
-              DevBuf<PcOut> &dres, cudaStream_t s, int nsm, PcCache C)
+              DevBuf<PcOut> &dres, cudaStream_t s, PcCache C)
 {
     DevBuf<PcTask> dt;
     PC_CK(upload(dt, tasks, s));
@@ -1069,11 +1120,13 @@ int run_tasks(const PkDev *dP, const std::vector<PcTask> &tasks, std::vector<PcO
     const int n = (int)tasks.size();
     const char *fc = std::getenv("G3L_PC_FIRST_CAP");
     if (fc && std::atoi(fc) == PC_CAP_TINY)
-        k_pc_integrate<PC_CAP_TINY><<<std::min(n, nsm * 8), PC_THREADS, pc_smem(PC_CAP_TINY), s>>>(
-            dP, dt.p, nullptr, n, dres.p, C);
+        k_pc_integrate<PC_CAP_TINY, PC_THREADS_SMALL>
+            <<<n, PC_THREADS_SMALL, pc_smem(PC_CAP_TINY), s>>>(
+                dP, dt.p, nullptr, n, dres.p, C);
     else
-        k_pc_integrate<PC_CAP_SMALL><<<std::min(n, nsm * 4), PC_THREADS, pc_smem(PC_CAP_SMALL),
-                                       s>>>(dP, dt.p, nullptr, n, dres.p, C);
+        k_pc_integrate<PC_CAP_SMALL, PC_THREADS_SMALL>
+            <<<n, PC_THREADS_SMALL, pc_smem(PC_CAP_SMALL), s>>>(
+                dP, dt.p, nullptr, n, dres.p, C);
     PC_CK(cudaGetLastError());
     res.resize(n);
     PC_CK(cudaMemcpyAsync(res.data(), dres.p, n * sizeof(PcOut), cudaMemcpyDeviceToHost, s));
@@ -1085,8 +1138,9 @@ int run_tasks(const PkDev *dP, const std::vector<PcTask> &tasks, std::vector<PcO
         DevBuf<int> di;
         PC_CK(upload(di, big, s));
         const int nb = (int)big.size();
-        k_pc_integrate<PC_CAP_LARGE><<<std::min(nb, nsm), PC_THREADS, pc_smem(PC_CAP_LARGE), s>>>(
-            dP, dt.p, di.p, nb, dres.p, C);
+        k_pc_integrate<PC_CAP_LARGE, PC_THREADS_LARGE>
+            <<<nb, PC_THREADS_LARGE, pc_smem(PC_CAP_LARGE), s>>>(
+                dP, dt.p, di.p, nb, dres.p, C);
         PC_CK(cudaGetLastError());
         PC_CK(cudaMemcpyAsync(res.data(), dres.p, n * sizeof(PcOut), cudaMemcpyDeviceToHost, s));
         PC_CK(cudaStreamSynchronize(s));
@@ -1272,12 +1326,7 @@ int precompute_impl(const g3l_precompute_in *in, int device, g3l_precompute_out 
             return G3L_ERR_INVALID;
         }
     PC_CK(cudaSetDevice(device));
-    int nsm = 0;
-    PC_CK(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, device));
-    PC_CK(cudaFuncSetAttribute(k_pc_integrate<PC_CAP_SMALL>,
-                               cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               (int)pc_smem(PC_CAP_SMALL)));
-    PC_CK(cudaFuncSetAttribute(k_pc_integrate<PC_CAP_LARGE>,
+    PC_CK(cudaFuncSetAttribute(k_pc_integrate<PC_CAP_LARGE, PC_THREADS_LARGE>,
                                cudaFuncAttributeMaxDynamicSharedMemorySize,
                                (int)pc_smem(PC_CAP_LARGE)));
     cudaStream_t s;
@@ -1322,7 +1371,7 @@ int precompute_impl(const g3l_precompute_in *in, int device, g3l_precompute_out 
 
     // pass 1: the amplitude (src/Powerspectrum.cpp:67-77) and the comoving distances
     std::vector<PcTask> t1;
-    t1.push_back(PcTask{PC_AMP, 0, 0, 0, 0, 0.0, 1e12});
+    t1.push_back(PcTask{PC_AMP, 0, 8. / P.H0 * 100, 0, 0, 0.0, 1e12});
     for (int i = 0; i < N; ++i) t1.push_back(PcTask{PC_CHI, 0, 0, 0, 0, 0.0, zs[i]});
     for (int j = 0; j < Ns; ++j) t1.push_back(PcTask{PC_CHI, 0, 0, 0, 0, 0.0, in->nz_z[j]});
     DevBuf<PkDev> dP;
@@ -1330,7 +1379,15 @@ int precompute_impl(const g3l_precompute_in *in, int device, g3l_precompute_out 
     PC_CK(cudaMemcpyAsync(dP.p, &P, sizeof P, cudaMemcpyHostToDevice, s));
     std::vector<PcOut> r1;
     DevBuf<PcOut> dr1;
-    int st = run_tasks(dP.p, t1, r1, dr1, s, nsm, PcCache{});
+    DevBuf<PcNode> cnode;
+    DevBuf<unsigned> cstate;
+    PC_CK(cnode.alloc((size_t)1 << PC_CACHE_LOG2));
+    PC_CK(cstate.alloc((size_t)1 << PC_CACHE_LOG2));
+    PC_CK(cudaMemsetAsync(cstate.p, 0, sizeof(unsigned) << PC_CACHE_LOG2, s));
+    const PcCache cache{cnode.p, cstate.p};
+    k_pc_warm<<<((PC_WARM_DEPTH + 1) * PC_WARM * 16 + 63) / 64, 64, 0, s>>>(dP.p, 1e12, cache);
+    PC_CK(cudaGetLastError());
+    int st = run_tasks(dP.p, t1, r1, dr1, s, cache);
     if (st) return st;
     const double factor = kPi * in->cosmo[3];
     P.amplitude = 2 * factor * factor / r1[0].val;
@@ -1361,12 +1418,7 @@ int precompute_impl(const g3l_precompute_in *in, int device, g3l_precompute_out 
         }
     std::vector<PcOut> r2;
     DevBuf<PcOut> dr2;
-    DevBuf<PcNode> cnode;
-    DevBuf<unsigned> cstate;
-    PC_CK(cnode.alloc((size_t)1 << PC_CACHE_LOG2));
-    PC_CK(cstate.alloc((size_t)1 << PC_CACHE_LOG2));
-    PC_CK(cudaMemsetAsync(cstate.p, 0, sizeof(unsigned) << PC_CACHE_LOG2, s));
-    st = run_tasks(dP.p, t2, r2, dr2, s, nsm, PcCache{cnode.p, cstate.p});
+    st = run_tasks(dP.p, t2, r2, dr2, s, cache);
     if (st) return st;
 
     // the tables
