@@ -1,14 +1,14 @@
 // eval_fp64.cu -- all-FP64 rule evaluation: the plain FP64 form of the engine.
 //
-// One warp evaluates one work item: it cuts a selected parent region along its
-// split dimension (cut_region, src/hcubature.cpp:206-218) and applies the
-// Genz-Malik 7/5 rule to both children (rule75genzmalik_evalError,
-// src/hcubature.cpp:456-577), or evaluates a root region.  The per-dimension
-// coordinate variants (c, c-+lambda*h) are computed once per child together
-// with everything that depends on one coordinate only (10^x, aperture filter,
-// HOD occupations, bin indices); each lane then evaluates whole points.  The
-// rule sums are formed by one lane per child in the reference's summation
-// order.  Compiled with -fmad=false so every product and sum rounds as in the
+// A warp (or, when a round has few cuts, a block) evaluates one work item: it cuts a
+// selected parent region along its split dimension (cut_region,
+// src/hcubature.cpp:206-218) and applies the Genz-Malik 7/5 rule to both children
+// (rule75genzmalik_evalError, src/hcubature.cpp:456-577), or evaluates a root region.
+// The per-dimension coordinate variants (c, c-+lambda*h) are computed once per child
+// together with everything that depends on one coordinate only (10^x, aperture filter,
+// HOD occupations, bin indices), then what depends on a few coordinates once per
+// projection of the points onto them; each lane then evaluates whole points.  The rule
+// sums are formed in the reference's summation order.  Compiled with -fmad=false so every product and sum rounds as in the
 // reference's CPU build.
 #include "phys64.cuh"
 
@@ -339,16 +339,155 @@ __device__ void combine64(const double *v, double vol, double &val, double &err,
     split = dimDiffMax;
 }
 
-// One work item on one warp: `cut` = bisect the region at pslot along its split
-// dimension into pslot (lower half) and qslot (upper half) and evaluate both;
-// otherwise evaluate the region at pslot in place (roots, FP64 re-evaluation).
+// Point tables of a group's re-evaluation passes: the point codes, the (l, m, z)
+// combinations of the cached u_NFW (ucache_tables) and the projections of the k3 u_NFW
+// (u3_tables) and of the auxiliary functions (aux_tables).  The same for every launch, so
+// k_re_tables builds them once per context into P.retab and each block copies them to
+// shared memory (building them per block cost more than the cached work saves).
 template <int KIND, int TERM>
-__device__ void warp_item64(const DevTables &T, const IntDesc &d, const Pool &P, long long pslot,
-                            long long qslot, bool cut, Slot64 *slots, double *vals,
-                            const uint32_t *sdesc, unsigned long long *ties, double *dbg)
+struct ReTab {
+    static constexpr int DIM = TERM + 4, NP = rule_points(DIM), NF = ucache_nf(TERM);
+    static constexpr int NU3 = u3_nfun(TERM) > 0 ? u3_nfun(TERM) : 1, NA = aux_nfun(TERM);
+    uint32_t sdesc[NP];
+    int ucn[NF];
+    uint16_t ucl[NF * UC_MAX];
+    uint8_t ucidx[NF * NP];
+    uint8_t u3rep[NU3 * NP];
+    uint8_t u3list[NU3 * U3_MAX];
+    uint8_t auxrep[NA * NP];
+    uint8_t auxlist[AUX_MAX];
+};
+
+template <int KIND, int TERM>
+__global__ void __launch_bounds__(128) k_re_tables(unsigned char *out)
 {
-    constexpr int DIM = TERM + 4;
-    constexpr int NP = rule_points(DIM);
+    using RT = ReTab<KIND, TERM>;
+    static_assert(sizeof(RT) <= RETAB_BYTES && sizeof(RT) % 4 == 0, "re-evaluation table size");
+    __shared__ __align__(16) unsigned char buf[sizeof(RT)];
+    __shared__ uint8_t map[RT::NF * 343];
+    RT &t = *reinterpret_cast<RT *>(buf);
+    ucache_tables<KIND, TERM>(t.ucidx, t.ucl, t.ucn, map);
+    for (int p = threadIdx.x; p < RT::NP; p += blockDim.x) t.sdesc[p] = point_variants(RT::DIM, p);
+    __syncthreads();
+    u3_tables<KIND, TERM>(t.sdesc, t.u3rep, t.u3list, map);  // map is free again
+    aux_tables<TERM>(t.sdesc, t.auxrep, t.auxlist, map);
+    uint32_t *dst = reinterpret_cast<uint32_t *>(out + (KIND * 3 + TERM - 1) * RETAB_BYTES);
+    for (int i = threadIdx.x; i < (int)(sizeof(RT) / 4); i += blockDim.x)
+        dst[i] = reinterpret_cast<const uint32_t *>(buf)[i];
+}
+
+// copy group (KIND, TERM)'s tables to shared memory buf (every thread calls it)
+template <int KIND, int TERM>
+__device__ inline const ReTab<KIND, TERM> &load_retab(const Pool &P, unsigned char *buf)
+{
+    using RT = ReTab<KIND, TERM>;
+    const uint32_t *src =
+        reinterpret_cast<const uint32_t *>(P.retab + (KIND * 3 + TERM - 1) * RETAB_BYTES);
+    for (int i = threadIdx.x; i < (int)(sizeof(RT) / 4); i += blockDim.x)
+        reinterpret_cast<uint32_t *>(buf)[i] = __ldg(src + i);
+    __syncthreads();
+    return *reinterpret_cast<const RT *>(buf);
+}
+
+// Threads that share one work item: a warp, or the whole block.
+struct Group {
+    int size, rank;  // 32 or 128; rank of this thread
+    __device__ void sync() const
+    {
+        if (size == 32) __syncwarp();
+        else __syncthreads();
+    }
+};
+
+// Shared memory of one work item.  Child 1 has its own copy of a cached function only when
+// the split dimension is among the function's dimensions.
+template <int KIND, int TERM>
+struct Item64 {
+    static constexpr int DIM = TERM + 4, NP = rule_points(DIM), NF = ucache_nf(TERM);
+    static constexpr int NU3 = u3_nfun(TERM), NA = aux_nfun(TERM);
+    static constexpr int NAUX = aux_off(TERM, NA - 1) + aux_count(TERM, NA - 1);
+    Slot64 slots[(DIM + 1) * NVAR];
+    double mz[2][TERM][MZ_PAIRS][MZ_VALS];
+    double uc[2][NF][UC_MAX];
+    double u3[2][NU3 > 0 ? NU3 : 1][NU3 > 0 ? U3_MAX : 1];
+    double aux[2][NAUX];
+    double vals[2 * NP];
+};
+
+// Rule sums of both children by one warp, each sum in the reference's order
+// (src/hcubature.cpp:512-576): eight lanes per child form the axis sums, the pair sum, the
+// corner sum and one fourth difference each.  An FP64 instruction occupies the pipe for 64
+// cycles however few lanes take part, so the sums run side by side, not one after another.
+// Valid in lanes 0 (child 0) and 8 (child 1).
+template <int DIM>
+__device__ void combine64_warp(const double *v, double vol, double &val, double &err, int &split)
+{
+    const int r = threadIdx.x & 7;
+    const double ratio = (G3L_LAMBDA2 * G3L_LAMBDA2) / (G3L_LAMBDA4 * G3L_LAMBDA4);
+    const double weight1 = (double)(12824 - 9120 * DIM + 400 * DIM * DIM) / (double)19683;
+    const double weight3 = (double)(1820 - 400 * DIM) / (double)19683;
+    const double weight5 = (double)6859 / (double)19683 / (double)(1u << DIM);
+    const double weightE1 = (double)(729 - 950 * DIM + 50 * DIM * DIM) / (double)729;
+    const double weightE3 = (double)(265 - 100 * DIM) / (double)1458;
+    const double weight2 = 980. / 6561., weight4 = 200. / 19683.;
+    const double weightE2 = 245. / 486., weightE4 = 25. / 729.;
+    constexpr int NRR = 2 * DIM * (DIM - 1), NC = 1 << DIM;
+    const double val0 = v[0];
+    // lane r = 0, 1: pairs of axis points at lambda2, lambda4; 2: (+-, +-) points; 3: corners
+    const double *p = v + (r == 2 ? 1 + 4 * DIM : (r == 3 ? 1 + 4 * DIM + NRR : 1 + 2 * r));
+    const int n = r < 2 ? DIM : (r == 2 ? NRR : (r == 3 ? NC : 0));
+    double s = 0;
+    constexpr int NMAX = NRR > NC ? NRR : NC;
+    for (int k = 0; k < NMAX; ++k)
+        if (k < n) s += r < 2 ? p[4 * k] + p[4 * k + 1] : p[k];
+    // fourth difference of dimension r
+    long long db = 0;
+    if (r < DIM) {
+        const double *q = v + 1 + 4 * r;
+        double diff = 0;
+        diff += fabs(q[0] + q[1] - 2 * val0 - ratio * (q[2] + q[3] - 2 * val0));
+        if (diff > 0) db = __double_as_longlong(diff);  // NaN never exceeds the maximum
+    }
+    const double sum2 = __shfl_sync(0xffffffffu, s, 0, 8), sum3 = __shfl_sync(0xffffffffu, s, 1, 8);
+    const double sum4 = __shfl_sync(0xffffffffu, s, 2, 8), sum5 = __shfl_sync(0xffffffffu, s, 3, 8);
+    long long maxdiff = 0;
+    int dimDiffMax = 0;
+    for (int k = 0; k < DIM; ++k) {  // the first maximum
+        const long long o = __shfl_sync(0xffffffffu, db, k, 8);
+        if (o > maxdiff) {
+            maxdiff = o;
+            dimDiffMax = k;
+        }
+    }
+    const double result = vol * (weight1 * val0 + weight2 * sum2 + weight3 * sum3 + weight4 * sum4 +
+                                 weight5 * sum5);
+    const double res5th =
+        vol * (weightE1 * val0 + weightE2 * sum2 + weightE3 * sum3 + weightE4 * sum4);
+    val = result;
+    err = fabs(res5th - result);
+    split = dimDiffMax;
+}
+
+// One work item on a group of threads: `cut` = bisect the region at pslot along its split
+// dimension into pslot (lower half) and qslot (upper half) and evaluate both; otherwise
+// evaluate the region at pslot in place (roots).  Four passes with a barrier between:
+// coordinate slots; (mass, z) values and the auxiliary functions; every u_NFW that several
+// points share; the points.  A quantity is evaluated once per projection of the rule's
+// points onto the dimensions it depends on, and for child 1 only if the split dimension is
+// one of them, by the expressions of the per-point code (bit-identical values).  The FP64
+// pipe bounds this kernel (one warp instruction per 64 cycles per SM quarter), so what
+// counts is the number of warp instructions: the 2-halo rule takes 132 + 186 u_NFW per
+// child at most instead of 894, the 3-halo rule 66 + 93 instead of 723.
+template <int KIND, int TERM>
+__device__ void group_item64(const DevTables &T, const IntDesc &d, const Pool &P, long long pslot,
+                             long long qslot, bool cut, Item64<KIND, TERM> &I,
+                             const ReTab<KIND, TERM> &tb, const Group &gr,
+                             unsigned long long *ties, double *dbg)
+{
+    using M = Model64<KIND, TERM>;
+    using It = Item64<KIND, TERM>;
+    constexpr int DIM = It::DIM, NP = It::NP, NF = It::NF, NU3 = It::NU3, NA = It::NA;
+    constexpr int ZD = DIM - 1;
     const int lane = threadIdx.x & 31;
     const long long stride = P.stride;
     const int sdim = cut ? P.split[pslot] : 0;
@@ -359,76 +498,204 @@ __device__ void warp_item64(const DevTables &T, const IntDesc &d, const Pool &P,
         c_l = P.center[lane * stride + pslot];
         lev = P.level[lane * stride + pslot];
     }
-    double cL = 0, cR = 0;
     const int levs = __shfl_sync(0xffffffffu, lev, sdim) + (cut ? 1 : 0);
     const double cs = __shfl_sync(0xffffffffu, c_l, sdim);
-    const double hws = ldexp(d.hw0[sdim], -levs);
+    double cL = cs, cR = cs;
     if (cut) {
+        const double hws = ldexp(d.hw0[sdim], -levs);
         cL = cs - hws;
         cR = cs + hws;
     }
     const int levsum = __reduce_add_sync(0xffffffffu, lane < DIM ? lev : 0) + (cut ? 1 : 0);
-    // coordinate variant slots: dims 0..DIM-1 of child 0, then dim sdim of child 1
-    const int nslot = (DIM + nchild - 1) * NVAR;
-    for (int t = lane; t < nslot; t += 32) {
-        int dd = t / NVAR, v = t - dd * NVAR;
-        int dim = dd < DIM ? dd : sdim;
-        double c = P.center[dim * stride + pslot];
-        int L = P.level[dim * stride + pslot];
-        if (cut && dim == sdim) {
-            L += 1;
-            c = (dd < DIM) ? cL : cR;
+    // does child 1 need its own values of a function of the dimensions dims?
+    auto own = [&](uint32_t dims) { return cut && ((dims >> sdim) & 1u); };
+    // coordinate slots, masses first (the longest path), then l, phi, z: the warps then
+    // diverge least.  Slots of child 1's split dimension follow those of its kind.
+    {
+        const bool smass = cut && sdim >= 3 && sdim < 3 + TERM;
+        const int nm = TERM * NVAR, nms = nm + (smass ? NVAR : 0);
+        const int nslot = (DIM + nchild - 1) * NVAR;
+        for (int t = gr.rank; t < nslot; t += gr.size) {
+            int sd;  // slot row: dimension, or DIM for child 1's split dimension
+            if (t < nms) {
+                sd = t / NVAR < TERM ? 3 + t / NVAR : DIM;
+            } else {
+                const int q = (t - nms) / NVAR;
+                sd = q < 3 ? q : (q == 3 ? ZD : DIM);
+            }
+            const int v = t % NVAR, dim = sd < DIM ? sd : sdim;
+            int L = P.level[dim * stride + pslot];
+            double c = P.center[dim * stride + pslot];
+            if (cut && dim == sdim) {
+                L += 1;
+                c = sd < DIM ? cL : cR;
+            }
+            M::fill(T, d, dim, variant_x(c, ldexp(d.hw0[dim], -L), v), I.slots[sd * NVAR + v], ties);
         }
-        double hw = ldexp(d.hw0[dim], -L);
-        double x = c;
-        if (v > 0) {
-            double lam = (v <= 2) ? G3L_LAMBDA2 : (v <= 4 ? G3L_LAMBDA4 : G3L_LAMBDA5);
-            double r = hw * lam;
-            x = (v & 1) ? c - r : c + r;
-        }
-        Model64<KIND, TERM>::fill(T, d, dim, x, slots[t], ties);
     }
-    __syncwarp();
-    for (int p = lane; p < nchild * NP; p += 32) {
-        int ch = p >= NP ? 1 : 0;
-        int pp = p - ch * NP;
-        uint32_t vv = sdesc[pp];
+    gr.sync();
+    auto slot = [&](int ch, int dim, int v) -> const Slot64 & {
+        return I.slots[((ch && dim == sdim) ? DIM : dim) * NVAR + v];
+    };
+    // r_200 and F per (mass, z) pair; auxiliary functions per projection
+    {
+        int nmz[TERM], nax[NA], tot = 0;
+#pragma unroll
+        for (int k = 0; k < TERM; ++k) {
+            nmz[k] = MZ_PAIRS * (own((8u << k) | (1u << ZD)) ? 2 : 1);
+            tot += nmz[k];
+        }
+#pragma unroll
+        for (int a = 0; a < NA; ++a) {
+            nax[a] = aux_count(TERM, a) * (own(aux_dims(TERM, a)) ? 2 : 1);
+            tot += nax[a];
+        }
+        for (int t0 = gr.rank; t0 < tot; t0 += gr.size) {
+            int t = t0, k = 0, a = -1;
+#pragma unroll
+            for (int q = 0; q < TERM; ++q)
+                if (k == q && t >= nmz[q]) {
+                    t -= nmz[q];
+                    ++k;
+                }
+            if (k < TERM) {
+                const int ch = t >= MZ_PAIRS, j = t - ch * MZ_PAIRS;
+                const int vm = mz_vm_of(j), vz = mz_vz_of(j);
+                M::mz_values(T, d, slot(ch, 3 + k, vm), slot(ch, ZD, vz).i1, KIND == 0 ? 3 : 2,
+                             I.mz[ch][k][j]);
+                continue;
+            }
+            a = 0;
+#pragma unroll
+            for (int q = 0; q < NA - 1; ++q)
+                if (a == q && t >= nax[q]) {
+                    t -= nax[q];
+                    ++a;
+                }
+            const int na = aux_count(TERM, a);
+            const int ch = t >= na, j = t - ch * na;
+            const uint32_t vv = tb.sdesc[tb.auxlist[aux_off(TERM, a) + j]];
+            const Slot64 *sp[DIM];
+#pragma unroll
+            for (int dd = 0; dd < DIM; ++dd) sp[dd] = &slot(ch, dd, (vv >> (3 * dd)) & 7);
+            I.aux[ch][aux_off(TERM, a) + j] = M::aux(T, d, a, sp);
+        }
+    }
+    gr.sync();
+    // shared u_NFW: (l, m, z) combinations, then k3 projections
+    {
+        int nu[NF], n3[NU3 > 0 ? NU3 : 1] = {0}, tot = 0;
+#pragma unroll
+        for (int f = 0; f < NF; ++f) {
+            const uint32_t dims = (1u << ucache_fun(KIND, TERM, f, 0)) |
+                                  (1u << ucache_fun(KIND, TERM, f, 1)) | (1u << ZD);
+            nu[f] = tb.ucn[f] * (own(dims) ? 2 : 1);
+            tot += nu[f];
+        }
+#pragma unroll
+        for (int f = 0; f < NU3; ++f) {
+            n3[f] = U3_MAX * (own(7u | (1u << u3_mass(KIND, TERM, f)) | (1u << ZD)) ? 2 : 1);
+            tot += n3[f];
+        }
+        for (int t0 = gr.rank; t0 < tot; t0 += gr.size) {
+            int t = t0, f = 0;
+            bool lmz = true;
+#pragma unroll
+            for (int q = 0; q < NF; ++q)
+                if (f == q && t >= nu[q]) {
+                    t -= nu[q];
+                    ++f;
+                }
+            if (f == NF) {
+                lmz = false;
+                f = 0;
+                if (NU3 == 2 && t >= n3[0]) {
+                    t -= n3[0];
+                    f = 1;
+                }
+            }
+            if (lmz) {
+                const int n = tb.ucn[f], ch = t >= n, j = t - ch * n;
+                const uint32_t key = tb.ucl[f * UC_MAX + j];
+                const int vl = key & 7, vm = (key >> 3) & 7, vz = (key >> 6) & 7;
+                const int dl = ucache_fun(KIND, TERM, f, 0), dm = ucache_fun(KIND, TERM, f, 1);
+                const int mc = ch && own((1u << dm) | (1u << ZD));
+                I.uc[ch][f][j] = M::ucached(T, d, f, slot(ch, dl, vl), slot(ch, dm, vm),
+                                            slot(ch, ZD, vz), I.mz[mc][dm - 3][mz_index(vm, vz)]);
+            } else {
+                const int ch = t >= U3_MAX, j = t - ch * U3_MAX;
+                const uint32_t vv = tb.sdesc[tb.u3list[f * U3_MAX + j]];
+                const int dm = u3_mass(KIND, TERM, f);
+                const int mc = ch && own((1u << dm) | (1u << ZD));
+                const Slot64 *sp[DIM];
+#pragma unroll
+                for (int dd = 0; dd < DIM; ++dd) sp[dd] = &slot(ch, dd, (vv >> (3 * dd)) & 7);
+                I.u3[ch][f][j] = M::u3(T, f, sp,
+                                       I.mz[mc][dm - 3][mz_index((vv >> (3 * dm)) & 7, (vv >> (3 * ZD)) & 7)]);
+            }
+        }
+    }
+    gr.sync();
+    for (int p = gr.rank; p < nchild * NP; p += gr.size) {
+        const int ch = p >= NP ? 1 : 0;
+        const int pp = p - ch * NP;
+        const uint32_t vv = tb.sdesc[pp];
         const Slot64 *sp[DIM];
 #pragma unroll
-        for (int dd = 0; dd < DIM; ++dd) {
-            int v = (vv >> (3 * dd)) & 7;
-            sp[dd] = (ch && dd == sdim) ? &slots[DIM * NVAR + v] : &slots[dd * NVAR + v];
+        for (int dd = 0; dd < DIM; ++dd) sp[dd] = &slot(ch, dd, (vv >> (3 * dd)) & 7);
+        double uc[NF], u3c[NU3 > 0 ? NU3 : 1], ax[NA];
+#pragma unroll
+        for (int f = 0; f < NF; ++f) {
+            const uint32_t dims = (1u << ucache_fun(KIND, TERM, f, 0)) |
+                                  (1u << ucache_fun(KIND, TERM, f, 1)) | (1u << ZD);
+            uc[f] = I.uc[ch && own(dims)][f][tb.ucidx[f * NP + pp]];
         }
-        vals[p] = Model64<KIND, TERM>::point(T, d, sp);
-        if (dbg) dbg[p] = vals[p];
+#pragma unroll
+        for (int f = 0; f < NU3; ++f)
+            u3c[f] = I.u3[ch && own(7u | (1u << u3_mass(KIND, TERM, f)) | (1u << ZD))][f]
+                         [tb.u3rep[f * NP + pp]];
+#pragma unroll
+        for (int a = 0; a < NA; ++a)
+            ax[a] = I.aux[ch && own(aux_dims(TERM, a))][aux_off(TERM, a) + tb.auxrep[a * NP + pp]];
+        const double *mz = TERM == 1 ? I.mz[ch && own(8u | (1u << ZD))][0]
+                                           [mz_index((vv >> 9) & 7, (vv >> (3 * ZD)) & 7)]
+                                     : nullptr;
+        const double v = M::point(T, d, sp, uc, NU3 > 0 ? u3c : nullptr, ax, mz);
+        I.vals[p] = v;
+        if (dbg) dbg[p] = v;
     }
-    __syncwarp();
-    // rule sums: lane 0 -> child 0, lane 1 -> child 1
-    if (lane < nchild) {
-        double vol = ldexp(d.rootvol, -levsum);
+    gr.sync();
+    if (gr.rank < 32) {
         double val, err;
         int split;
-        combine64<DIM>(vals + lane * NP, vol, val, err, split);
-        long long slot = lane == 0 ? pslot : qslot;
-        P.val[slot] = val;
-        P.err[slot] = err;
-        P.split[slot] = (unsigned char)split;
-        if (P.unc) P.unc[slot] = 0.f;
-        if (P.uval) P.uval[slot] = 0.f;
-    }
-    if (cut && lane < DIM) {
-        double cnew = c_l;
-        int lnew = lev;
-        if (lane == sdim) {
-            lnew = levs;
-            cnew = cL;
+        const int ch = (lane >> 3) & 1;
+        combine64_warp<DIM>(I.vals + (ch < nchild ? ch : 0) * NP, ldexp(d.rootvol, -levsum), val, err,
+                            split);
+        if ((lane & 7) == 0 && lane < 8 * nchild) {
+            const long long slot = lane == 0 ? pslot : qslot;
+            P.val[slot] = val;
+            P.err[slot] = err;
+            P.split[slot] = (unsigned char)split;
+            if (P.unc) P.unc[slot] = 0.f;
+            if (P.uval) P.uval[slot] = 0.f;
         }
-        P.center[lane * stride + pslot] = cnew;
-        P.level[lane * stride + pslot] = (unsigned char)lnew;
-        P.center[lane * stride + qslot] = lane == sdim ? cR : c_l;
-        P.level[lane * stride + qslot] = (unsigned char)lnew;
+        if (cut && lane < DIM) {
+            const int lnew = lane == sdim ? levs : lev;
+            P.center[lane * stride + pslot] = lane == sdim ? cL : c_l;
+            P.level[lane * stride + pslot] = (unsigned char)lnew;
+            P.center[lane * stride + qslot] = lane == sdim ? cR : c_l;
+            P.level[lane * stride + qslot] = (unsigned char)lnew;
+        }
     }
-    __syncwarp();
+    gr.sync();
+}
+
+// Dynamic shared memory: the group's point tables and one Item64 per warp.
+constexpr int EVAL64_WARPS = 4;
+template <int KIND, int TERM>
+constexpr size_t eval64_smem()
+{
+    return (sizeof(ReTab<KIND, TERM>) + 15) / 16 * 16 + EVAL64_WARPS * sizeof(Item64<KIND, TERM>);
 }
 
 template <int KIND, int TERM>
@@ -436,22 +703,28 @@ __global__ void __launch_bounds__(128) k_eval64(DevTables T, const IntDesc *__re
                                                 IntState *__restrict__ S, Pool P, BatchHdr *H,
                                                 const long long *__restrict__ woff)
 {
-    constexpr int DIM = TERM + 4;
-    constexpr int NP = rule_points(DIM);
-    constexpr int NSLOT = (DIM + 1) * NVAR;
-    constexpr int WPB = 4;
-    __shared__ uint32_t sdesc[NP];
-    __shared__ Slot64 sslot[WPB][NSLOT];
-    __shared__ double svals[WPB][2 * NP];
+    extern __shared__ __align__(16) unsigned char smem64[];
+    using RT = ReTab<KIND, TERM>;
     const int g = KIND * 3 + TERM - 1;
-    for (int p = threadIdx.x; p < NP; p += blockDim.x) sdesc[p] = point_variants(DIM, p);
-    __syncthreads();
-    const int wib = threadIdx.x >> 5;
     const int gb = H->gbeg[g], ge = H->gbeg[g + 1];
     if (gb >= ge) return;
     const long long wbeg = woff[gb], wend = woff[ge];
-    const long long nwarps = (long long)gridDim.x * WPB;
-    for (long long w = wbeg + (long long)blockIdx.x * WPB + wib; w < wend; w += nwarps) {
+    // Few items: the whole block takes one, so that a round of few cuts is not as long as one
+    // warp's evaluation of a whole cut.  The warps of a full grid otherwise take one each
+    // (no idle lanes at the ends of the passes, no block barriers).  The line lies where a
+    // block per item would take a second turn.
+    const bool wide = wend - wbeg <= (long long)gridDim.x;
+    const int wib = threadIdx.x >> 5;
+    const long long first = wide ? blockIdx.x : (long long)blockIdx.x * EVAL64_WARPS + wib;
+    const long long step = wide ? (long long)gridDim.x : (long long)gridDim.x * EVAL64_WARPS;
+    // no work for the block: skip the tables
+    if (wbeg + (wide ? first : (long long)blockIdx.x * EVAL64_WARPS) >= wend) return;
+    const RT &tb = load_retab<KIND, TERM>(P, smem64);
+    Item64<KIND, TERM> *items =
+        reinterpret_cast<Item64<KIND, TERM> *>(smem64 + (sizeof(RT) + 15) / 16 * 16);
+    const Group gr{wide ? 128 : 32, wide ? (int)threadIdx.x : (int)(threadIdx.x & 31)};
+    Item64<KIND, TERM> &I = items[wide ? 0 : wib];
+    for (long long w = wbeg + first; w < wend; w += step) {
         int lo = gb, hi = ge - 1;  // last integral i with woff[i] <= w
         while (lo < hi) {
             int mid = (lo + hi + 1) >> 1;
@@ -465,8 +738,7 @@ __global__ void __launch_bounds__(128) k_eval64(DevTables T, const IntDesc *__re
         const bool cut = cj >= 0;  // cj < 0: a fresh integral's root region
         const long long pslot = d.base + (cut ? cj : 0);
         const long long qslot = cut ? d.base + (S[i].nR - S[i].K) + j : -1;
-        warp_item64<KIND, TERM>(T, d, P, pslot, qslot, cut, sslot[wib], svals[wib], sdesc,
-                                &H->ties, H->dbg);
+        group_item64<KIND, TERM>(T, d, P, pslot, qslot, cut, I, tb, gr, &H->ties, H->dbg);
     }
 }
 
@@ -535,56 +807,6 @@ struct Reeval {
         return n < P.rcap ? n : P.rcap;
     }
 };
-
-// Point tables of a group's re-evaluation passes: the point codes, the (l, m, z)
-// combinations of the cached u_NFW (ucache_tables) and the projections of the k3 u_NFW
-// (u3_tables) and of the auxiliary functions (aux_tables).  The same for every launch, so
-// k_re_tables builds them once per context into P.retab and each block copies them to
-// shared memory (building them per block cost more than the cached work saves).
-template <int KIND, int TERM>
-struct ReTab {
-    static constexpr int DIM = TERM + 4, NP = rule_points(DIM), NF = ucache_nf(TERM);
-    static constexpr int NU3 = u3_nfun(TERM) > 0 ? u3_nfun(TERM) : 1, NA = aux_nfun(TERM);
-    uint32_t sdesc[NP];
-    int ucn[NF];
-    uint16_t ucl[NF * UC_MAX];
-    uint8_t ucidx[NF * NP];
-    uint8_t u3rep[NU3 * NP];
-    uint8_t u3list[NU3 * U3_MAX];
-    uint8_t auxrep[NA * NP];
-    uint8_t auxlist[AUX_MAX];
-};
-
-template <int KIND, int TERM>
-__global__ void __launch_bounds__(128) k_re_tables(unsigned char *out)
-{
-    using RT = ReTab<KIND, TERM>;
-    static_assert(sizeof(RT) <= RETAB_BYTES && sizeof(RT) % 4 == 0, "re-evaluation table size");
-    __shared__ __align__(16) unsigned char buf[sizeof(RT)];
-    __shared__ uint8_t map[RT::NF * 343];
-    RT &t = *reinterpret_cast<RT *>(buf);
-    ucache_tables<KIND, TERM>(t.ucidx, t.ucl, t.ucn, map);
-    for (int p = threadIdx.x; p < RT::NP; p += blockDim.x) t.sdesc[p] = point_variants(RT::DIM, p);
-    __syncthreads();
-    u3_tables<KIND, TERM>(t.sdesc, t.u3rep, t.u3list, map);  // map is free again
-    aux_tables<TERM>(t.sdesc, t.auxrep, t.auxlist, map);
-    uint32_t *dst = reinterpret_cast<uint32_t *>(out + (KIND * 3 + TERM - 1) * RETAB_BYTES);
-    for (int i = threadIdx.x; i < (int)(sizeof(RT) / 4); i += blockDim.x)
-        dst[i] = reinterpret_cast<const uint32_t *>(buf)[i];
-}
-
-// copy group (KIND, TERM)'s tables to shared memory buf (every thread calls it)
-template <int KIND, int TERM>
-__device__ inline const ReTab<KIND, TERM> &load_retab(const Pool &P, unsigned char *buf)
-{
-    using RT = ReTab<KIND, TERM>;
-    const uint32_t *src =
-        reinterpret_cast<const uint32_t *>(P.retab + (KIND * 3 + TERM - 1) * RETAB_BYTES);
-    for (int i = threadIdx.x; i < (int)(sizeof(RT) / 4); i += blockDim.x)
-        reinterpret_cast<uint32_t *>(buf)[i] = __ldg(src + i);
-    __syncthreads();
-    return *reinterpret_cast<const RT *>(buf);
-}
 
 template <int KIND, int TERM>
 __global__ void __launch_bounds__(128) k_re_fill(DevTables T, const IntDesc *__restrict__ D,
@@ -970,6 +1192,14 @@ void *reeval64_kernel(int kind, int term)
     static void *tab[2][3] = {
         {(void *)k_reeval64<0, 1>, (void *)k_reeval64<0, 2>, (void *)k_reeval64<0, 3>},
         {(void *)k_reeval64<1, 1>, (void *)k_reeval64<1, 2>, (void *)k_reeval64<1, 3>}};
+    return tab[kind][term - 1];
+}
+
+// dynamic shared memory of a group's k_eval64
+size_t eval64_smem_bytes(int kind, int term)
+{
+    static const size_t tab[2][3] = {{eval64_smem<0, 1>(), eval64_smem<0, 2>(), eval64_smem<0, 3>()},
+                                     {eval64_smem<1, 1>(), eval64_smem<1, 2>(), eval64_smem<1, 3>()}};
     return tab[kind][term - 1];
 }
 
