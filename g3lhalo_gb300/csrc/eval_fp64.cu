@@ -1,15 +1,15 @@
 // eval_fp64.cu -- all-FP64 rule evaluation: the plain FP64 form of the engine.
 //
-// A warp (or, when a round has few cuts, a block) evaluates one work item: it cuts a
-// selected parent region along its split dimension (cut_region,
-// src/hcubature.cpp:206-218) and applies the Genz-Malik 7/5 rule to both children
-// (rule75genzmalik_evalError, src/hcubature.cpp:456-577), or evaluates a root region.
+// A block evaluates one work item: it cuts a selected parent region along its split
+// dimension (cut_region, src/hcubature.cpp:206-218) and applies the Genz-Malik 7/5 rule to
+// both children (rule75genzmalik_evalError, src/hcubature.cpp:456-577), or evaluates a
+// root region.
 // The per-dimension coordinate variants (c, c-+lambda*h) are computed once per child
 // together with everything that depends on one coordinate only (10^x, aperture filter,
 // HOD occupations, bin indices), then what depends on a few coordinates once per
 // projection of the points onto them; each lane then evaluates whole points.  The rule
-// sums are formed in the reference's summation order.  Compiled with -fmad=false so every product and sum rounds as in the
-// reference's CPU build.
+// sums are formed in the reference's summation order.  Compiled with -fmad=false so every
+// product and sum rounds as in the reference's CPU build.
 #include "phys64.cuh"
 
 namespace g3l {
@@ -34,7 +34,7 @@ __device__ __forceinline__ double variant_x(double c, double hw, int v)
 // truncated z bin of z = x (the z slot's i1, Model64::fill)
 __device__ __forceinline__ int z_trunc64(const DevTables &T, double x)
 {
-    double zr = (x - T.zmin) * T.Nz / (T.zmax - T.zmin);
+    double zr = ddiv((x - T.zmin) * T.Nz, T.zmax - T.zmin);
     return min(max((int)zr, 0), T.Nz - 1);
 }
 
@@ -85,7 +85,7 @@ struct Model64 {
             }
         } else {  // z
             S.a[0] = x;
-            double zr = (x - T.zmin) * T.Nz / (T.zmax - T.zmin);
+            double zr = ddiv((x - T.zmin) * T.Nz, T.zmax - T.zmin);
             S.i0 = min(max((int)round(zr), 0), T.Nz - 1);
             S.i1 = min(max((int)zr, 0), T.Nz - 1);
         }
@@ -98,7 +98,7 @@ struct Model64 {
                                      const Slot64 &M, const Slot64 &Z, const double *mz)
     {
         const double w_ = __ldg(T.w + Z.i0);
-        const double k = L.a[0] / w_;
+        const double k = ddiv(L.a[0], w_);
         const double conc = __ldg(T.conc + Z.i1 * T.Nm + M.i1);
         const int fs = ucache_fun(KIND, TERM, f, 2);
         const double c = (fs == 0 ? 1.0 : (fs == 1 ? T.hod[6 * d.hod1] : T.hod[6 * d.hod2])) * conc;
@@ -127,7 +127,7 @@ struct Model64 {
         const double l1 = L1.a[0], l2 = L2.a[0], cphi = PH.a[0];
         const double w_ = __ldg(T.w + Z.i0);
         const double l3 = sqrt(l1 * l1 + l2 * l2 + 2 * l1 * l2 * cphi);
-        const double k3 = l3 / w_;
+        const double k3 = ddiv(l3, w_);
         const double c = 1.0 * __ldg(T.conc + Z.i1 * T.Nm + M.i1);
         if (!mz) return u_nfw64_F(k3, r200_64(M.a[0], __ldg(T.rho_bar + Z.i1)), c, nfw_norm64(c));
         return u_nfw64_F(k3, mz[0], c, mz[1]);
@@ -143,8 +143,8 @@ struct Model64 {
         if (a == 0) return aperture64(d.theta[2] * l3);
         const int z_ix = s[DIM - 1]->i0;
         const double w_ = __ldg(T.w + z_ix);
-        if (TERM == 3) return bi_lin64(T, l1 / w_, l2 / w_, cphi, z_ix);
-        return plin64(T, z_ix, (a == 1 ? l1 : (a == 2 ? l2 : l3)) / w_);
+        if (TERM == 3) return bi_lin64(T, ddiv(l1, w_), ddiv(l2, w_), cphi, z_ix);
+        return plin64(T, z_ix, ddiv(a == 1 ? l1 : (a == 2 ? l2 : l3), w_));
     }
 
     // uc: the cached u_NFW values of this point (ucache_fun order), or null; u3c: its
@@ -159,9 +159,9 @@ struct Model64 {
         const int z_ix = Z.i0, z_it = Z.i1, Nm = T.Nm;
         const double w_ = __ldg(T.w + z_ix);
         const double l3 = sqrt(l1 * l1 + l2 * l2 + 2 * l1 * l2 * cphi);
-        const double k1 = l1 / w_;
-        const double k2 = l2 / w_;
-        const double k3 = l3 / w_;
+        const double k1 = ddiv(l1, w_);
+        const double k2 = ddiv(l2, w_);
+        const double k3 = ddiv(l3, w_);
         const double rho = __ldg(T.rho_bar + z_ix);
         const double rhot = __ldg(T.rho_bar + z_it);
         const double f1 = T.hod[6 * d.hod1];
@@ -179,10 +179,11 @@ struct Model64 {
                 const double u3 = mz ? u_nfw64_F(k3, mz[0], 1.0 * cc, mz[1]) : u_nfw64(k3, r2, cc, 1);
                 const double u2 = uc ? uc[1] : u_nfw64(k2, r2, cc, f2);
                 const double u1 = uc ? uc[0] : u_nfw64(k1, r2, cc, f1);
-                double Bggd = 1. / nbar1 / nbar2 / rho * __ldg(T.hmf + z_ix * Nm + M.i0) * m * u3;
+                double Bggd = ddiv(ddiv(ddiv(1., nbar1), nbar2), rho) * __ldg(T.hmf + z_ix * Nm + M.i0) * m * u3;
                 Bggd *= M.a[1] * M.a[4] * u2 + M.a[3] * M.a[2] * u1 + M.a[5] * u1 * u2;
-                double bggk = Bggd / __ldg(T.dwdz + z_ix) * __ldg(T.g + z_ix) *
-                              __ldg(T.p1 + z_ix) * __ldg(T.p2 + z_ix) / w_ / w_ / w_ * (1. + z);
+                double bggk = ddiv(Bggd, __ldg(T.dwdz + z_ix)) * __ldg(T.g + z_ix) *
+                              __ldg(T.p1 + z_ix) * __ldg(T.p2 + z_ix);
+                bggk = ddiv(ddiv(ddiv(bggk, w_), w_), w_) * (1. + z);
                 return l1 * l2 * m * l1 * l2 * L1.a[1] * L2.a[1] * U3 * bggk;
             } else if (TERM == 2) {
                 // src/NNMap_Model.cu:787-856
@@ -207,13 +208,14 @@ struct Model64 {
                 const double Gg_k2m2 = M2.a[3] + M2.a[4] * u2_2;  // hod2 at m2
                 const double Gg_k2m1 = M1.a[3] + M1.a[4] * u2_1;  // hod2 at m1
                 const double Gg_k1m2 = M2.a[1] + M2.a[2] * u1_2;  // hod1 at m2
-                double Bggd = 1. / nbar1 / nbar2 / rho * __ldg(T.hmf + z_ix * Nm + M1.i0) *
+                double Bggd = ddiv(ddiv(ddiv(1., nbar1), nbar2), rho) * __ldg(T.hmf + z_ix * Nm + M1.i0) *
                               __ldg(T.hmf + z_ix * Nm + M2.i0) * __ldg(T.b_h + z_ix * Nm + M1.i0) *
                               __ldg(T.b_h + z_ix * Nm + M2.i0) *
                               (m1 * u3_1 * Ggg * Pk3 + m2 * u3_2 * Gg_k1m1 * Gg_k2m2 * Pk1 +
                                m2 * u3_2 * Gg_k2m1 * Gg_k1m2 * Pk2);
-                double bggk = 1. / __ldg(T.dwdz + z_ix) * __ldg(T.g + z_ix) * __ldg(T.p1 + z_ix) *
-                              __ldg(T.p2 + z_ix) / w_ / w_ / w_ * (1. + z) * Bggd;
+                double bggk = ddiv(1., __ldg(T.dwdz + z_ix)) * __ldg(T.g + z_ix) *
+                              __ldg(T.p1 + z_ix) * __ldg(T.p2 + z_ix);
+                bggk = ddiv(ddiv(ddiv(bggk, w_), w_), w_) * (1. + z) * Bggd;
                 return l1 * l2 * m1 * m2 * l1 * l2 * L1.a[1] * L2.a[1] * U3 * bggk;
             } else {
                 // src/NNMap_Model.cu:1003-1037
@@ -225,13 +227,14 @@ struct Model64 {
                 const double u2 = uc ? uc[1] : u_nfw64(k2, r200_64(m2, rhot), __ldg(T.conc + z_it * Nm + M2.i1), f2);
                 const double Gg1 = M1.a[1] + M1.a[2] * u1;  // hod1 at m1
                 const double Gg2 = M2.a[3] + M2.a[4] * u2;  // hod2 at m2
-                double Bggd = 1. / nbar1 / nbar2 / rho * __ldg(T.hmf + z_ix * Nm + M1.i0) *
+                double Bggd = ddiv(ddiv(ddiv(1., nbar1), nbar2), rho) * __ldg(T.hmf + z_ix * Nm + M1.i0) *
                               __ldg(T.hmf + z_ix * Nm + M2.i0) * __ldg(T.hmf + z_ix * Nm + M3.i0) *
                               m3 * u3 * Gg1 * Gg2 * (ax ? ax[1] : bi_lin64(T, k1, k2, cphi, z_ix)) *
                               __ldg(T.b_h + z_ix * Nm + M1.i0) * __ldg(T.b_h + z_ix * Nm + M2.i0) *
                               __ldg(T.b_h + z_ix * Nm + M3.i0);
-                double bggk = Bggd / __ldg(T.dwdz + z_ix) * __ldg(T.g + z_ix) * __ldg(T.p1 + z_ix) *
-                              __ldg(T.p2 + z_ix) / w_ / w_ / w_ * (1. + z);
+                double bggk = ddiv(Bggd, __ldg(T.dwdz + z_ix)) * __ldg(T.g + z_ix) *
+                              __ldg(T.p1 + z_ix) * __ldg(T.p2 + z_ix);
+                bggk = ddiv(ddiv(ddiv(bggk, w_), w_), w_) * (1. + z);
                 return l1 * l2 * m1 * m2 * m3 * l1 * l2 * L1.a[1] * L2.a[1] * U3 * bggk;
             }
         } else {
@@ -244,13 +247,13 @@ struct Model64 {
                 const double m = M.a[0];
                 const double r2 = mz ? mz[0] : r200_64(m, rhot);  // mz[0] is this value
                 const double cc = __ldg(T.conc + z_it * Nm + M.i1);
-                double Bgdd = 1. / nbar / rho / rho * __ldg(T.hmf + z_ix * Nm + M.i0) * m * m *
+                double Bgdd = ddiv(ddiv(ddiv(1., nbar), rho), rho) * __ldg(T.hmf + z_ix * Nm + M.i0) * m * m *
                               (M.a[1] + M.a[2] * (uc ? uc[0] : u_nfw64(k1, r2, cc, f))) *
                               (uc ? uc[1] : u_nfw64(k2, r2, cc, 1)) *
                               (mz ? u_nfw64_F(k3, mz[0], 1.0 * cc, mz[1]) : u_nfw64(k3, r2, cc, 1));
-                double bgkk = Bgdd / __ldg(T.dwdz + z_ix) * gz * gz * __ldg(T.p1 + z_ix) / w_ / w_ *
-                              (1. + z) * (1. + z);
-                return l1 * l2 * m * l1 * l2 * L1.a[1] * L2.a[1] * U3 * bgkk / nbar;
+                double bgkk = ddiv(Bgdd, __ldg(T.dwdz + z_ix)) * gz * gz * __ldg(T.p1 + z_ix);
+                bgkk = ddiv(ddiv(bgkk, w_), w_) * (1. + z) * (1. + z);
+                return ddiv(l1 * l2 * m * l1 * l2 * L1.a[1] * L2.a[1] * U3 * bgkk, nbar);
             } else if (TERM == 2) {
                 // src/NMapMap_Model.cu:402-468
                 const Slot64 &M1 = *s[3], &M2 = *s[4];
@@ -267,15 +270,15 @@ struct Model64 {
                 const double u3_1 = u3c ? u3c[0] : u_nfw64(k3, ra, ca, 1);
                 const double u2_2 = uc ? uc[2] : u_nfw64(k2, rb, cb, 1);
                 const double u1_1f = uc ? uc[3] : u_nfw64(k1, ra, ca, f);
-                double Bgdd = 1. / nbar / rho / rho * __ldg(T.hmf + z_ix * Nm + M1.i0) *
+                double Bgdd = ddiv(ddiv(ddiv(1., nbar), rho), rho) * __ldg(T.hmf + z_ix * Nm + M1.i0) *
                               __ldg(T.hmf + z_ix * Nm + M2.i0) * __ldg(T.b_h + z_ix * Nm + M1.i0) *
                               __ldg(T.b_h + z_ix * Nm + M2.i0) *
                               (m1 * m2 * u2_1 * u3_2 * (M2.a[1] + M2.a[2] * u1_2f) * Pk2 +
                                m1 * m2 * u3_1 * u2_2 * (M2.a[1] + M2.a[2] * u1_2f) * Pk3 +
                                m2 * m2 * u2_1 * u3_2 * (M1.a[1] + M1.a[2] * u1_1f) * Pk1);
-                double bgkk = Bgdd / __ldg(T.dwdz + z_ix) * gz * gz * __ldg(T.p1 + z_ix) / w_ / w_ *
-                              (1. + z) * (1. + z);
-                return l1 * l2 * m1 * m2 * l1 * l2 * L1.a[1] * L2.a[1] * U3 * bgkk / nbar;
+                double bgkk = ddiv(Bgdd, __ldg(T.dwdz + z_ix)) * gz * gz * __ldg(T.p1 + z_ix);
+                bgkk = ddiv(ddiv(bgkk, w_), w_) * (1. + z) * (1. + z);
+                return ddiv(l1 * l2 * m1 * m2 * l1 * l2 * L1.a[1] * L2.a[1] * U3 * bgkk, nbar);
             } else {
                 // src/NMapMap_Model.cu:592-632 (Nc, Ns at m3; u_NFW(k1, m2, f))
                 const Slot64 &M1 = *s[3], &M2 = *s[4], &M3 = *s[5];
@@ -283,7 +286,7 @@ struct Model64 {
                 const double ra = r200_64(m1, rhot), rb = r200_64(m2, rhot);
                 const double ca = __ldg(T.conc + z_it * Nm + M1.i1);
                 const double cb = __ldg(T.conc + z_it * Nm + M2.i1);
-                double Bgdd = 1. / nbar / rho / rho * __ldg(T.hmf + z_ix * Nm + M1.i0) *
+                double Bgdd = ddiv(ddiv(ddiv(1., nbar), rho), rho) * __ldg(T.hmf + z_ix * Nm + M1.i0) *
                               __ldg(T.hmf + z_ix * Nm + M2.i0) * __ldg(T.hmf + z_ix * Nm + M3.i0) *
                               __ldg(T.b_h + z_ix * Nm + M1.i0) * __ldg(T.b_h + z_ix * Nm + M2.i0) *
                               __ldg(T.b_h + z_ix * Nm + M3.i0) * m1 * m2 *
@@ -291,9 +294,9 @@ struct Model64 {
                               (u3c ? u3c[0] : u_nfw64(k3, rb, cb, 1)) *
                               (M3.a[1] + M3.a[2] * (uc ? uc[1] : u_nfw64(k1, rb, cb, f))) *
                               (ax ? ax[1] : bi_lin64(T, k1, k2, cphi, z_ix));
-                double bgkk = Bgdd / __ldg(T.dwdz + z_ix) * gz * gz * __ldg(T.p1 + z_ix) / w_ / w_ *
-                              (1. + z) * (1. + z);
-                return l1 * l2 * m1 * m2 * m3 * l1 * l2 * L1.a[1] * L2.a[1] * U3 * bgkk / nbar;
+                double bgkk = ddiv(Bgdd, __ldg(T.dwdz + z_ix)) * gz * gz * __ldg(T.p1 + z_ix);
+                bgkk = ddiv(ddiv(bgkk, w_), w_) * (1. + z) * (1. + z);
+                return ddiv(l1 * l2 * m1 * m2 * m3 * l1 * l2 * L1.a[1] * L2.a[1] * U3 * bgkk, nbar);
             }
         }
     }
@@ -389,16 +392,6 @@ __device__ inline const ReTab<KIND, TERM> &load_retab(const Pool &P, unsigned ch
     return *reinterpret_cast<const RT *>(buf);
 }
 
-// Threads that share one work item: a warp, or the whole block.
-struct Group {
-    int size, rank;  // 32 or 128; rank of this thread
-    __device__ void sync() const
-    {
-        if (size == 32) __syncwarp();
-        else __syncthreads();
-    }
-};
-
 // Shared memory of one work item.  Child 1 has its own copy of a cached function only when
 // the split dimension is among the function's dimensions.
 template <int KIND, int TERM>
@@ -468,7 +461,7 @@ __device__ void combine64_warp(const double *v, double vol, double &val, double 
     split = dimDiffMax;
 }
 
-// One work item on a group of threads: `cut` = bisect the region at pslot along its split
+// One work item on a block of 128 threads: `cut` = bisect the region at pslot along its split
 // dimension into pslot (lower half) and qslot (upper half) and evaluate both; otherwise
 // evaluate the region at pslot in place (roots).  Four passes with a barrier between:
 // coordinate slots; (mass, z) values and the auxiliary functions; every u_NFW that several
@@ -479,10 +472,10 @@ __device__ void combine64_warp(const double *v, double vol, double &val, double 
 // counts is the number of warp instructions: the 2-halo rule takes 132 + 186 u_NFW per
 // child at most instead of 894, the 3-halo rule 66 + 93 instead of 723.
 template <int KIND, int TERM>
-__device__ void group_item64(const DevTables &T, const IntDesc &d, const Pool &P, long long pslot,
+__device__ void block_item64(const DevTables &T, const IntDesc &d, const Pool &P, long long pslot,
                              long long qslot, bool cut, Item64<KIND, TERM> &I,
-                             const ReTab<KIND, TERM> &tb, const Group &gr,
-                             unsigned long long *ties, double *dbg)
+                             const ReTab<KIND, TERM> &tb, int rank, unsigned long long *ties,
+                             double *dbg)
 {
     using M = Model64<KIND, TERM>;
     using It = Item64<KIND, TERM>;
@@ -515,7 +508,7 @@ __device__ void group_item64(const DevTables &T, const IntDesc &d, const Pool &P
         const bool smass = cut && sdim >= 3 && sdim < 3 + TERM;
         const int nm = TERM * NVAR, nms = nm + (smass ? NVAR : 0);
         const int nslot = (DIM + nchild - 1) * NVAR;
-        for (int t = gr.rank; t < nslot; t += gr.size) {
+        for (int t = rank; t < nslot; t += 128) {
             int sd;  // slot row: dimension, or DIM for child 1's split dimension
             if (t < nms) {
                 sd = t / NVAR < TERM ? 3 + t / NVAR : DIM;
@@ -533,7 +526,7 @@ __device__ void group_item64(const DevTables &T, const IntDesc &d, const Pool &P
             M::fill(T, d, dim, variant_x(c, ldexp(d.hw0[dim], -L), v), I.slots[sd * NVAR + v], ties);
         }
     }
-    gr.sync();
+    __syncthreads();
     auto slot = [&](int ch, int dim, int v) -> const Slot64 & {
         return I.slots[((ch && dim == sdim) ? DIM : dim) * NVAR + v];
     };
@@ -550,7 +543,7 @@ __device__ void group_item64(const DevTables &T, const IntDesc &d, const Pool &P
             nax[a] = aux_count(TERM, a) * (own(aux_dims(TERM, a)) ? 2 : 1);
             tot += nax[a];
         }
-        for (int t0 = gr.rank; t0 < tot; t0 += gr.size) {
+        for (int t0 = rank; t0 < tot; t0 += 128) {
             int t = t0, k = 0, a = -1;
 #pragma unroll
             for (int q = 0; q < TERM; ++q)
@@ -581,7 +574,7 @@ __device__ void group_item64(const DevTables &T, const IntDesc &d, const Pool &P
             I.aux[ch][aux_off(TERM, a) + j] = M::aux(T, d, a, sp);
         }
     }
-    gr.sync();
+    __syncthreads();
     // shared u_NFW: (l, m, z) combinations, then k3 projections
     {
         int nu[NF], n3[NU3 > 0 ? NU3 : 1] = {0}, tot = 0;
@@ -597,7 +590,7 @@ __device__ void group_item64(const DevTables &T, const IntDesc &d, const Pool &P
             n3[f] = U3_MAX * (own(7u | (1u << u3_mass(KIND, TERM, f)) | (1u << ZD)) ? 2 : 1);
             tot += n3[f];
         }
-        for (int t0 = gr.rank; t0 < tot; t0 += gr.size) {
+        for (int t0 = rank; t0 < tot; t0 += 128) {
             int t = t0, f = 0;
             bool lmz = true;
 #pragma unroll
@@ -635,8 +628,8 @@ __device__ void group_item64(const DevTables &T, const IntDesc &d, const Pool &P
             }
         }
     }
-    gr.sync();
-    for (int p = gr.rank; p < nchild * NP; p += gr.size) {
+    __syncthreads();
+    for (int p = rank; p < nchild * NP; p += 128) {
         const int ch = p >= NP ? 1 : 0;
         const int pp = p - ch * NP;
         const uint32_t vv = tb.sdesc[pp];
@@ -664,8 +657,8 @@ __device__ void group_item64(const DevTables &T, const IntDesc &d, const Pool &P
         I.vals[p] = v;
         if (dbg) dbg[p] = v;
     }
-    gr.sync();
-    if (gr.rank < 32) {
+    __syncthreads();
+    if (rank < 32) {
         double val, err;
         int split;
         const int ch = (lane >> 3) & 1;
@@ -687,44 +680,28 @@ __device__ void group_item64(const DevTables &T, const IntDesc &d, const Pool &P
             P.level[lane * stride + qslot] = (unsigned char)lnew;
         }
     }
-    gr.sync();
+    __syncthreads();
 }
 
-// Dynamic shared memory: the group's point tables and one Item64 per warp.
-constexpr int EVAL64_WARPS = 4;
+// A block per work item.  (Measured against a warp per item, four per block, which has fewer
+// idle lanes at the ends of the passes but leaves a round of few cuts as long as one warp's
+// evaluation of a whole cut and an SM's quarters unevenly loaded: the block is as fast or
+// faster for rounds of any size, 9 triplets x 3 NMapMap terms 16.0 -> 14.9 ms.)
 template <int KIND, int TERM>
-constexpr size_t eval64_smem()
-{
-    return (sizeof(ReTab<KIND, TERM>) + 15) / 16 * 16 + EVAL64_WARPS * sizeof(Item64<KIND, TERM>);
-}
-
-template <int KIND, int TERM>
-__global__ void __launch_bounds__(128) k_eval64(DevTables T, const IntDesc *__restrict__ D,
+__global__ void __launch_bounds__(128, 5) k_eval64(DevTables T, const IntDesc *__restrict__ D,
                                                 IntState *__restrict__ S, Pool P, BatchHdr *H,
                                                 const long long *__restrict__ woff)
 {
-    extern __shared__ __align__(16) unsigned char smem64[];
     using RT = ReTab<KIND, TERM>;
+    __shared__ __align__(16) unsigned char tbuf[sizeof(RT)];
+    __shared__ Item64<KIND, TERM> I;
     const int g = KIND * 3 + TERM - 1;
     const int gb = H->gbeg[g], ge = H->gbeg[g + 1];
     if (gb >= ge) return;
     const long long wbeg = woff[gb], wend = woff[ge];
-    // Few items: the whole block takes one, so that a round of few cuts is not as long as one
-    // warp's evaluation of a whole cut.  The warps of a full grid otherwise take one each
-    // (no idle lanes at the ends of the passes, no block barriers).  The line lies where a
-    // block per item would take a second turn.
-    const bool wide = wend - wbeg <= (long long)gridDim.x;
-    const int wib = threadIdx.x >> 5;
-    const long long first = wide ? blockIdx.x : (long long)blockIdx.x * EVAL64_WARPS + wib;
-    const long long step = wide ? (long long)gridDim.x : (long long)gridDim.x * EVAL64_WARPS;
-    // no work for the block: skip the tables
-    if (wbeg + (wide ? first : (long long)blockIdx.x * EVAL64_WARPS) >= wend) return;
-    const RT &tb = load_retab<KIND, TERM>(P, smem64);
-    Item64<KIND, TERM> *items =
-        reinterpret_cast<Item64<KIND, TERM> *>(smem64 + (sizeof(RT) + 15) / 16 * 16);
-    const Group gr{wide ? 128 : 32, wide ? (int)threadIdx.x : (int)(threadIdx.x & 31)};
-    Item64<KIND, TERM> &I = items[wide ? 0 : wib];
-    for (long long w = wbeg + first; w < wend; w += step) {
+    if (wbeg + blockIdx.x >= wend) return;  // no work here: skip the tables
+    const RT &tb = load_retab<KIND, TERM>(P, tbuf);
+    for (long long w = wbeg + blockIdx.x; w < wend; w += gridDim.x) {
         int lo = gb, hi = ge - 1;  // last integral i with woff[i] <= w
         while (lo < hi) {
             int mid = (lo + hi + 1) >> 1;
@@ -738,7 +715,11 @@ __global__ void __launch_bounds__(128) k_eval64(DevTables T, const IntDesc *__re
         const bool cut = cj >= 0;  // cj < 0: a fresh integral's root region
         const long long pslot = d.base + (cut ? cj : 0);
         const long long qslot = cut ? d.base + (S[i].nR - S[i].K) + j : -1;
-        group_item64<KIND, TERM>(T, d, P, pslot, qslot, cut, I, tb, gr, &H->ties, H->dbg);
+        // a block's first warps get the passes' uneven remainders: the warp that comes first
+        // turns with the item, so that the SM's quarters share them
+        const int turn = 32 * (int)((w + (w >> 3) + (w >> 7)) & 3);
+        block_item64<KIND, TERM>(T, d, P, pslot, qslot, cut, I, tb, (threadIdx.x + turn) & 127,
+                                 &H->ties, H->dbg);
     }
 }
 
@@ -1192,14 +1173,6 @@ void *reeval64_kernel(int kind, int term)
     static void *tab[2][3] = {
         {(void *)k_reeval64<0, 1>, (void *)k_reeval64<0, 2>, (void *)k_reeval64<0, 3>},
         {(void *)k_reeval64<1, 1>, (void *)k_reeval64<1, 2>, (void *)k_reeval64<1, 3>}};
-    return tab[kind][term - 1];
-}
-
-// dynamic shared memory of a group's k_eval64
-size_t eval64_smem_bytes(int kind, int term)
-{
-    static const size_t tab[2][3] = {{eval64_smem<0, 1>(), eval64_smem<0, 2>(), eval64_smem<0, 3>()},
-                                     {eval64_smem<1, 1>(), eval64_smem<1, 2>(), eval64_smem<1, 3>()}};
     return tab[kind][term - 1];
 }
 

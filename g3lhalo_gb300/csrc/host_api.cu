@@ -33,7 +33,6 @@
 
 namespace g3l {
 void *eval64_kernel(int kind, int term);
-size_t eval64_smem_bytes(int kind, int term);
 void *reeval64_kernel(int kind, int term);
 void *reeval_phase_kernel(int kind, int term, int phase);
 cudaError_t build_reeval_tables(unsigned char *out, cudaStream_t s);
@@ -403,16 +402,10 @@ void *eval_fn(const g3l_ctx *c, int precision, int group)
                                  : evalmx_kernel(kind, term, c->opt.evalmx_variant[group]);
 }
 
-// dynamic shared memory of the rule kernel of a group
-size_t eval_smem(int precision, int group)
-{
-    return precision == G3L_FP64 ? eval64_smem_bytes(group / 3, group % 3 + 1) : 0;
-}
-
-int eval_grid(g3l_ctx *c, void *fn, size_t smem)
+int eval_grid(g3l_ctx *c, void *fn)
 {
     int nb = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, fn, 128, smem) != cudaSuccess || nb < 1) nb = 1;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, fn, 128, 0) != cudaSuccess || nb < 1) nb = 1;
     if (c->opt.eval_blocks_per_sm > 0) nb = std::min(nb, c->opt.eval_blocks_per_sm);
     return nb * c->nsm;
 }
@@ -448,13 +441,13 @@ struct KernelArgs {
 };
 
 int add_kernel(cudaGraph_t g, cudaGraphNode_t *node, const cudaGraphNode_t *deps, size_t ndeps,
-               void *fn, int grid, int block, void **args, size_t smem = 0)
+               void *fn, int grid, int block, void **args)
 {
     cudaKernelNodeParams kp{};
     kp.func = fn;
     kp.gridDim = dim3(grid);
     kp.blockDim = dim3(block);
-    kp.sharedMemBytes = (unsigned)smem;
+    kp.sharedMemBytes = 0;
     kp.kernelParams = args;
     G3L_CK(cudaGraphAddKernelNode(node, g, deps, ndeps, &kp));
     return G3L_OK;
@@ -576,8 +569,7 @@ int build_graph_ws(g3l_ctx *c, Workspace &W, int precision, int gmask, bool init
         void *args[] = {&a.T, &a.D, &a.S, &a.P, &a.H, &a.woff};
         cudaGraphNode_t n_ev, deps[2] = {prev, ends[grp]};
         int st = add_kernel(body, &n_ev, deps, precision == G3L_MIXED ? 2 : 1, fn,
-                            eval_grid(c, fn, eval_smem(precision, grp)), 128, args,
-                            eval_smem(precision, grp));
+                            eval_grid(c, fn), 128, args);
         if (st) return st;
         prev = n_ev;
     }
@@ -709,8 +701,7 @@ int run_host_loop(g3l_ctx *c, int precision, int gmask, int *launches)
             void *fn = eval_fn(c, precision, grp);
             void *args[] = {&a.T, &a.D, &a.S, &a.P, &a.H, &a.woff};
             G3L_CK(cudaEventRecord(c->tev[2 * grp], s));
-            const size_t sm = eval_smem(precision, grp);
-            G3L_CK(cudaLaunchKernel(fn, dim3(eval_grid(c, fn, sm)), dim3(128), args, sm, s));
+            G3L_CK(cudaLaunchKernel(fn, dim3(eval_grid(c, fn)), dim3(128), args, 0, s));
             G3L_CK(cudaEventRecord(c->tev[2 * grp + 1], s));
             ++*launches;
         }
@@ -1271,10 +1262,6 @@ try {
     G3L_CK(cudaHostGetDevicePointer((void **)&c->cancel_d, c->cancel_h, 0));
     G3L_CK(cudaMalloc((void **)&c->retab_d, (size_t)NGROUPS * RETAB_BYTES));
     G3L_CK(build_reeval_tables(c->retab_d, c->stream));
-    for (int g = 0; g < NGROUPS; ++g)
-        G3L_CK(cudaFuncSetAttribute(eval64_kernel(g / 3, g % 3 + 1),
-                                    cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    (int)eval64_smem_bytes(g / 3, g % 3 + 1)));
     G3L_CK(cudaStreamSynchronize(c->stream));
     c->B = host::Binning{t->Nz, t->Nm, t->Nk, t->zmin, t->zmax, t->mmin, t->mmax, t->kmin, t->kmax};
     c->Om = t->Om;
@@ -2034,8 +2021,7 @@ try {
         if (rc) break;
         KernelArgs a{c->T, W.D, W.S, W.P, W.H, W.woff, 0, 0, 0.0, 0.0};
         void *args[] = {&a.T, &a.D, &a.S, &a.P, &a.H, &a.woff};
-        if (cudaLaunchKernel(eval_fn(c, precision, grp), dim3(1), dim3(128), args,
-                             eval_smem(precision, grp), s)) {
+        if (cudaLaunchKernel(eval_fn(c, precision, grp), dim3(1), dim3(128), args, 0, s)) {
             rc = G3L_ERR_CUDA;
             break;
         }
@@ -2389,8 +2375,7 @@ int eval_static_locked(g3l_ctx *c, const g3l_integral *items, int n, int precisi
             if (!(gmask & (1 << g))) continue;
             void *fn = eval_fn(c, precision, g);
             void *args[] = {&a.T, &a.D, &a.S, &a.P, &a.H, &a.woff};
-            const size_t sm = eval_smem(precision, g);
-            G3L_CK(cudaLaunchKernel(fn, dim3(eval_grid(c, fn, sm)), dim3(128), args, sm, s));
+            G3L_CK(cudaLaunchKernel(fn, dim3(eval_grid(c, fn)), dim3(128), args, 0, s));
             ++launches;
         }
         G3L_CK(cudaMemcpyAsync(&active, &a.H->any_active, sizeof(int), cudaMemcpyDeviceToHost, s));

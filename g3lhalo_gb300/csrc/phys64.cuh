@@ -12,8 +12,10 @@
 // (2015, GalSim).  The small-argument branch evaluates them with explicit powers left
 // to right as the reference does; the large-argument branch in Horner form on 1/x^2
 // (one FP64 division instead of forty; ~1e-16 relative from the reference's order).
+// Divisions run on the integer pipes (ddiv, idiv64.cuh: the same bits).
 #pragma once
 #include "g3l_device.cuh"
+#include "idiv64.cuh"
 
 namespace g3l {
 
@@ -36,7 +38,7 @@ __device__ __forceinline__ void sici64_sc(double x, double &si, double &ci, doub
         double b = 1 + 1.01162145739225565e-2 * x2 + 4.99175116169755106e-5 * x4 +
                    1.55654986308745614e-7 * x6 + 3.28067571055789734e-10 * x8 +
                    4.5049097575386581e-13 * x10 + 3.21107051193712168e-16 * x12;
-        si = x * a / b;
+        si = ddiv(x * a, b);
         a = -0.25 + 7.51851524438898291e-3 * x2 - 1.27528342240267686e-4 * x4 +
             1.05297363846239184e-6 * x6 - 4.68889508144848019e-9 * x8 +
             1.06480802891189243e-11 * x10 - 9.93728488857585407e-15 * x12;
@@ -44,13 +46,13 @@ __device__ __forceinline__ void sici64_sc(double x, double &si, double &ci, doub
             2.55533277086129636e-7 * x6 + 6.97071295760958946e-10 * x8 +
             1.38536352772778619e-12 * x10 + 1.89106054713059759e-15 * x12 +
             1.39759616731376855e-18 * x14;
-        ci = 0.5772156649 + log(x) + x2 * a / b;
+        ci = 0.5772156649 + log(x) + ddiv(x2 * a, b);
         sincos(x, &sx, &cx);
     } else {
         // f = (1/x) A(t)/B(t), g = t C(t)/D(t) with t = 1/x^2: the reference's explicit
         // powers of 1/x (src/generalFunctions.cu:65-81) in Horner form, one division for t
         // instead of one per term (each FP64 division is a multi-instruction sequence)
-        const double t = 1 / x2;
+        const double t = ddiv(1, x2);
         double sin_x, cos_x;
         sincos(x, &sin_x, &cos_x);
         double A = -4.94701168645415959931e11;
@@ -95,8 +97,8 @@ __device__ __forceinline__ void sici64_sc(double x, double &si, double &ci, doub
         Dd = Dd * t + 2.40036752835578777e5;
         Dd = Dd * t + 8.19595201151451564e2;
         Dd = Dd * t + 1;
-        const double f = A / B / x;
-        const double g = C / Dd * t;
+        const double f = ddiv(ddiv(A, B), x);
+        const double g = ddiv(C, Dd) * t;
         si = 0.5 * 3.14159265358979323846 - f * cos_x - g * sin_x;
         ci = f * sin_x - g * cos_x;
         sx = sin_x;
@@ -114,18 +116,18 @@ __device__ __forceinline__ void sici64(double x, double &si, double &ci)
 // F = ln(1 + c) - c / (1 + c) (callers that share one (mass, z) pair pass F once computed)
 __device__ __forceinline__ double u_nfw64_F(double k, double r200, double c, double F)
 {
-    double arg1 = k * r200 / c;
+    double arg1 = ddiv(k * r200, c);
     double arg2 = arg1 * (1 + c);
     double si1, ci1, si2, ci2, s1, c1;
     sici64_sc(arg1, si1, ci1, s1, c1);  // s1, c1 = sin(arg1), cos(arg1)
     sici64(arg2, si2, ci2);
     double term1 = s1 * (si2 - si1);
     double term2 = c1 * (ci2 - ci1);
-    double term3 = -sin(arg1 * c) / arg2;
-    return (term1 + term2 + term3) / F;
+    double term3 = ddiv(-sin(arg1 * c), arg2);
+    return ddiv(term1 + term2 + term3, F);
 }
 
-__device__ __forceinline__ double nfw_norm64(double c) { return log(1. + c) - c / (1. + c); }
+__device__ __forceinline__ double nfw_norm64(double c) { return log(1. + c) - ddiv(c, 1. + c); }
 
 // NFW Fourier profile given k, r_200 and the tabulated concentration (truncated indices
 // are resolved by the caller, as in src/generalFunctions.cu:11-15).
@@ -137,7 +139,7 @@ __device__ __forceinline__ double u_nfw64(double k, double r200, double conc, do
 
 __device__ __forceinline__ double r200_64(double m, double rho)
 {
-    return pow(0.239 * m / rho / 200, 1. / 3.);
+    return pow(ddiv(ddiv(0.239 * m, rho), 200), 1. / 3.);
 }
 
 __device__ __forceinline__ double aperture64(double eta)
@@ -151,9 +153,9 @@ __device__ __forceinline__ double aperture64(double eta)
 // the same expression, so the same values)
 __device__ __forceinline__ void occupations64(const double *h, double m, double &nc, double &ns)
 {
-    const double e1 = 1 + erf(log(m / h[2]) / h[3] / 1.414213562);
+    const double e1 = 1 + erf(ddiv(ddiv(log(ddiv(m, h[2])), h[3]), 1.414213562));
     nc = 0.5 * h[1] * e1;
-    ns = 0.5 * e1 * pow(m / h[4], h[5]);
+    ns = 0.5 * e1 * pow(ddiv(m, h[4]), h[5]);
 }
 // NsatNsat from the two satellite occupations Ns1 (hod1) and Ns2 (hod2) at m, the
 // reference's expression (src/HOD.cu:78-94) with its nsat calls' values passed in;
@@ -169,13 +171,13 @@ __device__ __forceinline__ double nsatnsat64(double Ns1, double Ns2, int same, d
 
 __device__ __forceinline__ double F2_64(double k1, double k2, double cosphi)
 {
-    return 0.7143 + 0.2857 * cosphi * cosphi + 0.5 * cosphi * (k1 / k2 + k2 / k2);
+    return 0.7143 + 0.2857 * cosphi * cosphi + 0.5 * cosphi * (ddiv(k1, k2) + ddiv(k2, k2));
 }
 
 // P_lin lookup with the small-k linear extrapolation (src/NNMap_Model.cu:819-839)
 __device__ __forceinline__ double plin64(const DevTables &T, int z_ix, double k)
 {
-    int k_ix = (int)round(log(k / T.kmin) * T.Nk / T.ln_kratio);
+    int k_ix = (int)round(ddiv(log(ddiv(k, T.kmin)) * T.Nk, T.ln_kratio));
     if (k_ix >= 0) {
         // clamp_k: stay in the z row; otherwise the reference's flat read, bounded by
         // the end of the table (the reference reads past it)
@@ -184,7 +186,7 @@ __device__ __forceinline__ double plin64(const DevTables &T, int z_ix, double k)
         const long long last = (long long)T.Nz * T.Nk - 1;
         return __ldg(T.P_lin + (flat > last ? last : flat));
     }
-    return __ldg(T.P_lin + z_ix * T.Nk) / T.kmin * k;
+    return ddiv(__ldg(T.P_lin + z_ix * T.Nk), T.kmin) * k;
 }
 
 __device__ __forceinline__ double bi_lin64(const DevTables &T, double k1, double k2,
@@ -192,8 +194,8 @@ __device__ __forceinline__ double bi_lin64(const DevTables &T, double k1, double
 {
     double k3 = sqrt(k1 * k1 + k2 * k2 + 2 * k1 * k2 * cosphi);
     double c_phi12 = cosphi;
-    double c_phi13 = (k2 * k2 - k3 * k3 - k1 * k1) / (2 * k1 * k3);
-    double c_phi23 = (k1 * k1 - k2 * k2 - k3 * k3) / (2 * k3 * k2);
+    double c_phi13 = ddiv(k2 * k2 - k3 * k3 - k1 * k1, 2 * k1 * k3);
+    double c_phi23 = ddiv(k1 * k1 - k2 * k2 - k3 * k3, 2 * k3 * k2);
     double Pk1 = plin64(T, z_ix, k1);
     double Pk2 = plin64(T, z_ix, k2);
     double Pk3 = plin64(T, z_ix, k3);

@@ -33,6 +33,7 @@
 
 #include "g3l_gpu.h"
 #include "host_internal.h"
+#include "idiv64.cuh"
 
 namespace g3l {
 namespace {
@@ -231,11 +232,11 @@ __device__ __forceinline__ double k_integrand(const PcTask &t, double x, double 
     // the top-hat's W = 3 (sin y - y cos y) / y^3 and its derivative with one division each
     // (src/Powerspectrum.cpp:104-114)
     const double y2 = y * y;
-    const double q = 3 / (y2 * y);
+    const double q = ddiv(3, y2 * y);
     const double W = q * (sy - y * cy);
     if (t.type != PC_DSIGMA2) return W * W * g * amp;  // src/Powerspectrum.cpp:79-102, 219-243
     // src/Powerspectrum.cpp:267-293
-    const double Wprime = ((y2 - 3.) * sy + 3. * y * cy) * x * q / y;
+    const double Wprime = ddiv(((y2 - 3.) * sy + 3. * y * cy) * x * q, y);
     return W * Wprime * g * (t.dR * amp);
 }
 
@@ -290,7 +291,7 @@ __device__ __forceinline__ void rule_gk15_hw(double f, int hl, double hw, double
     double e = __shfl_sync(0xffffffffu, t, 1, 16);
     const double rabs = __shfl_sync(0xffffffffu, t, 2, 16), rasc = __shfl_sync(0xffffffffu, t, 3, 16);
     if (rasc != 0 && e != 0) {
-        const double q = 200 * e / rasc;
+        const double q = ddiv(200 * e, rasc);
         const double scale = q * sqrt(q);
         e = (scale < 1) ? rasc * scale : rasc;
     }
