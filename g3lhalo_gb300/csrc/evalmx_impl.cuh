@@ -2,8 +2,8 @@
 // evalmx_impl.cuh -- mixed-precision rule evaluation: FP32 integrand, wide accumulation
 // (instantiated in evalmx_k0.cu and evalmx_k1.cu).
 //
-// Same work decomposition as eval_fp64.cu (one warp cuts one parent region and
-// applies the Genz-Malik 7/5 rule to both children), with the arithmetic
+// One warp, or a block when a round has few cuts, cuts one parent region and applies the
+// Genz-Malik 7/5 rule to both children, with the arithmetic
 // rearranged for a GPU whose FP64 rate is ~1/60 of its FP32 rate:
 //  * Region centres stay FP64 in HBM; each is split into a double-float with
 //    integer operations, and the 7 coordinate variants c, c-+lambda h of every
@@ -746,12 +746,23 @@ __device__ __forceinline__ df hw_sum(df a)
 // integral (default 0: always); the selection kernel has it re-taken in FP64 if the
 // region is cut.  The error estimate's bound (unc) decides selection boundaries.
 
+// Threads that share one work item: a warp, or the whole block of 128.
+struct Group {
+    int size, rank;
+    __device__ void sync() const
+    {
+        if (size == 32) __syncwarp();
+        else __syncthreads();
+    }
+};
+
 template <int KIND, int TERM>
-__device__ void warp_itemF(const DevTables &T, const IntDesc &d, int iint, double Vcur,
-                           const Pool &P, BatchHdr *H, long long pslot, long long qslot, bool cut,
-                           SlotF *slots, float *vals, Child &C, const uint32_t *sdesc,
-                           unsigned &ties, int &small, const uint8_t *ucidx,
-                           const uint16_t *ucl, const int *ucn, float *ucache)
+__device__ void group_itemF(const Group &gr, const DevTables &T, const IntDesc &d, int iint,
+                            double Vcur, const Pool &P, BatchHdr *H, long long pslot,
+                            long long qslot, bool cut, SlotF *slots, float *vals, Child &C,
+                            const uint32_t *sdesc, unsigned &ties, int &small,
+                            const uint8_t *ucidx, const uint16_t *ucl, const int *ucn,
+                            float *ucache)
 {
     constexpr int DIM = TERM + 4;
     constexpr int NP = rule_points(DIM);
@@ -778,18 +789,18 @@ __device__ void warp_itemF(const DevTables &T, const IntDesc &d, int iint, doubl
     const double cL = __shfl_sync(0xffffffffu, cchild, 0);
     const double cR = __shfl_sync(0xffffffffu, cchild, 1);
     const int levsum = __reduce_add_sync(0xffffffffu, lane < DIM ? lev : 0) + (cut ? 1 : 0);
-    if (lane < DIM) {
+    if (gr.rank < DIM) {
         C.c64[lane] = (cut && lane == sdim) ? cL : c_l;
         C.lev[lane] = (cut && lane == sdim) ? levs : lev;
     }
-    if (lane == DIM) {
+    if (gr.rank == DIM) {
         C.c64[DIM] = cR;
         C.lev[DIM] = levs;
     }
-    __syncwarp();
+    gr.sync();
     // coordinate-variant slots
     const int nslot = (DIM + nchild - 1) * NVAR;
-    for (int t = lane; t < nslot; t += 32) {
+    for (int t = gr.rank; t < nslot; t += gr.size) {
         const int sd = t / NVAR, v = t - sd * NVAR;
         const int dim = sd < DIM ? sd : sdim;
         df x = df_from_double(C.c64[sd]);
@@ -800,10 +811,10 @@ __device__ void warp_itemF(const DevTables &T, const IntDesc &d, int iint, doubl
         }
         ModelF<KIND, TERM>::fill(T, d, C, sd, dim, v, x, slots[t], ties);
     }
-    __syncwarp();
+    gr.sync();
     // u_NFW of the (l, m, z) variant combinations the points share, per child
     constexpr int NF = ModelF<KIND, TERM>::NF;
-    for (int t = lane; ModelF<KIND, TERM>::UC && t < nchild * NF * UC_MAX; t += 32) {
+    for (int t = gr.rank; ModelF<KIND, TERM>::UC && t < nchild * NF * UC_MAX; t += gr.size) {
         const int ch = t / (NF * UC_MAX), r = t - ch * NF * UC_MAX;
         const int f = r / UC_MAX, j = r - f * UC_MAX;
         if (j >= ucn[f]) continue;
@@ -816,9 +827,9 @@ __device__ void warp_itemF(const DevTables &T, const IntDesc &d, int iint, doubl
         ucache[(ch * NF + f) * UC_MAX + j] =
             ModelF<KIND, TERM>::ucached(T, d, f, sl(dl, vl), sl(dm, vm), sl(DIM - 1, vz), small);
     }
-    __syncwarp();
+    gr.sync();
     // points
-    for (int p = lane; p < nchild * NP; p += 32) {
+    for (int p = gr.rank; p < nchild * NP; p += gr.size) {
         const int ch = p >= NP ? 1 : 0;
         const int pp = p - ch * NP;
         const uint32_t vv = sdesc[pp];
@@ -836,7 +847,8 @@ __device__ void warp_itemF(const DevTables &T, const IntDesc &d, int iint, doubl
         vals[p] = ModelF<KIND, TERM>::point(T, d, sp, C, ch, sdim, vv, ties, small, uc);
         if (H->dbg) H->dbg[p] = (double)vals[p];
     }
-    __syncwarp();
+    gr.sync();
+    if (gr.rank >= 32) return;  // the first warp forms the sums (the caller synchronises)
     // rule sums in double-float, uncertainty sums in FP32: half-warp hh serves child hh
     const int hh = lane >> 4, hl = lane & 15;
     const bool active = hh < nchild;
@@ -974,7 +986,6 @@ __device__ void warp_itemF(const DevTables &T, const IntDesc &d, int iint, doubl
         P.center[lane * stride + qslot] = lane == sdim ? cR : c_l;
         P.level[lane * stride + qslot] = (unsigned char)C.lev[lane];
     }
-    __syncwarp();
 }
 
 // MINB: the blocks per SM the register budget is cut for (6: 80 registers per thread,
@@ -1008,8 +1019,16 @@ __global__ void __launch_bounds__(128, MINB) k_evalmx(DevTables T, const IntDesc
     const long long wbeg = woff[gb], wend = woff[ge];
     unsigned ties = 0;
     int small = 0;
-    const long long nwarps = (long long)gridDim.x * WPB;
-    for (long long w = wbeg + (long long)blockIdx.x * WPB + wib; w < wend; w += nwarps) {
+    // Few items: a block takes one, so that a round of few cuts is not as long as one warp's
+    // evaluation of a whole cut.  The warps of a full grid take one each otherwise (no idle
+    // lanes at the ends of the passes, no block barriers).  The line lies where a block per
+    // item would take a second turn.  One triplet, 3 terms: 9.3 -> 7.7 ms.
+    const bool wide = wend - wbeg <= (long long)gridDim.x;
+    const Group gr{wide ? 128 : 32, wide ? (int)threadIdx.x : lane};
+    const int buf = wide ? 0 : wib;
+    const long long first = wide ? blockIdx.x : (long long)blockIdx.x * WPB + wib;
+    const long long step = (long long)gridDim.x * (wide ? 1 : WPB);
+    for (long long w = wbeg + first; w < wend; w += step) {
         int lo = gb, hi = ge - 1;
         while (lo < hi) {
             int mid = (lo + hi + 1) >> 1;
@@ -1023,9 +1042,10 @@ __global__ void __launch_bounds__(128, MINB) k_evalmx(DevTables T, const IntDesc
         const bool cut = cj >= 0;
         const long long pslot = d.base + (cut ? cj : 0);
         const long long qslot = cut ? d.base + (S[i].nR - S[i].K) + j : -1;
-        warp_itemF<KIND, TERM>(T, d, i, S[i].val, P, H, pslot, qslot, cut, sslot[wib],
-                               svals[wib], schild[wib], sdesc, ties, small, ucidx, ucl, ucn,
-                               ucache[wib]);
+        group_itemF<KIND, TERM>(gr, T, d, i, S[i].val, P, H, pslot, qslot, cut, sslot[buf],
+                                svals[buf], schild[buf], sdesc, ties, small, ucidx, ucl, ucn,
+                                ucache[buf]);
+        gr.sync();
     }
     // warp-aggregated diagnostics
     unsigned tw = __reduce_add_sync(0xffffffffu, ties);

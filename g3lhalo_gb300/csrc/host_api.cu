@@ -106,6 +106,7 @@ struct Workspace {
 
 struct GraphEntry {
     int gen, precision, gmask;
+    bool side;  // the groups' rule kernels side by side
     cudaGraph_t graph;
     cudaGraphExec_t exec;
 };
@@ -467,10 +468,19 @@ void set_esc_queues(const IntDesc *D, int n, BatchHdr &H)
     }
 }
 
+// The groups' rule kernels run side by side in a call whose region pools hold at most this
+// many regions, in a chain otherwise.  A call cuts a region pool's worth of regions over
+// ~25 rounds: below the line a round leaves each kernel's grid partly empty and its length
+// is the sum of three short kernels; above it each kernel fills the device and concurrent
+// ones contend for caches and registers.  Measured, chain against side by side: mixed 32k
+// regions (one triplet) 7.67 / 6.81 ms, 310k 19.2 / 18.0, 2.4M 64.8 / 69.3; FP64 700 regions
+// 5.33 / 3.26 ms, 7.7k 10.5 / 9.6, 16k 14.1 / 15.0.
+constexpr long long kSideMaxMixed = 600000, kSideMaxFp64 = 10000;
+
 // The device loop as one graph: init, then WHILE (conditional node) { select, [mixed:
 // FP64 re-evaluations, second selection pass], scan, [mixed: re-evaluations], rule
 // evaluation per group }.  `init` = false leaves the states as they are (serving).
-int build_graph_ws(g3l_ctx *c, Workspace &W, int precision, int gmask, bool init,
+int build_graph_ws(g3l_ctx *c, Workspace &W, int precision, int gmask, bool init, bool side,
                    GraphEntry &out)
 {
     KernelArgs a{c->T, W.D, W.S, W.P, W.H, W.woff, 0, 1, c->T.tau_sel, c->T.tau_val};
@@ -559,29 +569,30 @@ int build_graph_ws(g3l_ctx *c, Workspace &W, int precision, int gmask, bool init
         int st = add_reevals(prev, ends);
         if (st) return st;
     }
-    // the groups' rule kernels in a chain (side-by-side branches measured slower: each
-    // kernel fills the device, and concurrent ones contend for it); a group's kernel
-    // waits for the previous one and its own re-evaluations, so the other groups'
-    // re-evaluations run beside it
+    // the groups' rule kernels in a chain, or side by side (kSideMaxMixed); a group's
+    // kernel waits for the previous one, if chained, and its own re-evaluations, so the
+    // other groups' re-evaluations run beside it
     for (int grp = 0; grp < NGROUPS; ++grp) {
         if (!(gmask & (1 << grp))) continue;
         void *fn = eval_fn(c, precision, grp);
         void *args[] = {&a.T, &a.D, &a.S, &a.P, &a.H, &a.woff};
-        cudaGraphNode_t n_ev, deps[2] = {prev, ends[grp]};
-        int st = add_kernel(body, &n_ev, deps, precision == G3L_MIXED ? 2 : 1, fn,
-                            eval_grid(c, fn), 128, args);
+        cudaGraphNode_t n_ev, deps[2];
+        int nd = 0;
+        if (!side || precision != G3L_MIXED) deps[nd++] = prev;
+        if (precision == G3L_MIXED) deps[nd++] = ends[grp];
+        int st = add_kernel(body, &n_ev, deps, nd, fn, eval_grid(c, fn), 128, args);
         if (st) return st;
-        prev = n_ev;
+        if (!side) prev = n_ev;
     }
     cudaGraphExec_t ex;
     G3L_CK(cudaGraphInstantiate(&ex, g, 0));
-    out = GraphEntry{W.gen, precision, gmask, g, ex};
+    out = GraphEntry{W.gen, precision, gmask, side, g, ex};
     return G3L_OK;
 }
 
-int build_graph(g3l_ctx *c, int precision, int gmask, GraphEntry &out)
+int build_graph(g3l_ctx *c, int precision, int gmask, bool side, GraphEntry &out)
 {
-    return build_graph_ws(c, c->W, precision, gmask, true, out);
+    return build_graph_ws(c, c->W, precision, gmask, true, side, out);
 }
 
 // descriptor of one integral: bounds and root geometry as the reference computes them
@@ -1046,7 +1057,7 @@ int srv_create(g3l_ctx *c, int precision, int per_group, uint64_t pool_regions, 
     if (cudaStreamCreateWithFlags(&v->s, cudaStreamNonBlocking) != cudaSuccess) st = G3L_ERR_CUDA;
     if (!st) st = alloc_workspace(v->W, v->n, v->pool, c->retab_d);
     if (!st) st = dalloc(&v->d_new, (size_t)v->n) | dalloc(&v->d_idx, (size_t)v->n);
-    if (!st) st = build_graph_ws(c, v->W, precision, (1 << NGROUPS) - 1, false, v->G);
+    if (!st) st = build_graph_ws(c, v->W, precision, (1 << NGROUPS) - 1, false, true, v->G);
     if (!st) v->graph_ok = true;
     if (!st) {
         // every slot starts free: a finished state, never selected
@@ -1820,12 +1831,14 @@ try {
     int launches = 0;
     G3L_CK(cudaEventRecord(c->ev0, c->stream));
     if (c->opt.use_graph) {
+        const bool side = base <= (precision == G3L_FP64 ? kSideMaxFp64 : kSideMaxMixed);
         GraphEntry *ge = nullptr;
         for (auto &g : c->graphs)
-            if (g.gen == W.gen && g.precision == precision && g.gmask == gmask) ge = &g;
+            if (g.gen == W.gen && g.precision == precision && g.gmask == gmask && g.side == side)
+                ge = &g;
         if (!ge) {
             GraphEntry e;
-            st = build_graph(c, precision, gmask, e);
+            st = build_graph(c, precision, gmask, side, e);
             if (st) return st;
             c->graphs.push_back(e);
             ge = &c->graphs.back();
