@@ -9,10 +9,10 @@
 //              converged(): err <= |val| rtol, src/converged.h:10-14) and picks
 //              the regions the heap would pop: the largest errors, in order,
 //              until the remaining error is <= rtol |val| (Gladwell), capped by
-//              the evaluation budget.  Both cut-offs are found with an MSD radix
-//              select on the IEEE bit pattern of the errors; the running error
-//              sums use 64-bit fixed point, so the choice is deterministic and
-//              independent of thread scheduling.
+//              the evaluation budget.  Both cut-offs are found with histograms of
+//              the IEEE bit patterns of the errors; the running error sums use
+//              64-bit fixed point, so the choice is deterministic and independent
+//              of thread scheduling.
 //   k_scan   : prefix sum of the per-integral pop counts -> flat work list; sets
 //              the graph's WHILE condition (no host round trip).
 //   k_eval*  : cut + rule evaluation (eval_fp64.cu / evalmx_impl.cuh).
@@ -25,6 +25,8 @@ namespace g3l {
 
 constexpr int SEL_BS = 256;
 constexpr int SEL_WARPS = SEL_BS / 32;
+constexpr int SEL_BUCKETS = 1024;  // histogram of one selection pass (a multiple of SEL_BS)
+constexpr int SEL_PER = SEL_BUCKETS / SEL_BS;
 
 __device__ __forceinline__ unsigned long long ekey(const double *err, long long s)
 {
@@ -49,152 +51,246 @@ __device__ T block_sum(T v, T *sh)
     return r;
 }
 
-// exclusive block scan of 0/1 flags; returns prefix, writes the total
-__device__ int block_flag_scan(int flag, int *sh, int &total)
+// x 2^s as FP32, truncated (x >= 0); odd is set where x does not fit
+__device__ __forceinline__ float f32_scaled(double x, int s, bool &odd)
 {
-    unsigned b = __ballot_sync(0xffffffffu, flag);
-    int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    int pre = __popc(b & ((1u << lane) - 1u));
-    if (lane == 0) sh[w] = __popc(b);
-    __syncthreads();
-    int off = 0, tot = 0;
-    for (int k = 0; k < SEL_WARPS; ++k) {
-        if (k < w) off += sh[k];
-        tot += sh[k];
-    }
-    __syncthreads();
-    total = tot;
-    return off + pre;
+    const unsigned long long u = (unsigned long long)__double_as_longlong(x);
+    const int e = (int)((u >> 52) & 0x7ffu) - 1023 + s;
+    if (u == 0) return 0.f;
+    if (e < -126 || e > 60) odd = true;
+    const unsigned m = (unsigned)(u >> 29) & 0x7fffffu;
+    return e < -126 ? 0.f : __uint_as_float(((unsigned)min(e, 60) + 127u) << 23 | m);
 }
 
-__device__ float block_max(float v, float *sh)
+// floor(t) of t >= 0, all ones from 1.8e19 on, by integer operations (an FP64 compare and
+// conversion occupy the FP64 pipe for 64 cycles each)
+__device__ __forceinline__ unsigned long long floor_u64(double t)
 {
-    for (int o = 16; o > 0; o >>= 1) v = fmaxf(v, __shfl_down_sync(0xffffffffu, v, o));
-    if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = v;
-    __syncthreads();
-    float r = 0.f;
-    if (threadIdx.x == 0) {
-        for (int w = 0; w < SEL_WARPS; ++w) r = fmaxf(r, sh[w]);
-        sh[0] = r;
-    }
-    __syncthreads();
-    r = sh[0];
-    __syncthreads();
-    return r;
+    const unsigned long long u = (unsigned long long)__double_as_longlong(t);
+    if (u >= 0x43EF399B1438A100ull) return 0xFFFFFFFFFFFFFFFFull;  // 1.8e19
+    const int e = (int)(u >> 52) - 1075;
+    const unsigned long long m = (u & 0xFFFFFFFFFFFFFull) | 0x10000000000000ull;
+    return e >= 0 ? m << e : (e > -64 ? m >> -e : 0ull);
 }
 
 struct SelShared {
-    unsigned int cnt[256];
-    unsigned long long sum[256];
-    unsigned long long prefix, mask;
-    unsigned long long sum_above;
-    unsigned int cnt_above;
-    int chosen, unique;
-    double dred[SEL_WARPS];
+    unsigned int cnt[SEL_BUCKETS];
+    unsigned long long sum[SEL_BUCKETS];
+    unsigned long long ck[32], cq[32];  // candidates of the boundary bucket
+    unsigned long long wk[2][SEL_WARPS];
+    unsigned int wc[SEL_WARPS];
+    unsigned long long bkey, qb, sum_above;
+    unsigned int cnt_above, chosen, chosen_cnt, ncand;
+    double dred[2 * SEL_WARPS];
     unsigned long long ured[SEL_WARPS];
-    int ired[SEL_WARPS];
-    float fred[SEL_WARPS];
+    float fred[2 * SEL_WARPS];
+    int ired[2][SEL_WARPS];
+    int odd, ubits;
 };
 
-// MSD radix select over the live errors of one integral, descending.  by_sum:
-// find the bucket where the cumulative fixed-point error first reaches `need`;
-// otherwise where the cumulative count reaches `need`.  Returns the boundary key
-// and the count/sum of strictly larger keys.
-__device__ void radix_select(const double *err, const unsigned long long *q, long long base, int R,
-                             bool by_sum, unsigned long long need, SelShared &sh,
-                             unsigned long long &bkey, unsigned int &cnt_above,
-                             unsigned long long &sum_above)
+// Block sums of two doubles (in block_sum's order) and of the two FP32 bounds, which stay
+// in sh.fred[0], sh.fred[1]; sh.odd: any odd.
+__device__ void block_totals(double sv, double se, float fue, float fuv, bool odd, SelShared &sh,
+                             double &V, double &E)
 {
-    if (threadIdx.x == 0) {
-        sh.prefix = 0;
-        sh.mask = 0;
-        sh.sum_above = 0;
-        sh.cnt_above = 0;
-        sh.unique = 0;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    for (int o = 16; o > 0; o >>= 1) {
+        sv += __shfl_down_sync(0xffffffffu, sv, o);
+        se += __shfl_down_sync(0xffffffffu, se, o);
+        fue += __shfl_down_sync(0xffffffffu, fue, o);
+        fuv += __shfl_down_sync(0xffffffffu, fuv, o);
+    }
+    if (lane == 0) {
+        sh.dred[warp] = sv;
+        sh.dred[SEL_WARPS + warp] = se;
+        sh.fred[warp] = fue;
+        sh.fred[SEL_WARPS + warp] = fuv;
+    }
+    odd = __syncthreads_or(odd);
+    double r = 0;
+    float f = 0.f;
+    if (threadIdx.x < 2) {
+        for (int w = 0; w < SEL_WARPS; ++w) {
+            r += sh.dred[threadIdx.x * SEL_WARPS + w];
+            f += sh.fred[threadIdx.x * SEL_WARPS + w];
+        }
     }
     __syncthreads();
-    for (int pass = 0; pass < 8; ++pass) {
-        const int shift = 56 - 8 * pass;
-        sh.cnt[threadIdx.x] = 0;
-        sh.sum[threadIdx.x] = 0;
-        __syncthreads();
-        const unsigned long long prefix = sh.prefix, mask = sh.mask;
-        for (int j = threadIdx.x; j < R; j += SEL_BS) {
-            unsigned long long k = ekey(err, base + j);
-            if ((k & mask) == prefix) {
-                int dg = (int)((k >> shift) & 255ull);
+    if (threadIdx.x < 2) {
+        sh.dred[threadIdx.x] = r;
+        sh.fred[threadIdx.x] = f;
+    }
+    if (threadIdx.x == 0) sh.odd = odd;
+    __syncthreads();
+    V = sh.dred[0];
+    E = sh.dred[1];
+}
+
+// Boundary of a selection of the largest keys of one integral (err: keys as doubles >= 0,
+// descending by bit pattern).  by_sum: the key at which the cumulative q first reaches
+// `need`; otherwise at which the cumulative count does.  Returns that key, the count and sum
+// of the strictly larger keys and (by_sum) the q of the key.
+//
+// One pass histograms the keys' bit patterns linearly between the smallest and the largest
+// (a logarithmic scale), which spreads them over the 1024 buckets: digits of the pattern
+// itself start with bytes of sign and exponent that nearly all keys share, and the 64-bit
+// atomics of a whole integral then queue at one or two addresses (8 such passes were most
+// of k_select's time).  The boundary bucket is narrowed the same way until it holds at most
+// 32 keys, which one warp ranks.  All sums are integers: the result does not depend on the
+// order of the threads.
+__device__ void boundary_select(const double *err, const unsigned long long *q, long long base, int R,
+                                bool by_sum, unsigned long long need, SelShared &sh,
+                                unsigned long long &bkey, unsigned int &cnt_above,
+                                unsigned long long &sum_above, unsigned long long &qb)
+{
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    unsigned long long kmn = ~0ull, kmx = 0;
+    for (int j = tid; j < R; j += SEL_BS) {
+        const unsigned long long k = ekey(err, base + j);
+        kmn = k < kmn ? k : kmn;
+        kmx = k > kmx ? k : kmx;
+    }
+    for (int o = 16; o > 0; o >>= 1) {
+        const unsigned long long a = __shfl_xor_sync(0xffffffffu, kmn, o);
+        const unsigned long long b = __shfl_xor_sync(0xffffffffu, kmx, o);
+        kmn = a < kmn ? a : kmn;
+        kmx = b > kmx ? b : kmx;
+    }
+    if (lane == 0) {
+        sh.wk[0][warp] = kmn;
+        sh.wk[1][warp] = kmx;
+    }
+    for (int b = 0; b < SEL_PER; ++b) {
+        sh.cnt[b * SEL_BS + tid] = 0;
+        sh.sum[b * SEL_BS + tid] = 0;
+    }
+    __syncthreads();
+    kmn = sh.wk[0][0];
+    kmx = sh.wk[1][0];
+    for (int w = 1; w < SEL_WARPS; ++w) {
+        kmn = sh.wk[0][w] < kmn ? sh.wk[0][w] : kmn;
+        kmx = sh.wk[1][w] > kmx ? sh.wk[1][w] : kmx;
+    }
+    unsigned long long lo = kmn, span = kmx - kmn, sa = 0;
+    unsigned int ca = 0;
+    for (;;) {
+        const int bits = 64 - __clzll((long long)span);
+        const int shift = bits > 10 ? bits - 10 : 0;
+        for (int j = tid; j < R; j += SEL_BS) {
+            const unsigned long long d = ekey(err, base + j) - lo;  // wraps below lo
+            if (d <= span) {
+                const unsigned dg = (unsigned)(d >> shift);
                 atomicAdd(&sh.cnt[dg], 1u);
                 if (by_sum) atomicAdd(&sh.sum[dg], q[base + j]);
             }
         }
         __syncthreads();
-        if (threadIdx.x < 32) {
-            // lane l owns buckets 255-8l .. 248-8l (descending)
-            const int lane = threadIdx.x;
-            unsigned long long s = 0, c = 0;
-            for (int b = 0; b < 8; ++b) {
-                int dg = 255 - 8 * lane - b;
-                s += sh.sum[dg];
-                c += sh.cnt[dg];
-            }
-            unsigned long long v = by_sum ? s : c;
-            unsigned long long inc = v;  // inclusive scan in descending bucket order
-            for (int o = 1; o < 32; o <<= 1) {
-                unsigned long long t = __shfl_up_sync(0xffffffffu, inc, o);
-                if (lane >= o) inc += t;
-            }
-            const unsigned long long base_v = by_sum ? sh.sum_above : sh.cnt_above;
-            unsigned hit = __ballot_sync(0xffffffffu, base_v + inc >= need);
-            int first = hit ? __ffs(hit) - 1 : 31;
-            unsigned long long exs = 0, exc_c = 0;
-            // exclusive sums of both quantities at the owning lane
-            unsigned long long sc = s, cc = c;
-            for (int o = 1; o < 32; o <<= 1) {
-                unsigned long long t1 = __shfl_up_sync(0xffffffffu, sc, o);
-                unsigned long long t2 = __shfl_up_sync(0xffffffffu, cc, o);
-                if (lane >= o) {
-                    sc += t1;
-                    cc += t2;
-                }
-            }
-            exs = sc - s;
-            exc_c = cc - c;
-            if (lane == first) {
-                unsigned long long sa = sh.sum_above + exs, ca = sh.cnt_above + exc_c;
-                int chosen = 255 - 8 * lane - 7;
-                for (int b = 0; b < 8; ++b) {
-                    int dg = 255 - 8 * lane - b;
-                    unsigned long long nv = by_sum ? sa + sh.sum[dg] : ca + sh.cnt[dg];
-                    if (nv >= need) {
-                        chosen = dg;
-                        break;
-                    }
-                    sa += sh.sum[dg];
-                    ca += sh.cnt[dg];
-                }
-                sh.sum_above = sa;
-                sh.cnt_above = (unsigned int)ca;
-                sh.chosen = chosen;
-                sh.prefix = prefix | ((unsigned long long)chosen << shift);
-                sh.mask = mask | (0xFFull << shift);
-                sh.unique = (sh.cnt[chosen] == 1u);
+        // thread t owns buckets 1023 - 4 t .. 1020 - 4 t (descending)
+        const int top = SEL_BUCKETS - 1 - SEL_PER * tid;
+        unsigned long long s = 0;
+        unsigned int c = 0;
+        for (int b = 0; b < SEL_PER; ++b) {
+            s += sh.sum[top - b];
+            c += sh.cnt[top - b];
+        }
+        unsigned long long si = s;
+        unsigned int ci = c;
+        for (int o = 1; o < 32; o <<= 1) {
+            const unsigned long long ts = __shfl_up_sync(0xffffffffu, si, o);
+            const unsigned int tc = __shfl_up_sync(0xffffffffu, ci, o);
+            if (lane >= o) {
+                si += ts;
+                ci += tc;
             }
         }
+        if (lane == 31) {
+            sh.wk[0][warp] = si;
+            sh.wc[warp] = ci;
+        }
         __syncthreads();
-        if (sh.unique) {
-            // a single element carries the boundary: find its full key
-            const unsigned long long p2 = sh.prefix, m2 = sh.mask;
-            for (int j = threadIdx.x; j < R; j += SEL_BS) {
-                unsigned long long k = ekey(err, base + j);
-                if ((k & m2) == p2) sh.prefix = k;  // exactly one writer
+        unsigned long long se = sa + si - s;  // larger keys' sum and count before this thread's
+        unsigned int ce = ca + ci - c;
+        for (int w = 0; w < warp; ++w) {
+            se += sh.wk[0][w];
+            ce += sh.wc[w];
+        }
+        const unsigned long long before = by_sum ? se : ce, here = by_sum ? s : c;
+        if ((before < need && before + here >= need) || (tid == SEL_BS - 1 && before + here < need)) {
+            int chosen = top;
+            for (int b = 0; b < SEL_PER; ++b) {
+                chosen = top - b;
+                const unsigned long long v = by_sum ? se + sh.sum[chosen] : ce + sh.cnt[chosen];
+                if (v >= need || b == SEL_PER - 1) break;
+                se += sh.sum[chosen];
+                ce += sh.cnt[chosen];
             }
+            sh.chosen = (unsigned)chosen;
+            sh.chosen_cnt = sh.cnt[chosen];
+            sh.sum_above = se;
+            sh.cnt_above = ce;
+            sh.ncand = 0;
+        }
+        __syncthreads();
+        lo += (unsigned long long)sh.chosen << shift;
+        span = (1ull << shift) - 1;
+        sa = sh.sum_above;
+        ca = sh.cnt_above;
+        if (shift == 0) {  // one key (and its equals) left
+            if (by_sum)
+                for (int j = tid; j < R; j += SEL_BS)
+                    if (ekey(err, base + j) == lo) sh.qb = q[base + j];  // the same for all equals
+            if (tid == 0) sh.bkey = lo;
             __syncthreads();
             break;
         }
+        if (sh.chosen_cnt <= 32) {
+            for (int j = tid; j < R; j += SEL_BS) {
+                const unsigned long long k = ekey(err, base + j);
+                if (k - lo <= span) {
+                    const unsigned at = atomicAdd(&sh.ncand, 1u);
+                    sh.ck[at] = k;
+                    sh.cq[at] = by_sum ? q[base + j] : 1ull;
+                }
+            }
+            __syncthreads();
+            if (tid < 32) {
+                const int n = (int)sh.ncand;
+                const unsigned long long k = lane < n ? sh.ck[lane] : 0, v = lane < n ? sh.cq[lane] : 0;
+                unsigned long long gt = 0, ge = 0;
+                unsigned int ngt = 0;
+                for (int j = 0; j < n; ++j) {
+                    const unsigned long long kj = sh.ck[j], vj = sh.cq[j];
+                    if (kj > k) {
+                        gt += vj;
+                        ++ngt;
+                    }
+                    if (kj >= k) ge += vj;
+                }
+                const unsigned long long from = by_sum ? sa : ca;
+                // the smallest key where the total is never reached (not met by the callers)
+                const bool last = from + ge < need && gt + v == ge && ngt + 1u >= (unsigned)n;
+                if (lane < n && ((from + gt < need && from + ge >= need) || last)) {
+                    sh.bkey = k;
+                    sh.qb = v;
+                    sh.cnt_above = ca + ngt;
+                    sh.sum_above = sa + (by_sum ? gt : 0);
+                }
+            }
+            __syncthreads();
+            sa = sh.sum_above;
+            ca = sh.cnt_above;
+            break;
+        }
+        for (int b = 0; b < SEL_PER; ++b) {
+            sh.cnt[b * SEL_BS + tid] = 0;
+            sh.sum[b * SEL_BS + tid] = 0;
+        }
+        __syncthreads();
     }
-    bkey = sh.prefix;
-    cnt_above = sh.cnt_above;
-    sum_above = sh.sum_above;
+    bkey = sh.bkey;
+    qb = sh.qb;
+    cnt_above = ca;
+    sum_above = sa;
     __syncthreads();
 }
 
@@ -209,8 +305,7 @@ __device__ void escalate_keys(const IntDesc &d, IntState *S, const Pool &P, Batc
     const double sc = 1152921504606846976.0 / U;  // 2^60 / U
     unsigned long long ql = 0;
     for (int j = threadIdx.x; j < R; j += SEL_BS) {
-        const double t = P.key[base + j] * sc;
-        const unsigned long long qq = t >= 1.8e19 ? 0xFFFFFFFFFFFFFFFFull : (unsigned long long)t;
+        const unsigned long long qq = floor_u64(P.key[base + j] * sc);
         P.q[base + j] = qq;
         ql += qq;
     }
@@ -218,9 +313,9 @@ __device__ void escalate_keys(const IntDesc &d, IntState *S, const Pool &P, Batc
     const double kq = keep * sc;
     const unsigned long long qk = kq >= 1.8e19 ? 0xFFFFFFFFFFFFFFFFull : (unsigned long long)kq;
     const unsigned long long needp = Qk > qk ? Qk - qk : 1;
-    unsigned long long pb, ps;
+    unsigned long long pb, ps, pq;
     unsigned int pc;
-    radix_select(P.key, P.q, base, R, true, needp, sh, pb, pc, ps);
+    boundary_select(P.key, P.q, base, R, true, needp, sh, pb, pc, ps, pq);
     for (int j = threadIdx.x; j < R; j += SEL_BS) {
         const unsigned long long kb = (unsigned long long)__double_as_longlong(P.key[base + j]);
         if (kb >= pb && P.key[base + j] > 0.0) push_esc(H, P, d.kind * 3 + d.term - 1, i, j | (1 << 30));
@@ -279,24 +374,40 @@ __global__ void __launch_bounds__(SEL_BS) k_select(const IntDesc *__restrict__ D
             __syncthreads();
             continue;
         }
-        // totals over live regions (mixed: and the FP32 uncertainty of each total)
-        double sv = 0, se = 0, sue = 0, suv = 0;
+        // Totals over live regions.  Mixed: and the FP32 uncertainty of each total, which
+        // only thresholds are compared with.  In FP64 each of its terms takes three
+        // instructions of a pipe that issues one per 64 cycles, so it is first bounded in
+        // FP32 from the operands' leading bits, relative to 2^-sref, and summed in FP64 only
+        // where that does not settle the comparison.
+        const double eref = S[i].err > 0 ? S[i].err : P.err[base];
+        const int sref = 1023 - (int)(((unsigned long long)__double_as_longlong(eref) >> 52) & 0x7ffu);
+        double sv = 0, se = 0;
+        float fue = 0.f, fuv = 0.f;
+        bool odd = false;
         for (int j = threadIdx.x; j < R; j += SEL_BS) {
             const double v = P.val[base + j], e = P.err[base + j];
             sv += v;
             se += e;
             if (gthr > 0.0) {
-                sue += e * (double)P.unc[base + j];
-                suv += fabs(v) * (double)P.uval[base + j];
+                fue = fmaf(f32_scaled(e, sref, odd), P.unc[base + j], fue);
+                fuv = fmaf(f32_scaled(fabs(v), sref, odd), P.uval[base + j], fuv);
             }
         }
-        double V = block_sum(sv, sh.dred);
-        double E = block_sum(se, sh.dred);
-        double UE = 0, UV = 0;
-        if (gthr > 0.0) {
+        double V, E;
+        block_totals(sv, se, fue, fuv, odd, sh, V, E);
+        // FP64 totals of the uncertainty, formed on demand
+        const double f2 = ldexp(1.0, -sref);  // unit of the FP32 bounds
+        const double fUE = gthr * (double)sh.fred[0] * f2, fUV = gthr * vr * (double)sh.fred[1] * f2;
+        const bool fodd = sh.odd != 0 || !(fUE < 1e300) || !(fUV < 1e300);
+        auto exact_unc = [&](double &UE, double &UV) {
+            double sue = 0, suv = 0;
+            for (int j = threadIdx.x; j < R; j += SEL_BS) {
+                sue += P.err[base + j] * (double)P.unc[base + j];
+                suv += fabs(P.val[base + j]) * (double)P.uval[base + j];
+            }
             UE = gthr * block_sum(sue, sh.dred);
             UV = gthr * vr * block_sum(suv, sh.dred);
-        }
+        };
         if (threadIdx.x == 0) {
             IntState st = S[i];
             int fin = 0, status = ST_OK;
@@ -321,13 +432,25 @@ __global__ void __launch_bounds__(SEL_BS) k_select(const IntDesc *__restrict__ D
             s_flag[2] = st.pad;  // polish passes so far
             s_tot[0] = V;
             s_tot[1] = E;
-            // the convergence test E <= rtol |V| decided within the FP32 uncertainty
             const bool tested = !s_cancel && isfinite(V) && isfinite(E) &&
                                 !(d.max_eval && st.neval >= d.max_eval);
-            s_flag[3] = gthr > 0.0 && tested && (UE + d.rtol * UV) > 0.0 &&
-                        fabs(E - fabs(V) * d.rtol) <= UE + d.rtol * UV;
+            // the convergence test E <= rtol |V| decided within the FP32 uncertainty: 1 = yes,
+            // 2 = the FP32 bound of the uncertainty does not tell
+            s_flag[3] = 0;
+            if (gthr > 0.0 && tested) {
+                const double dist = fabs(E - fabs(V) * d.rtol), f = fUE + d.rtol * fUV;
+                s_flag[3] = fodd || (dist > 0.999 * f && dist < 1.001 * f) || !(f > 0.0) ? 2 : dist <= f;
+            }
         }
         __syncthreads();
+        if (s_flag[3] == 2) {
+            double UE, UV;
+            exact_unc(UE, UV);
+            if (threadIdx.x == 0)
+                s_flag[3] = (UE + d.rtol * UV) > 0.0 &&
+                            fabs(s_tot[1] - fabs(s_tot[0]) * d.rtol) <= UE + d.rtol * UV;
+            __syncthreads();
+        }
         if (s_flag[3]) {
             const double margin = fabs(s_tot[1] - fabs(s_tot[0]) * d.rtol);
             double ul = 0;
@@ -360,8 +483,7 @@ __global__ void __launch_bounds__(SEL_BS) k_select(const IntDesc *__restrict__ D
                     const double sc = 1152921504606846976.0 / U;
                     unsigned long long ql = 0;
                     for (int j = threadIdx.x; j < R; j += SEL_BS) {
-                        double t = P.key[base + j] * sc;
-                        unsigned long long qq = t >= 1.8e19 ? 0xFFFFFFFFFFFFFFFFull : (unsigned long long)t;
+                        const unsigned long long qq = floor_u64(P.key[base + j] * sc);
                         P.q[base + j] = qq;
                         ql += qq;
                     }
@@ -371,8 +493,8 @@ __global__ void __launch_bounds__(SEL_BS) k_select(const IntDesc *__restrict__ D
                     const unsigned long long needp = Qk > qk ? Qk - qk : 1;
                     unsigned long long pb;
                     unsigned int pc;
-                    unsigned long long ps;
-                    radix_select(P.key, P.q, base, R, true, needp, sh, pb, pc, ps);
+                    unsigned long long ps, pq;
+                    boundary_select(P.key, P.q, base, R, true, needp, sh, pb, pc, ps, pq);
                     for (int j = threadIdx.x; j < R; j += SEL_BS) {
                         const unsigned long long kb =
                             (unsigned long long)__double_as_longlong(P.key[base + j]);
@@ -410,8 +532,7 @@ __global__ void __launch_bounds__(SEL_BS) k_select(const IntDesc *__restrict__ D
         const double scale = 1152921504606846976.0 / E;  // 2^60 / E
         unsigned long long qs = 0;
         for (int j = threadIdx.x; j < R; j += SEL_BS) {
-            double t = P.err[base + j] * scale;
-            unsigned long long qq = t >= 1.8e19 ? 0xFFFFFFFFFFFFFFFFull : (unsigned long long)t;
+            const unsigned long long qq = floor_u64(P.err[base + j] * scale);
             P.q[base + j] = qq;
             qs += qq;
         }
@@ -427,15 +548,8 @@ __global__ void __launch_bounds__(SEL_BS) k_select(const IntDesc *__restrict__ D
         if (need == 0) {
             Kconv = 1;
         } else {
-            radix_select(P.err, P.q, base, R, true, need, sh, bkey, cnt_above, sum_above);
-            // all keys equal to bkey carry the same q (any writer stores the same value)
-            if (threadIdx.x == 0) sh.ured[0] = 0;
-            __syncthreads();
-            for (int j = threadIdx.x; j < R; j += SEL_BS)
-                if (ekey(P.err, base + j) == bkey) sh.ured[0] = P.q[base + j];
-            __syncthreads();
-            unsigned long long qb = sh.ured[0];
-            __syncthreads();
+            unsigned long long qb;
+            boundary_select(P.err, P.q, base, R, true, need, sh, bkey, cnt_above, sum_above, qb);
             unsigned long long rest = need - sum_above;
             tneed = qb ? (rest + qb - 1) / qb : 1;
             Kconv = (unsigned long long)cnt_above + tneed;
@@ -453,12 +567,26 @@ __global__ void __launch_bounds__(SEL_BS) k_select(const IntDesc *__restrict__ D
                 if (Kconv < Kcap && Kconv < (unsigned long long)R) m = m_hi;
                 if (Kconv > 1 && m_lo < m) m = m_lo;
                 if (m != 0xFFFFFFFFFFFFFFFFull) {
-                    double ur = 0;
+                    const double m_abs = (double)m / scale;
+                    // the bound in FP32 first, as above
+                    float fur = 0.f;
+                    bool od = false;
                     for (int j = threadIdx.x; j < R; j += SEL_BS)
                         if (ekey(P.err, base + j) <= bkey)
-                            ur += P.err[base + j] * (double)P.unc[base + j];
-                    const double dlt = gthr * block_sum(ur, sh.dred) + d.rtol * UV;
-                    const double m_abs = (double)m / scale;
+                            fur = fmaf(f32_scaled(P.err[base + j], sref, od), P.unc[base + j], fur);
+                    od = __syncthreads_or(od);
+                    fur = block_sum(fur, sh.fred);
+                    const double f = gthr * (double)fur * f2 + d.rtol * fUV;
+                    double dlt = f;
+                    if (od || fodd || (m_abs > 0.999 * f && m_abs < 1.001 * f) || !(f > 0.0)) {
+                        double ur = 0, UE, UV;
+                        for (int j = threadIdx.x; j < R; j += SEL_BS)
+                            if (ekey(P.err, base + j) <= bkey)
+                                ur += P.err[base + j] * (double)P.unc[base + j];
+                        ur = block_sum(ur, sh.dred);
+                        exact_unc(UE, UV);
+                        dlt = gthr * ur + d.rtol * UV;
+                    }
                     if (dlt > 0.0 && m_abs <= dlt) {
                         double ul = 0;
                         for (int j = threadIdx.x; j < R; j += SEL_BS) {
@@ -485,7 +613,8 @@ __global__ void __launch_bounds__(SEL_BS) k_select(const IntDesc *__restrict__ D
                 cnt_above = 0;
                 tneed = R;  // every key >= 0: take all
             } else {
-                radix_select(P.err, P.q, base, R, false, K, sh, bkey, cnt_above, sum_above);
+                unsigned long long qb;
+                boundary_select(P.err, P.q, base, R, false, K, sh, bkey, cnt_above, sum_above, qb);
                 tneed = K - cnt_above;
             }
         }
@@ -495,27 +624,34 @@ __global__ void __launch_bounds__(SEL_BS) k_select(const IntDesc *__restrict__ D
         if (H->mixed && K < (unsigned long long)R) {
             const double b = __longlong_as_double((long long)bkey);
             if (b > tau_sel * fabs(V)) {
-                float ub = 0.f;
-                for (int j = threadIdx.x; j < R; j += SEL_BS)
-                    if (ekey(P.err, base + j) == bkey) ub = fmaxf(ub, P.unc[base + j]);
-                ub = block_max(ub, sh.fred);
+                if (threadIdx.x == 0) sh.ubits = 0;
+                __syncthreads();
+                for (int j = threadIdx.x; j < R; j += SEL_BS)  // bounds are >= 0: order as integers
+                    if (ekey(P.err, base + j) == bkey) atomicMax(&sh.ubits, __float_as_int(P.unc[base + j]));
+                __syncthreads();
+                const float ub = __int_as_float(sh.ubits);
                 const double blo = b * (1.0 - ub), bhi = b * (1.0 + ub);
-                int amb = 0;
-                for (int j = threadIdx.x; j < R; j += SEL_BS) {
+                // do the bounds of region j overlap the boundary's?  |key difference| 2^-52 is
+                // at most 2 |ln(e / b)|, and an overlap with bounds below 1/4 has |ln(e / b)| <=
+                // 2 (u + ub): what differs by more is told apart without FP64
+                auto overlaps = [&](unsigned long long k, double e, float u) {
+                    const int dk = abs((int)((long long)(k >> 20) - (long long)(bkey >> 20)));
+                    if (u < 0.25f && ub < 0.25f && (float)dk * 2.3283064e-10f > 4.1f * (u + ub) + 1e-6f)
+                        return false;
+                    return e * (1.0 + u) >= blo && e * (1.0 - u) <= bhi;
+                };
+                bool some = false;
+                for (int j = threadIdx.x; j < R && !some; j += SEL_BS) {
                     const unsigned long long k = ekey(P.err, base + j);
-                    if (k == bkey) continue;
-                    const double e = P.err[base + j];
                     const float u = P.unc[base + j];
-                    if ((u > 0.f || ub > 0.f) && e * (1.0 + u) >= blo && e * (1.0 - u) <= bhi) ++amb;
+                    some = k != bkey && (u > 0.f || ub > 0.f) && overlaps(k, P.err[base + j], u);
                 }
-                amb = block_sum(amb, sh.ired);
+                const int amb = __syncthreads_or(some);
                 if (amb > 0) {
                     for (int j = threadIdx.x; j < R; j += SEL_BS) {
-                        const double e = P.err[base + j];
                         const float u = P.unc[base + j];
-                        if (u > 0.f && e * (1.0 + u) >= blo && e * (1.0 - u) <= bhi) {
+                        if (u > 0.f && overlaps(ekey(P.err, base + j), P.err[base + j], u))
                             push_esc(H, P, d.kind * 3 + d.term - 1, i, j | (1 << 30));
-                        }
                     }
                     if (threadIdx.x == 0) {
                         S[i].K = 0;
@@ -537,31 +673,46 @@ __global__ void __launch_bounds__(SEL_BS) k_select(const IntDesc *__restrict__ D
             __syncthreads();
             continue;
         }
-        // compact the selection in slot order
-        int run_sel = 0, run_tie = 0;
-        for (int c0 = 0; c0 < R; c0 += SEL_BS) {
-            int j = c0 + threadIdx.x;
-            unsigned long long k = j < R ? ekey(P.err, base + j) : 0;
-            int is_eq = (j < R && k == bkey && !(K == (unsigned long long)R)) ? 1 : 0;
-            int is_gt = (j < R && (K == (unsigned long long)R || k > bkey)) ? 1 : 0;
-            int ntie;
-            int tr = run_tie + block_flag_scan(is_eq, sh.ired, ntie);
-            int sel = is_gt || (is_eq && (unsigned long long)tr < tneed);
-            int nsel;
-            int pos = run_sel + block_flag_scan(sel, sh.ired, nsel);
-            if (sel) P.cand[base + pos] = j;
-            run_tie += ntie;
-            run_sel += nsel;
-        }
-        // Mixed precision: selected parents whose split is flagged unsettled get it
-        // re-taken in FP64 before this round's cut.
-        if (H->mixed) {
+        // Compact the selection in slot order: each warp counts its part of the regions, then
+        // writes it behind the other warps' counts.  Mixed precision: selected parents whose
+        // split is flagged unsettled get it re-taken in FP64 before this round's cut.
+        {
+            const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+            const int part = ((R + SEL_WARPS - 1) / SEL_WARPS + 31) & ~31;
+            const int j0 = warp * part, j1 = min(R, j0 + part);
+            const bool all = K == (unsigned long long)R;
+            int ngt = 0, neq = 0;
+            for (int c0 = j0; c0 < j1; c0 += 32) {
+                const int j = c0 + lane;
+                const unsigned long long k = j < j1 ? ekey(P.err, base + j) : 0;
+                ngt += __popc(__ballot_sync(0xffffffffu, j < j1 && (all || k > bkey)));
+                neq += __popc(__ballot_sync(0xffffffffu, j < j1 && !all && k == bkey));
+            }
+            if (lane == 0) {
+                sh.ired[0][warp] = ngt;
+                sh.ired[1][warp] = neq;
+            }
             __syncthreads();
-            for (int j = threadIdx.x; j < (int)K; j += SEL_BS) {
-                const int r = P.cand[base + j];
-                if (P.split[base + r] & 0x80) {
-                    push_esc(H, P, d.kind * 3 + d.term - 1, i, r);
+            long long ties = 0;  // equal keys before this warp's part
+            int pos = 0;
+            for (int w = 0; w < warp; ++w) {
+                const long long left = (long long)tneed - ties, ne = sh.ired[1][w];
+                pos += sh.ired[0][w] + (int)(left < 0 ? 0 : (left < ne ? left : ne));
+                ties += ne;
+            }
+            for (int c0 = j0; c0 < j1; c0 += 32) {
+                const int j = c0 + lane;
+                const unsigned long long k = j < j1 ? ekey(P.err, base + j) : 0;
+                const bool gt = j < j1 && (all || k > bkey), eq = j < j1 && !all && k == bkey;
+                const unsigned be = __ballot_sync(0xffffffffu, eq), lower = (1u << lane) - 1u;
+                const bool sel = gt || (eq && ties + __popc(be & lower) < (long long)tneed);
+                const unsigned bs = __ballot_sync(0xffffffffu, sel);
+                if (sel) {
+                    P.cand[base + pos + __popc(bs & lower)] = j;
+                    if (H->mixed && (P.split[base + j] & 0x80)) push_esc(H, P, d.kind * 3 + d.term - 1, i, j);
                 }
+                pos += __popc(bs);
+                ties += __popc(be);
             }
         }
         if (threadIdx.x == 0) {
