@@ -300,7 +300,8 @@ __device__ void boundary_select(const double *err, const unsigned long long *q, 
 // when a threshold decision (convergence, the Gladwell count) lies within the FP32
 // uncertainty of the sums it compares.
 __device__ void escalate_keys(const IntDesc &d, IntState *S, const Pool &P, BatchHdr *H, int i,
-                              long long base, int R, double U, double keep, SelShared &sh)
+                              long long base, int R, double U, double keep, int pass,
+                              SelShared &sh)
 {
     const double sc = 1152921504606846976.0 / U;  // 2^60 / U
     unsigned long long ql = 0;
@@ -318,7 +319,7 @@ __device__ void escalate_keys(const IntDesc &d, IntState *S, const Pool &P, Batc
     boundary_select(P.key, P.q, base, R, true, needp, sh, pb, pc, ps, pq);
     for (int j = threadIdx.x; j < R; j += SEL_BS) {
         const unsigned long long kb = (unsigned long long)__double_as_longlong(P.key[base + j]);
-        if (kb >= pb && P.key[base + j] > 0.0) push_esc(H, P, d.kind * 3 + d.term - 1, i, j | (1 << 30));
+        if (kb >= pb && P.key[base + j] > 0.0) push_esc(H, P, pass, d.kind * 3 + d.term - 1, i, j | (1 << 30));
     }
     if (threadIdx.x == 0) {
         S[i].K = 0;
@@ -461,7 +462,7 @@ __global__ void __launch_bounds__(SEL_BS) k_select(const IntDesc *__restrict__ D
                 ul += kj;
             }
             const double U = block_sum(ul, sh.dred);
-            escalate_keys(d, S, P, H, i, base, R, U, 0.9 * margin, sh);
+            escalate_keys(d, S, P, H, i, base, R, U, 0.9 * margin, pass, sh);
             continue;
         }
         if (s_flag[0]) {
@@ -499,7 +500,7 @@ __global__ void __launch_bounds__(SEL_BS) k_select(const IntDesc *__restrict__ D
                         const unsigned long long kb =
                             (unsigned long long)__double_as_longlong(P.key[base + j]);
                         if (kb >= pb && P.uval[base + j] > 0.f) {
-                            push_esc(H, P, d.kind * 3 + d.term - 1, i, j | (1 << 30));
+                            push_esc(H, P, pass, d.kind * 3 + d.term - 1, i, j | (1 << 30));
                         }
                     }
                     if (threadIdx.x == 0) {
@@ -598,7 +599,7 @@ __global__ void __launch_bounds__(SEL_BS) k_select(const IntDesc *__restrict__ D
                             ul += kj;
                         }
                         const double U = block_sum(ul, sh.dred);
-                        escalate_keys(d, S, P, H, i, base, R, U, 0.9 * m_abs, sh);
+                        escalate_keys(d, S, P, H, i, base, R, U, 0.9 * m_abs, pass, sh);
                         continue;
                     }
                 }
@@ -651,7 +652,7 @@ __global__ void __launch_bounds__(SEL_BS) k_select(const IntDesc *__restrict__ D
                     for (int j = threadIdx.x; j < R; j += SEL_BS) {
                         const float u = P.unc[base + j];
                         if (u > 0.f && overlaps(ekey(P.err, base + j), P.err[base + j], u))
-                            push_esc(H, P, d.kind * 3 + d.term - 1, i, j | (1 << 30));
+                            push_esc(H, P, pass, d.kind * 3 + d.term - 1, i, j | (1 << 30));
                     }
                     if (threadIdx.x == 0) {
                         S[i].K = 0;
@@ -709,7 +710,7 @@ __global__ void __launch_bounds__(SEL_BS) k_select(const IntDesc *__restrict__ D
                 const unsigned bs = __ballot_sync(0xffffffffu, sel);
                 if (sel) {
                     P.cand[base + pos + __popc(bs & lower)] = j;
-                    if (H->mixed && (P.split[base + j] & 0x80)) push_esc(H, P, d.kind * 3 + d.term - 1, i, j);
+                    if (H->mixed && (P.split[base + j] & 0x80)) push_esc(H, P, pass, d.kind * 3 + d.term - 1, i, j);
                 }
                 pos += __popc(bs);
                 ties += __popc(be);
@@ -753,9 +754,16 @@ __global__ void __launch_bounds__(1024) k_scan(IntState *__restrict__ S, long lo
         long long tot = part[blockDim.x - 1];
         woff[n] = tot;
         H->total_work = tot;
-        // keep looping while there is work or a deferred FP64 re-evaluation
+        // Keep looping while there is work or a deferred FP64 re-evaluation.  The first stage's
+        // queues have been consumed: count the round's entries and clear them (the second
+        // stage's are cleared by the next round's first stage, k_re_fill).
         int pending = 0;
-        for (int g = 0; g < NGROUPS; ++g) pending |= H->n_esc[g];
+        for (int g = 0; g < NGROUPS; ++g) {
+            const int n0 = H->n_esc[0][g], n1 = H->n_esc[1][g], cap = H->esc_cap[g];
+            pending |= n1;
+            H->escalated += (unsigned long long)(min(n0, cap) + min(n1, cap));
+            H->n_esc[0][g] = 0;
+        }
         const int more = tot > 0 || pending > 0;
         H->any_active = more;
         H->regions += 2ull * (unsigned long long)tot;
@@ -810,7 +818,7 @@ __global__ void k_init(const IntDesc *__restrict__ D, IntState *__restrict__ S, 
         H->chunk_count = 0;
         H->ties = 0;
         H->small_arg = 0;
-        for (int g = 0; g < NGROUPS; ++g) H->n_esc[g] = 0;
+        for (int g = 0; g < NGROUPS; ++g) H->n_esc[0][g] = H->n_esc[1][g] = 0;
         H->escalated = 0;
         H->deferred = 0;
         H->polished = 0;
@@ -818,18 +826,6 @@ __global__ void k_init(const IntDesc *__restrict__ D, IntState *__restrict__ S, 
         H->thr_checks = 0;
         H->cancel = 0;
         H->t0_ns = global_timer_ns();
-    }
-}
-
-// end of a mixed-precision round: the FP64 re-evaluation queue has been consumed
-// End of a re-evaluation stage: count and clear the queues of every group (grp < 0) or
-// of group grp alone (the per-group ends of concurrent branches, hence the atomic count)
-__global__ void k_round_end(BatchHdr *H, int grp)
-{
-    for (int g = grp < 0 ? 0 : grp; g < (grp < 0 ? NGROUPS : grp + 1); ++g) {
-        const int n = H->n_esc[g];
-        atomicAdd(&H->escalated, (unsigned long long)(n < H->esc_cap[g] ? n : H->esc_cap[g]));
-        H->n_esc[g] = 0;
     }
 }
 
@@ -863,7 +859,6 @@ __global__ void k_admit(const IntDesc *__restrict__ Dn, const int *__restrict__ 
 }
 
 void *admit_kernel() { return (void *)k_admit; }
-void *round_end_kernel() { return (void *)k_round_end; }
 void *select_kernel() { return (void *)k_select; }
 void *scan_kernel() { return (void *)k_scan; }
 void *init_kernel() { return (void *)k_init; }

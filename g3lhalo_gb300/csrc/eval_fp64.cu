@@ -52,6 +52,29 @@ template <int KIND, int TERM>
 struct Model64 {
     static constexpr int DIM = TERM + 4;
 
+    // N_sat pair count of a mass slot: with the rescaling s of the hod1 slot at this mass's
+    // rounded bin (src/NNMap_Model.cu:563,808)
+    __device__ static double pairs(const DevTables &T, const IntDesc &d, const Slot64 &S)
+    {
+        return nsatnsat64(S.a[2], S.a[4], d.same, T.A, T.eps, S.a[0],
+                          __ldg(T.scale + (size_t)d.hod1 * T.Nm + S.i0));
+    }
+
+    // A halo mass's slot without the second population (two populations: S.a[3..5])
+    __device__ static void fill_mass(const DevTables &T, const IntDesc &d, double x, Slot64 &S,
+                                     unsigned long long *ties)
+    {
+        const double m = pow(10, x);
+        S.a[0] = m;
+        m_index(T, x, m, S.i0, S.i1, ties);
+        occupations64(T.hod + 6 * d.hod1, m, S.a[1], S.a[2]);
+        if (KIND == 0 && d.same) {  // the second population's occupations are the first's
+            S.a[3] = S.a[1];
+            S.a[4] = S.a[2];
+            S.a[5] = pairs(T, d, S);
+        }
+    }
+
     // Fill one coordinate-variant slot (everything that depends on one coordinate).
     __device__ static void fill(const DevTables &T, const IntDesc &d, int dimidx, double x,
                                 Slot64 &S, unsigned long long *ties)
@@ -63,25 +86,10 @@ struct Model64 {
         } else if (dimidx == 2) {  // phi
             S.a[0] = cos(x);
         } else if (dimidx < 3 + TERM) {  // halo masses (log10 m)
-            double m = pow(10, x);
-            S.a[0] = m;
-            m_index(T, x, m, S.i0, S.i1, ties);
-            const double *h1 = T.hod + 6 * d.hod1;
-            const double *h2 = T.hod + 6 * d.hod2;
-            occupations64(h1, m, S.a[1], S.a[2]);
-            if (KIND == 0) {
-                // the second population's occupations: the same values as the first's when
-                // the slots are the same
-                if (d.same) {
-                    S.a[3] = S.a[1];
-                    S.a[4] = S.a[2];
-                } else {
-                    occupations64(h2, m, S.a[3], S.a[4]);
-                }
-                // rescaling s of the hod1 slot at this mass's rounded bin
-                // (src/NNMap_Model.cu:563,808)
-                S.a[5] = nsatnsat64(S.a[2], S.a[4], d.same, T.A, T.eps, m,
-                                    __ldg(T.scale + (size_t)d.hod1 * T.Nm + S.i0));
+            fill_mass(T, d, x, S, ties);
+            if (KIND == 0 && !d.same) {
+                occupations64(T.hod + 6 * d.hod2, S.a[0], S.a[3], S.a[4]);
+                S.a[5] = pairs(T, d, S);
             }
         } else {  // z
             S.a[0] = x;
@@ -92,45 +100,57 @@ struct Model64 {
     }
 
     // Integrand at one point from its variant slots (kernel_function_* of the reference).
-    // cached u_NFW f (ucache_fun) at slots L (l), M (mass), Z (z): the expressions of point()
-    // mz: r_200 and F of the (M, Z) pair (MZ_VALS values, k_re_fill), or null
-    __device__ static double ucached(const DevTables &T, const IntDesc &d, int f, const Slot64 &L,
-                                     const Slot64 &M, const Slot64 &Z, const double *mz)
+    // Operands of the shared u_NFW, with the expressions of point(); mz: r_200 and F of the
+    // (mass, z) pair.  Cached u_NFW f (ucache_fun) at slots L (l), M (mass), Z (z):
+    __device__ static void ucached_args(const DevTables &T, const IntDesc &d, int f, const Slot64 &L,
+                                        const Slot64 &M, const Slot64 &Z, const double *mz,
+                                        double &k, double &r200, double &c, double &F)
     {
         const double w_ = __ldg(T.w + Z.i0);
-        const double k = ddiv(L.a[0], w_);
         const double conc = __ldg(T.conc + Z.i1 * T.Nm + M.i1);
         const int fs = ucache_fun(KIND, TERM, f, 2);
-        const double c = (fs == 0 ? 1.0 : (fs == 1 ? T.hod[6 * d.hod1] : T.hod[6 * d.hod2])) * conc;
-        if (!mz) return u_nfw64_F(k, r200_64(M.a[0], __ldg(T.rho_bar + Z.i1)), c, nfw_norm64(c));
-        return u_nfw64_F(k, mz[0], c, mz[1 + fs]);
+        k = ddiv(L.a[0], w_);
+        r200 = mz[0];
+        c = (fs == 0 ? 1.0 : (fs == 1 ? T.hod[6 * d.hod1] : T.hod[6 * d.hod2])) * conc;
+        F = mz[1 + fs];
     }
 
-    // r_200 and F at factors 1, f of hod1, f of hod2 (nf of them) of halo mass slot M at
-    // z bin zt, with the expressions of point(): o[0..nf]
-    __device__ static void mz_values(const DevTables &T, const IntDesc &d, const Slot64 &M, int zt,
-                                     int nf, double *o)
-    {
-        const double conc = __ldg(T.conc + zt * T.Nm + M.i1);
-        o[0] = r200_64(M.a[0], __ldg(T.rho_bar + zt));
-        for (int q = 0; q < nf; ++q)
-            o[1 + q] = nfw_norm64((q == 0 ? 1.0 : (q == 1 ? T.hod[6 * d.hod1] : T.hod[6 * d.hod2])) * conc);
-    }
-
-    // u_NFW(k3, mass u3_mass(f)) of the 2- and 3-halo terms, with the expressions of
-    // point(): shared by the points with the same projection (u3_drop)
-    // mz: r_200 and F of the (mass, z) pair (k_re_fill), or null
-    __device__ static double u3(const DevTables &T, int f, const Slot64 *const *s, const double *mz)
+    // u_NFW(k3, mass u3_mass(f)): shared by the points with the same projection (u3_drop)
+    __device__ static void u3_args(const DevTables &T, int f, const Slot64 *const *s,
+                                   const double *mz, double &k, double &r200, double &c, double &F)
     {
         const Slot64 &L1 = *s[0], &L2 = *s[1], &PH = *s[2], &Z = *s[DIM - 1];
         const Slot64 &M = *s[u3_mass(KIND, TERM, f)];
         const double l1 = L1.a[0], l2 = L2.a[0], cphi = PH.a[0];
         const double w_ = __ldg(T.w + Z.i0);
         const double l3 = sqrt(l1 * l1 + l2 * l2 + 2 * l1 * l2 * cphi);
-        const double k3 = ddiv(l3, w_);
-        const double c = 1.0 * __ldg(T.conc + Z.i1 * T.Nm + M.i1);
-        if (!mz) return u_nfw64_F(k3, r200_64(M.a[0], __ldg(T.rho_bar + Z.i1)), c, nfw_norm64(c));
-        return u_nfw64_F(k3, mz[0], c, mz[1]);
+        k = ddiv(l3, w_);
+        r200 = mz[0];
+        c = 1.0 * __ldg(T.conc + Z.i1 * T.Nm + M.i1);
+        F = mz[1];
+    }
+
+    // F at factors 1, f of hod1, f of hod2 (nf of them) of halo mass slot M at z bin zt, with
+    // the expressions of point(): o[1..nf]
+    __device__ static void mz_norms(const DevTables &T, const IntDesc &d, const Slot64 &M, int zt,
+                                    int nf, double *o)
+    {
+        const double conc = __ldg(T.conc + zt * T.Nm + M.i1);
+        double c0 = 0, F = 0;
+        for (int q = 0; q < nf; ++q) {
+            const double c = (q == 0 ? 1.0 : (q == 1 ? T.hod[6 * d.hod1] : T.hod[6 * d.hod2])) * conc;
+            if (q == 0 || c != c0) F = nfw_norm64(c);  // equal factors share it
+            c0 = c;
+            o[1 + q] = F;
+        }
+    }
+
+    // r_200 and the normalisations: o[0..nf]
+    __device__ static void mz_values(const DevTables &T, const IntDesc &d, const Slot64 &M, int zt,
+                                     int nf, double *o)
+    {
+        o[0] = r200_64(M.a[0], __ldg(T.rho_bar + zt));
+        mz_norms(T, d, M, zt, nf, o);
     }
 
     // auxiliary function a (aux_dims) with the expressions of point(): the aperture filter
@@ -148,11 +168,10 @@ struct Model64 {
     }
 
     // uc: the cached u_NFW values of this point (ucache_fun order), or null; u3c: its
-    // cached u_NFW at k3 (u3()), or null; ax: its cached auxiliary values (aux()), or null;
-    // mz: r_200 and F of its (mass, z) pair (1-halo terms), or null
+    // cached u_NFW at k3 (u3()), or null; ax: its cached auxiliary values (aux()), or null
     __device__ static double point(const DevTables &T, const IntDesc &d, const Slot64 *const *s,
                                    const double *uc = nullptr, const double *u3c = nullptr,
-                                   const double *ax = nullptr, const double *mz = nullptr)
+                                   const double *ax = nullptr)
     {
         const Slot64 &L1 = *s[0], &L2 = *s[1], &PH = *s[2], &Z = *s[DIM - 1];
         const double l1 = L1.a[0], l2 = L2.a[0], cphi = PH.a[0], z = Z.a[0];
@@ -174,9 +193,9 @@ struct Model64 {
                 // src/NNMap_Model.cu:544-593
                 const Slot64 &M = *s[3];
                 const double m = M.a[0];
-                const double r2 = mz ? mz[0] : r200_64(m, rhot);  // mz[0] is this value
+                const double r2 = r200_64(m, rhot);
                 const double cc = __ldg(T.conc + z_it * Nm + M.i1);
-                const double u3 = mz ? u_nfw64_F(k3, mz[0], 1.0 * cc, mz[1]) : u_nfw64(k3, r2, cc, 1);
+                const double u3 = u3c ? u3c[0] : u_nfw64(k3, r2, cc, 1);
                 const double u2 = uc ? uc[1] : u_nfw64(k2, r2, cc, f2);
                 const double u1 = uc ? uc[0] : u_nfw64(k1, r2, cc, f1);
                 double Bggd = ddiv(ddiv(ddiv(1., nbar1), nbar2), rho) * __ldg(T.hmf + z_ix * Nm + M.i0) * m * u3;
@@ -245,12 +264,12 @@ struct Model64 {
                 // src/NMapMap_Model.cu:263-301
                 const Slot64 &M = *s[3];
                 const double m = M.a[0];
-                const double r2 = mz ? mz[0] : r200_64(m, rhot);  // mz[0] is this value
+                const double r2 = r200_64(m, rhot);
                 const double cc = __ldg(T.conc + z_it * Nm + M.i1);
                 double Bgdd = ddiv(ddiv(ddiv(1., nbar), rho), rho) * __ldg(T.hmf + z_ix * Nm + M.i0) * m * m *
                               (M.a[1] + M.a[2] * (uc ? uc[0] : u_nfw64(k1, r2, cc, f))) *
                               (uc ? uc[1] : u_nfw64(k2, r2, cc, 1)) *
-                              (mz ? u_nfw64_F(k3, mz[0], 1.0 * cc, mz[1]) : u_nfw64(k3, r2, cc, 1));
+                              (u3c ? u3c[0] : u_nfw64(k3, r2, cc, 1));
                 double bgkk = ddiv(Bgdd, __ldg(T.dwdz + z_ix)) * gz * gz * __ldg(T.p1 + z_ix);
                 bgkk = ddiv(ddiv(bgkk, w_), w_) * (1. + z) * (1. + z);
                 return ddiv(l1 * l2 * m * l1 * l2 * L1.a[1] * L2.a[1] * U3 * bgkk, nbar);
@@ -302,65 +321,6 @@ struct Model64 {
     }
 };
 
-// Rule sums of one region in the reference's order (src/hcubature.cpp:512-576).
-template <int DIM>
-__device__ void combine64(const double *v, double vol, double &val, double &err, int &split)
-{
-    const double ratio = (G3L_LAMBDA2 * G3L_LAMBDA2) / (G3L_LAMBDA4 * G3L_LAMBDA4);
-    const double weight1 = (double)(12824 - 9120 * DIM + 400 * DIM * DIM) / (double)19683;
-    const double weight3 = (double)(1820 - 400 * DIM) / (double)19683;
-    const double weight5 = (double)6859 / (double)19683 / (double)(1u << DIM);
-    const double weightE1 = (double)(729 - 950 * DIM + 50 * DIM * DIM) / (double)729;
-    const double weightE3 = (double)(265 - 100 * DIM) / (double)1458;
-    const double weight2 = 980. / 6561., weight4 = 200. / 19683.;
-    const double weightE2 = 245. / 486., weightE4 = 25. / 729.;
-    double val0 = v[0], sum2 = 0, sum3 = 0, sum4 = 0, sum5 = 0;
-    double maxdiff = 0;
-    int dimDiffMax = 0;
-    int k0 = 1;
-    for (int k = 0; k < DIM; ++k) {
-        double v0 = v[k0 + 4 * k], v1 = v[k0 + 4 * k + 1];
-        double v2 = v[k0 + 4 * k + 2], v3 = v[k0 + 4 * k + 3];
-        sum2 += v0 + v1;
-        sum3 += v2 + v3;
-        double diff = 0;
-        diff += fabs(v0 + v1 - 2 * val0 - ratio * (v2 + v3 - 2 * val0));
-        if (diff > maxdiff) {
-            maxdiff = diff;
-            dimDiffMax = k;
-        }
-    }
-    k0 += 4 * DIM;
-    for (int k = 0; k < 2 * DIM * (DIM - 1); ++k) sum4 += v[k0 + k];
-    k0 += 2 * DIM * (DIM - 1);
-    for (int k = 0; k < (1 << DIM); ++k) sum5 += v[k0 + k];
-    double result = vol * (weight1 * val0 + weight2 * sum2 + weight3 * sum3 + weight4 * sum4 +
-                           weight5 * sum5);
-    double res5th = vol * (weightE1 * val0 + weightE2 * sum2 + weightE3 * sum3 + weightE4 * sum4);
-    val = result;
-    err = fabs(res5th - result);
-    split = dimDiffMax;
-}
-
-// Point tables of a group's re-evaluation passes: the point codes, the (l, m, z)
-// combinations of the cached u_NFW (ucache_tables) and the projections of the k3 u_NFW
-// (u3_tables) and of the auxiliary functions (aux_tables).  The same for every launch, so
-// k_re_tables builds them once per context into P.retab and each block copies them to
-// shared memory (building them per block cost more than the cached work saves).
-template <int KIND, int TERM>
-struct ReTab {
-    static constexpr int DIM = TERM + 4, NP = rule_points(DIM), NF = ucache_nf(TERM);
-    static constexpr int NU3 = u3_nfun(TERM) > 0 ? u3_nfun(TERM) : 1, NA = aux_nfun(TERM);
-    uint32_t sdesc[NP];
-    int ucn[NF];
-    uint16_t ucl[NF * UC_MAX];
-    uint8_t ucidx[NF * NP];
-    uint8_t u3rep[NU3 * NP];
-    uint8_t u3list[NU3 * U3_MAX];
-    uint8_t auxrep[NA * NP];
-    uint8_t auxlist[AUX_MAX];
-};
-
 template <int KIND, int TERM>
 __global__ void __launch_bounds__(128) k_re_tables(unsigned char *out)
 {
@@ -379,19 +339,6 @@ __global__ void __launch_bounds__(128) k_re_tables(unsigned char *out)
         dst[i] = reinterpret_cast<const uint32_t *>(buf)[i];
 }
 
-// copy group (KIND, TERM)'s tables to shared memory buf (every thread calls it)
-template <int KIND, int TERM>
-__device__ inline const ReTab<KIND, TERM> &load_retab(const Pool &P, unsigned char *buf)
-{
-    using RT = ReTab<KIND, TERM>;
-    const uint32_t *src =
-        reinterpret_cast<const uint32_t *>(P.retab + (KIND * 3 + TERM - 1) * RETAB_BYTES);
-    for (int i = threadIdx.x; i < (int)(sizeof(RT) / 4); i += blockDim.x)
-        reinterpret_cast<uint32_t *>(buf)[i] = __ldg(src + i);
-    __syncthreads();
-    return *reinterpret_cast<const RT *>(buf);
-}
-
 // Shared memory of one work item.  Child 1 has its own copy of a cached function only when
 // the split dimension is among the function's dimensions.
 template <int KIND, int TERM>
@@ -402,7 +349,7 @@ struct Item64 {
     Slot64 slots[(DIM + 1) * NVAR];
     double mz[2][TERM][MZ_PAIRS][MZ_VALS];
     double uc[2][NF][UC_MAX];
-    double u3[2][NU3 > 0 ? NU3 : 1][NU3 > 0 ? U3_MAX : 1];
+    double u3[2][NU3][U3_MAX];
     double aux[2][NAUX];
     double vals[2 * NP];
 };
@@ -577,7 +524,7 @@ __device__ void block_item64(const DevTables &T, const IntDesc &d, const Pool &P
     __syncthreads();
     // shared u_NFW: (l, m, z) combinations, then k3 projections
     {
-        int nu[NF], n3[NU3 > 0 ? NU3 : 1] = {0}, tot = 0;
+        int nu[NF], n3[NU3], tot = 0;
 #pragma unroll
         for (int f = 0; f < NF; ++f) {
             const uint32_t dims = (1u << ucache_fun(KIND, TERM, f, 0)) |
@@ -593,6 +540,7 @@ __device__ void block_item64(const DevTables &T, const IntDesc &d, const Pool &P
         for (int t0 = rank; t0 < tot; t0 += 128) {
             int t = t0, f = 0;
             bool lmz = true;
+            double kk, r200, cc, F, *out;
 #pragma unroll
             for (int q = 0; q < NF; ++q)
                 if (f == q && t >= nu[q]) {
@@ -613,8 +561,9 @@ __device__ void block_item64(const DevTables &T, const IntDesc &d, const Pool &P
                 const int vl = key & 7, vm = (key >> 3) & 7, vz = (key >> 6) & 7;
                 const int dl = ucache_fun(KIND, TERM, f, 0), dm = ucache_fun(KIND, TERM, f, 1);
                 const int mc = ch && own((1u << dm) | (1u << ZD));
-                I.uc[ch][f][j] = M::ucached(T, d, f, slot(ch, dl, vl), slot(ch, dm, vm),
-                                            slot(ch, ZD, vz), I.mz[mc][dm - 3][mz_index(vm, vz)]);
+                M::ucached_args(T, d, f, slot(ch, dl, vl), slot(ch, dm, vm), slot(ch, ZD, vz),
+                                I.mz[mc][dm - 3][mz_index(vm, vz)], kk, r200, cc, F);
+                out = &I.uc[ch][f][j];
             } else {
                 const int ch = t >= U3_MAX, j = t - ch * U3_MAX;
                 const uint32_t vv = tb.sdesc[tb.u3list[f * U3_MAX + j]];
@@ -623,9 +572,11 @@ __device__ void block_item64(const DevTables &T, const IntDesc &d, const Pool &P
                 const Slot64 *sp[DIM];
 #pragma unroll
                 for (int dd = 0; dd < DIM; ++dd) sp[dd] = &slot(ch, dd, (vv >> (3 * dd)) & 7);
-                I.u3[ch][f][j] = M::u3(T, f, sp,
-                                       I.mz[mc][dm - 3][mz_index((vv >> (3 * dm)) & 7, (vv >> (3 * ZD)) & 7)]);
+                M::u3_args(T, f, sp, I.mz[mc][dm - 3][mz_index((vv >> (3 * dm)) & 7, (vv >> (3 * ZD)) & 7)],
+                           kk, r200, cc, F);
+                out = &I.u3[ch][f][j];
             }
+            *out = u_nfw64_F(kk, r200, cc, F);
         }
     }
     __syncthreads();
@@ -636,7 +587,7 @@ __device__ void block_item64(const DevTables &T, const IntDesc &d, const Pool &P
         const Slot64 *sp[DIM];
 #pragma unroll
         for (int dd = 0; dd < DIM; ++dd) sp[dd] = &slot(ch, dd, (vv >> (3 * dd)) & 7);
-        double uc[NF], u3c[NU3 > 0 ? NU3 : 1], ax[NA];
+        double uc[NF], u3c[NU3], ax[NA];
 #pragma unroll
         for (int f = 0; f < NF; ++f) {
             const uint32_t dims = (1u << ucache_fun(KIND, TERM, f, 0)) |
@@ -650,10 +601,7 @@ __device__ void block_item64(const DevTables &T, const IntDesc &d, const Pool &P
 #pragma unroll
         for (int a = 0; a < NA; ++a)
             ax[a] = I.aux[ch && own(aux_dims(TERM, a))][aux_off(TERM, a) + tb.auxrep[a * NP + pp]];
-        const double *mz = TERM == 1 ? I.mz[ch && own(8u | (1u << ZD))][0]
-                                           [mz_index((vv >> 9) & 7, (vv >> (3 * ZD)) & 7)]
-                                     : nullptr;
-        const double v = M::point(T, d, sp, uc, NU3 > 0 ? u3c : nullptr, ax, mz);
+        const double v = M::point(T, d, sp, uc, u3c, ax);
         I.vals[p] = v;
         if (dbg) dbg[p] = v;
     }
@@ -730,36 +678,31 @@ static_assert(sizeof(Slot64) == reeval_slot_bytes, "re-evaluation scratch layout
 // and the 4 dim axis points enter the fourth differences, src/hcubature.cpp:527-575),
 // kind 1 = whole rule (value, error and split: ambiguous selection boundaries and the
 // final polish).  The FP64 pipe issues one warp instruction per 64 cycles per SM
-// sub-partition, so a round's re-evaluation time is set by the busiest sub-partition:
-// the work is spread evenly over the whole device in three passes over the first
-// P.rcap entries -- coordinate slots (one per thread), rule points (one per thread, each
-// entry's points padded to whole warps) and the sums (one thread per entry, in the
-// reference's order).  Entries beyond P.rcap take the batched kernel k_reeval64.
+// sub-partition, so a round's re-evaluation time is set by the busiest sub-partition and, in
+// a round of few entries, by the longest chain of one thread: the work is spread evenly over
+// the whole device in three passes over the first P.rcap entries.
+//   k_re_fill    coordinate slots; a mass's two populations, its r_200 and its NFW
+//                normalisations on threads of their own
+//   k_re_ucache  shared u_NFW, two threads each (Si and Ci of either argument), and the
+//                auxiliary functions
+//   k_re_finish  a block per entry: the points, then the sums in the reference's order
+// Every pass's kinds of task start on a warp boundary, so that a warp runs one kind.
+// Entries beyond P.rcap take the batched kernel k_reeval64.
 template <int KIND, int TERM>
 struct Reeval {
     static constexpr int DIM = TERM + 4;
     static constexpr int NP = rule_points(DIM);
     static constexpr int NAX = 1 + 4 * DIM;
     static constexpr int NS = DIM * NVAR;
-    static constexpr int NPAD = (NP + 31) / 32 * 32;
     static constexpr int G = KIND * 3 + TERM - 1;
-    // the pass of cached values (measured faster for every term): the points then
-    // evaluate no FP64 u_NFW of their own except the 1-halo terms' k3 one
-    static constexpr bool UCACHE = true;
-    // r_200 and F once per (mass, z) pair (k_re_fill) instead of per u_NFW call
-    static constexpr bool MZ = UCACHE;
     __device__ static Slot64 *slots(const Pool &P)
     {
         return (Slot64 *)(P.rscr + (long long)G * P.rscr_group);
     }
-    __device__ static double *vals(const Pool &P)
+    __device__ static double *ucv(const Pool &P)  // [rcap][UC_NF_MAX][UC_MAX]
     {
         return (double *)(P.rscr + (long long)G * P.rscr_group +
                           ((long long)P.rcap * MAX_DIM * NVAR * reeval_slot_bytes + 255) / 256 * 256);
-    }
-    __device__ static double *ucv(const Pool &P)  // [rcap][UC_NF_MAX][UC_MAX]
-    {
-        return vals(P) + (long long)P.rcap * 256;
     }
     __device__ static double *u3v(const Pool &P)  // [rcap][U3_NF_MAX][U3_MAX]
     {
@@ -781,266 +724,316 @@ struct Reeval {
     // auxiliary values per entry (124 for the 2-halo terms)
     static constexpr int NAUX = aux_off(TERM, aux_nfun(TERM) - 1) + aux_count(TERM, aux_nfun(TERM) - 1);
     static_assert(NAUX <= AUX_MAX, "auxiliary projections exceed AUX_MAX");
-    __device__ static int count(const Pool &P, const BatchHdr *H)
+    __device__ static int count(const Pool &P, const BatchHdr *H, int stage)
     {
         const int cap = H->esc_cap[G];
-        const int n = H->n_esc[G] < cap ? H->n_esc[G] : cap;
+        const int n = H->n_esc[stage][G] < cap ? H->n_esc[stage][G] : cap;
         return n < P.rcap ? n : P.rcap;
     }
+    // coordinate of variant v of dimension dim of entry ent
+    __device__ static double coord(const Pool &P, const IntDesc &d, int2 ent, int dim, int v)
+    {
+        const long long slot = d.base + (ent.y & 0x3FFFFFFF);
+        return variant_x(P.center[dim * P.stride + slot],
+                         ldexp(d.hw0[dim], -(int)P.level[dim * P.stride + slot]), v);
+    }
 };
+
+__host__ __device__ constexpr long long warps_up(long long n) { return (n + 31) / 32 * 32; }
 
 template <int KIND, int TERM>
 __global__ void __launch_bounds__(128) k_re_fill(DevTables T, const IntDesc *__restrict__ D,
                                                  IntState *__restrict__ S, Pool P, BatchHdr *H,
-                                                 const long long *__restrict__ woff)
+                                                 const long long *__restrict__ woff, int stage)
 {
     using R = Reeval<KIND, TERM>;
-    const int m = R::count(P, H);
+    using M = Model64<KIND, TERM>;
+    // the second stage's queue of the previous round has been consumed
+    if (stage == 0 && blockIdx.x == 0 && threadIdx.x == 0) H->n_esc[1][R::G] = 0;
+    const int m = R::count(P, H, stage);
     if (m == 0) return;
     const int2 *Q = P.esc + H->esc_beg[R::G];
     Slot64 *SL = R::slots(P);
-    const long long stride = P.stride;
-    const long long tot1 = (long long)m * R::NS;
-    // then the (mass, z) pairs' r_200 and F, one thread each (their mass and bin from the
-    // same expressions as the mass slot's)
-    constexpr int NMZ = R::MZ ? TERM * MZ_PAIRS : 0;
-    const long long tot = tot1 + (long long)m * NMZ;
+    constexpr int ZD = R::DIM - 1, NMS = TERM * NVAR, NLS = 4 * NVAR, NMZ = TERM * MZ_PAIRS;
+    // masses (the longest), the second population's occupations, r_200, the normalisations,
+    // then l1, l2, phi and z
+    const long long b1 = warps_up((long long)m * NMS), b2 = b1 + (KIND == 0 ? b1 : 0);
+    const long long nmz = warps_up((long long)m * NMZ), b3 = b2 + nmz, b4 = b3 + nmz;
+    const long long tot = b4 + (long long)m * NLS;
     for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < tot;
          t += (long long)gridDim.x * blockDim.x) {
-        if (NMZ > 0 && t >= tot1) {
-            constexpr int NMZ1 = NMZ > 0 ? NMZ : 1;
-            const long long t2 = t - tot1;
-            const int k = (int)(t2 / NMZ1), r = (int)(t2 - (long long)k * NMZ1);
+        if (t < b2) {
+            const bool second = t >= b1;
+            const long long q = second ? t - b1 : t;
+            const int k = (int)(q / NMS), r = (int)(q - (long long)k * NMS);
+            if (k >= m) continue;
+            const int dim = 3 + r / NVAR, v = r % NVAR;
+            const int2 ent = Q[k];
+            const IntDesc &d = D[ent.x];
+            if (second && d.same) continue;
+            // split only: the centre of every dimension, the contenders' axis variants
+            if (!(ent.y >> 30) && !split_variant(split_cmask(P, d, ent), dim, v)) continue;
+            const double x = R::coord(P, d, ent, dim, v);
+            Slot64 &sl = SL[(long long)k * R::NS + dim * NVAR + v];
+            if (!second) {
+                Slot64 f;
+                M::fill_mass(T, d, x, f, &H->ties);
+                sl.a[0] = f.a[0];
+                sl.a[1] = f.a[1];
+                sl.a[2] = f.a[2];
+                sl.i0 = f.i0;
+                sl.i1 = f.i1;
+                if (KIND == 0 && d.same) {
+                    sl.a[3] = f.a[3];
+                    sl.a[4] = f.a[4];
+                    sl.a[5] = f.a[5];
+                }
+            } else {
+                occupations64(T.hod + 6 * d.hod2, pow(10, x), sl.a[3], sl.a[4]);
+            }
+        } else if (t < b4) {
+            // r_200 and F of the (mass, z) pairs, from the mass slot's expressions
+            const bool norm = t >= b3;
+            const long long q = t - (norm ? b3 : b2);
+            const int k = (int)(q / NMZ), r = (int)(q - (long long)k * NMZ);
+            if (k >= m) continue;
             const int md = 3 + r / MZ_PAIRS, j = r - (md - 3) * MZ_PAIRS;
             const int vm = mz_vm_of(j), vz = mz_vz_of(j);
             const int2 ent = Q[k];
             const IntDesc &d = D[ent.x];
-            constexpr int zd = R::DIM - 1;
-            if (!(ent.y >> 30)) {  // split only: the centre and the contenders' axis variants
+            if (!(ent.y >> 30)) {
                 const unsigned cm = split_cmask(P, d, ent);
-                if ((vm && vz) || !split_variant(cm, md, vm) || !split_variant(cm, zd, vz)) continue;
+                if ((vm && vz) || !split_variant(cm, md, vm) || !split_variant(cm, ZD, vz)) continue;
             }
-            const long long slot = d.base + (ent.y & 0x3FFFFFFF);
-            Slot64 M;
-            const double xm = variant_x(P.center[md * stride + slot],
-                                        ldexp(d.hw0[md], -(int)P.level[md * stride + slot]), vm);
-            M.a[0] = pow(10, xm);
-            m_index(T, xm, M.a[0], M.i0, M.i1, nullptr);
-            const int zt = z_trunc64(T, variant_x(P.center[zd * stride + slot],
-                                                  ldexp(d.hw0[zd], -(int)P.level[zd * stride + slot]), vz));
-            Model64<KIND, TERM>::mz_values(T, d, M, zt, KIND == 0 ? 3 : 2,
-                                           R::mzv(P) + (((long long)k * 3 + (md - 3)) * MZ_PAIRS + j) * MZ_VALS);
-            continue;
+            const double xm = R::coord(P, d, ent, md, vm);
+            const int zt = z_trunc64(T, R::coord(P, d, ent, ZD, vz));
+            double *o = R::mzv(P) + (((long long)k * 3 + (md - 3)) * MZ_PAIRS + j) * MZ_VALS;
+            if (norm) {
+                Slot64 f;
+                m_index_x(T, xm, f.i0, f.i1);
+                M::mz_norms(T, d, f, zt, KIND == 0 ? 3 : 2, o);
+            } else {
+                o[0] = r200_64(pow(10, xm), __ldg(T.rho_bar + zt));
+            }
+        } else {
+            const long long q = t - b4;
+            const int k = (int)(q / NLS), r = (int)(q - (long long)k * NLS);
+            const int dim = r / NVAR < 3 ? r / NVAR : ZD, v = r % NVAR;
+            const int2 ent = Q[k];
+            const IntDesc &d = D[ent.x];
+            if (!(ent.y >> 30) && !split_variant(split_cmask(P, d, ent), dim, v)) continue;
+            M::fill(T, d, dim, R::coord(P, d, ent, dim, v), SL[(long long)k * R::NS + dim * NVAR + v],
+                    &H->ties);
         }
-        const int k = (int)(t / R::NS), r = (int)(t - (long long)k * R::NS);
-        const int dim = r / NVAR, v = r - dim * NVAR;
-        const int2 ent = Q[k];
-        const IntDesc &d = D[ent.x];
-        // split only: the centre of every dimension, the contenders' axis variants
-        if (!(ent.y >> 30) && !split_variant(split_cmask(P, d, ent), dim, v)) continue;
-        const long long slot = d.base + (ent.y & 0x3FFFFFFF);
-        const double c = P.center[dim * stride + slot];
-        const double hw = ldexp(d.hw0[dim], -(int)P.level[dim * stride + slot]);
-        Model64<KIND, TERM>::fill(T, d, dim, variant_x(c, hw, v), SL[(long long)k * R::NS + r], &H->ties);
     }
 }
 
-// cached u_NFW of each entry's (l, m, z) combinations (whole rules: all of them; split
-// only: those without corner variants, whose slots are not filled)
+// u_NFW of each entry's (l, m, z) combinations and k3 projections (whole rules: all of them;
+// split only: those that the centre and the contenders' axis points read), then the
+// auxiliary functions per projection and the satellite pair counts of two populations.
 template <int KIND, int TERM>
 __global__ void __launch_bounds__(128) k_re_ucache(DevTables T, const IntDesc *__restrict__ D,
                                                    IntState *__restrict__ S, Pool P, BatchHdr *H,
-                                                   const long long *__restrict__ woff)
+                                                   const long long *__restrict__ woff, int stage)
 {
     using R = Reeval<KIND, TERM>;
-    constexpr int NF = ucache_nf(TERM);
+    using M = Model64<KIND, TERM>;
+    constexpr int NF = ucache_nf(TERM), NU3 = u3_nfun(TERM), ZD = R::DIM - 1;
     __shared__ __align__(16) unsigned char tbuf[sizeof(ReTab<KIND, TERM>)];
-    const int m = R::count(P, H);
-    if (m == 0 || !R::UCACHE) return;
-    const long long tot1 = (long long)m * NF * UC_MAX;
-    // the k3 u_NFW of each projection (2- and 3-halo terms): after the (l, m, z) ones
-    const long long tot2 = tot1 + (long long)m * u3_nfun(TERM) * U3_MAX;
-    // the auxiliary functions of each projection: last
-    const long long tot = tot2 + (long long)m * R::NAUX;
-    if ((long long)blockIdx.x * blockDim.x >= tot) return;  // no work here: skip the tables
-    const ReTab<KIND, TERM> &tb = load_retab<KIND, TERM>(P, tbuf);
-    const uint32_t *sdesc = tb.sdesc;
-    const uint16_t *ucl = tb.ucl;
-    const int *ucn = tb.ucn;
-    const uint8_t *u3list = tb.u3list, *auxlist = tb.auxlist;
-    const int2 *Q = P.esc + H->esc_beg[R::G];
-    const Slot64 *SL = R::slots(P);
-    double *UC = R::ucv(P);
-    double *U3C = R::u3v(P);
-    double *AX = R::auxv(P);
-    for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < tot;
-         t += (long long)gridDim.x * blockDim.x) {
-        if (t >= tot2) {
-            const long long t3 = t - tot2;
-            const int k = (int)(t3 / R::NAUX), r = (int)(t3 - (long long)k * R::NAUX);
-            int a = 0;
-            while (a + 1 < aux_nfun(TERM) && r >= aux_off(TERM, a + 1)) ++a;
-            const int pr = auxlist[r];
-            const int2 ent = Q[k];
-            // split only: the projections of the centre and the contenders' axis points
-            if (!(ent.y >> 30) && !split_point(split_cmask(P, D[ent.x], ent), pr, R::NAX)) continue;
-            const uint32_t vv = sdesc[pr];
-            const Slot64 *base = SL + (long long)k * R::NS;
-            const Slot64 *sp[R::DIM];
-#pragma unroll
-            for (int dd = 0; dd < R::DIM; ++dd) sp[dd] = base + dd * NVAR + ((vv >> (3 * dd)) & 7);
-            AX[(long long)k * AUX_MAX + r] = Model64<KIND, TERM>::aux(T, D[ent.x], a, sp);
-            continue;
-        }
-        if (t >= tot1) {
-            const long long t2 = t - tot1;
-            const int k = (int)(t2 / (u3_nfun(TERM) * U3_MAX));
-            const int r = (int)(t2 - (long long)k * u3_nfun(TERM) * U3_MAX);
-            const int f = r / U3_MAX, j = r - f * U3_MAX;
-            const int pr = u3list[f * U3_MAX + j];  // every projection index is used (93)
-            const int2 ent = Q[k];
-            if (!(ent.y >> 30) && !split_point(split_cmask(P, D[ent.x], ent), pr, R::NAX)) continue;
-            const uint32_t vv = sdesc[pr];
-            const Slot64 *base = SL + (long long)k * R::NS;
-            const Slot64 *sp[R::DIM];
-#pragma unroll
-            for (int dd = 0; dd < R::DIM; ++dd) sp[dd] = base + dd * NVAR + ((vv >> (3 * dd)) & 7);
-            U3C[((long long)k * U3_NF_MAX + f) * U3_MAX + j] =
-                Model64<KIND, TERM>::u3(T, f, sp, R::MZ ? R::mz(P, k, u3_mass(KIND, TERM, f), vv) : nullptr);
-            continue;
-        }
-        const int k = (int)(t / (NF * UC_MAX)), r = (int)(t - (long long)k * NF * UC_MAX);
-        const int f = r / UC_MAX, j = r - f * UC_MAX;
-        if (j >= ucn[f]) continue;
-        const int2 ent = Q[k];
-        const uint32_t key = ucl[f * UC_MAX + j];
-        const int vl = key & 7, vm = (key >> 3) & 7, vz = (key >> 6) & 7;
-        const int dl = ucache_fun(KIND, TERM, f, 0), dm = ucache_fun(KIND, TERM, f, 1);
-        if (!(ent.y >> 30)) {  // split only: combinations of the centre and one contender axis
-            const unsigned cm = split_cmask(P, D[ent.x], ent);
-            if ((vl != 0) + (vm != 0) + (vz != 0) > 1 || !split_variant(cm, dl, vl) ||
-                !split_variant(cm, dm, vm) || !split_variant(cm, R::DIM - 1, vz))
-                continue;
-        }
-        const Slot64 *base = SL + (long long)k * R::NS;
-        UC[((long long)k * UC_NF_MAX + f) * UC_MAX + j] = Model64<KIND, TERM>::ucached(
-            T, D[ent.x], f, base[dl * NVAR + vl], base[dm * NVAR + vm], base[(R::DIM - 1) * NVAR + vz],
-            R::MZ ? R::mz(P, k, dm, ((uint32_t)vm << (3 * dm)) | ((uint32_t)vz << (3 * (R::DIM - 1))))
-                  : nullptr);
-    }
-}
-
-template <int KIND, int TERM>
-__global__ void __launch_bounds__(128) k_re_points(DevTables T, const IntDesc *__restrict__ D,
-                                                   IntState *__restrict__ S, Pool P, BatchHdr *H,
-                                                   const long long *__restrict__ woff)
-{
-    using R = Reeval<KIND, TERM>;
-    constexpr int DIM = R::DIM;
-    constexpr int NF = ucache_nf(TERM);
-    constexpr int NU3 = u3_nfun(TERM);
-    constexpr int NA = aux_nfun(TERM);
-    __shared__ __align__(16) unsigned char tbuf[sizeof(ReTab<KIND, TERM>)];
-    const int m = R::count(P, H);
+    __shared__ double ex[3][64];
+    const int m = R::count(P, H, stage);
     if (m == 0) return;
-    const long long tot = (long long)m * R::NPAD;
-    if ((long long)blockIdx.x * blockDim.x >= tot) return;  // no work here: skip the tables
+    const long long b1 = warps_up((long long)m * NF * UC_MAX), nu = b1 + (long long)m * NU3 * U3_MAX;
+    const long long a1 = warps_up((long long)m * R::NAUX);
+    const long long na = a1 + (KIND == 0 ? (long long)m * TERM * NVAR : 0);
+    const long long nchunk = (nu + 63) / 64;
+    // the auxiliary tasks start from the other end of the grid
+    const long long first_aux = (long long)(gridDim.x - 1 - blockIdx.x) * blockDim.x;
+    if (blockIdx.x >= nchunk && first_aux >= na) return;  // no work here: skip the tables
     const ReTab<KIND, TERM> &tb = load_retab<KIND, TERM>(P, tbuf);
-    const uint32_t *sdesc = tb.sdesc;
-    const uint8_t *ucidx = tb.ucidx, *u3rep = tb.u3rep, *auxrep = tb.auxrep;
-    const double *U3C = R::u3v(P);
-    const double *AX = R::auxv(P);
     const int2 *Q = P.esc + H->esc_beg[R::G];
-    const Slot64 *SL = R::slots(P);
-    double *VL = R::vals(P);
-    const double *UC = R::ucv(P);
-    for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < tot;
-         t += (long long)gridDim.x * blockDim.x) {
-        const int k = (int)(t / R::NPAD), p = (int)(t - (long long)k * R::NPAD);
+    Slot64 *SL = R::slots(P);
+    double *UC = R::ucv(P), *U3C = R::u3v(P), *AX = R::auxv(P);
+    const int part = threadIdx.x >> 6, q = threadIdx.x & 63;
+    for (long long c = blockIdx.x; c < nchunk; c += gridDim.x) {
+        const long long t = c * 64 + q;
+        double kk = 1, r200 = 1, cc = 1, F = 1;
+        double *out = nullptr;
+        if (t < b1) {
+            const int k = (int)(t / (NF * UC_MAX)), r = (int)(t - (long long)k * NF * UC_MAX);
+            const int f = r / UC_MAX, j = r - f * UC_MAX;
+            if (k < m && j < tb.ucn[f]) {
+                const int2 ent = Q[k];
+                const IntDesc &d = D[ent.x];
+                const uint32_t key = tb.ucl[f * UC_MAX + j];
+                const int vl = key & 7, vm = (key >> 3) & 7, vz = (key >> 6) & 7;
+                const int dl = ucache_fun(KIND, TERM, f, 0), dm = ucache_fun(KIND, TERM, f, 1);
+                bool need = true;
+                if (!(ent.y >> 30)) {  // combinations of the centre and one contender axis
+                    const unsigned cm = split_cmask(P, d, ent);
+                    need = (vl != 0) + (vm != 0) + (vz != 0) <= 1 && split_variant(cm, dl, vl) &&
+                           split_variant(cm, dm, vm) && split_variant(cm, ZD, vz);
+                }
+                if (need) {
+                    const Slot64 *base = SL + (long long)k * R::NS;
+                    M::ucached_args(T, d, f, base[dl * NVAR + vl], base[dm * NVAR + vm],
+                                    base[ZD * NVAR + vz],
+                                    R::mz(P, k, dm, ((uint32_t)vm << (3 * dm)) | ((uint32_t)vz << (3 * ZD))),
+                                    kk, r200, cc, F);
+                    out = UC + ((long long)k * UC_NF_MAX + f) * UC_MAX + j;
+                }
+            }
+        } else if (t < nu) {
+            const long long t2 = t - b1;
+            const int k = (int)(t2 / (NU3 * U3_MAX)), r = (int)(t2 - (long long)k * NU3 * U3_MAX);
+            const int f = r / U3_MAX, j = r - f * U3_MAX;
+            const int pr = tb.u3list[f * U3_MAX + j];  // every projection index is used (93)
+            const int2 ent = Q[k];
+            if ((ent.y >> 30) || split_point(split_cmask(P, D[ent.x], ent), pr, R::NAX)) {
+                const uint32_t vv = tb.sdesc[pr];
+                const Slot64 *base = SL + (long long)k * R::NS;
+                const Slot64 *sp[R::DIM];
+#pragma unroll
+                for (int dd = 0; dd < R::DIM; ++dd) sp[dd] = base + dd * NVAR + ((vv >> (3 * dd)) & 7);
+                M::u3_args(T, f, sp, R::mz(P, k, u3_mass(KIND, TERM, f), vv), kk, r200, cc, F);
+                out = U3C + ((long long)k * U3_NF_MAX + f) * U3_MAX + j;
+            }
+        }
+        // u_nfw64_F, each argument's Si and Ci on a thread of its own (64 apart)
+        const double arg1 = ddiv(kk * r200, cc);
+        const double arg2 = arg1 * (1 + cc);
+        double si = 0, ci = 0, sx = 0, cx = 0;
+        if (out) sici64_sc(part ? arg2 : arg1, si, ci, sx, cx);
+        if (part) {
+            ex[0][q] = si;
+            ex[1][q] = ci;
+            if (out) ex[2][q] = ddiv(-sin(arg1 * cc), arg2);
+        }
+        __syncthreads();
+        if (!part && out) {
+            const double term1 = sx * (ex[0][q] - si);
+            const double term2 = cx * (ex[1][q] - ci);
+            *out = ddiv(term1 + term2 + ex[2][q], F);
+        }
+        __syncthreads();
+    }
+    for (long long t = first_aux + threadIdx.x; t < na; t += (long long)gridDim.x * blockDim.x) {
+        if (t >= a1) {
+            const long long t2 = t - a1;
+            const int k = (int)(t2 / (TERM * NVAR)), r = (int)(t2 - (long long)k * (TERM * NVAR));
+            const int2 ent = Q[k];
+            const IntDesc &d = D[ent.x];
+            if (d.same || (!(ent.y >> 30) && !split_variant(split_cmask(P, d, ent), 3 + r / NVAR, r % NVAR)))
+                continue;
+            Slot64 &sl = SL[(long long)k * R::NS + 3 * NVAR + r];
+            sl.a[5] = M::pairs(T, d, sl);
+            continue;
+        }
+        const int k = (int)(t / R::NAUX), r = (int)(t - (long long)k * R::NAUX);
+        if (k >= m) continue;
+        int a = 0;
+        while (a + 1 < aux_nfun(TERM) && r >= aux_off(TERM, a + 1)) ++a;
+        const int pr = tb.auxlist[r];
         const int2 ent = Q[k];
-        if (p >= R::NP) continue;
-        const IntDesc &d = D[ent.x];
-        if (!(ent.y >> 30) && !split_point(split_cmask(P, d, ent), p, R::NAX)) continue;
-        const uint32_t vv = sdesc[p];
+        // split only: the projections of the centre and the contenders' axis points
+        if (!(ent.y >> 30) && !split_point(split_cmask(P, D[ent.x], ent), pr, R::NAX)) continue;
+        const uint32_t vv = tb.sdesc[pr];
         const Slot64 *base = SL + (long long)k * R::NS;
-        const Slot64 *sp[DIM];
+        const Slot64 *sp[R::DIM];
 #pragma unroll
-        for (int dd = 0; dd < DIM; ++dd) sp[dd] = base + dd * NVAR + ((vv >> (3 * dd)) & 7);
-        double uc[NF];
-        if (R::UCACHE) {
-#pragma unroll
-            for (int f = 0; f < NF; ++f)
-                uc[f] = UC[((long long)k * UC_NF_MAX + f) * UC_MAX + ucidx[f * R::NP + p]];
-        }
-        double u3c[NU3 > 0 ? NU3 : 1];
-        if (R::UCACHE) {
-#pragma unroll
-            for (int f = 0; f < NU3; ++f)
-                u3c[f] = U3C[((long long)k * U3_NF_MAX + f) * U3_MAX + u3rep[f * R::NP + p]];
-        }
-        double ax[NA];
-        if (R::UCACHE) {
-#pragma unroll
-            for (int a = 0; a < NA; ++a)
-                ax[a] = AX[(long long)k * AUX_MAX + aux_off(TERM, a) + auxrep[a * R::NP + p]];
-        }
-        VL[(long long)k * R::NPAD + p] = Model64<KIND, TERM>::point(
-            T, d, sp, R::UCACHE ? uc : nullptr, (R::UCACHE && NU3 > 0) ? u3c : nullptr,
-            R::UCACHE ? ax : nullptr, (R::MZ && TERM == 1) ? R::mz(P, k, 3, vv) : nullptr);
+        for (int dd = 0; dd < R::DIM; ++dd) sp[dd] = base + dd * NVAR + ((vv >> (3 * dd)) & 7);
+        AX[(long long)k * AUX_MAX + r] = M::aux(T, D[ent.x], a, sp);
     }
 }
 
-// the sums of one re-evaluated region (vl: its rule-point values)
+// the split dimension of one re-taken split (vl: its rule-point values; cm: the contenders)
+template <int DIM>
+__device__ int retaken_split(const double *vl, unsigned cm)
+{
+    const double ratio = (G3L_LAMBDA2 * G3L_LAMBDA2) / (G3L_LAMBDA4 * G3L_LAMBDA4);
+    const double val0 = vl[0];
+    double maxdiff = 0;
+    int dimDiffMax = 0;
+    for (int q = 0; q < DIM; ++q) {
+        if (!((cm >> q) & 1u)) continue;  // not a contender (its points were not taken)
+        double v0 = vl[1 + 4 * q], v1 = vl[2 + 4 * q];
+        double v2 = vl[3 + 4 * q], v3 = vl[4 + 4 * q];
+        double diff = 0;
+        diff += fabs(v0 + v1 - 2 * val0 - ratio * (v2 + v3 - 2 * val0));
+        if (diff > maxdiff) {
+            maxdiff = diff;
+            dimDiffMax = q;
+        }
+    }
+    return dimDiffMax;
+}
+
+// the sums of one re-evaluated region by one warp (vl: its rule-point values)
 template <int DIM>
 __device__ void reeval_finish(const IntDesc &d, const Pool &P, long long slot, bool full,
                               const double *vl, unsigned cm)
 {
-    const long long stride = P.stride;
+    const int lane = threadIdx.x & 31;
     if (full) {
-        int lsum = 0;
-        for (int q = 0; q < DIM; ++q) lsum += P.level[q * stride + slot];
+        const int lsum = __reduce_add_sync(0xffffffffu, lane < DIM ? (int)P.level[lane * P.stride + slot] : 0);
         double val, err;
         int split;
-        combine64<DIM>(vl, ldexp(d.rootvol, -lsum), val, err, split);
-        P.val[slot] = val;
-        P.err[slot] = err;
-        P.split[slot] = (unsigned char)split;
-        P.unc[slot] = 0.f;
-        P.uval[slot] = 0.f;
-    } else {
-        const double ratio = (G3L_LAMBDA2 * G3L_LAMBDA2) / (G3L_LAMBDA4 * G3L_LAMBDA4);
-        const double val0 = vl[0];
-        double maxdiff = 0;
-        int dimDiffMax = 0;
-        for (int q = 0; q < DIM; ++q) {
-            if (!((cm >> q) & 1u)) continue;  // not a contender (its points were not taken)
-            double v0 = vl[1 + 4 * q], v1 = vl[2 + 4 * q];
-            double v2 = vl[3 + 4 * q], v3 = vl[4 + 4 * q];
-            double diff = 0;
-            diff += fabs(v0 + v1 - 2 * val0 - ratio * (v2 + v3 - 2 * val0));
-            if (diff > maxdiff) {
-                maxdiff = diff;
-                dimDiffMax = q;
-            }
+        combine64_warp<DIM>(vl, ldexp(d.rootvol, -lsum), val, err, split);
+        if (lane == 0) {
+            P.val[slot] = val;
+            P.err[slot] = err;
+            P.split[slot] = (unsigned char)split;
+            P.unc[slot] = 0.f;
+            P.uval[slot] = 0.f;
         }
-        P.split[slot] = (unsigned char)dimDiffMax;
+    } else if (lane == 0) {
+        P.split[slot] = (unsigned char)retaken_split<DIM>(vl, cm);
     }
 }
 
 template <int KIND, int TERM>
-__global__ void __launch_bounds__(128) k_re_combine(DevTables T, const IntDesc *__restrict__ D,
-                                                    IntState *__restrict__ S, Pool P, BatchHdr *H,
-                                                    const long long *__restrict__ woff)
+__global__ void __launch_bounds__(128) k_re_finish(DevTables T, const IntDesc *__restrict__ D,
+                                                   IntState *__restrict__ S, Pool P, BatchHdr *H,
+                                                   const long long *__restrict__ woff, int stage)
 {
     using R = Reeval<KIND, TERM>;
-    const int m = R::count(P, H);
+    constexpr int DIM = R::DIM, NF = ucache_nf(TERM), NU3 = u3_nfun(TERM), NA = aux_nfun(TERM);
+    __shared__ __align__(16) unsigned char tbuf[sizeof(ReTab<KIND, TERM>)];
+    __shared__ double vals[R::NP];
+    const int m = R::count(P, H, stage);
+    if ((int)blockIdx.x >= m) return;  // no work here: skip the tables
+    const ReTab<KIND, TERM> &tb = load_retab<KIND, TERM>(P, tbuf);
     const int2 *Q = P.esc + H->esc_beg[R::G];
-    const double *VL = R::vals(P);
-    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < m; k += gridDim.x * blockDim.x) {
+    const Slot64 *SL = R::slots(P);
+    const double *UC = R::ucv(P), *U3C = R::u3v(P), *AX = R::auxv(P);
+    for (int k = blockIdx.x; k < m; k += gridDim.x) {
         const int2 ent = Q[k];
         const IntDesc &d = D[ent.x];
-        reeval_finish<R::DIM>(d, P, d.base + (ent.y & 0x3FFFFFFF), (ent.y >> 30) != 0,
-                              VL + (long long)k * R::NPAD, (ent.y >> 30) ? 0u : split_cmask(P, d, ent));
+        const bool full = (ent.y >> 30) != 0;
+        const unsigned cm = full ? 0u : split_cmask(P, d, ent);
+        for (int p = threadIdx.x; p < (full ? R::NP : R::NAX); p += 128) {
+            if (!full && !split_point(cm, p, R::NAX)) continue;
+            const uint32_t vv = tb.sdesc[p];
+            const Slot64 *base = SL + (long long)k * R::NS;
+            const Slot64 *sp[DIM];
+#pragma unroll
+            for (int dd = 0; dd < DIM; ++dd) sp[dd] = base + dd * NVAR + ((vv >> (3 * dd)) & 7);
+            double uc[NF], u3c[NU3], ax[NA];
+#pragma unroll
+            for (int f = 0; f < NF; ++f)
+                uc[f] = UC[((long long)k * UC_NF_MAX + f) * UC_MAX + tb.ucidx[f * R::NP + p]];
+#pragma unroll
+            for (int f = 0; f < NU3; ++f)
+                u3c[f] = U3C[((long long)k * U3_NF_MAX + f) * U3_MAX + tb.u3rep[f * R::NP + p]];
+#pragma unroll
+            for (int a = 0; a < NA; ++a)
+                ax[a] = AX[(long long)k * AUX_MAX + aux_off(TERM, a) + tb.auxrep[a * R::NP + p]];
+            vals[p] = Model64<KIND, TERM>::point(T, d, sp, uc, u3c, ax);
+        }
+        __syncthreads();
+        if (threadIdx.x < 32)
+            reeval_finish<DIM>(d, P, d.base + (ent.y & 0x3FFFFFFF), full, vals, cm);
+        __syncthreads();
     }
 }
 
@@ -1049,7 +1042,7 @@ __global__ void __launch_bounds__(128) k_re_combine(DevTables T, const IntDesc *
 template <int KIND, int TERM>
 __global__ void __launch_bounds__(128) k_reeval64(DevTables T, const IntDesc *__restrict__ D,
                                                   IntState *__restrict__ S, Pool P, BatchHdr *H,
-                                                  const long long *__restrict__ woff)
+                                                  const long long *__restrict__ woff, int stage)
 {
     constexpr int DIM = TERM + 4;
     constexpr int NP = rule_points(DIM);
@@ -1062,7 +1055,7 @@ __global__ void __launch_bounds__(128) k_reeval64(DevTables T, const IntDesc *__
     __shared__ int2 sent[RB];
     const int g = KIND * 3 + TERM - 1;
     const int cap = H->esc_cap[g];
-    const int n = H->n_esc[g] < cap ? H->n_esc[g] : cap;
+    const int n = H->n_esc[stage][g] < cap ? H->n_esc[stage][g] : cap;
     const int first = P.rcap;
     if (n <= first) return;
     for (int p = threadIdx.x; p < NP; p += blockDim.x) sdesc[p] = point_variants(DIM, p);
@@ -1112,11 +1105,12 @@ __global__ void __launch_bounds__(128) k_reeval64(DevTables T, const IntDesc *__
             vals[k][p] = Model64<KIND, TERM>::point(T, d, sp);
         }
         __syncthreads();
-        if (threadIdx.x < ne) {
-            const int2 ent = sent[threadIdx.x];
+        static_assert(RB <= 4, "one warp per entry");
+        if ((int)threadIdx.x >> 5 < ne) {
+            const int2 ent = sent[threadIdx.x >> 5];
             const IntDesc &d = D[ent.x];
             reeval_finish<DIM>(d, P, d.base + (ent.y & 0x3FFFFFFF), (ent.y >> 30) != 0,
-                               vals[threadIdx.x], (ent.y >> 30) ? 0u : split_cmask(P, d, ent));
+                               vals[threadIdx.x >> 5], (ent.y >> 30) ? 0u : split_cmask(P, d, ent));
         }
     }
 }
@@ -1125,15 +1119,13 @@ __global__ void __launch_bounds__(128) k_reeval64(DevTables T, const IntDesc *__
     template __global__ void k_eval64<K, Tm>(DevTables, const IntDesc *, IntState *, Pool,      \
                                              BatchHdr *, const long long *);                     \
     template __global__ void k_reeval64<K, Tm>(DevTables, const IntDesc *, IntState *, Pool,    \
-                                               BatchHdr *, const long long *);                   \
+                                               BatchHdr *, const long long *, int);              \
     template __global__ void k_re_fill<K, Tm>(DevTables, const IntDesc *, IntState *, Pool,     \
-                                              BatchHdr *, const long long *);                    \
+                                              BatchHdr *, const long long *, int);               \
     template __global__ void k_re_ucache<K, Tm>(DevTables, const IntDesc *, IntState *, Pool,   \
-                                                BatchHdr *, const long long *);                  \
-    template __global__ void k_re_points<K, Tm>(DevTables, const IntDesc *, IntState *, Pool,   \
-                                                BatchHdr *, const long long *);                  \
-    template __global__ void k_re_combine<K, Tm>(DevTables, const IntDesc *, IntState *, Pool,  \
-                                                 BatchHdr *, const long long *);                 \
+                                                BatchHdr *, const long long *, int);             \
+    template __global__ void k_re_finish<K, Tm>(DevTables, const IntDesc *, IntState *, Pool,   \
+                                                BatchHdr *, const long long *, int);             \
     template __global__ void k_re_tables<K, Tm>(unsigned char *);
 G3L_INST64(0, 1)
 G3L_INST64(0, 2)
@@ -1155,25 +1147,17 @@ cudaError_t build_reeval_tables(unsigned char *out, cudaStream_t s)
     return cudaGetLastError();
 }
 
-// re-evaluation kernels of a group: 0 = fill, 1 = cached u_NFW, 2 = points, 3 = combine,
-// 4 = batched tail
+// re-evaluation kernels of a group: 0 = fill, 1 = cached values, 2 = points and sums,
+// 3 = batched tail
 void *reeval_phase_kernel(int kind, int term, int phase)
 {
 #define G3L_RE_ROW(K, Tm)                                                                       \
-    {(void *)k_re_fill<K, Tm>, (void *)k_re_ucache<K, Tm>, (void *)k_re_points<K, Tm>,           \
-     (void *)k_re_combine<K, Tm>, (void *)k_reeval64<K, Tm>}
-    static void *tab[2][3][5] = {{G3L_RE_ROW(0, 1), G3L_RE_ROW(0, 2), G3L_RE_ROW(0, 3)},
+    {(void *)k_re_fill<K, Tm>, (void *)k_re_ucache<K, Tm>, (void *)k_re_finish<K, Tm>,           \
+     (void *)k_reeval64<K, Tm>}
+    static void *tab[2][3][4] = {{G3L_RE_ROW(0, 1), G3L_RE_ROW(0, 2), G3L_RE_ROW(0, 3)},
                                  {G3L_RE_ROW(1, 1), G3L_RE_ROW(1, 2), G3L_RE_ROW(1, 3)}};
 #undef G3L_RE_ROW
     return tab[kind][term - 1][phase];
-}
-
-void *reeval64_kernel(int kind, int term)
-{
-    static void *tab[2][3] = {
-        {(void *)k_reeval64<0, 1>, (void *)k_reeval64<0, 2>, (void *)k_reeval64<0, 3>},
-        {(void *)k_reeval64<1, 1>, (void *)k_reeval64<1, 2>, (void *)k_reeval64<1, 3>}};
-    return tab[kind][term - 1];
 }
 
 void *eval64_kernel(int kind, int term)

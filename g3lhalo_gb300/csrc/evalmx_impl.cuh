@@ -29,6 +29,8 @@
 //  * Rule sums, fourth differences and the 7th/5th-degree combination are
 //    double-float; the final value and error are formed in FP64 by four lanes
 //    at once.
+#include <cstddef>
+
 #include "dfloat.cuh"
 #include "g3l_device.cuh"
 #include "phys64.cuh"
@@ -999,20 +1001,16 @@ __global__ void __launch_bounds__(128, MINB) k_evalmx(DevTables T, const IntDesc
     constexpr int NP = rule_points(DIM);
     constexpr int NSLOT = (DIM + 1) * NVAR;
     constexpr int WPB = 4;
-    __shared__ uint32_t sdesc[NP];
+    // the point codes and the tables of the shared u_NFW (the head of the group's ReTab)
+    using RT = ReTab<KIND, TERM>;
+    constexpr int TAB = (int)offsetof(RT, u3rep);
+    __shared__ __align__(16) unsigned char tbuf[(TAB + 3) / 4 * 4];
     __shared__ SlotF sslot[WPB][NSLOT];
     __shared__ float svals[WPB][2 * NP];
     __shared__ Child schild[WPB];
     constexpr int NF = ModelF<KIND, TERM>::NF;
-    __shared__ uint8_t ucidx[NF * NP];           // combination of each point, per function
-    __shared__ uint16_t ucl[NF * UC_MAX];        // variants (l | m << 3 | z << 6) of each
-    __shared__ int ucn[NF];
     __shared__ float ucache[WPB][2 * NF * UC_MAX];
-    __shared__ uint8_t ucmap[NF * 343];
-    if (ModelF<KIND, TERM>::UC) ucache_tables<KIND, TERM>(ucidx, ucl, ucn, ucmap);
     const int g = KIND * 3 + TERM - 1;
-    for (int p = threadIdx.x; p < NP; p += blockDim.x) sdesc[p] = point_variants(DIM, p);
-    __syncthreads();
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
     const int gb = H->gbeg[g], ge = H->gbeg[g + 1];
     if (gb >= ge) return;
@@ -1027,6 +1025,12 @@ __global__ void __launch_bounds__(128, MINB) k_evalmx(DevTables T, const IntDesc
     const Group gr{wide ? 128 : 32, wide ? (int)threadIdx.x : lane};
     const int buf = wide ? 0 : wib;
     const long long first = wide ? blockIdx.x : (long long)blockIdx.x * WPB + wib;
+    if (wbeg + (wide ? (long long)blockIdx.x : (long long)blockIdx.x * WPB) >= wend) return;  // no work here
+    const RT &tb = load_retab<KIND, TERM>(P, tbuf, TAB);
+    const uint32_t *sdesc = tb.sdesc;
+    const uint8_t *ucidx = tb.ucidx;
+    const uint16_t *ucl = tb.ucl;
+    const int *ucn = tb.ucn;
     const long long step = (long long)gridDim.x * (wide ? 1 : WPB);
     for (long long w = wbeg + first; w < wend; w += step) {
         int lo = gb, hi = ge - 1;

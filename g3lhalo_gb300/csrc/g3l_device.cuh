@@ -118,7 +118,7 @@ struct Pool {
     double *key;            // selection scratch (polish keys |val| * uval)
     int2 *esc;              // regions queued for FP64 re-evaluation: (integral, local slot)
     long long stride;
-    // FP64 re-evaluation scratch: per group, coordinate slots and rule-point values of the
+    // FP64 re-evaluation scratch: per group, coordinate slots and cached values of the
     // first rcap queued entries of a round (later entries take the batched kernel)
     unsigned char *rscr;
     long long rscr_group;   // bytes per group
@@ -129,22 +129,24 @@ struct Pool {
 };
 constexpr int RETAB_BYTES = 4096;
 
-// u_NFW at k3 = |l1 + l2| / w with one halo mass (2- and 3-halo terms) does not depend
-// on the other mass dimensions, so the rule points that differ only there share it:
+// u_NFW at k3 = |l1 + l2| / w with one halo mass does not depend on the other mass
+// dimensions (2- and 3-halo terms), so the rule points that differ only there share it:
 // function f (u3_nfun(term) of them) uses mass dimension u3_mass(kind, term, f) and
-// ignores the variant fields u3_drop(kind, term, f) of the point code.  Dropping one of 6
-// or two of 7 dimensions leaves U3_MAX = rule_points(5) = 93 distinct projections.
+// ignores the variant fields u3_drop(kind, term, f) of the point code.  Dropping none of 5,
+// one of 6 or two of 7 dimensions leaves U3_MAX = rule_points(5) = 93 distinct projections
+// (for the 1-halo terms one per point: their u_NFW at k3 goes with the other shared ones).
 constexpr int U3_MAX = 93;
 constexpr int U3_NF_MAX = 2;
-__host__ __device__ constexpr int u3_nfun(int term) { return term == 1 ? 0 : (term == 2 ? 2 : 1); }
+__host__ __device__ constexpr int u3_nfun(int term) { return term == 2 ? 2 : 1; }
 __host__ __device__ constexpr int u3_mass(int kind, int term, int f)
 {
-    return term == 2 ? 3 + f : (kind == 0 ? 5 : 4);
+    return term == 1 ? 3 : (term == 2 ? 3 + f : (kind == 0 ? 5 : 4));
 }
 __host__ __device__ constexpr uint32_t u3_drop(int kind, int term, int f)
 {
-    return term == 2 ? (7u << (3 * (4 - f)))
-                     : (kind == 0 ? ((7u << 9) | (7u << 12)) : ((7u << 9) | (7u << 15)));
+    return term == 1 ? 0u
+                     : (term == 2 ? (7u << (3 * (4 - f)))
+                                  : (kind == 0 ? ((7u << 9) | (7u << 12)) : ((7u << 9) | (7u << 15))));
 }
 
 // Other quantities of a point that depend on a few of its dimensions only, cached per
@@ -230,7 +232,7 @@ constexpr long long reeval_slot_bytes = 56;  // sizeof(Slot64)
 __host__ __device__ constexpr long long reeval_scratch_group_bytes(int rcap)
 {
     return ((long long)rcap * MAX_DIM * NVAR * reeval_slot_bytes + 255) / 256 * 256 +
-           (long long)rcap * 256 * 8 + (long long)rcap * UC_NF_MAX * UC_MAX * 8 +
+           (long long)rcap * UC_NF_MAX * UC_MAX * 8 +
            (long long)rcap * U3_NF_MAX * U3_MAX * 8 + (long long)rcap * AUX_MAX * 8 +
            (long long)rcap * 3 * MZ_PAIRS * MZ_VALS * 8;
 }
@@ -252,7 +254,10 @@ struct BatchHdr {
     int chunk_rounds;            // > 0: stop the device loop after this many rounds (serving)
     int chunk_count;             //   rounds run in the current launch
     int mixed;                   // 1: mixed-precision pass (uncertainty bookkeeping on)
-    int n_esc[NGROUPS];          // FP64 re-evaluation queue of each group: fill,
+    // FP64 re-evaluation queue of each group: fill, per stage of the round (entries pushed by
+    // the first and by the second selection pass; the second stage's reuse the storage of
+    // the first, which has been consumed by then),
+    int n_esc[2][NGROUPS];
     int esc_cap[NGROUPS];        //   capacity (the group's pool slots)
     long long esc_beg[NGROUPS];  //   and first entry in Pool::esc
     unsigned long long escalated;// statistics: regions re-evaluated in FP64
@@ -307,10 +312,10 @@ __host__ __device__ constexpr int ucache_fun(int kind, int term, int f, int k)
 }
 
 // Queue region `code` (local slot | whole-rule flag << 30) of integral i, group g, for
-// FP64 re-evaluation in this round.
-__device__ inline void push_esc(BatchHdr *H, const Pool &P, int g, int i, int code)
+// FP64 re-evaluation in stage `stage` of this round.
+__device__ inline void push_esc(BatchHdr *H, const Pool &P, int stage, int g, int i, int code)
 {
-    const int k = atomicAdd(&H->n_esc[g], 1);
+    const int k = atomicAdd(&H->n_esc[stage][g], 1);
     if (k < H->esc_cap[g]) P.esc[H->esc_beg[g] + k] = make_int2(i, code);
     if (code >> 30) atomicAdd(&H->esc_full, 1ull);
 }
@@ -457,6 +462,41 @@ __device__ inline void aux_tables(const uint32_t *sdesc, uint8_t *auxrep, uint8_
     for (int a = 0; a < aux_nfun(TERM); ++a)
         proj_tables(sdesc, NP, aux_keep(TERM, a), auxrep + a * NP, auxlist + aux_off(TERM, a),
                     aux_count(TERM, a), tmp);
+}
+
+// Point tables of a group's kernels: the point codes, the (l, m, z)
+// combinations of the cached u_NFW (ucache_tables) and the projections of the k3 u_NFW
+// (u3_tables) and of the auxiliary functions (aux_tables).  The same for every launch, so
+// k_re_tables builds them once per context into P.retab and each block copies what it needs
+// to shared memory (building them per block cost more than the cached work saves).
+// The members up to ucidx are all that the FP32 rule kernels read.
+template <int KIND, int TERM>
+struct ReTab {
+    static constexpr int DIM = TERM + 4, NP = rule_points(DIM), NF = ucache_nf(TERM);
+    static constexpr int NU3 = u3_nfun(TERM), NA = aux_nfun(TERM);
+    uint32_t sdesc[NP];
+    int ucn[NF];
+    uint16_t ucl[NF * UC_MAX];
+    uint8_t ucidx[NF * NP];
+    uint8_t u3rep[NU3 * NP];
+    uint8_t u3list[NU3 * U3_MAX];
+    uint8_t auxrep[NA * NP];
+    uint8_t auxlist[AUX_MAX];
+};
+
+// copy group (KIND, TERM)'s tables to shared memory buf (every thread calls it)
+// (its first `bytes` bytes)
+template <int KIND, int TERM>
+__device__ inline const ReTab<KIND, TERM> &load_retab(const Pool &P, unsigned char *buf,
+                                                      int bytes = (int)sizeof(ReTab<KIND, TERM>))
+{
+    using RT = ReTab<KIND, TERM>;
+    const uint32_t *src =
+        reinterpret_cast<const uint32_t *>(P.retab + (KIND * 3 + TERM - 1) * RETAB_BYTES);
+    for (int i = threadIdx.x; i < (bytes + 3) / 4; i += blockDim.x)
+        reinterpret_cast<uint32_t *>(buf)[i] = __ldg(src + i);
+    __syncthreads();
+    return *reinterpret_cast<const RT *>(buf);
 }
 
 }  // namespace g3l

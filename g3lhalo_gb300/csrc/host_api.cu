@@ -36,7 +36,6 @@ void *eval64_kernel(int kind, int term);
 void *reeval64_kernel(int kind, int term);
 void *reeval_phase_kernel(int kind, int term, int phase);
 cudaError_t build_reeval_tables(unsigned char *out, cudaStream_t s);
-void *round_end_kernel();
 void *evalmx_kernel_k0(int term, int variant);
 void *evalmx_kernel_k1(int term, int variant);
 inline void *evalmx_kernel(int kind, int term, int variant = 0)
@@ -79,8 +78,8 @@ int dalloc(T **p, size_t n)
 }
 
 // FP64 re-evaluation entries per group and round that take the device-wide passes
-// (10.0 kB of scratch each): 4 per integral, between 8192 (82 MB per group) and 524288
-// (5.2 GB per group); further entries take the batched kernel k_reeval64, which
+// (7.9 kB of scratch each): 4 per integral, between 8192 (65 MB per group) and 524288
+// (4.2 GB per group); further entries take the batched kernel k_reeval64, which
 // evaluates every point on its own.  G3L_REEVAL_CAP=<n> (read when a workspace is
 // allocated) sets the count instead: 0 sends every entry through the batched kernel, so
 // that tests can hold the passes' cached values against it.
@@ -418,13 +417,6 @@ int grid128(g3l_ctx *c, void *fn)
     return nb * c->nsm;
 }
 
-int reeval_grid(g3l_ctx *c, void *fn)
-{
-    int nb = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, fn, 128, 0) != cudaSuccess || nb < 1) nb = 1;
-    return nb * c->nsm;
-}
-
 struct KernelArgs {
     DevTables T;
     IntDesc *D;
@@ -436,9 +428,7 @@ struct KernelArgs {
     int use_cond;
     double tau_sel;
     double tau_val;
-    int pass0 = 0, pass1 = 1;
-    int all_groups = -1;
-    int grp_id[NGROUPS] = {0, 1, 2, 3, 4, 5};
+    int pass0 = 0, pass1 = 1;  // selection passes and the re-evaluation stages behind them
 };
 
 int add_kernel(cudaGraph_t g, cudaGraphNode_t *node, const cudaGraphNode_t *deps, size_t ndeps,
@@ -503,44 +493,26 @@ int build_graph_ws(g3l_ctx *c, Workspace &W, int precision, int gmask, bool init
     cudaGraph_t body = cp.conditional.phGraph_out[0];
     cudaGraphNode_t n_sel, n_scan, prev;
     // mixed: FP64 re-evaluations queued by a selection pass (unsettled splits of the
-    // parents about to be cut, ambiguous boundary regions, polish), then the round end
-    // (one branch per group, side by side: each group reads only its own queue).  With
-    // ends != null each group's branch gets its own end node (ends[grp]) and dep is left
-    // as it is: the rule kernel of a group then waits for its own re-evaluations only.
-    auto add_reevals = [&](cudaGraphNode_t &dep, cudaGraphNode_t *ends) -> int {
-        cudaGraphNode_t br[2 * NGROUPS];
-        int nbr = 0;
+    // parents about to be cut, ambiguous boundary regions, polish), one branch per group,
+    // side by side: each group reads only its own queue.  ends[2 grp], ends[2 grp + 1]: the
+    // last nodes of group grp's branch.
+    auto add_reevals = [&](cudaGraphNode_t dep, int &stage, cudaGraphNode_t *ends) -> int {
         for (int grp = 0; grp < NGROUPS; ++grp) {
             if (!(gmask & (1 << grp))) continue;
-            const int nbr0 = nbr;
-            void *args[] = {&a.T, &a.D, &a.S, &a.P, &a.H, &a.woff};
+            void *args[] = {&a.T, &a.D, &a.S, &a.P, &a.H, &a.woff, &stage};
             cudaGraphNode_t chain = dep;
-            for (int ph = 0; ph < 4; ++ph) {
+            for (int ph = 0; ph < 3; ++ph) {
                 void *fn = reeval_phase_kernel(grp / 3, grp % 3 + 1, ph);
                 cudaGraphNode_t nd;
-                int st = add_kernel(body, &nd, &chain, 1, fn, ph == 3 ? c->nsm : grid128(c, fn), 128,
-                                    args);
+                int st = add_kernel(body, &nd, &chain, 1, fn, grid128(c, fn), 128, args);
                 if (st) return st;
                 chain = nd;
             }
-            br[nbr++] = chain;
-            void *fn = reeval_phase_kernel(grp / 3, grp % 3 + 1, 4);
-            int st = add_kernel(body, &br[nbr], &dep, 1, fn, reeval_grid(c, fn), 128, args);
+            ends[2 * grp] = chain;
+            void *fn = reeval_phase_kernel(grp / 3, grp % 3 + 1, 3);
+            int st = add_kernel(body, &ends[2 * grp + 1], &dep, 1, fn, grid128(c, fn), 128, args);
             if (st) return st;
-            ++nbr;
-            if (ends) {
-                void *eargs[] = {&a.H, &a.grp_id[grp]};
-                st = add_kernel(body, &ends[grp], &br[nbr0], 2, round_end_kernel(), 1, 1, eargs);
-                if (st) return st;
-            }
         }
-        if (ends) return G3L_OK;
-        void *args[] = {&a.H, &a.all_groups};
-        cudaGraphNode_t n_end;
-        int st = add_kernel(body, &n_end, nbr ? br : &dep, nbr ? nbr : 1, round_end_kernel(), 1,
-                            1, args);
-        if (st) return st;
-        dep = n_end;
         return G3L_OK;
     };
     {
@@ -549,12 +521,17 @@ int build_graph_ws(g3l_ctx *c, Workspace &W, int precision, int gmask, bool init
         if (st) return st;
     }
     prev = n_sel;
+    cudaGraphNode_t ends[2 * NGROUPS];
     if (precision == G3L_MIXED) {
-        int st = add_reevals(prev, nullptr);
+        int st = add_reevals(prev, a.pass0, ends);
         if (st) return st;
+        cudaGraphNode_t deps[2 * NGROUPS];
+        int nd = 0;
+        for (int grp = 0; grp < NGROUPS; ++grp)
+            for (int e = 0; e < 2 && (gmask & (1 << grp)); ++e) deps[nd++] = ends[2 * grp + e];
         void *args[] = {&a.D, &a.S, &a.P, &a.H, &a.tau_sel, &a.tau_val, &a.pass1};
         cudaGraphNode_t n_sel1;
-        st = add_kernel(body, &n_sel1, &prev, 1, select_kernel(), c->nsm * 8, 256, args);
+        st = add_kernel(body, &n_sel1, deps, nd, select_kernel(), c->nsm * 8, 256, args);
         if (st) return st;
         prev = n_sel1;
     }
@@ -564,9 +541,8 @@ int build_graph_ws(g3l_ctx *c, Workspace &W, int precision, int gmask, bool init
         if (st) return st;
     }
     prev = n_scan;
-    cudaGraphNode_t ends[NGROUPS];
     if (precision == G3L_MIXED) {
-        int st = add_reevals(prev, ends);
+        int st = add_reevals(prev, a.pass1, ends);
         if (st) return st;
     }
     // the groups' rule kernels in a chain, or side by side (kSideMaxMixed); a group's
@@ -576,10 +552,10 @@ int build_graph_ws(g3l_ctx *c, Workspace &W, int precision, int gmask, bool init
         if (!(gmask & (1 << grp))) continue;
         void *fn = eval_fn(c, precision, grp);
         void *args[] = {&a.T, &a.D, &a.S, &a.P, &a.H, &a.woff};
-        cudaGraphNode_t n_ev, deps[2];
+        cudaGraphNode_t n_ev, deps[3];
         int nd = 0;
         if (!side || precision != G3L_MIXED) deps[nd++] = prev;
-        if (precision == G3L_MIXED) deps[nd++] = ends[grp];
+        for (int e = 0; e < 2 && precision == G3L_MIXED; ++e) deps[nd++] = ends[2 * grp + e];
         int st = add_kernel(body, &n_ev, deps, nd, fn, eval_grid(c, fn), 128, args);
         if (st) return st;
         if (!side) prev = n_ev;
@@ -655,22 +631,18 @@ int run_host_loop(g3l_ctx *c, int precision, int gmask, int *launches)
     c->stats.reeval_ms = 0;
     c->stats.select_ms = 0;
     float ms;
-    auto reevals = [&]() -> int {
+    auto reevals = [&](int &stage) -> int {
         G3L_CK(cudaEventRecord(c->tev[12], s));
         for (int grp = 0; grp < NGROUPS; ++grp) {
             if (!(gmask & (1 << grp))) continue;
-            void *args[] = {&a.T, &a.D, &a.S, &a.P, &a.H, &a.woff};
-            for (int ph = 0; ph < 5; ++ph) {
+            void *args[] = {&a.T, &a.D, &a.S, &a.P, &a.H, &a.woff, &stage};
+            for (int ph = 0; ph < 4; ++ph) {
                 void *fn = reeval_phase_kernel(grp / 3, grp % 3 + 1, ph);
-                const int grid = ph == 3 ? c->nsm : (ph == 4 ? reeval_grid(c, fn) : grid128(c, fn));
-                G3L_CK(cudaLaunchKernel(fn, dim3(grid), dim3(128), args, 0, s));
+                G3L_CK(cudaLaunchKernel(fn, dim3(grid128(c, fn)), dim3(128), args, 0, s));
                 ++*launches;
             }
         }
         G3L_CK(cudaEventRecord(c->tev[13], s));
-        void *eargs[] = {&a.H, &a.all_groups};
-        G3L_CK(cudaLaunchKernel(round_end_kernel(), dim3(1), dim3(1), eargs, 0, s));
-        ++*launches;
         G3L_CK(cudaEventSynchronize(c->tev[13]));
         cudaEventElapsedTime(&ms, c->tev[12], c->tev[13]);
         c->stats.reeval_ms += ms;
@@ -687,7 +659,7 @@ int run_host_loop(g3l_ctx *c, int precision, int gmask, int *launches)
         cudaEventElapsedTime(&ms, c->tev[14], c->tev[15]);
         c->stats.select_ms += ms;
         if (precision == G3L_MIXED) {
-            int st = reevals();
+            int st = reevals(a.pass0);
             if (st) return st;
             void *sargs1[] = {&a.D, &a.S, &a.P, &a.H, &a.tau_sel, &a.tau_val, &a.pass1};
             G3L_CK(cudaEventRecord(c->tev[14], s));
@@ -704,7 +676,7 @@ int run_host_loop(g3l_ctx *c, int precision, int gmask, int *launches)
         cudaEventElapsedTime(&ms, c->tev[14], c->tev[15]);
         c->stats.select_ms += ms;
         if (precision == G3L_MIXED) {
-            int st = reevals();
+            int st = reevals(a.pass1);
             if (st) return st;
         }
         for (int grp = 0; grp < NGROUPS; ++grp) {
@@ -1878,7 +1850,7 @@ try {
                                        : (uint64_t)(1 + (Hout.rounds_done + 1) *
                                                            (2 + ngroups +
                                                             (precision == G3L_MIXED
-                                                                 ? 2 * (ngroups + 1) + 1
+                                                                 ? 8 * ngroups + 1
                                                                  : 0)));
     sx.regions_evaluated = Hout.regions;
     sx.tie_fallbacks = Hout.ties;
@@ -2353,20 +2325,16 @@ int eval_static_locked(g3l_ctx *c, const g3l_integral *items, int n, int precisi
         ++launches;
     }
     int active = 1;
-    auto reevals = [&]() -> int {
+    auto reevals = [&](int &stage) -> int {
         for (int g = 0; g < NGROUPS; ++g) {
             if (!(gmask & (1 << g))) continue;
-            void *args[] = {&a.T, &a.D, &a.S, &a.P, &a.H, &a.woff};
-            for (int ph = 0; ph < 5; ++ph) {
+            void *args[] = {&a.T, &a.D, &a.S, &a.P, &a.H, &a.woff, &stage};
+            for (int ph = 0; ph < 4; ++ph) {
                 void *fn = reeval_phase_kernel(g / 3, g % 3 + 1, ph);
-                const int grid = ph == 3 ? c->nsm : (ph == 4 ? reeval_grid(c, fn) : grid128(c, fn));
-                G3L_CK(cudaLaunchKernel(fn, dim3(grid), dim3(128), args, 0, s));
+                G3L_CK(cudaLaunchKernel(fn, dim3(grid128(c, fn)), dim3(128), args, 0, s));
                 ++launches;
             }
         }
-        void *eargs[] = {&a.H, &a.all_groups};
-        G3L_CK(cudaLaunchKernel(round_end_kernel(), dim3(1), dim3(1), eargs, 0, s));
-        ++launches;
         return G3L_OK;
     };
     for (int r = 0; r < c->opt.max_rounds + 4 && active; ++r) {
@@ -2374,7 +2342,7 @@ int eval_static_locked(g3l_ctx *c, const g3l_integral *items, int n, int precisi
         G3L_CK(cudaLaunchKernel(select_kernel(), dim3(c->nsm * 8), dim3(256), sargs, 0, s));
         ++launches;
         if (precision == G3L_MIXED) {
-            if ((st = reevals())) return st;
+            if ((st = reevals(a.pass0))) return st;
             void *sargs1[] = {&a.D, &a.S, &a.P, &a.H, &a.tau_sel, &a.tau_val, &a.pass1};
             G3L_CK(cudaLaunchKernel(select_kernel(), dim3(c->nsm * 8), dim3(256), sargs1, 0, s));
             ++launches;
@@ -2383,7 +2351,7 @@ int eval_static_locked(g3l_ctx *c, const g3l_integral *items, int n, int precisi
         G3L_CK(cudaLaunchKernel(scan_kernel(), dim3(1), dim3(1024), cargs, 0, s));
         ++launches;
         if (precision == G3L_MIXED)
-            if ((st = reevals())) return st;
+            if ((st = reevals(a.pass1))) return st;
         for (int g = 0; g < NGROUPS; ++g) {
             if (!(gmask & (1 << g))) continue;
             void *fn = eval_fn(c, precision, g);

@@ -239,4 +239,13 @@ __device__ __forceinline__ void m_index(const DevTables &T, double x, double m, 
     if (ties) atomicAdd(ties, 1ull);
 }
 
+// the same from x alone (m = 10^x is formed only where the reference expression is needed)
+__device__ __forceinline__ void m_index_x(const DevTables &T, double x, int &ir, int &it)
+{
+    const double a = (x - T.m_x0) * T.m_scale;
+    const double fr = a - floor(a);
+    const bool edge = !(fabs(fr - 0.5) > 1e-9 && fr > 1e-9 && fr < 1 - 1e-9);
+    m_index(T, x, edge ? pow(10, x) : 0.0, ir, it, nullptr);
+}
+
 }  // namespace g3l
