@@ -29,8 +29,6 @@
 //  * Rule sums, fourth differences and the 7th/5th-degree combination are
 //    double-float; the final value and error are formed in FP64 by four lanes
 //    at once.
-#include <cstddef>
-
 #include "dfloat.cuh"
 #include "g3l_device.cuh"
 #include "phys64.cuh"
@@ -523,63 +521,83 @@ struct ModelF {
     // (l, m, z) variant combination of a work item (ucached) and passed to point() in uc[].
     // {l dim, m dim, concentration factor: 0 = 1, 1 = f of hod1, 2 = f of hod2}
     static constexpr int NF = ucache_nf(TERM);
-    // cache the (l, m, z) u_NFW for every term (measured faster for all six)
-    static constexpr bool UC = true;
     __host__ __device__ static constexpr int ufun(int f, int k)
     {
         return ucache_fun(KIND, TERM, f, k);
     }
 
-    // the cached u_NFW f at slots L (l), M (mass), Z (z), with the expressions of point()
-    __device__ static float ucached(const DevTables &T, const IntDesc &d, int f, const SlotF &L,
-                                    const SlotF &M, const SlotF &Z, int &small)
+    // Operands kr, c of the shared u_NFW (u_nfw32).  f-th of the (l, m, z) ones, at slots
+    // L (l), M (mass), Z (z):
+    __device__ static void ucached_args(const DevTables &T, const IntDesc &d, int f, const SlotF &L,
+                                        const SlotF &M, const SlotF &Z, float &kr, float &c)
     {
         const float kx = L.f[0] * Z.f[1];
         const float r = cbrtf(M.f[0] * Z.f[2]);
         const float cc = __ldg(T.f_conc + Z.i1 * T.Nm + M.i1);
         const int fs = ufun(f, 2);
-        const float fac = fs == 0 ? cc : (fs == 1 ? T.f_hodp[8 * d.hod1] : T.f_hodp[8 * d.hod2]) * cc;
-        return u_nfw32(kx * r, fac, T.small_arg, small);
+        c = fs == 0 ? cc : (fs == 1 ? T.f_hodp[8 * d.hod1] : T.f_hodp[8 * d.hod2]) * cc;
+        kr = kx * r;
     }
 
-    __device__ static float point(const DevTables &T, const IntDesc &d, const SlotF *const *s,
-                                  const Child &C, int ch, int sdim, uint32_t vv, unsigned &ties,
-                                  int &small, const float *uc)
+    // l3 = |l1 + l2| in the cancellation-free form
+    __device__ static float l3_of(const SlotF &L1, const SlotF &L2, const SlotF &PH)
     {
-        const SlotF &L1 = *s[0], &L2 = *s[1], &PH = *s[2], &Z = *s[DIM - 1];
-        const float l1 = L1.f[0], l2 = L2.f[0], cphi = PH.f[0];
+        const float l1 = L1.f[0], l2 = L2.f[0];
         const float dl = l1 - l2;
-        const float l3 = sqrtf(fmaf(dl, dl, 2.f * l1 * l2 * PH.f[1]));
-        const float U3 = aperture32(d.th_s[2] * l3);
-        const float kw = Z.f[1], k200 = Z.f[2];
-        const int zr = Z.i0, zt = Z.i1, Nm = T.Nm;
-        const float k1 = l1 * kw, k2 = l2 * kw, k3 = l3 * kw;
+        return sqrtf(fmaf(dl, dl, 2.f * l1 * l2 * PH.f[1]));
+    }
+
+    // u_NFW at k3, mass dimension u3_mass(f): shared by the points of one projection (u3_drop)
+    __device__ static void u3_args(const DevTables &T, int f, const SlotF *const *s, float &kr, float &c)
+    {
+        const SlotF &Z = *s[DIM - 1], &M = *s[u3_mass(KIND, TERM, f)];
+        const float k3 = l3_of(*s[0], *s[1], *s[2]) * Z.f[1];
+        const float r = cbrtf(M.f[0] * Z.f[2]);
+        c = __ldg(T.f_conc + Z.i1 * T.Nm + M.i1);
+        kr = k3 * r;
+    }
+
+    // auxiliary function a (aux_dims): the aperture filter of l3; P_lin at k1, k2, k3
+    // (2-halo); the tree-level bispectrum (3-halo)
+    __device__ static float aux(const DevTables &T, const IntDesc &d, int a, const SlotF *const *s,
+                                const Child &C, int ch, int sdim, uint32_t vv, unsigned &ties)
+    {
+        const SlotF &L1 = *s[0], &L2 = *s[1], &PH = *s[2];
+        if (TERM == 1 || a == 0) return aperture32(d.th_s[2] * l3_of(L1, L2, PH));
+        const SlotF &Z = *s[DIM - 1];
+        const float kw = Z.f[1];
+        const int zr = Z.i0;
+        if (TERM == 2 && a < 3) {  // k1, k2: one copy of the index code
+            const SlotF &L = a == 1 ? L1 : L2;
+            const int kx = kidx_l(T, d, C, ch, sdim, vv, a - 1, L, zr, ties);
+            return plin32(T, zr, kx, L.f[0] * kw);
+        }
+        const float k3 = l3_of(L1, L2, PH) * kw;
+        if (TERM == 2) return plin32(T, zr, kidx_k3(T, d, C, ch, sdim, vv, zr, k3, false, ties), k3);
+        return bi32(T, d, C, ch, sdim, vv, zr, L1.f[0] * kw, L2.f[0] * kw, k3, PH.f[0], L1, L2, ties);
+    }
+
+    // Integrand at one point from its variant slots, its shared u_NFW (uc, u3c) and its
+    // auxiliary values (ax)
+    __device__ static float point(const DevTables &T, const SlotF *const *s, const float *uc,
+                                  const float *u3c, const float *ax)
+    {
+        const SlotF &L1 = *s[0], &L2 = *s[1], &Z = *s[DIM - 1];
+        const float U3 = ax[0];
+        const int zr = Z.i0, Nm = T.Nm;
         const float A12 = L1.f[1] * L2.f[1];
-        const float sa = T.small_arg;
         if (KIND == 0) {
-            const float f1 = T.f_hodp[8 * d.hod1], f2 = T.f_hodp[8 * d.hod2];
             if (TERM == 1) {
                 const SlotF &M = *s[3];
-                const float r2 = cbrtf(M.f[0] * k200);
-                const float cc = __ldg(T.f_conc + zt * Nm + M.i1);
-                const float u3 = u_nfw32(k3 * r2, cc, sa, small);
-                const float u1 = uc[0];
-                const float u2 = uc[1];
+                const float u3 = u3c[0], u1 = uc[0], u2 = uc[1];
                 const float H = __ldg(T.f_hmf + zr * Nm + M.i0);
                 const float Ggg = M.f[1] * M.f[4] * u2 + M.f[3] * M.f[2] * u1 + M.f[5] * u1 * u2;
                 return A12 * U3 * Z.f[0] * (H * M.f[0] * M.f[0]) * u3 * Ggg;
             } else if (TERM == 2) {
                 const SlotF &M1 = *s[3], &M2 = *s[4];
-                const int kx3 = kidx_k3(T, d, C, ch, sdim, vv, zr, k3, false, ties);
-                float P1, P2;
-                plin_l12(T, d, C, ch, sdim, vv, L1, L2, zr, k1, k2, ties, P1, P2);
-                const float P3 = plin32(T, zr, kx3, k3);
-                float u3_1, u3_2;
-                u3_pair(T, M1, M2, k3, k200, zt, small, u3_1, u3_2);
-                const float u1_1 = uc[0];
-                const float u2_1 = uc[1];
-                const float u1_2 = uc[2];
-                const float u2_2 = uc[3];
+                const float P1 = ax[1], P2 = ax[2], P3 = ax[3];
+                const float u3_1 = u3c[0], u3_2 = u3c[1];
+                const float u1_1 = uc[0], u2_1 = uc[1], u1_2 = uc[2], u2_2 = uc[3];
                 const float Ggg = M2.f[1] * M2.f[4] * u2_2 + M2.f[3] * M2.f[2] * u1_2 +
                                   M2.f[5] * u1_2 * u2_2;
                 const float G11 = M1.f[1] + M1.f[2] * u1_1, G22 = M2.f[3] + M2.f[4] * u2_2;
@@ -593,11 +611,9 @@ struct ModelF {
             } else {
                 const SlotF &M1 = *s[3], &M2 = *s[4], &M3 = *s[5];
                 const float m1 = M1.f[0], m2 = M2.f[0], m3 = M3.f[0];
-                const float u3 = u_nfw32(k3 * cbrtf(m3 * k200), __ldg(T.f_conc + zt * Nm + M3.i1), sa, small);
-                const float u1 = UC ? uc[0] : u_nfw32(k1 * cbrtf(m1 * k200), f1 * __ldg(T.f_conc + zt * Nm + M1.i1), sa, small);
-                const float u2 = UC ? uc[1] : u_nfw32(k2 * cbrtf(m2 * k200), f2 * __ldg(T.f_conc + zt * Nm + M2.i1), sa, small);
+                const float u3 = u3c[0], u1 = uc[0], u2 = uc[1];
                 const float G1 = M1.f[1] + M1.f[2] * u1, G2 = M2.f[3] + M2.f[4] * u2;
-                const float Bi = bi32(T, d, C, ch, sdim, vv, zr, k1, k2, k3, cphi, L1, L2, ties);
+                const float Bi = ax[1];
                 const float HB = (__ldg(T.f_hmf + zr * Nm + M1.i0) * m1) *
                                  (__ldg(T.f_hmf + zr * Nm + M2.i0) * m2) *
                                  (__ldg(T.f_hmf + zr * Nm + M3.i0) * m3 * m3) *
@@ -606,28 +622,17 @@ struct ModelF {
                 return A12 * U3 * Z.f[0] * HB * u3 * G1 * G2 * Bi;
             }
         } else {
-            const float f = T.f_hodp[8 * d.hod1];
             if (TERM == 1) {
                 const SlotF &M = *s[3];
-                const float r2 = cbrtf(M.f[0] * k200);
-                const float cc = __ldg(T.f_conc + zt * Nm + M.i1);
                 const float m = M.f[0];
                 const float G = M.f[1] + M.f[2] * uc[0];
-                const float u2 = uc[1];
-                const float u3 = u_nfw32(k3 * r2, cc, sa, small);
+                const float u2 = uc[1], u3 = u3c[0];
                 return A12 * U3 * Z.f[0] * (__ldg(T.f_hmf + zr * Nm + M.i0) * m * m * m) * G * u2 * u3;
             } else if (TERM == 2) {
                 const SlotF &M1 = *s[3], &M2 = *s[4];
-                const int kx3 = kidx_k3(T, d, C, ch, sdim, vv, zr, k3, false, ties);
-                float P1, P2;
-                plin_l12(T, d, C, ch, sdim, vv, L1, L2, zr, k1, k2, ties, P1, P2);
-                const float P3 = plin32(T, zr, kx3, k3);
-                float u3_1, u3_2;
-                u3_pair(T, M1, M2, k3, k200, zt, small, u3_1, u3_2);
-                const float u2_1 = uc[0];
-                const float u1_2f = uc[1];
-                const float u2_2 = uc[2];
-                const float u1_1f = uc[3];
+                const float P1 = ax[1], P2 = ax[2], P3 = ax[3];
+                const float u3_1 = u3c[0], u3_2 = u3c[1];
+                const float u2_1 = uc[0], u1_2f = uc[1], u2_2 = uc[2], u1_1f = uc[3];
                 const float G2 = M2.f[1] + M2.f[2] * u1_2f, G1 = M1.f[1] + M1.f[2] * u1_1f;
                 const float m1 = M1.f[0], m2 = M2.f[0];
                 const float HB = (__ldg(T.f_hmf + zr * Nm + M1.i0) * m1) *
@@ -639,13 +644,9 @@ struct ModelF {
             } else {
                 const SlotF &M1 = *s[3], &M2 = *s[4], &M3 = *s[5];
                 const float m1 = M1.f[0], m2 = M2.f[0], m3 = M3.f[0];
-                const float ra = cbrtf(m1 * k200), rb = cbrtf(m2 * k200);
-                const float ca = __ldg(T.f_conc + zt * Nm + M1.i1);
-                const float cb = __ldg(T.f_conc + zt * Nm + M2.i1);
-                const float u2_1 = UC ? uc[0] : u_nfw32(k2 * ra, ca, sa, small);
-                const float u3_2 = u_nfw32(k3 * rb, cb, sa, small);
-                const float G = M3.f[1] + M3.f[2] * (UC ? uc[1] : u_nfw32(k1 * rb, f * cb, sa, small));
-                const float Bi = bi32(T, d, C, ch, sdim, vv, zr, k1, k2, k3, cphi, L1, L2, ties);
+                const float u2_1 = uc[0], u3_2 = u3c[0];
+                const float G = M3.f[1] + M3.f[2] * uc[1];
+                const float Bi = ax[1];
                 const float HB = (__ldg(T.f_hmf + zr * Nm + M1.i0) * m1 * m1) *
                                  (__ldg(T.f_hmf + zr * Nm + M2.i0) * m2 * m2) *
                                  (__ldg(T.f_hmf + zr * Nm + M3.i0) * m3) *
@@ -673,25 +674,6 @@ struct ModelF {
         }
         P1 = P[0];
         P2 = P[1];
-    }
-
-    // u_NFW(k3 r_200(m_a), c(m_a)) for the two masses of a 2-halo point, through one call
-    // site (a single copy of u_nfw32 in the kernel's hot loop)
-    __device__ static void u3_pair(const DevTables &T, const SlotF &M1, const SlotF &M2,
-                                   float k3, float k200, int zt, int &small, float &u1, float &u2)
-    {
-        float u[2];
-#pragma unroll 1
-        for (int q = 0; q < 2; ++q) {
-            const SlotF &M = q ? M2 : M1;
-            const float r = cbrtf(M.f[0] * k200);
-            const float c = __ldg(T.f_conc + zt * T.Nm + M.i1);
-            const float v = u_nfw32(k3 * r, c, T.small_arg, small);
-            if (q == 0) u[0] = v;
-            else u[1] = v;
-        }
-        u1 = u[0];
-        u2 = u[1];
     }
 
     // tree-level bispectrum (src/generalFunctions.cu:94-147), scaled by the P_lin scale^2;
@@ -748,6 +730,21 @@ __device__ __forceinline__ df hw_sum(df a)
 // integral (default 0: always); the selection kernel has it re-taken in FP64 if the
 // region is cut.  The error estimate's bound (unc) decides selection boundaries.
 
+// Shared memory of one work item.  Child 1 has its own copy of a cached function only when
+// the split dimension is among the function's dimensions.
+template <int KIND, int TERM>
+struct ItemF {
+    static constexpr int DIM = TERM + 4, NP = rule_points(DIM), NF = ucache_nf(TERM);
+    static constexpr int NU3 = u3_nfun(TERM), NA = aux_nfun(TERM);
+    static constexpr int NAUX = aux_off(TERM, NA - 1) + aux_count(TERM, NA - 1);
+    SlotF slots[(DIM + 1) * NVAR];
+    Child child;
+    float uc[2][NF][UC_MAX];
+    float u3[2][NU3][U3_MAX];
+    float aux[2][NAUX];
+    float vals[2 * NP];
+};
+
 // Threads that share one work item: a warp, or the whole block of 128.
 struct Group {
     int size, rank;
@@ -761,11 +758,15 @@ struct Group {
 template <int KIND, int TERM>
 __device__ void group_itemF(const Group &gr, const DevTables &T, const IntDesc &d, int iint,
                             double Vcur, const Pool &P, BatchHdr *H, long long pslot,
-                            long long qslot, bool cut, SlotF *slots, float *vals, Child &C,
-                            const uint32_t *sdesc, unsigned &ties, int &small,
-                            const uint8_t *ucidx, const uint16_t *ucl, const int *ucn,
-                            float *ucache)
+                            long long qslot, bool cut, ItemF<KIND, TERM> &I,
+                            const ReTab<KIND, TERM> &tb, unsigned &ties, int &small)
 {
+    using M = ModelF<KIND, TERM>;
+    using It = ItemF<KIND, TERM>;
+    constexpr int NF = It::NF, NU3 = It::NU3, NA = It::NA, ZD = It::DIM - 1;
+    SlotF *slots = I.slots;
+    float *vals = I.vals;
+    Child &C = I.child;
     constexpr int DIM = TERM + 4;
     constexpr int NP = rule_points(DIM);
     constexpr int NRR = 2 * DIM * (DIM - 1);
@@ -814,39 +815,103 @@ __device__ void group_itemF(const Group &gr, const DevTables &T, const IntDesc &
         ModelF<KIND, TERM>::fill(T, d, C, sd, dim, v, x, slots[t], ties);
     }
     gr.sync();
-    // u_NFW of the (l, m, z) variant combinations the points share, per child
-    constexpr int NF = ModelF<KIND, TERM>::NF;
-    for (int t = gr.rank; ModelF<KIND, TERM>::UC && t < nchild * NF * UC_MAX; t += gr.size) {
-        const int ch = t / (NF * UC_MAX), r = t - ch * NF * UC_MAX;
-        const int f = r / UC_MAX, j = r - f * UC_MAX;
-        if (j >= ucn[f]) continue;
-        const uint32_t key = ucl[f * UC_MAX + j];
-        const int dl = ModelF<KIND, TERM>::ufun(f, 0), dm = ModelF<KIND, TERM>::ufun(f, 1);
-        const int vl = key & 7, vm = (key >> 3) & 7, vz = (key >> 6) & 7;
-        auto sl = [&](int dim, int v) -> const SlotF & {
-            return (ch && dim == sdim) ? slots[DIM * NVAR + v] : slots[dim * NVAR + v];
-        };
-        ucache[(ch * NF + f) * UC_MAX + j] =
-            ModelF<KIND, TERM>::ucached(T, d, f, sl(dl, vl), sl(dm, vm), sl(DIM - 1, vz), small);
+    // does child 1 need its own values of a function of the dimensions dims?
+    auto own = [&](uint32_t dims) { return cut && ((dims >> sdim) & 1u); };
+    auto slot = [&](int ch, int dim, int v) -> const SlotF & {
+        return slots[((ch && dim == sdim) ? DIM : dim) * NVAR + v];
+    };
+    // What several points share, once per projection of the points onto the dimensions it
+    // depends on: u_NFW of the (l, m, z) combinations and at k3 ...
+    {
+        int nu[NF], n3[NU3], tot = 0;
+#pragma unroll
+        for (int f = 0; f < NF; ++f) {
+            nu[f] = tb.ucn[f] * (own((1u << M::ufun(f, 0)) | (1u << M::ufun(f, 1)) | (1u << ZD)) ? 2 : 1);
+            tot += nu[f];
+        }
+#pragma unroll
+        for (int f = 0; f < NU3; ++f) {
+            n3[f] = U3_MAX * (own(7u | (1u << u3_mass(KIND, TERM, f)) | (1u << ZD)) ? 2 : 1);
+            tot += n3[f];
+        }
+        for (int t0 = gr.rank; t0 < tot; t0 += gr.size) {
+            int t = t0, f = 0;
+#pragma unroll
+            for (int q = 0; q < NF; ++q)
+                if (f == q && t >= nu[q]) {
+                    t -= nu[q];
+                    ++f;
+                }
+            float kr, c, *out;
+            if (f < NF) {
+                const int n = tb.ucn[f], ch = t >= n, j = t - ch * n;
+                const uint32_t key = tb.ucl[f * UC_MAX + j];
+                M::ucached_args(T, d, f, slot(ch, M::ufun(f, 0), key & 7),
+                                slot(ch, M::ufun(f, 1), (key >> 3) & 7), slot(ch, ZD, (key >> 6) & 7), kr, c);
+                out = &I.uc[ch][f][j];
+            } else {
+                f = 0;
+                if (NU3 == 2 && t >= n3[0]) {
+                    t -= n3[0];
+                    f = 1;
+                }
+                const int ch = t >= U3_MAX, j = t - ch * U3_MAX;
+                const uint32_t vv = tb.sdesc[tb.u3list[f * U3_MAX + j]];
+                const SlotF *sp[DIM];
+#pragma unroll
+                for (int dd = 0; dd < DIM; ++dd) sp[dd] = &slot(ch, dd, (vv >> (3 * dd)) & 7);
+                M::u3_args(T, f, sp, kr, c);
+                out = &I.u3[ch][f][j];
+            }
+            *out = u_nfw32(kr, c, T.small_arg, small);
+        }
+    }
+    // ... and the auxiliary functions
+    {
+        int nax[NA], tot = 0;
+#pragma unroll
+        for (int a = 0; a < NA; ++a) {
+            nax[a] = aux_count(TERM, a) * (own(aux_dims(TERM, a)) ? 2 : 1);
+            tot += nax[a];
+        }
+        for (int t0 = gr.rank; t0 < tot; t0 += gr.size) {
+            int t = t0, a = 0;
+#pragma unroll
+            for (int q = 0; q < NA - 1; ++q)
+                if (a == q && t >= nax[q]) {
+                    t -= nax[q];
+                    ++a;
+                }
+            const int na = aux_count(TERM, a);
+            const int ch = t >= na, j = t - ch * na;
+            const uint32_t vv = tb.sdesc[tb.auxlist[aux_off(TERM, a) + j]];
+            const SlotF *sp[DIM];
+#pragma unroll
+            for (int dd = 0; dd < DIM; ++dd) sp[dd] = &slot(ch, dd, (vv >> (3 * dd)) & 7);
+            I.aux[ch][aux_off(TERM, a) + j] = M::aux(T, d, a, sp, C, ch, sdim, vv, ties);
+        }
     }
     gr.sync();
     // points
     for (int p = gr.rank; p < nchild * NP; p += gr.size) {
         const int ch = p >= NP ? 1 : 0;
         const int pp = p - ch * NP;
-        const uint32_t vv = sdesc[pp];
+        const uint32_t vv = tb.sdesc[pp];
         const SlotF *sp[DIM];
 #pragma unroll
-        for (int dd = 0; dd < DIM; ++dd) {
-            const int v = (vv >> (3 * dd)) & 7;
-            sp[dd] = (ch && dd == sdim) ? &slots[DIM * NVAR + v] : &slots[dd * NVAR + v];
-        }
-        float uc[NF] = {};
-        if (ModelF<KIND, TERM>::UC) {
+        for (int dd = 0; dd < DIM; ++dd) sp[dd] = &slot(ch, dd, (vv >> (3 * dd)) & 7);
+        float uc[NF], u3c[NU3], ax[NA];
 #pragma unroll
-            for (int f = 0; f < NF; ++f) uc[f] = ucache[(ch * NF + f) * UC_MAX + ucidx[f * NP + pp]];
-        }
-        vals[p] = ModelF<KIND, TERM>::point(T, d, sp, C, ch, sdim, vv, ties, small, uc);
+        for (int f = 0; f < NF; ++f)
+            uc[f] = I.uc[ch && own((1u << M::ufun(f, 0)) | (1u << M::ufun(f, 1)) | (1u << ZD))][f]
+                        [tb.ucidx[f * NP + pp]];
+#pragma unroll
+        for (int f = 0; f < NU3; ++f)
+            u3c[f] = I.u3[ch && own(7u | (1u << u3_mass(KIND, TERM, f)) | (1u << ZD))][f][tb.u3rep[f * NP + pp]];
+#pragma unroll
+        for (int a = 0; a < NA; ++a)
+            ax[a] = I.aux[ch && own(aux_dims(TERM, a))][aux_off(TERM, a) + tb.auxrep[a * NP + pp]];
+        vals[p] = M::point(T, sp, uc, u3c, ax);
         if (H->dbg) H->dbg[p] = (double)vals[p];
     }
     gr.sync();
@@ -997,19 +1062,10 @@ __global__ void __launch_bounds__(128, MINB) k_evalmx(DevTables T, const IntDesc
                                                 IntState *__restrict__ S, Pool P, BatchHdr *H,
                                                 const long long *__restrict__ woff)
 {
-    constexpr int DIM = TERM + 4;
-    constexpr int NP = rule_points(DIM);
-    constexpr int NSLOT = (DIM + 1) * NVAR;
     constexpr int WPB = 4;
-    // the point codes and the tables of the shared u_NFW (the head of the group's ReTab)
     using RT = ReTab<KIND, TERM>;
-    constexpr int TAB = (int)offsetof(RT, u3rep);
-    __shared__ __align__(16) unsigned char tbuf[(TAB + 3) / 4 * 4];
-    __shared__ SlotF sslot[WPB][NSLOT];
-    __shared__ float svals[WPB][2 * NP];
-    __shared__ Child schild[WPB];
-    constexpr int NF = ModelF<KIND, TERM>::NF;
-    __shared__ float ucache[WPB][2 * NF * UC_MAX];
+    __shared__ __align__(16) unsigned char tbuf[sizeof(RT)];
+    __shared__ ItemF<KIND, TERM> items[WPB];
     const int g = KIND * 3 + TERM - 1;
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
     const int gb = H->gbeg[g], ge = H->gbeg[g + 1];
@@ -1026,11 +1082,7 @@ __global__ void __launch_bounds__(128, MINB) k_evalmx(DevTables T, const IntDesc
     const int buf = wide ? 0 : wib;
     const long long first = wide ? blockIdx.x : (long long)blockIdx.x * WPB + wib;
     if (wbeg + (wide ? (long long)blockIdx.x : (long long)blockIdx.x * WPB) >= wend) return;  // no work here
-    const RT &tb = load_retab<KIND, TERM>(P, tbuf, TAB);
-    const uint32_t *sdesc = tb.sdesc;
-    const uint8_t *ucidx = tb.ucidx;
-    const uint16_t *ucl = tb.ucl;
-    const int *ucn = tb.ucn;
+    const RT &tb = load_retab<KIND, TERM>(P, tbuf);
     const long long step = (long long)gridDim.x * (wide ? 1 : WPB);
     for (long long w = wbeg + first; w < wend; w += step) {
         int lo = gb, hi = ge - 1;
@@ -1046,9 +1098,8 @@ __global__ void __launch_bounds__(128, MINB) k_evalmx(DevTables T, const IntDesc
         const bool cut = cj >= 0;
         const long long pslot = d.base + (cut ? cj : 0);
         const long long qslot = cut ? d.base + (S[i].nR - S[i].K) + j : -1;
-        group_itemF<KIND, TERM>(gr, T, d, i, S[i].val, P, H, pslot, qslot, cut, sslot[buf],
-                                svals[buf], schild[buf], sdesc, ties, small, ucidx, ucl, ucn,
-                                ucache[buf]);
+        group_itemF<KIND, TERM>(gr, T, d, i, S[i].val, P, H, pslot, qslot, cut, items[buf], tb, ties,
+                                small);
         gr.sync();
     }
     // warp-aggregated diagnostics
