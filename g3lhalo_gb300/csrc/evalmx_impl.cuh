@@ -190,16 +190,15 @@ static __device__ __noinline__ float u_nfw32(float kr, float c, float small_arg,
         ++small_hits;
         return u_nfw_small64(kr, c);
     }
-    float s1, c1, sk, ck;
-    sincosf(a1, &s1, &c1);
-    sincosf(kr, &sk, &ck);
-    // (a, b, e) of a1 and of a2: small form (Si, Ci polynomial, 0) below 4, else
-    // (f, g, f - 1/x)
+    // sin and cos of a1 and of kr; (a, b, e) of a1 and of a2: small form (Si, Ci polynomial,
+    // 0) below 4, else (f, g, f - 1/x)
+    float s1 = 0.f, c1 = 0.f, sk = 0.f, ck = 0.f;
     float a1a = 0.f, a1b = 0.f, a2a = 0.f, a2b = 0.f, a2e = 0.f;
 #pragma unroll 1
     for (int q = 0; q < 2; ++q) {
         const float x = q ? a2 : a1;
-        float a, b, e;
+        float a, b, e, sq, cq;
+        sincosf(q ? kr : a1, &sq, &cq);
         if (x < 4.f) {
             a = si_small(x);
             b = ci_small_poly(x);
@@ -208,30 +207,36 @@ static __device__ __noinline__ float u_nfw32(float kr, float c, float small_arg,
             fg_large(x, a, b, e);
         }
         if (q == 0) {
+            s1 = sq;
+            c1 = cq;
             a1a = a;
             a1b = b;
         } else {
+            sk = sq;
+            ck = cq;
             a2a = a;
             a2b = b;
             a2e = e;
         }
     }
+    // which product of a pair is fused is written out: left to the compiler it changes with
+    // the code around it, and with it the last bit
     float N;
     if (a2 < 4.f) {
         const float dS = a2a - a1a;
         const float dC = lnopc + (a2b - a1b);
-        N = s1 * dS + c1 * dC - __fdividef(sk, a2);
+        N = fmaf(s1, dS, c1 * dC) - __fdividef(sk, a2);
     } else if (a1 >= 4.f) {
         N = a1b - a2b * ck + a2e * sk;  // g(a1) - g(a2) cos(kr) + (f(a2) - 1/a2) sin(kr)
     } else {
         const float f2 = a2a, g2 = a2b;
-        const float s2 = s1 * ck + c1 * sk;  // sin(a1 + a1 c)
-        const float c2 = c1 * ck - s1 * sk;
+        const float s2 = fmaf(s1, ck, c1 * sk);  // sin(a1 + a1 c)
+        const float c2 = fmaf(c1, ck, -(s1 * sk));
         const float Si2 = HALF_PI_F - f2 * c2 - g2 * s2;
-        const float Ci2 = f2 * s2 - g2 * c2;
+        const float Ci2 = fmaf(f2, s2, -(g2 * c2));
         const float Si1 = a1a;
         const float Ci1 = GAMMA_F + __logf(a1) + a1b;
-        N = s1 * (Si2 - Si1) + c1 * (Ci2 - Ci1) - __fdividef(sk, a2);
+        N = fmaf(s1, Si2 - Si1, c1 * (Ci2 - Ci1)) - __fdividef(sk, a2);
     }
     return __fdividef(N, F);
 }
@@ -280,6 +285,16 @@ __device__ __forceinline__ bool tie_lookup(const unsigned long long *bits, const
     return false;
 }
 
+// One out-of-line copy of each library function that several places of a kernel use: the
+// rule kernels are bound by instruction fetch.
+static __device__ __noinline__ float exp10_32(float x) { return exp10f(x); }
+static __device__ __noinline__ float2 sincos_32(float x)
+{
+    float s, c;
+    sincosf(x, &s, &c);
+    return make_float2(s, c);
+}
+
 constexpr float IDX_TOL = 1e-7f;   // double-float index arguments
 constexpr float K3_TOL = 3e-5f;    // FP32 argument of the l3-based k index
 
@@ -326,13 +341,37 @@ __device__ __forceinline__ df ln_df(float v)
     return df_add_f(el, logf(m));
 }
 
+struct Child {
+    double c64[MAX_DIM + 1];  // FP64 centres: dims of child 0, then child 1's split dim
+    int lev[MAX_DIM + 1];
+};
+
+// exact FP64 coordinate of a variant (the reference's c -+ (h lambda))
+__device__ __forceinline__ double coord64(const IntDesc &d, const Child &C, int slotdim, int dim, int v)
+{
+    double c = C.c64[slotdim];
+    if (v == 0) return c;
+    double hw = ldexp(d.hw0[dim], -C.lev[slotdim]);
+    double lam = (v <= 2) ? G3L_LAMBDA2 : (v <= 4 ? G3L_LAMBDA4 : G3L_LAMBDA5);
+    double r = __dmul_rn(hw, lam);
+    return (v & 1) ? __dsub_rn(c, r) : __dadd_rn(c, r);
+}
+
+// FP64 coordinate dim of the point with code vv; own1: child 1's split dimension, else -1
+__device__ __forceinline__ double px64(const IntDesc &d, const Child &C, int own1, int dim, uint32_t vv)
+{
+    return coord64(d, C, dim == own1 ? d.dim : dim, dim, (vv >> (3 * dim)) & 7);
+}
+
 // Exact nearest-bin / truncated indices for arguments within IDX_TOL of a rounding
 // boundary: the tie table for the dyadic centre values (v == 0), else the reference's FP64
 // expression (src/NNMap_Model.cu:555-556, 796-799).  Out of line, like the k indices
 // below: they are rare, and their FP64 code would otherwise crowd the rule kernels'
 // instruction cache.  Return 1 when the FP64 expression was evaluated (counted).
-static __device__ __noinline__ int m_index_exact(const DevTables &T, double x64, int v, int &ir, int &it)
+static __device__ __noinline__ int m_index_exact(const DevTables &T, const IntDesc &d, const Child &C,
+                                                 int slotdim, int dim, int v, int &ir, int &it)
 {
+    const double x64 = coord64(d, C, slotdim, dim, v);
     if (v == 0 && tie_lookup(T.tie_m_bits, T.tie_m_round, T.tie_m_trunc, T.n_tie_m, x64, ir, it))
         return 0;
     double m = pow(10.0, x64);
@@ -342,8 +381,10 @@ static __device__ __noinline__ int m_index_exact(const DevTables &T, double x64,
     return 1;
 }
 
-static __device__ __noinline__ int z_index_exact(const DevTables &T, double x64, int v, int &ir, int &it)
+static __device__ __noinline__ int z_index_exact(const DevTables &T, const IntDesc &d, const Child &C,
+                                                 int slotdim, int dim, int v, int &ir, int &it)
 {
+    const double x64 = coord64(d, C, slotdim, dim, v);
     if (v == 0 && tie_lookup(T.tie_z_bits, T.tie_z_round, T.tie_z_trunc, T.n_tie_z, x64, ir, it))
         return 0;
     double zr = (x64 - T.zmin) * T.Nz / (T.zmax - T.zmin);
@@ -353,20 +394,21 @@ static __device__ __noinline__ int z_index_exact(const DevTables &T, double x64,
 }
 
 // the k index of k = 10^x / w(z), by the reference's expression
-static __device__ __noinline__ int kidx_l_exact(const DevTables &T, double x, int zr)
+static __device__ __noinline__ int kidx_l_exact(const DevTables &T, const IntDesc &d, const Child &C,
+                                                int own1, int dim, uint32_t vv, int zr)
 {
-    const double l = pow(10.0, x);
+    const double l = pow(10.0, px64(d, C, own1, dim, vv));
     return kix_exact64(T, l / T.w[zr]);
 }
 
 // the k index of k3 from the FP64 coordinates of l1, l2 and phi: |l1 + l2| / w
 // (src/NNMap_Model.cu:814-817), or the bispectrum's k3 from k1 = l1 / w, k2 = l2 / w
 // (src/generalFunctions.cu:99)
-static __device__ __noinline__ int kidx_k3_exact(const DevTables &T, double x1, double x2, double xphi,
-                                          int zr, bool from_k)
+static __device__ __noinline__ int kidx_k3_exact(const DevTables &T, const IntDesc &d, const Child &C,
+                                                 int own1, uint32_t vv, int zr, bool from_k)
 {
-    const double cph = cos(xphi);
-    double p1 = pow(10.0, x1), p2 = pow(10.0, x2);
+    const double cph = cos(px64(d, C, own1, 2, vv));
+    double p1 = pow(10.0, px64(d, C, own1, 0, vv)), p2 = pow(10.0, px64(d, C, own1, 1, vv));
     const double wz = T.w[zr];
     if (from_k) {
         p1 = p1 / wz;
@@ -380,52 +422,35 @@ static __device__ __noinline__ int kidx_k3_exact(const DevTables &T, double x1, 
 }
 
 // ------------------------------------------------------------------ per-term models
-struct Child {
-    double c64[MAX_DIM + 1];  // FP64 centres: dims of child 0, then child 1's split dim
-    int lev[MAX_DIM + 1];
-};
-
 template <int KIND, int TERM>
 struct ModelF {
     static constexpr int DIM = TERM + 4;
-
-    // exact FP64 coordinate of a variant (the reference's c -+ (h lambda))
-    __device__ static double coord64(const IntDesc &d, const Child &C, int slotdim, int dim, int v)
-    {
-        double c = C.c64[slotdim];
-        if (v == 0) return c;
-        double hw = ldexp(d.hw0[dim], -C.lev[slotdim]);
-        double lam = (v <= 2) ? G3L_LAMBDA2 : (v <= 4 ? G3L_LAMBDA4 : G3L_LAMBDA5);
-        double r = __dmul_rn(hw, lam);
-        return (v & 1) ? __dsub_rn(c, r) : __dadd_rn(c, r);
-    }
 
     __device__ static void fill(const DevTables &T, const IntDesc &d, const Child &C, int slotdim,
                                 int dim, int v, df x, SlotF &S, unsigned &ties)
     {
         if (dim < 2) {  // l1, l2: ls = 10^x / L0, A = ls^2 * U(theta l)
-            float ls = exp10f(x.hi) * fmaf(2.302585093f, x.lo, 1.f) * 1e-3f;
+            float ls = exp10_32(x.hi) * fmaf(2.302585093f, x.lo, 1.f) * 1e-3f;
             float U = aperture32(d.th_s[dim] * ls);
             S.f[0] = ls;
             S.f[1] = ls * ls * U;
             S.f[2] = x.hi;
             S.f[3] = x.lo;
         } else if (dim == 2) {  // phi: cos and 1 + cos = 2 cos^2(phi/2)
-            float s, c;
-            sincosf(x.hi, &s, &c);
+            const float2 sc = sincos_32(x.hi), sch = sincos_32(0.5f * x.hi);
+            const float s = sc.x, c = sc.y, sh = sch.x;
+            float ch = sch.y;
             S.f[0] = c - s * x.lo;
-            float sh, ch;
-            sincosf(0.5f * x.hi, &sh, &ch);
             ch = ch - sh * 0.5f * x.lo;
             S.f[1] = 2.f * ch * ch;
         } else if (dim < 3 + TERM) {  // halo mass (log10 m)
             int ir, it;
             df a = df_mul(df_add(x, df_neg({T.m_x02.x, T.m_x02.y})), {T.m_s2.x, T.m_s2.y});
             if (idx_df(a, T.Nm, IDX_TOL, ir, it))
-                ties += m_index_exact(T, coord64(d, C, slotdim, dim, v), v, ir, it);
+                ties += m_index_exact(T, d, C, slotdim, dim, v, ir, it);
             S.i0 = ir;
             S.i1 = it;
-            S.f[0] = exp10f(x.hi - 12.f) * fmaf(2.302585093f, x.lo, 1.f);  // m / 1e12
+            S.f[0] = exp10_32(x.hi - 12.f) * fmaf(2.302585093f, x.lo, 1.f);  // m / 1e12
             // occupations (src/HOD.cu:35-76) from log10 m; hodp = {f, alpha, log10 Mth (df),
             // ln10 / (sigma 1.414213562), log10 M' (df), beta}.  erfc keeps 1 + erf accurate
             // far below the threshold mass.
@@ -438,7 +463,7 @@ struct ModelF {
                 const float *h = T.f_hodp + 8 * (q ? d.hod2 : d.hod1);
                 const float e = erfcf(-((x.hi - h[2]) + (x.lo - h[3])) * h[4]);
                 const float nc = 0.5f * h[1] * e;
-                const float ns = 0.5f * e * exp10f(h[7] * ((x.hi - h[5]) + (x.lo - h[6])));
+                const float ns = 0.5f * e * exp10_32(h[7] * ((x.hi - h[5]) + (x.lo - h[6])));
                 if (q == 0) {
                     S.f[1] = nc;
                     S.f[2] = ns;
@@ -454,7 +479,7 @@ struct ModelF {
                     S.f[5] = (S.f[2] + __ldg(T.f_scale + d.hod1 * T.Nm + ir)) * S.f[2];
                 } else {
                     float n12 = S.f[2] * S.f[4];
-                    float r = n12 + T.fA * exp10f(T.feps * xm) * sqrtf(n12);
+                    float r = n12 + T.fA * exp10_32(T.feps * xm) * sqrtf(n12);
                     S.f[5] = r < 0.f ? 0.f : r;
                 }
             }
@@ -462,7 +487,7 @@ struct ModelF {
             int ir, it;
             df a = df_mul(df_add(x, df_neg({T.z_02.x, T.z_02.y})), {T.z_s2.x, T.z_s2.y});
             if (idx_df(a, T.Nz, IDX_TOL, ir, it))
-                ties += z_index_exact(T, coord64(d, C, slotdim, dim, v), v, ir, it);
+                ties += z_index_exact(T, d, C, slotdim, dim, v, ir, it);
             S.i0 = ir;
             S.i1 = it;
             const float opz = 1.f + (x.hi + x.lo);
@@ -479,15 +504,6 @@ struct ModelF {
         }
     }
 
-    // FP64 coordinate of point (for the rare exact k-index fallback)
-    __device__ static double px64(const IntDesc &d, const Child &C, int ch, int sdim, int dim,
-                                  uint32_t vv)
-    {
-        int v = (vv >> (3 * dim)) & 7;
-        int sd = (ch && dim == sdim) ? DIM : dim;
-        return coord64(d, C, sd, dim, v);
-    }
-
     // k index of k = l/w for the l coordinate of dimension dl, exact on a boundary
     __device__ static int kidx_l(const DevTables &T, const IntDesc &d, const Child &C, int ch,
                                  int sdim, uint32_t vv, int dl, const SlotF &L, int zr,
@@ -499,7 +515,7 @@ struct ModelF {
         int ix = round_df(a, IDX_TOL, near);
         if (!near) return ix;
         ++ties;
-        return kidx_l_exact(T, px64(d, C, ch, sdim, dl, vv), zr);
+        return kidx_l_exact(T, d, C, ch ? sdim : -1, dl, vv, zr);
     }
 
     // k index of k3 (|l1 + l2| / w, or from k1, k2 in the bispectrum), exact on a boundary
@@ -513,8 +529,7 @@ struct ModelF {
         int ix = round_df(a, K3_TOL, near);
         if (!near) return ix;
         ++ties;
-        return kidx_k3_exact(T, px64(d, C, ch, sdim, 0, vv), px64(d, C, ch, sdim, 1, vv),
-                             px64(d, C, ch, sdim, 2, vv), zr, from_k);
+        return kidx_k3_exact(T, d, C, ch ? sdim : -1, vv, zr, from_k);
     }
 
     // u_NFW calls that depend on one l, one mass and z only: evaluated once per distinct
@@ -716,13 +731,6 @@ __device__ __forceinline__ df shfl_xor_df(df a, int m, unsigned mask = 0xfffffff
     return {__shfl_xor_sync(mask, a.hi, m), __shfl_xor_sync(mask, a.lo, m)};
 }
 
-// half-warp (16-lane) reductions; lanes 0-15 serve child 0, 16-31 child 1
-__device__ __forceinline__ df hw_sum(df a)
-{
-    for (int m = 8; m > 0; m >>= 1) a = df_add(a, shfl_xor_df(a, m));
-    return a;
-}
-
 // The bound on the FP32 error of one point value has a relative part (the FP32
 // chain) and an absolute part (values so small that intermediate products may
 // have lost range): T.unc_eps |v| + T.unc_abs.  A split the bounds do not settle is
@@ -803,6 +811,7 @@ __device__ void group_itemF(const Group &gr, const DevTables &T, const IntDesc &
     gr.sync();
     // coordinate-variant slots
     const int nslot = (DIM + nchild - 1) * NVAR;
+#pragma unroll 1
     for (int t = gr.rank; t < nslot; t += gr.size) {
         const int sd = t / NVAR, v = t - sd * NVAR;
         const int dim = sd < DIM ? sd : sdim;
@@ -834,6 +843,7 @@ __device__ void group_itemF(const Group &gr, const DevTables &T, const IntDesc &
             n3[f] = U3_MAX * (own(7u | (1u << u3_mass(KIND, TERM, f)) | (1u << ZD)) ? 2 : 1);
             tot += n3[f];
         }
+#pragma unroll 1
         for (int t0 = gr.rank; t0 < tot; t0 += gr.size) {
             int t = t0, f = 0;
 #pragma unroll
@@ -874,6 +884,7 @@ __device__ void group_itemF(const Group &gr, const DevTables &T, const IntDesc &
             nax[a] = aux_count(TERM, a) * (own(aux_dims(TERM, a)) ? 2 : 1);
             tot += nax[a];
         }
+#pragma unroll 1
         for (int t0 = gr.rank; t0 < tot; t0 += gr.size) {
             int t = t0, a = 0;
 #pragma unroll
@@ -893,6 +904,7 @@ __device__ void group_itemF(const Group &gr, const DevTables &T, const IntDesc &
     }
     gr.sync();
     // points
+#pragma unroll 1
     for (int p = gr.rank; p < nchild * NP; p += gr.size) {
         const int ch = p >= NP ? 1 : 0;
         const int pp = p - ch * NP;
@@ -948,22 +960,25 @@ __device__ void group_itemF(const Group &gr, const DevTables &T, const IntDesc &
         udiff = ua + RATIO * ub + (2.f - 2.f * RATIO) * u0;
     }
     if (active) {
+#pragma unroll 1
         for (int k = hl; k < NRR; k += 16) {
             const float x = v[1 + 4 * DIM + k];
             s4 = df_add_f(s4, x);
             u4 += fmaf(EPS_REL, fabsf(x), TAU_ABS);
         }
+#pragma unroll 1
         for (int k = hl; k < (1 << DIM); k += 16) {
             const float x = v[1 + 4 * DIM + NRR + k];
             s45 = df_add_f(s45, x);
             u5 += fmaf(EPS_REL, fabsf(x), TAU_ABS);
         }
     }
-    s2 = hw_sum(s2);
-    s3 = hw_sum(s3);
-    s4 = hw_sum(s4);
-    s45 = hw_sum(s45);
+#pragma unroll 1
     for (int m = 8; m > 0; m >>= 1) {
+        s2 = df_add(s2, shfl_xor_df(s2, m));
+        s3 = df_add(s3, shfl_xor_df(s3, m));
+        s4 = df_add(s4, shfl_xor_df(s4, m));
+        s45 = df_add(s45, shfl_xor_df(s45, m));
         u2 += __shfl_xor_sync(0xffffffffu, u2, m);
         u3 += __shfl_xor_sync(0xffffffffu, u3, m);
         u4 += __shfl_xor_sync(0xffffffffu, u4, m);
@@ -973,6 +988,7 @@ __device__ void group_itemF(const Group &gr, const DevTables &T, const IntDesc &
     int sidx = hl;
     df best = diff;
     float ubest = udiff;
+#pragma unroll 1
     for (int m = 8; m > 0; m >>= 1) {
         df od = shfl_xor_df(best, m);
         int oi = __shfl_xor_sync(0xffffffffu, sidx, m);
@@ -985,6 +1001,7 @@ __device__ void group_itemF(const Group &gr, const DevTables &T, const IntDesc &
     }
     df second = (hl == sidx) ? df{-1.f, 0.f} : diff;
     float usecond = (hl == sidx) ? 0.f : udiff;
+#pragma unroll 1
     for (int m = 8; m > 0; m >>= 1) {
         df od = shfl_xor_df(second, m);
         float ou = __shfl_xor_sync(0xffffffffu, usecond, m);
@@ -1003,16 +1020,20 @@ __device__ void group_itemF(const Group &gr, const DevTables &T, const IntDesc &
                          diff.hi + udiff >= (best.hi - ubest) - 1e-6f * fabsf(best.hi));
     const unsigned cmask = (cbits >> (16 * hh)) & ((1u << DIM) - 1u);
     // 7th- and 5th-degree brackets (double-float), then FP64 on four lanes
-    df b7 = df_mul_f({df_hi_of(W::w1), df_lo_of(W::w1)}, val0);
-    b7 = df_add(b7, df_mul(s2, {df_hi_of(W::w2), df_lo_of(W::w2)}));
-    b7 = df_add(b7, df_mul(s3, {df_hi_of(W::w3), df_lo_of(W::w3)}));
-    b7 = df_add(b7, df_mul(s4, {df_hi_of(W::w4), df_lo_of(W::w4)}));
-    df b5 = df_mul_f({df_hi_of(W::wE1), df_lo_of(W::wE1)}, val0);
-    b5 = df_add(b5, df_mul(s2, {df_hi_of(W::wE2), df_lo_of(W::wE2)}));
-    b5 = df_add(b5, df_mul(s3, {df_hi_of(W::wE3), df_lo_of(W::wE3)}));
-    b5 = df_add(b5, df_mul(s4, {df_hi_of(W::wE4), df_lo_of(W::wE4)}));
-    df e = df_add(b5, df_neg(df_add(b7, df_mul(s45, {df_hi_of(W::w5), df_lo_of(W::w5)}))));
+    // odd lanes form the 5th-degree bracket beside the even lanes' 7th-degree one
+    const bool deg5 = hl & 1;
+    auto weight = [&](double w7, double w5) {
+        return deg5 ? df{df_hi_of(w5), df_lo_of(w5)} : df{df_hi_of(w7), df_lo_of(w7)};
+    };
+    df br = df_mul_f(weight(W::w1, W::wE1), val0);
+    br = df_add(br, df_mul(s2, weight(W::w2, W::wE2)));
+    br = df_add(br, df_mul(s3, weight(W::w3, W::wE3)));
+    br = df_add(br, df_mul(s4, weight(W::w4, W::wE4)));
+    const df brx = shfl_xor_df(br, 1);
+    df b7 = deg5 ? brx : br;
+    const df b5 = deg5 ? br : brx;
     b7 = df_add(b7, df_mul(s45, {df_hi_of(W::w5), df_lo_of(W::w5)}));
+    df e = df_add(b5, df_neg(b7));
     if (e.hi < 0.f) e = df_neg(e);
     // bound on the error of e from the point-value bounds (weights of res7 - res5)
     const float ue = fabsf((float)(W::w1 - W::wE1)) * u0 + fabsf((float)(W::w2 - W::wE2)) * u2 +
@@ -1076,8 +1097,9 @@ __global__ void __launch_bounds__(128, MINB) k_evalmx(DevTables T, const IntDesc
     // Few items: a block takes one, so that a round of few cuts is not as long as one warp's
     // evaluation of a whole cut.  The warps of a full grid take one each otherwise (no idle
     // lanes at the ends of the passes, no block barriers).  The line lies where a block per
-    // item would take a second turn.  One triplet, 3 terms: 9.3 -> 7.7 ms.
-    const bool wide = wend - wbeg <= (long long)gridDim.x;
+    // item would take a third turn (one to four turns measured within 1%).  One triplet, 3
+    // terms: 9.3 -> 7.7 ms; a block per item throughout would cost 220 triplets 10%.
+    const bool wide = wend - wbeg <= 2 * (long long)gridDim.x;
     const Group gr{wide ? 128 : 32, wide ? (int)threadIdx.x : lane};
     const int buf = wide ? 0 : wib;
     const long long first = wide ? blockIdx.x : (long long)blockIdx.x * WPB + wib;
