@@ -215,7 +215,8 @@ __device__ void boundary_select(const double *err, const unsigned long long *q, 
             ce += sh.wc[w];
         }
         const unsigned long long before = by_sum ? se : ce, here = by_sum ? s : c;
-        if ((before < need && before + here >= need) || (tid == SEL_BS - 1 && before + here < need)) {
+        // exactly one thread (the first or last where `need` lies outside the total)
+        if ((before < need || tid == 0) && (before + here >= need || tid == SEL_BS - 1)) {
             int chosen = top;
             for (int b = 0; b < SEL_PER; ++b) {
                 chosen = top - b;
@@ -248,28 +249,32 @@ __device__ void boundary_select(const double *err, const unsigned long long *q, 
                 const unsigned long long k = ekey(err, base + j);
                 if (k - lo <= span) {
                     const unsigned at = atomicAdd(&sh.ncand, 1u);
-                    sh.ck[at] = k;
-                    sh.cq[at] = by_sum ? q[base + j] : 1ull;
+                    if (at < 32) {
+                        sh.ck[at] = k;
+                        sh.cq[at] = by_sum ? q[base + j] : 1ull;
+                    }
                 }
             }
             __syncthreads();
             if (tid < 32) {
-                const int n = (int)sh.ncand;
+                const int n = min((int)sh.ncand, 32);
                 const unsigned long long k = lane < n ? sh.ck[lane] : 0, v = lane < n ? sh.cq[lane] : 0;
                 unsigned long long gt = 0, ge = 0;
-                unsigned int ngt = 0;
+                unsigned int ngt = 0, nge = 0;
                 for (int j = 0; j < n; ++j) {
                     const unsigned long long kj = sh.ck[j], vj = sh.cq[j];
                     if (kj > k) {
                         gt += vj;
                         ++ngt;
                     }
-                    if (kj >= k) ge += vj;
+                    if (kj >= k) {
+                        ge += vj;
+                        ++nge;
+                    }
                 }
                 const unsigned long long from = by_sum ? sa : ca;
-                // the smallest key where the total is never reached (not met by the callers)
-                const bool last = from + ge < need && gt + v == ge && ngt + 1u >= (unsigned)n;
-                if (lane < n && ((from + gt < need && from + ge >= need) || last)) {
+                // (the largest or smallest key where `need` lies outside the total)
+                if (lane < n && (from + gt < need || ngt == 0) && (from + ge >= need || nge == (unsigned)n)) {
                     sh.bkey = k;
                     sh.qb = v;
                     sh.cnt_above = ca + ngt;
@@ -344,7 +349,7 @@ __global__ void __launch_bounds__(SEL_BS) k_select(const IntDesc *__restrict__ D
     // threshold guard (mixed precision): bound multiplier (gthr) and the value bounds' basis
     const double gthr = H->mixed ? (double)H->thr_ratio : 0.0;
     const double vr = (double)H->val_ratio;
-    const int n = H->n;
+    const int end = H->gbeg[NGROUPS];
     // a stop request: k_scan's (cancel or deadline), or a host cancel that arrived since
     // (one read of the host-mapped word per block)
     if (threadIdx.x == 0) {
@@ -353,7 +358,7 @@ __global__ void __launch_bounds__(SEL_BS) k_select(const IntDesc *__restrict__ D
         s_cancel = cz;
     }
     __syncthreads();
-    for (int i = blockIdx.x; i < n; i += gridDim.x) {
+    for (int i = H->gbeg[0] + blockIdx.x; i < end; i += gridDim.x) {
         if (pass == 1 && !S[i].defer) continue;  // block-uniform
         __syncthreads();
         if (threadIdx.x == 0) S[i].defer = 0;
@@ -365,7 +370,9 @@ __global__ void __launch_bounds__(SEL_BS) k_select(const IntDesc *__restrict__ D
         const long long base = d.base;
         const int R = S[i].nR;
         if (R == 0) {
-            // fresh integral: its root region is this round's single work item
+            // fresh integral: its root region is this round's single work item (every warp has
+            // to have read nR before it changes)
+            __syncthreads();
             if (threadIdx.x == 0) {
                 P.cand[base] = -1;
                 S[i].K = 1;
@@ -732,9 +739,9 @@ __global__ void __launch_bounds__(1024) k_scan(IntState *__restrict__ S, long lo
                                                int use_cond)
 {
     __shared__ long long part[1024];
-    const int n = H->n;
-    const int per = (n + blockDim.x - 1) / blockDim.x;
-    const int b = threadIdx.x * per, e = min(n, b + per);
+    const int beg = H->gbeg[0], n = H->gbeg[NGROUPS];
+    const int per = (n - beg + blockDim.x - 1) / blockDim.x;
+    const int b = beg + threadIdx.x * per, e = min(n, b + per);
     long long loc = 0;
     for (int i = b; i < e; ++i) loc += S[i].K;
     part[threadIdx.x] = loc;
@@ -787,8 +794,8 @@ __global__ void __launch_bounds__(1024) k_scan(IntState *__restrict__ S, long lo
 __global__ void k_init(const IntDesc *__restrict__ D, IntState *__restrict__ S, Pool P,
                        BatchHdr *H)
 {
-    const int n = H->n;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    const int beg = H->gbeg[0], n = H->gbeg[NGROUPS];
+    for (int i = beg + blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const IntDesc &d = D[i];
         for (int k = 0; k < MAX_DIM; ++k) {
             if (k < d.dim) {
@@ -813,7 +820,7 @@ __global__ void k_init(const IntDesc *__restrict__ D, IntState *__restrict__ S, 
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         H->any_active = 1;
         H->total_work = 0;
-        H->regions = (unsigned long long)n;
+        H->regions = (unsigned long long)(n - beg);
         H->rounds_done = 0;
         H->chunk_count = 0;
         H->ties = 0;
@@ -858,6 +865,13 @@ __global__ void k_admit(const IntDesc *__restrict__ Dn, const int *__restrict__ 
     }
 }
 
+// Serving: a group's loop is entered only if the host counted unfinished integrals in it
+__global__ void k_gate(const BatchHdr *H, cudaGraphConditionalHandle handle)
+{
+    cudaGraphSetConditional(handle, H->n > 0 ? 1u : 0u);
+}
+
+void *gate_kernel() { return (void *)k_gate; }
 void *admit_kernel() { return (void *)k_admit; }
 void *select_kernel() { return (void *)k_select; }
 void *scan_kernel() { return (void *)k_scan; }

@@ -237,9 +237,11 @@ __host__ __device__ constexpr long long reeval_scratch_group_bytes(int rcap)
            (long long)rcap * 3 * MZ_PAIRS * MZ_VALS * 8;
 }
 
-// Per-call header kept in device memory so one instantiated graph serves any batch.
+// Header of one refinement loop, kept in device memory so one instantiated graph serves any
+// batch.  The loop covers the integrals [gbeg[0], gbeg[NGROUPS]): those of one group when
+// the groups' loops run side by side (graph), all of them in host-driven rounds.
 struct BatchHdr {
-    int n;                       // integrals (sorted by group)
+    int n;                       // integrals of the loop (serving: unfinished ones)
     int gbeg[NGROUPS + 1];       // group g = integrals [gbeg[g], gbeg[g+1])
     int max_rounds;
     int cancel;                  // nonzero stops the loop at the next selection: 1 =

@@ -46,6 +46,7 @@ void *select_kernel();
 void *scan_kernel();
 void *init_kernel();
 void *admit_kernel();
+void *gate_kernel();
 namespace host {
 const char *last_error_cstr();
 }
@@ -105,7 +106,6 @@ struct Workspace {
 
 struct GraphEntry {
     int gen, precision, gmask;
-    bool side;  // the groups' rule kernels side by side
     cudaGraph_t graph;
     cudaGraphExec_t exec;
 };
@@ -365,8 +365,8 @@ int alloc_workspace(Workspace &W, int ncap, size_t pcap, const unsigned char *re
     st |= dalloc(&W.P.rscr, (size_t)(NGROUPS * W.P.rscr_group));
     st |= dalloc(&W.D, (size_t)ncap);
     st |= dalloc(&W.S, (size_t)ncap);
-    st |= dalloc(&W.woff, (size_t)ncap + 1);
-    st |= dalloc(&W.H, 1);
+    st |= dalloc(&W.woff, (size_t)ncap + NGROUPS);  // group g: entries [beg + g, end + g]
+    st |= dalloc(&W.H, NGROUPS);
     if (st) {
         free_workspace(W);
         return G3L_ERR_NOMEM;
@@ -458,117 +458,119 @@ void set_esc_queues(const IntDesc *D, int n, BatchHdr &H)
     }
 }
 
-// The groups' rule kernels run side by side in a call whose region pools hold at most this
-// many regions, in a chain otherwise.  A call cuts a region pool's worth of regions over
-// ~25 rounds: below the line a round leaves each kernel's grid partly empty and its length
-// is the sum of three short kernels; above it each kernel fills the device and concurrent
-// ones contend for caches and registers.  Measured, chain against side by side: mixed 32k
-// regions (one triplet) 7.67 / 6.81 ms, 310k 19.2 / 18.0, 2.4M 64.8 / 69.3; FP64 700 regions
-// 5.33 / 3.26 ms, 7.7k 10.5 / 9.6, 16k 14.1 / 15.0.
-constexpr long long kSideMaxMixed = 600000, kSideMaxFp64 = 10000;
-
-// The device loop as one graph: init, then WHILE (conditional node) { select, [mixed:
-// FP64 re-evaluations, second selection pass], scan, [mixed: re-evaluations], rule
-// evaluation per group }.  `init` = false leaves the states as they are (serving).
-int build_graph_ws(g3l_ctx *c, Workspace &W, int precision, int gmask, bool init, bool side,
-                   GraphEntry &out)
+// Headers of the groups' loops from the call's header: loop g covers group g alone.
+void split_header(const BatchHdr &H, BatchHdr *Hg)
 {
-    KernelArgs a{c->T, W.D, W.S, W.P, W.H, W.woff, 0, 1, c->T.tau_sel, c->T.tau_val};
+    for (int g = 0; g < NGROUPS; ++g) {
+        Hg[g] = H;
+        Hg[g].n = H.gbeg[g + 1] - H.gbeg[g];
+        for (int k = 0; k <= NGROUPS; ++k) Hg[g].gbeg[k] = k <= g ? H.gbeg[g] : H.gbeg[g + 1];
+    }
+}
+
+// the statistics of the groups' loops as one header
+BatchHdr merge_headers(const BatchHdr *Hg, int gmask)
+{
+    BatchHdr H{};
+    for (int g = 0; g < NGROUPS; ++g) {
+        if (!(gmask & (1 << g))) continue;
+        H.rounds_done = std::max(H.rounds_done, Hg[g].rounds_done);
+        H.regions += Hg[g].regions;
+        H.ties += Hg[g].ties;
+        H.small_arg += Hg[g].small_arg;
+        H.escalated += Hg[g].escalated;
+        H.deferred += Hg[g].deferred;
+        H.polished += Hg[g].polished;
+        H.esc_full += Hg[g].esc_full;
+        H.thr_checks += Hg[g].thr_checks;
+    }
+    return H;
+}
+
+// One refinement loop per group, side by side in one graph: init, then WHILE (conditional
+// node) { select, [mixed: FP64 re-evaluations, second selection pass], scan, [mixed:
+// re-evaluations], rule evaluation }.  The groups' integrals are independent, so a loop
+// waits for nothing of the others: rounds of one group's FP64 re-evaluations (FP64 pipe)
+// run beside another's rule kernels (FP32), and a call of few integrals has each round as
+// long as its own group's work instead of the slowest group's (one loop over all groups:
+// 220 triplets 53.1 ms, one triplet 4.3 ms).  `init` = false leaves the states as they are
+// and enters a loop only if its header counts unfinished integrals (serving).
+int build_graph_ws(g3l_ctx *c, Workspace &W, int precision, int gmask, bool init, GraphEntry &out)
+{
     cudaGraph_t g;
     G3L_CK(cudaGraphCreate(&g, 0));
-    cudaGraphNode_t n_init;
-    if (init) {
-        void *args[] = {&a.D, &a.S, &a.P, &a.H};
-        int st = add_kernel(g, &n_init, nullptr, 0, init_kernel(), c->nsm * 4, 256, args);
-        if (st) return st;
-    }
-    G3L_CK(cudaGraphConditionalHandleCreate(&a.handle, g, 1, cudaGraphCondAssignDefault));
-    cudaGraphNodeParams cp{};
-    cp.type = cudaGraphNodeTypeConditional;
-    cp.conditional.handle = a.handle;
-    cp.conditional.type = cudaGraphCondTypeWhile;
-    cp.conditional.size = 1;
-    cudaGraphNode_t n_while;
-    G3L_CK(cudaGraphAddNode(&n_while, g, init ? &n_init : nullptr, nullptr, init ? 1 : 0, &cp));
-    cudaGraph_t body = cp.conditional.phGraph_out[0];
-    cudaGraphNode_t n_sel, n_scan, prev;
-    // mixed: FP64 re-evaluations queued by a selection pass (unsettled splits of the
-    // parents about to be cut, ambiguous boundary regions, polish), one branch per group,
-    // side by side: each group reads only its own queue.  ends[2 grp], ends[2 grp + 1]: the
-    // last nodes of group grp's branch.
-    auto add_reevals = [&](cudaGraphNode_t dep, int &stage, cudaGraphNode_t *ends) -> int {
-        for (int grp = 0; grp < NGROUPS; ++grp) {
-            if (!(gmask & (1 << grp))) continue;
-            void *args[] = {&a.T, &a.D, &a.S, &a.P, &a.H, &a.woff, &stage};
-            cudaGraphNode_t chain = dep;
-            for (int ph = 0; ph < 3; ++ph) {
-                void *fn = reeval_phase_kernel(grp / 3, grp % 3 + 1, ph);
-                cudaGraphNode_t nd;
-                int st = add_kernel(body, &nd, &chain, 1, fn, grid128(c, fn), 128, args);
-                if (st) return st;
-                chain = nd;
-            }
-            ends[2 * grp] = chain;
-            void *fn = reeval_phase_kernel(grp / 3, grp % 3 + 1, 3);
-            int st = add_kernel(body, &ends[2 * grp + 1], &dep, 1, fn, grid128(c, fn), 128, args);
-            if (st) return st;
-        }
-        return G3L_OK;
-    };
-    {
-        void *args[] = {&a.D, &a.S, &a.P, &a.H, &a.tau_sel, &a.tau_val, &a.pass0};
-        int st = add_kernel(body, &n_sel, nullptr, 0, select_kernel(), c->nsm * 8, 256, args);
-        if (st) return st;
-    }
-    prev = n_sel;
-    cudaGraphNode_t ends[2 * NGROUPS];
-    if (precision == G3L_MIXED) {
-        int st = add_reevals(prev, a.pass0, ends);
-        if (st) return st;
-        cudaGraphNode_t deps[2 * NGROUPS];
-        int nd = 0;
-        for (int grp = 0; grp < NGROUPS; ++grp)
-            for (int e = 0; e < 2 && (gmask & (1 << grp)); ++e) deps[nd++] = ends[2 * grp + e];
-        void *args[] = {&a.D, &a.S, &a.P, &a.H, &a.tau_sel, &a.tau_val, &a.pass1};
-        cudaGraphNode_t n_sel1;
-        st = add_kernel(body, &n_sel1, deps, nd, select_kernel(), c->nsm * 8, 256, args);
-        if (st) return st;
-        prev = n_sel1;
-    }
-    {
-        void *args[] = {&a.S, &a.woff, &a.H, &a.handle, &a.use_cond};
-        int st = add_kernel(body, &n_scan, &prev, 1, scan_kernel(), 1, 1024, args);
-        if (st) return st;
-    }
-    prev = n_scan;
-    if (precision == G3L_MIXED) {
-        int st = add_reevals(prev, a.pass1, ends);
-        if (st) return st;
-    }
-    // the groups' rule kernels in a chain, or side by side (kSideMaxMixed); a group's
-    // kernel waits for the previous one, if chained, and its own re-evaluations, so the
-    // other groups' re-evaluations run beside it
     for (int grp = 0; grp < NGROUPS; ++grp) {
         if (!(gmask & (1 << grp))) continue;
+        KernelArgs a{c->T, W.D, W.S, W.P, W.H + grp, W.woff + grp, 0, 1, c->T.tau_sel, c->T.tau_val};
+        G3L_CK(cudaGraphConditionalHandleCreate(&a.handle, g, 1, cudaGraphCondAssignDefault));
+        cudaGraphNode_t n_init;
+        int st;
+        if (init) {
+            void *args[] = {&a.D, &a.S, &a.P, &a.H};
+            st = add_kernel(g, &n_init, nullptr, 0, init_kernel(), c->nsm, 256, args);
+        } else {
+            void *args[] = {&a.H, &a.handle};
+            st = add_kernel(g, &n_init, nullptr, 0, gate_kernel(), 1, 1, args);
+        }
+        if (st) return st;
+        cudaGraphNodeParams cp{};
+        cp.type = cudaGraphNodeTypeConditional;
+        cp.conditional.handle = a.handle;
+        cp.conditional.type = cudaGraphCondTypeWhile;
+        cp.conditional.size = 1;
+        cudaGraphNode_t n_while;
+        G3L_CK(cudaGraphAddNode(&n_while, g, &n_init, nullptr, 1, &cp));
+        cudaGraph_t body = cp.conditional.phGraph_out[0];
+        // nodes of one step, each depending on all nodes of the previous one
+        cudaGraphNode_t prev[2];
+        int nprev = 0;
+        auto step = [&](void *fn, int grid, int block, void **args) -> int {
+            cudaGraphNode_t nd;
+            const int r = add_kernel(body, &nd, prev, nprev, fn, grid, block, args);
+            prev[0] = nd;
+            nprev = 1;
+            return r;
+        };
+        // FP64 re-evaluations queued by a selection pass (unsettled splits of the parents
+        // about to be cut, ambiguous boundary regions, polish): the three device-wide
+        // passes, and beside them the batched kernel for what exceeds their scratch
+        auto reevals = [&](int &stage) -> int {
+            void *args[] = {&a.T, &a.D, &a.S, &a.P, &a.H, &a.woff, &stage};
+            const cudaGraphNode_t from[2] = {prev[0], prev[1]};
+            const int nfrom = nprev;
+            int r = G3L_OK;
+            for (int ph = 0; ph < 3 && !r; ++ph) {
+                void *fn = reeval_phase_kernel(grp / 3, grp % 3 + 1, ph);
+                r = step(fn, grid128(c, fn), 128, args);
+            }
+            void *tail = reeval_phase_kernel(grp / 3, grp % 3 + 1, 3);
+            if (!r) r = add_kernel(body, &prev[nprev++], from, nfrom, tail, grid128(c, tail), 128, args);
+            return r;
+        };
+        void *sel[] = {&a.D, &a.S, &a.P, &a.H, &a.tau_sel, &a.tau_val, &a.pass0};
+        st = step(select_kernel(), c->nsm * 8, 256, sel);
+        if (!st && precision == G3L_MIXED) {
+            st = reevals(a.pass0);
+            sel[6] = &a.pass1;
+            if (!st) st = step(select_kernel(), c->nsm * 8, 256, sel);
+        }
+        void *scan[] = {&a.S, &a.woff, &a.H, &a.handle, &a.use_cond};
+        if (!st) st = step(scan_kernel(), 1, 1024, scan);
+        if (!st && precision == G3L_MIXED) st = reevals(a.pass1);
         void *fn = eval_fn(c, precision, grp);
         void *args[] = {&a.T, &a.D, &a.S, &a.P, &a.H, &a.woff};
-        cudaGraphNode_t n_ev, deps[3];
-        int nd = 0;
-        if (!side || precision != G3L_MIXED) deps[nd++] = prev;
-        for (int e = 0; e < 2 && precision == G3L_MIXED; ++e) deps[nd++] = ends[2 * grp + e];
-        int st = add_kernel(body, &n_ev, deps, nd, fn, eval_grid(c, fn), 128, args);
+        if (!st) st = step(fn, eval_grid(c, fn), 128, args);
         if (st) return st;
-        if (!side) prev = n_ev;
     }
     cudaGraphExec_t ex;
     G3L_CK(cudaGraphInstantiate(&ex, g, 0));
-    out = GraphEntry{W.gen, precision, gmask, side, g, ex};
+    out = GraphEntry{W.gen, precision, gmask, g, ex};
     return G3L_OK;
 }
 
-int build_graph(g3l_ctx *c, int precision, int gmask, bool side, GraphEntry &out)
+int build_graph(g3l_ctx *c, int precision, int gmask, GraphEntry &out)
 {
-    return build_graph_ws(c, c->W, precision, gmask, true, side, out);
+    return build_graph_ws(c, c->W, precision, gmask, true, out);
 }
 
 // descriptor of one integral: bounds and root geometry as the reference computes them
@@ -791,7 +793,8 @@ struct g3l_server {
     Workspace W;
     GraphEntry G{};
     bool graph_ok = false;
-    std::vector<IntState> Sh;       // host copy of the states after each launch
+    IntState *Sh = nullptr;         // host copy of the states after each launch (pinned)
+    BatchHdr *Hs = nullptr;         // headers of a launch (pinned)
     std::vector<int64_t> slot_req;  // slot -> ticket (0 = free)
     std::vector<int> slot_item;
     std::vector<std::vector<int>> free_slots;  // per group
@@ -896,6 +899,7 @@ void srv_loop(g3l_server *v)
         ni.clear();
         cancel_slots.clear();
         long long cnt[NGROUPS] = {};
+        int live[NGROUPS] = {};
         {
             std::unique_lock<std::mutex> lk(v->mu);
             v->cv_work.wait(lk, [&] { return v->stop || !v->pending.empty() || v->active > 0; });
@@ -909,6 +913,7 @@ void srv_loop(g3l_server *v)
                 if (q.cancel && !v->Sh[i].done) cancel_slots.push_back(i);
                 const IntDesc &d = q.desc[v->slot_item[i]];
                 cnt[d.kind * 3 + d.term - 1] += d.cap;
+                ++live[d.kind * 3 + d.term - 1];
             }
             if (v->active == 0) continue;
         }
@@ -943,10 +948,17 @@ void srv_loop(g3l_server *v)
             H.esc_cap[g] = (int)std::min<long long>(cnt[g], 0x7fffffff);
             beg += cnt[g];
         }
-        SRV_CK(cudaMemcpyAsync(v->W.H, &H, sizeof H, cudaMemcpyHostToDevice, s));
+        split_header(H, v->Hs);
+        for (int g = 0; g < NGROUPS; ++g) v->Hs[g].n = live[g];
+        SRV_CK(cudaMemcpyAsync(v->W.H, v->Hs, sizeof(BatchHdr) * NGROUPS, cudaMemcpyHostToDevice, s));
         NvtxScope nv("server launch");
         SRV_CK(cudaGraphLaunch(v->G.exec, s));
-        SRV_CK(cudaMemcpyAsync(v->Sh.data(), v->W.S, sizeof(IntState) * v->n, cudaMemcpyDeviceToHost, s));
+        for (int g = 0; g < NGROUPS; ++g) {  // the states of the groups that ran
+            if (!live[g]) continue;
+            const size_t at = (size_t)g * v->per_group;
+            SRV_CK(cudaMemcpyAsync(v->Sh + at, v->W.S + at, sizeof(IntState) * v->per_group,
+                                   cudaMemcpyDeviceToHost, s));
+        }
         SRV_CK(cudaStreamSynchronize(s));
         SRV_CK(cudaGetLastError());
         {
@@ -1001,6 +1013,8 @@ void srv_destroy(g3l_server *v)
     free_workspace(v->W);
     if (v->d_new) cudaFree(v->d_new);
     if (v->d_idx) cudaFree(v->d_idx);
+    if (v->Sh) cudaFreeHost(v->Sh);
+    if (v->Hs) cudaFreeHost(v->Hs);
     if (v->s) cudaStreamDestroy(v->s);
     delete v;
 }
@@ -1028,14 +1042,19 @@ int srv_create(g3l_ctx *c, int precision, int per_group, uint64_t pool_regions, 
     int st = G3L_OK;
     if (cudaStreamCreateWithFlags(&v->s, cudaStreamNonBlocking) != cudaSuccess) st = G3L_ERR_CUDA;
     if (!st) st = alloc_workspace(v->W, v->n, v->pool, c->retab_d);
+    if (!st && (cudaMallocHost(&v->Sh, sizeof(IntState) * v->n) != cudaSuccess ||
+                cudaMallocHost(&v->Hs, sizeof(BatchHdr) * NGROUPS) != cudaSuccess))
+        st = G3L_ERR_NOMEM;
     if (!st) st = dalloc(&v->d_new, (size_t)v->n) | dalloc(&v->d_idx, (size_t)v->n);
-    if (!st) st = build_graph_ws(c, v->W, precision, (1 << NGROUPS) - 1, false, true, v->G);
+    if (!st) st = build_graph_ws(c, v->W, precision, (1 << NGROUPS) - 1, false, v->G);
     if (!st) v->graph_ok = true;
     if (!st) {
         // every slot starts free: a finished state, never selected
-        v->Sh.assign(v->n, IntState{});
-        for (auto &x : v->Sh) x.done = 1;
-        if (cudaMemcpy(v->W.S, v->Sh.data(), sizeof(IntState) * v->n, cudaMemcpyHostToDevice) !=
+        for (int i = 0; i < v->n; ++i) {
+            v->Sh[i] = IntState{};
+            v->Sh[i].done = 1;
+        }
+        if (cudaMemcpy(v->W.S, v->Sh, sizeof(IntState) * v->n, cudaMemcpyHostToDevice) !=
             cudaSuccess)
             st = G3L_ERR_CUDA;
     }
@@ -1780,8 +1799,10 @@ try {
     set_stop_fields(c, H);
     H.dbg = nullptr;
     // stage through pinned host memory: descriptors + header in, states + header out
-    const size_t in_bytes = sizeof(IntDesc) * n + sizeof(BatchHdr);
-    const size_t out_bytes = sizeof(IntState) * n + sizeof(BatchHdr);
+    // (host-driven rounds: one loop over all groups, in the first header)
+    const size_t hdr_bytes = sizeof(BatchHdr) * (c->opt.use_graph ? NGROUPS : 1);
+    const size_t in_bytes = sizeof(IntDesc) * n + hdr_bytes;
+    const size_t out_bytes = sizeof(IntState) * n + hdr_bytes;
     if (c->stage_bytes < in_bytes + out_bytes) {
         if (c->stage) cudaFreeHost(c->stage);
         c->stage_bytes = (in_bytes + out_bytes) * 5 / 4 + 4096;
@@ -1794,23 +1815,24 @@ try {
     }
     char *stg = (char *)c->stage;
     std::memcpy(stg, D.data(), sizeof(IntDesc) * n);
-    std::memcpy(stg + sizeof(IntDesc) * n, &H, sizeof(BatchHdr));
+    BatchHdr Hg[NGROUPS];
+    if (c->opt.use_graph) split_header(H, Hg);
+    else Hg[0] = H;
+    std::memcpy(stg + sizeof(IntDesc) * n, Hg, hdr_bytes);
     c->last_h2d = in_bytes;
     c->last_d2h = out_bytes;
     G3L_CK(cudaMemcpyAsync(W.D, stg, sizeof(IntDesc) * n, cudaMemcpyHostToDevice, c->stream));
-    G3L_CK(cudaMemcpyAsync(W.H, stg + sizeof(IntDesc) * n, sizeof(BatchHdr),
-                           cudaMemcpyHostToDevice, c->stream));
+    G3L_CK(cudaMemcpyAsync(W.H, stg + sizeof(IntDesc) * n, hdr_bytes, cudaMemcpyHostToDevice,
+                           c->stream));
     int launches = 0;
     G3L_CK(cudaEventRecord(c->ev0, c->stream));
     if (c->opt.use_graph) {
-        const bool side = base <= (precision == G3L_FP64 ? kSideMaxFp64 : kSideMaxMixed);
         GraphEntry *ge = nullptr;
         for (auto &g : c->graphs)
-            if (g.gen == W.gen && g.precision == precision && g.gmask == gmask && g.side == side)
-                ge = &g;
+            if (g.gen == W.gen && g.precision == precision && g.gmask == gmask) ge = &g;
         if (!ge) {
             GraphEntry e;
-            st = build_graph(c, precision, gmask, side, e);
+            st = build_graph(c, precision, gmask, e);
             if (st) return st;
             c->graphs.push_back(e);
             ge = &c->graphs.back();
@@ -1824,17 +1846,16 @@ try {
     G3L_CK(cudaEventRecord(c->ev1, c->stream));
     char *ostg = stg + in_bytes;
     G3L_CK(cudaMemcpyAsync(ostg, W.S, sizeof(IntState) * n, cudaMemcpyDeviceToHost, c->stream));
-    G3L_CK(cudaMemcpyAsync(ostg + sizeof(IntState) * n, W.H, sizeof(BatchHdr),
-                           cudaMemcpyDeviceToHost, c->stream));
+    G3L_CK(cudaMemcpyAsync(ostg + sizeof(IntState) * n, W.H, hdr_bytes, cudaMemcpyDeviceToHost,
+                           c->stream));
     G3L_CK(cudaStreamSynchronize(c->stream));
     std::vector<IntState> S(n);
     std::memcpy(S.data(), ostg, sizeof(IntState) * n);
-    BatchHdr Hout;
-    std::memcpy(&Hout, ostg + sizeof(IntState) * n, sizeof(BatchHdr));
+    std::memcpy(Hg, ostg + sizeof(IntState) * n, hdr_bytes);
+    const BatchHdr Hout = c->opt.use_graph ? merge_headers(Hg, gmask) : Hg[0];
     G3L_CK(cudaGetLastError());
     float ms = 0;
     cudaEventElapsedTime(&ms, c->ev0, c->ev1);
-    int ngroups = __builtin_popcount((unsigned)gmask);
     g3l_stats &sx = c->stats;
     {
         g3l_stats keep = sx;
@@ -1846,12 +1867,13 @@ try {
         }
     }
     sx.rounds = (uint64_t)Hout.rounds_done;
-    sx.kernel_launches = launches >= 0 ? (uint64_t)launches
-                                       : (uint64_t)(1 + (Hout.rounds_done + 1) *
-                                                           (2 + ngroups +
-                                                            (precision == G3L_MIXED
-                                                                 ? 8 * ngroups + 1
-                                                                 : 0)));
+    if (launches >= 0) {
+        sx.kernel_launches = (uint64_t)launches;
+    } else {  // per group: init, then each round's nodes
+        const int per_round = precision == G3L_MIXED ? 12 : 3;
+        for (int g = 0; g < NGROUPS; ++g)
+            if (gmask & (1 << g)) sx.kernel_launches += 1 + (uint64_t)(Hg[g].rounds_done + 1) * per_round;
+    }
     sx.regions_evaluated = Hout.regions;
     sx.tie_fallbacks = Hout.ties;
     sx.small_arg_fp64 = Hout.small_arg;
