@@ -244,9 +244,9 @@ __device__ __forceinline__ double k_integrand(const PcTask &t, double x, double 
 // 675-740), formed across the 16 lanes of a half-warp (lane i holds the value at abscissa i
 // of gk_point's order; lane 15 holds nothing): the reference's sums in another order.  An
 // FP64 instruction occupies the pipe for 64 cycles however few lanes take part, so one lane
-// per region summing 15 values three times cost more than the integrand; the power 3/2 is
-// x sqrt(x) (an FP64 pow is ~75 instructions).  Valid in lane 0 of the half-warp.
-__device__ __forceinline__ void rule_gk15_hw(double f, int hl, double hw, double &val, double &err)
+// per region summing 15 values three times cost more than the integrand.  Returns, in lanes
+// 0-3 of the half-warp: the value, |rk - rg| hw, rabs and rasc.
+__device__ __forceinline__ double rule_gk15_sums(double f, int hl, double hw)
 {
     // abscissa i: 0 centre, then pairs (2j+1, 2j+2): Gauss-Kronrod pair j (Kronrod-only
     // nodes for j = 0, 2, 4, 6 of cXgk; Gauss nodes for odd j)
@@ -286,20 +286,33 @@ __device__ __forceinline__ void rule_gk15_hw(double f, int hl, double hw, double
     for (int o = 8; o > 0; o >>= 1) rs += __shfl_xor_sync(0xffffffffu, rs, o, 16);
     // times the half-width, one lane each: value, |rk - rg|, rabs, rasc
     const double rg = __shfl_sync(0xffffffffu, s0, 4, 16), ra = __shfl_sync(0xffffffffu, s0, 8, 16);
-    const double t = (hl == 0 ? rk : hl == 1 ? fabs(rk - rg) : hl == 2 ? ra : rs) * hw;
-    val = t;
-    double e = __shfl_sync(0xffffffffu, t, 1, 16);
-    const double rabs = __shfl_sync(0xffffffffu, t, 2, 16), rasc = __shfl_sync(0xffffffffu, t, 3, 16);
-    if (rasc != 0 && e != 0) {
+    return (hl == 0 ? rk : hl == 1 ? fabs(rk - rg) : hl == 2 ? ra : rs) * hw;
+}
+
+// the error from |rk - rg| hw, rabs and rasc.  Its operands are >= 0 and compared by bit
+// pattern; the power 3/2 is x sqrt(x) (an FP64 pow is ~86 instructions).
+__device__ __forceinline__ double rule_gk15_err(double e, double rabs, double rasc)
+{
+    auto bits = [](double x) { return __double_as_longlong(x); };
+    if (bits(rasc) != 0 && bits(e) != 0) {
         const double q = ddiv(200 * e, rasc);
         const double scale = q * sqrt(q);
-        e = (scale < 1) ? rasc * scale : rasc;
+        e = bits(scale) < bits(1.0) ? rasc * scale : rasc;
     }
-    if (rabs > DBL_MIN / (50 * DBL_EPSILON)) {
+    if (bits(rabs) > bits(DBL_MIN / (50 * DBL_EPSILON))) {
         const double min_err = 50 * DBL_EPSILON * rabs;
-        if (min_err > e) e = min_err;
+        if (bits(min_err) > bits(e)) e = min_err;
     }
-    err = e;
+    return e;
+}
+
+// value and error in lane 0 of the half-warp
+__device__ __forceinline__ void rule_gk15_hw(double f, int hl, double hw, double &val, double &err)
+{
+    val = rule_gk15_sums(f, hl, hw);
+    const double e = __shfl_sync(0xffffffffu, val, 1, 16);
+    const double rabs = __shfl_sync(0xffffffffu, val, 2, 16), rasc = __shfl_sync(0xffffffffu, val, 3, 16);
+    err = rule_gk15_err(e, rabs, rasc);
 }
 
 // the i-th Gauss-Kronrod abscissa of the region (c, hw), in the reference's order
@@ -485,13 +498,60 @@ __device__ PcOut gk_integrate(double lo, double hi, double *sm, const Eval &ev)
     return o;
 }
 
+// Sort P2 (a power of two, >= 32) keys with their indices, largest key first, equal keys by
+// index, by the whole block: a bitonic network whose steps over fewer than 32 elements run
+// in registers between shuffles (15 block barriers for the wide steps of 1024 elements and
+// 6 for the others, instead of 55).
+__device__ void sort_desc(long long *key, int *ord, int P2)
+{
+    const int tid = threadIdx.x, nth = blockDim.x;
+    auto before = [](long long ka, int a, long long kb, int b) { return ka > kb || (ka == kb && a < b); };
+    for (int k = 32; k <= P2; k <<= 1) {
+        for (int j = k >> 1; j >= 32; j >>= 1) {
+            for (int t = tid; t < P2; t += nth) {
+                const int u = t ^ j;
+                if (u > t) {
+                    const long long ka = key[t], kb = key[u];
+                    const int a = ord[t], b = ord[u];
+                    if (before(ka, a, kb, b) != ((t & k) == 0)) {  // descending blocks first
+                        key[t] = kb;
+                        key[u] = ka;
+                        ord[t] = b;
+                        ord[u] = a;
+                    }
+                }
+            }
+            __syncthreads();
+        }
+        for (int t = tid; t < P2; t += nth) {  // whole warps: P2 and nth are multiples of 32
+            long long ka = key[t];
+            int a = ord[t];
+            for (int kk = k == 32 ? 2 : k; kk <= k; kk <<= 1)
+                for (int j = min(kk >> 1, 16); j > 0; j >>= 1) {
+                    const long long kb = __shfl_xor_sync(0xffffffffu, ka, j);
+                    const int b = __shfl_xor_sync(0xffffffffu, a, j);
+                    const bool lower = (t & j) == 0, desc = (t & kk) == 0;
+                    if (before(ka, a, kb, b) != (lower == desc)) {
+                        ka = kb;
+                        a = b;
+                    }
+                }
+            key[t] = ka;
+            ord[t] = a;
+        }
+        __syncthreads();
+    }
+}
+
 // The same refinement with the live regions in plain arrays instead of a heap, for
 // integrals whose result needs agree with the reference's to ~1e-12 rather than in the
-// last bit (n_bar): each round the whole block sorts the live regions by error
-// (bitonic, descending) and thread 0 walks that order with the reference's Gladwell
-// rule (pop the largest errors until the rest is within tolerance), so the regions cut
-// are the heap's; only the order among exactly equal errors and the summation order of
-// the totals differ.  Shared memory: pc_smem(CAP) plus CAP ints.
+// last bit (n_bar): each round the whole block sorts the live regions by error and thread
+// 0 walks that order with the reference's Gladwell rule (pop the largest errors until the
+// rest is within tolerance), so the regions cut are the heap's; only the order among
+// exactly equal errors and the summation order of the totals differ.  A popped region's
+// place goes to its lower half, the upper halves are appended.  FP64 work is kept off the
+// threads that need not do it: the block's warps share one FP64 pipe per SM quarter.
+// Shared memory: nbar_smem(CAP).
 template <int CAP, class Eval>
 __device__ PcOut gk_integrate_sorted(double lo, double hi, double *sm, const Eval &ev)
 {
@@ -499,22 +559,12 @@ __device__ PcOut gk_integrate_sorted(double lo, double hi, double *sm, const Eva
     double *lc = sm, *lh = sm + CAP, *lv = sm + 2 * CAP, *le = sm + 3 * CAP;
     double *bc = sm + 4 * CAP, *bh = bc + PC_BATCH, *bv = bh + PC_BATCH, *be = bv + PC_BATCH;
     int *ord = (int *)(be + PC_BATCH);
-    __shared__ int s_nb, s_done, s_n, s_K, s_status, s_rounds;
-    __shared__ double s_red[2][32];
-    __shared__ unsigned long long s_neval;
-    const int tid = threadIdx.x, nth = blockDim.x;
-    if (tid == 0) {
-        bc[0] = 0.5 * (lo + hi);
-        bh[0] = 0.5 * (hi - lo);
-        s_nb = 1;
-        s_done = 0;
-        s_n = 0;
-        s_status = 0;
-        s_rounds = 0;
-        s_neval = 15;
-    }
-    __syncthreads();
-    // deterministic block sums of val and err over the live regions
+    long long *key = (long long *)bv;  // during a sort (the batch's values have been taken over)
+    __shared__ int s_K, s_status;
+    __shared__ double s_red[2][32], s_tot[2];
+    const int tid = threadIdx.x, nth = blockDim.x, nw = nth / 32;
+    // deterministic block sums of val and err over the live regions: thread 0 the values,
+    // thread 1 the errors
     auto totals = [&](int n, double &V, double &E) {
         double v = 0, e = 0;
         for (int i = tid; i < n; i += nth) {
@@ -530,80 +580,73 @@ __device__ PcOut gk_integrate_sorted(double lo, double hi, double *sm, const Eva
             s_red[1][tid >> 5] = e;
         }
         __syncthreads();
-        V = 0;
-        E = 0;
-        for (int w = 0; w < nth / 32; ++w) {
-            V += s_red[0][w];
-            E += s_red[1][w];
+        if (tid < 2) {
+            double r = 0;
+            for (int w = 0; w < nw; ++w) r += s_red[tid][w];
+            s_tot[tid] = r;
         }
         __syncthreads();
+        V = s_tot[0];
+        E = s_tot[1];
     };
-    while (true) {
-        ev(s_nb, bc, bh, bv, be);
+    int n = 0, K = 0, rounds = 0, status = 0;  // the same in every thread
+    unsigned long long neval = 15;
+    if (tid == 0) {
+        bc[0] = 0.5 * (lo + hi);
+        bh[0] = 0.5 * (hi - lo);
+        s_status = 0;
+    }
+    __syncthreads();
+    double hv, he;
+    for (;;) {
+        const int nb = n == 0 ? 1 : 2 * K;
+        ev(nb, bc, bh, bv, be);
         __syncthreads();
         // the batch joins the live regions
-        const int n0 = s_n, nb = s_nb;
         for (int b = tid; b < nb; b += nth) {
-            lc[n0 + b] = bc[b];
-            lh[n0 + b] = bh[b];
-            lv[n0 + b] = bv[b];
-            le[n0 + b] = be[b];
+            const int at = n == 0 ? 0 : ((b & 1) ? n + (b >> 1) : ord[b >> 1]);
+            lc[at] = bc[b];
+            lh[at] = bh[b];
+            lv[at] = bv[b];
+            le[at] = be[b];
         }
-        const int n = n0 + nb;
+        n += n == 0 ? 1 : K;
         __syncthreads();
-        if (tid == 0) s_n = n;  // every thread has read n0 (barrier above)
-        double hv, he;
         totals(n, hv, he);
         if (converged(he, hv)) break;
-        // largest errors first
-        int P2 = 1;
+        if (++rounds > PC_MAX_ROUNDS) {
+            status = G3L_ERR_ROUNDS;
+            break;
+        }
+        // largest errors first (they are >= 0: their bit patterns order as integers)
+        int P2 = 32;
         while (P2 < n) P2 <<= 1;
-        for (int i = tid; i < P2; i += nth) ord[i] = i;
-        __syncthreads();
-        for (int k = 2; k <= P2; k <<= 1)
-            for (int j = k >> 1; j > 0; j >>= 1) {
-                for (int t = tid; t < P2; t += nth) {
-                    const int u = t ^ j;
-                    if (u > t) {
-                        const int a = ord[t], b = ord[u];
-                        // errors are >= 0: their bit patterns order as integers (integer
-                        // compares; FP64 ones run at 1/64 of the FP32 rate)
-                        const long long ka = a < n ? __double_as_longlong(le[a]) : -1ll;
-                        const long long kb = b < n ? __double_as_longlong(le[b]) : -1ll;
-                        // descending overall: the first half of each k-block descending
-                        const bool desc = (t & k) == 0;
-                        if (desc ? (ka < kb || (ka == kb && a > b)) : (ka > kb || (ka == kb && a < b))) {
-                            ord[t] = b;
-                            ord[u] = a;
-                        }
-                    }
-                }
-                __syncthreads();
-            }
-        if (tid == 0) {
-            int K = 0;
-            if (++s_rounds > PC_MAX_ROUNDS) {
-                s_status = G3L_ERR_ROUNDS;
-                s_done = 1;
-            } else {
-                double eErr = he;
-                const double eVal = hv;
-                do {
-                    if (n + K + 1 > CAP) {  // live regions and children after this pop
-                        s_status = G3L_ERR_POOL;
-                        s_done = 1;
-                        break;
-                    }
-                    eErr -= le[ord[K]];
-                    ++K;
-                    if (converged(eErr, eVal)) break;
-                } while (K < n);
-            }
-            s_K = K;
+        for (int i = tid; i < P2; i += nth) {
+            key[i] = i < n ? __double_as_longlong(le[i]) : -1ll;
+            ord[i] = i;
         }
         __syncthreads();
-        if (s_done) break;
-        const int K = s_K;
+        sort_desc(key, ord, P2);
+        if (tid == 0) {
+            // pop until the error left is within tolerance: err > 0 && err > |val| 1e-4 by bit
+            // patterns (a negative rest has the sign bit)
+            const long long tol = __double_as_longlong(fabs(hv) * 1e-4);
+            double eErr = he;
+            int k = 0;
+            do {
+                if (n + k + 1 > CAP) {  // live regions after this pop's children
+                    s_status = G3L_ERR_POOL;
+                    break;
+                }
+                eErr -= __longlong_as_double(key[k]);
+                ++k;
+            } while (k < n && __double_as_longlong(eErr) > 0 && __double_as_longlong(eErr) > tol);
+            s_K = k;
+        }
+        __syncthreads();
+        status = s_status;
+        if (status) break;
+        K = s_K;
         // children of the popped regions (cut, src/hcubature.cpp:206-218)
         for (int k = tid; k < K; k += nth) {
             const int r = ord[k];
@@ -613,32 +656,10 @@ __device__ PcOut gk_integrate_sorted(double lo, double hi, double *sm, const Eva
             bc[2 * k + 1] = lc[r] + h2;
             bh[2 * k + 1] = h2;
         }
-        // the rest stays live (gathered through the batch's value arrays)
-        const int m = n - K;
-        for (int k = tid; k < m; k += nth) {
-            const int r = ord[K + k];
-            bv[k] = lc[r];
-            bv[CAP + k] = lh[r];
-            be[k] = lv[r];
-            be[CAP + k] = le[r];
-        }
-        __syncthreads();
-        for (int k = tid; k < m; k += nth) {
-            lc[k] = bv[k];
-            lh[k] = bv[CAP + k];
-            lv[k] = be[k];
-            le[k] = be[CAP + k];
-        }
-        if (tid == 0) {
-            s_n = m;
-            s_nb = 2 * K;
-            s_neval += 30ull * (unsigned long long)K;
-        }
+        neval += 30ull * (unsigned long long)K;
         __syncthreads();
     }
-    double V, E;
-    totals(s_n, V, E);
-    PcOut o{V, E, s_neval, s_status, s_rounds};
+    PcOut o{hv, he, neval, status, rounds};
     __syncthreads();
     return o;
 }
@@ -871,7 +892,10 @@ struct NbarEval {
         const int warp = threadIdx.x >> 5, nwarps = blockDim.x / 32;
         const double *h = A.hods + 6 * t.hod;
         const double *row = A.hmf + (size_t)t.z_ix * A.Nm;
-        for (int r0 = 2 * warp; r0 < nb; r0 += 2 * nwarps) {
+        // a lane keeps the sums of one of the warp's last 32 regions, whose errors are then
+        // formed together
+        double kv = 0, ke = 0, ka = 0, ks = 0;
+        for (int r0 = 2 * warp, step = 0; r0 < nb; r0 += 2 * nwarps, ++step) {
             const int r = r0 + half;
             const bool live = r < nb;
             double f = 0;
@@ -912,18 +936,29 @@ struct NbarEval {
                 if (!have) nbar_factors(A, h, gk_point(c, hw, hl), m, S, mix);
                 f = m * row[mix] * S;  // src/generalFunctions.cu:233-245
             }
-            double v, e;
-            rule_gk15_hw(f, hl, hw, v, e);
-            if (live && hl == 0) {
-                bv[r] = v;
-                be[r] = e;
+            const double t = rule_gk15_sums(f, hl, hw);
+            const int src = (lane & 1) * 16;
+            const double tv = __shfl_sync(0xffffffffu, t, src), te = __shfl_sync(0xffffffffu, t, src + 1);
+            const double ta = __shfl_sync(0xffffffffu, t, src + 2), ts = __shfl_sync(0xffffffffu, t, src + 3);
+            if ((lane >> 1) == (step & 15)) {
+                kv = tv;
+                ke = te;
+                ka = ta;
+                ks = ts;
+            }
+            if ((step & 15) == 15 || r0 + 2 * nwarps >= nb) {
+                const int rr = r0 + 2 * nwarps * ((lane >> 1) - (step & 15)) + (lane & 1);
+                if ((lane >> 1) <= (step & 15) && rr < nb) {
+                    bv[rr] = kv;
+                    be[rr] = rule_gk15_err(ke, ka, ks);
+                }
             }
         }
     }
 };
 
-// 16 warps per integral: the batch of a round (up to ~800 regions) takes a few passes
-constexpr int NBAR_THREADS = 512;
+// 8 warps per integral (16 measured slower: more threads at the barriers, no more FP64)
+constexpr int NBAR_THREADS = 256;
 
 template <int CAP>
 __global__ void __launch_bounds__(NBAR_THREADS) k_nbar(NbarArgs A, const NbarTask *__restrict__ tasks,
