@@ -562,7 +562,7 @@ __device__ PcOut gk_integrate_sorted(double lo, double hi, double *sm, const Eva
     long long *key = (long long *)bv;  // during a sort (the batch's values have been taken over)
     __shared__ int s_K, s_status;
     __shared__ double s_red[2][32], s_tot[2];
-    const int tid = threadIdx.x, nth = blockDim.x, nw = nth / 32;
+    const int tid = threadIdx.x, nth = blockDim.x, nw = nth / 32;  // nth = 256
     // deterministic block sums of val and err over the live regions: thread 0 the values,
     // thread 1 the errors
     auto totals = [&](int n, double &V, double &E) {
@@ -659,7 +659,29 @@ __device__ PcOut gk_integrate_sorted(double lo, double hi, double *sm, const Eva
         neval += 30ull * (unsigned long long)K;
         __syncthreads();
     }
-    PcOut o{hv, he, neval, status, rounds};
+    // The value as 512 strided partial sums over the regions in the order of the last sort, the
+    // children of its pops behind the rest: an order of its own, kept because a last-bit change
+    // of n_bar can tip an exact tie in the cubatures that divide by it.
+    {
+        const int m = n - 2 * K;  // regions the last round left (0 before the first)
+        auto at = [&](int p) {
+            if (rounds == 0) return p;
+            if (p < m) return ord[K + p];
+            const int b = p - m;
+            return (b & 1) ? n - K + (b >> 1) : ord[b >> 1];
+        };
+        double v[2] = {0, 0};
+        for (int h = 0; h < 2; ++h) {
+            for (int p = tid + h * 256; p < n; p += 512) v[h] += lv[at(p)];
+            for (int o = 16; o > 0; o >>= 1) v[h] += __shfl_down_sync(0xffffffffu, v[h], o);
+            if ((tid & 31) == 0) s_red[0][h * 8 + (tid >> 5)] = v[h];
+        }
+        __syncthreads();
+        hv = 0;
+        if (tid == 0)
+            for (int w = 0; w < 16; ++w) hv += s_red[0][w];
+    }
+    PcOut o{hv, he, neval, status, rounds};  // the value in thread 0
     __syncthreads();
     return o;
 }
@@ -756,14 +778,17 @@ __global__ void __launch_bounds__(THREADS) k_pc_integrate(const PkDev *__restric
 // the call, spread over the whole device and reproducing that arithmetic bit for bit;
 // the integrals then read them by node index and evaluate only deeper regions
 // themselves.  Either way a factor is the same expression of the same abscissa.
-constexpr int NBAR_DEPTH = 12;
+constexpr int NBAR_DEPTH = 9;
 constexpr int NBAR_NODES = (2 << NBAR_DEPTH) - 1;  // depths 0..NBAR_DEPTH
 // Below depth NBAR_DEPTH the refinement follows the mass-bin edges (the nearest-bin
 // lookup makes n(m, z) jump there; elsewhere the integrand is smooth): at every depth the
-// two children of the node that contains an edge.  k_nbar_deep evaluates those, for the
+// two children of the node that contains an edge.  k_nbar_factors evaluates those too, for the
 // Nm - 1 edges and depths NBAR_DEPTH + 1 .. NBAR_DEEP, by the same path arithmetic.
-constexpr int NBAR_DEEP = 44;
+constexpr int NBAR_DEEP = 20;
 constexpr int NBAR_NDEEP = NBAR_DEEP - NBAR_DEPTH;
+// (Depths measured over 1 to 128 vectors: 8 to 10 shallow within 2%, 12 up to 20% slower; deep
+// 44 / 36 / 28 / 20: 14.3 / 13.0 / 9.6 / 9.0 ms for 50 vectors -- most integrals stop above
+// depth 20, and what goes deeper is evaluated in place.)
 
 struct NbarTask {
     double lo, hi;
@@ -777,34 +802,34 @@ struct NbarArgs {
     double mmin, ln_mratio;  // mass bin = round(log(m / mmin) Nm / ln_mratio)
     double lo, hi;           // integration range in log10 m
     double inv_hw0;          // 1 / root half-width
-    // factors of node n of HOD h at abscissa i: [(h * NBAR_NODES + n) * 15 + i]
+    // Entry q: shallow node n at q = n; then the deep nodes, of edge e (e + 1 = the index whose
+    // bin starts there) at x = xm0 + (e + 0.5) dx, depth NBAR_DEPTH + 1 + dd, side s, at
+    // q = NBAR_NODES + (e * NBAR_NDEEP + dd) * 2 + s, with their node index at that depth in
+    // dkey.  At abscissa i: mass fm[q * 15 + i], bin fmix[q * 15 + i], and of HOD vector h
+    // N_c + N_s in fS[(h * nent + q) * 15 + i].
     double *fm, *fS;
     int *fmix;
-    // deep nodes: edge e (e + 1 = the index whose bin starts there) at x = xm0 + (e + 0.5) dx,
-    // depth NBAR_DEPTH + 1 + dd, side s: entry q = ((h * ne + e) * NBAR_NDEEP + dd) * 2 + s,
-    // its node index at that depth dkey[q], factors [q * 15 + i]
+    long long *dkey;
     double xm0, dx, inv_dx;
     int ne;
-    long long *dkey;
-    double *dm, *dS;
-    int *dmix;
+    long long nent;
 };
 
-constexpr size_t kNbarNodeBytes = 15 * (8 + 8 + 4);
-constexpr size_t kNbarDeepBytes = 8 + kNbarNodeBytes;  // key + factors
-
-// N_c + N_s (src/HOD.cu:35-76; erf taken once, the same argument in both) and the
-// nearest mass bin (src/NNMap_Model.cu:556) at x = log10 m
-__device__ __forceinline__ void nbar_factors(const NbarArgs &A, const double *h, double x,
-                                             double &m, double &S, int &mix)
+// m = 10^x and the nearest mass bin (src/NNMap_Model.cu:556) at x = log10 m
+__device__ __forceinline__ void nbar_mass(const NbarArgs &A, double x, double &m, int &mix)
 {
     m = pow(10.0, x);
-    const double e = erf(log(m / h[2]) / h[3] / 1.414213562);
-    const double Nc = 0.5 * h[1] * (1 + e);
-    const double Ns = 0.5 * (1 + e) * pow(m / h[4], h[5]);
-    S = Nc + Ns;
-    mix = (int)round(log(m / A.mmin) * A.Nm / A.ln_mratio);
+    mix = (int)round(ddiv(log(ddiv(m, A.mmin)) * A.Nm, A.ln_mratio));
     mix = min(max(mix, 0), A.Nm - 1);  // in range for every abscissa of the interval
+}
+
+// N_c + N_s at m (src/HOD.cu:35-76; erf taken once, the same argument in both)
+__device__ __forceinline__ double nbar_occupation(const double *h, double m)
+{
+    const double e = erf(ddiv(ddiv(log(ddiv(m, h[2])), h[3]), 1.414213562));
+    const double Nc = 0.5 * h[1] * (1 + e);
+    const double Ns = 0.5 * (1 + e) * pow(ddiv(m, h[4]), h[5]);
+    return Nc + Ns;
 }
 
 // centre and half-width of node n (heap numbering: root 0, children 2n+1 and 2n+2 the
@@ -822,61 +847,53 @@ __device__ __forceinline__ void nbar_node(double lo, double hi, int n, double &c
     }
 }
 
-// one thread per (HOD, node, abscissa)
+// The factor tables: one thread per (chunk of HOD vectors, entry, abscissa).  Entries are the
+// NBAR_NODES shallow nodes, then the deep ones (edge, depth, side): walk from the root
+// towards the edge (upper half when the edge is at or above the centre), then take the
+// child on that side.  The mass and its bin are the same for every HOD vector.
+constexpr int NBAR_HCHUNK = 8;
 __global__ void __launch_bounds__(256) k_nbar_factors(NbarArgs A, int nh)
 {
-    const long long total = (long long)nh * NBAR_NODES * 15;
+    const long long ndeep = (long long)A.ne * NBAR_NDEEP * 2, nent = NBAR_NODES + ndeep;
+    const int nchunk = (nh + NBAR_HCHUNK - 1) / NBAR_HCHUNK;
+    const long long total = (long long)nchunk * nent * 15;
     for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total;
          t += (long long)gridDim.x * blockDim.x) {
         const int i = (int)(t % 15);
-        const long long hn = t / 15;
-        const int n = (int)(hn % NBAR_NODES), h = (int)(hn / NBAR_NODES);
+        const long long q = t / 15 % nent;
+        const int h0 = (int)(t / 15 / nent) * NBAR_HCHUNK, h1 = min(nh, h0 + NBAR_HCHUNK);
         double c, hw;
-        nbar_node(A.lo, A.hi, n, c, hw);
-        double m, S;
-        int mix;
-        nbar_factors(A, A.hods + 6 * h, gk_point(c, hw, i), m, S, mix);
-        A.fm[t] = m;
-        A.fS[t] = S;
-        A.fmix[t] = mix;
-    }
-}
-
-// one thread per (HOD, edge, depth, side, abscissa): walk from the root towards the edge
-// (upper half when the edge is at or above the centre), then take the child on side s
-__global__ void __launch_bounds__(256) k_nbar_deep(NbarArgs A, int nh)
-{
-    const long long total = (long long)nh * A.ne * NBAR_NDEEP * 2 * 15;
-    for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total;
-         t += (long long)gridDim.x * blockDim.x) {
-        const int i = (int)(t % 15);
-        const long long q = t / 15;
-        const int side = (int)(q & 1);
-        const int dd = (int)((q >> 1) % NBAR_NDEEP);
-        const long long he = (q >> 1) / NBAR_NDEEP;
-        const int e = (int)(he % A.ne), h = (int)(he / A.ne);
-        const double xe = A.xm0 + (e + 0.5) * A.dx;
-        const int d = NBAR_DEPTH + 1 + dd;
-        double c = 0.5 * (A.lo + A.hi), hw = 0.5 * (A.hi - A.lo);
-        long long k = 0;
-        for (int l = 1; l < d; ++l) {  // to the depth-(d-1) node containing the edge
+        if (q < NBAR_NODES) {
+            nbar_node(A.lo, A.hi, (int)q, c, hw);
+        } else {
+            const long long qd = q - NBAR_NODES;
+            const int side = (int)(qd & 1);
+            const int dd = (int)((qd >> 1) % NBAR_NDEEP), e = (int)((qd >> 1) / NBAR_NDEEP);
+            const double xe = A.xm0 + (e + 0.5) * A.dx;
+            const int d = NBAR_DEPTH + 1 + dd;
+            c = 0.5 * (A.lo + A.hi);
+            hw = 0.5 * (A.hi - A.lo);
+            long long k = 0;
+            for (int l = 1; l < d; ++l) {  // to the depth-(d-1) node containing the edge
+                const double h2 = hw * 0.5;
+                const bool up = xe >= c;
+                c = up ? c + h2 : c - h2;
+                hw = h2;
+                k = 2 * k + (up ? 1 : 0);
+            }
             const double h2 = hw * 0.5;
-            const bool up = xe >= c;
-            c = up ? c + h2 : c - h2;
+            c = side ? c + h2 : c - h2;
             hw = h2;
-            k = 2 * k + (up ? 1 : 0);
+            if (i == 0 && h0 == 0) A.dkey[qd] = 2 * k + side;
         }
-        const double h2 = hw * 0.5;
-        c = side ? c + h2 : c - h2;
-        hw = h2;
-        k = 2 * k + side;
-        double m, S;
+        double m;
         int mix;
-        nbar_factors(A, A.hods + 6 * h, gk_point(c, hw, i), m, S, mix);
-        A.dm[t] = m;
-        A.dS[t] = S;
-        A.dmix[t] = mix;
-        if (i == 0) A.dkey[q] = k;
+        nbar_mass(A, gk_point(c, hw, i), m, mix);
+        if (h0 == 0) {
+            A.fm[q * 15 + i] = m;
+            A.fmix[q * 15 + i] = mix;
+        }
+        for (int h = h0; h < h1; ++h) A.fS[((long long)h * nent + q) * 15 + i] = nbar_occupation(A.hods + 6 * h, m);
     }
 }
 
@@ -908,38 +925,33 @@ struct NbarEval {
                               (int)((__double_as_longlong(hw) >> 52) & 0x7ff);
                 double m, S;
                 int mix;
-                bool have = false;
+                long long q = -1;  // entry of the region's node
+                const long long k = (long long)floor((c - A.lo) * ldexp(A.inv_hw0, d - 1));
                 if (d >= 0 && d <= NBAR_DEPTH) {
-                    const long long k = (long long)floor((c - A.lo) * ldexp(A.inv_hw0, d - 1));
-                    const long long n = (1ll << d) - 1 + k;
-                    const size_t q = ((size_t)t.hod * NBAR_NODES + n) * 15 + hl;
-                    m = A.fm[q];
-                    S = A.fS[q];
-                    mix = A.fmix[q];
-                    have = true;
+                    q = (1ll << d) - 1 + k;
                 } else if (d > NBAR_DEPTH && d <= NBAR_DEEP) {
                     // a node on the path to the nearest mass-bin edge, if it is one
-                    const long long k = (long long)floor((c - A.lo) * ldexp(A.inv_hw0, d - 1));
                     const int e = (int)floor((c - A.xm0) * A.inv_dx);
                     if (e >= 0 && e < A.ne) {
-                        const long long q =
-                            (((long long)t.hod * A.ne + e) * NBAR_NDEEP + (d - NBAR_DEPTH - 1)) * 2 +
-                            (k & 1);
-                        if (A.dkey[q] == k) {
-                            m = A.dm[q * 15 + hl];
-                            S = A.dS[q * 15 + hl];
-                            mix = A.dmix[q * 15 + hl];
-                            have = true;
-                        }
+                        const long long qd =
+                            ((long long)e * NBAR_NDEEP + (d - NBAR_DEPTH - 1)) * 2 + (k & 1);
+                        if (A.dkey[qd] == k) q = NBAR_NODES + qd;
                     }
                 }
-                if (!have) nbar_factors(A, h, gk_point(c, hw, hl), m, S, mix);
+                if (q >= 0) {
+                    m = A.fm[q * 15 + hl];
+                    mix = A.fmix[q * 15 + hl];
+                    S = A.fS[((long long)t.hod * A.nent + q) * 15 + hl];
+                } else {
+                    nbar_mass(A, gk_point(c, hw, hl), m, mix);
+                    S = nbar_occupation(h, m);
+                }
                 f = m * row[mix] * S;  // src/generalFunctions.cu:233-245
             }
-            const double t = rule_gk15_sums(f, hl, hw);
+            const double sm = rule_gk15_sums(f, hl, hw);
             const int src = (lane & 1) * 16;
-            const double tv = __shfl_sync(0xffffffffu, t, src), te = __shfl_sync(0xffffffffu, t, src + 1);
-            const double ta = __shfl_sync(0xffffffffu, t, src + 2), ts = __shfl_sync(0xffffffffu, t, src + 3);
+            const double tv = __shfl_sync(0xffffffffu, sm, src), te = __shfl_sync(0xffffffffu, sm, src + 1);
+            const double ta = __shfl_sync(0xffffffffu, sm, src + 2), ts = __shfl_sync(0xffffffffu, sm, src + 3);
             if ((lane >> 1) == (step & 15)) {
                 kv = tv;
                 ke = te;
@@ -1203,7 +1215,7 @@ void free_nbar_device(NbarDevice &W)
 }
 
 namespace {
-constexpr int kNbarChunk = 64;  // HOD vectors per launch (157 MB of factor tables)
+constexpr int kNbarChunk = 64;  // HOD vectors per launch (29 MB of factor tables)
 constexpr int kNbarCapSmall = 1024;      // live regions of the first pass
 }  // namespace
 
@@ -1240,20 +1252,17 @@ int n_bar_device(NbarDevice &W, const Binning &B, const double *d_hmf, const dou
             PC_CK(cudaMalloc(&W.idx, sizeof(int) * ntask));
             W.ntask_cap = (size_t)ntask;
         }
-        if ((size_t)nk > W.nhod_cap) {  // HOD vectors and their factor tables
+        const size_t nent = NBAR_NODES + (size_t)(B.Nm - 1) * NBAR_NDEEP * 2;  // nodes in the tables
+        if ((size_t)nk > W.nhod_cap) {  // HOD vectors and the factor tables
             if (W.hods) cudaFree(W.hods);
             if (W.cache) cudaFree(W.cache);
             W.hods = nullptr;
             W.cache = nullptr;
             W.nhod_cap = 0;
             PC_CK(cudaMalloc((void **)&W.hods, sizeof(double) * 6 * nk));
-            PC_CK(cudaMalloc(&W.cache, (size_t)nk * (NBAR_NODES * kNbarNodeBytes +
-                                                     (size_t)(B.Nm - 1) * NBAR_NDEEP * 2 *
-                                                         kNbarDeepBytes) +
-                                   8));  // + alignment of the deep keys
+            PC_CK(cudaMalloc(&W.cache, nent * (8 + 15 * (8 + 4)) + nent * 15 * 8 * (size_t)nk));
             W.nhod_cap = (size_t)nk;
         }
-        const size_t E = (size_t)W.nhod_cap * NBAR_NODES * 15;
         NbarArgs A{};
         A.hmf = d_hmf;
         A.hods = W.hods;
@@ -1263,31 +1272,24 @@ int n_bar_device(NbarDevice &W, const Binning &B, const double *d_hmf, const dou
         A.lo = lo;
         A.hi = hi;
         A.inv_hw0 = 1.0 / (0.5 * (hi - lo));
-        A.fm = (double *)W.cache;
-        A.fS = A.fm + E;
-        A.fmix = (int *)(A.fS + E);
+        A.nent = (long long)nent;
+        A.dkey = (long long *)W.cache;
+        A.fm = (double *)(A.dkey + nent);
+        A.fS = A.fm + nent * 15;
+        A.fmix = (int *)(A.fS + (size_t)W.nhod_cap * nent * 15);
         // deep nodes along the mass-bin edges
         A.xm0 = std::log10(B.mmin);
         A.dx = std::log(B.mmax / B.mmin) / (std::log(10.0) * B.Nm);
         A.inv_dx = 1 / A.dx;
         A.ne = B.Nm - 1;
-        const size_t E2 = (size_t)W.nhod_cap * A.ne * NBAR_NDEEP * 2;
-        A.dkey = (long long *)(A.fmix + E + (E & 1));  // 8-byte aligned
-        A.dm = (double *)(A.dkey + E2);
-        A.dS = A.dm + E2 * 15;
-        A.dmix = (int *)(A.dS + E2 * 15);
         PC_CK(cudaMemcpyAsync(W.tasks, tasks.data(), sizeof(NbarTask) * ntask,
                               cudaMemcpyHostToDevice, s));
         PC_CK(cudaMemcpyAsync(W.hods, hods + (size_t)6 * h0, sizeof(double) * 6 * nk,
                               cudaMemcpyHostToDevice, s));
         {
-            const long long nthr = (long long)nk * NBAR_NODES * 15;
+            const long long nthr = (long long)((nk + NBAR_HCHUNK - 1) / NBAR_HCHUNK) * nent * 15;
             const int grid = (int)std::min<long long>((nthr + 255) / 256, (long long)nsm * 16);
             k_nbar_factors<<<grid, 256, 0, s>>>(A, nk);
-            PC_CK(cudaGetLastError());
-            const long long nthr2 = (long long)nk * A.ne * NBAR_NDEEP * 2 * 15;
-            const int grid2 = (int)std::min<long long>((nthr2 + 255) / 256, (long long)nsm * 16);
-            if (nthr2 > 0) k_nbar_deep<<<grid2, 256, 0, s>>>(A, nk);
             PC_CK(cudaGetLastError());
         }
         k_nbar<kNbarCapSmall><<<std::min(ntask, nsm * 2), NBAR_THREADS, nbar_smem(kNbarCapSmall), s>>>(
