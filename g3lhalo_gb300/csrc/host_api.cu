@@ -1531,6 +1531,7 @@ try {
 int g3l_set_correlation(g3l_ctx *c, double A, double eps)
 {
     if (!c || !std::isfinite(A) || !std::isfinite(eps)) return G3L_ERR_INVALID;
+    if (A == c->A && eps == c->eps) return G3L_OK;  // the graphs hold these values already
     c->A = A;
     c->eps = eps;
     c->T.A = A;
