@@ -20,6 +20,7 @@
 #include <cuda_runtime.h>
 
 #include "g3l_device.cuh"
+#include "idiv64.cuh"
 
 namespace g3l {
 
@@ -85,45 +86,84 @@ struct SelShared {
     unsigned long long ured[SEL_WARPS];
     float fred[2 * SEL_WARPS];
     int ired[2][SEL_WARPS];
-    int odd, ubits;
+    int ubits, cancel;
+    // set between the totals and the selection, each by one thread
+    double scale;                    // 2^60 / E
+    unsigned long long qthr, kcap;   // rtol |V| in units of 1 / scale; budget's region count
+    double tau_thr, tau_sel;         // the two tolerances times |V|
 };
 
-// Block sums of two doubles (in block_sum's order) and of the two FP32 bounds, which stay
-// in sh.fred[0], sh.fred[1]; sh.odd: any odd.
-__device__ void block_totals(double sv, double se, float fue, float fuv, bool odd, SelShared &sh,
-                             double &V, double &E)
+// Block sums of two doubles (in block_sum's order) and of two FP32 values, over R regions
+// (zeros from the threads without one); returns any odd.  The two doubles are added in one
+// instruction, one in each half of the warp, and the warps without a region add nothing:
+// on a pipe that issues one FP64 instruction per 64 cycles the additions are the time.
+__device__ bool block_totals(double sv, double se, float fue, float fuv, bool odd, int R, SelShared &sh,
+                             double &V, double &E, float &UE, float &UV)
 {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    for (int o = 16; o > 0; o >>= 1) {
-        sv += __shfl_down_sync(0xffffffffu, sv, o);
-        se += __shfl_down_sync(0xffffffffu, se, o);
-        fue += __shfl_down_sync(0xffffffffu, fue, o);
-        fuv += __shfl_down_sync(0xffffffffu, fuv, o);
-    }
-    if (lane == 0) {
-        sh.dred[warp] = sv;
-        sh.dred[SEL_WARPS + warp] = se;
-        sh.fred[warp] = fue;
-        sh.fred[SEL_WARPS + warp] = fuv;
-    }
-    odd = __syncthreads_or(odd);
-    double r = 0;
-    float f = 0.f;
-    if (threadIdx.x < 2) {
-        for (int w = 0; w < SEL_WARPS; ++w) {
-            r += sh.dred[threadIdx.x * SEL_WARPS + w];
-            f += sh.fred[threadIdx.x * SEL_WARPS + w];
+    const int nw = min(SEL_WARPS, (R + 31) >> 5);
+    if (warp < nw) {
+        double x = lane < 16 ? sv : se;
+        x += __shfl_xor_sync(0xffffffffu, lane < 16 ? se : sv, 16);
+        for (int o = 8; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o, 16);
+        for (int o = 16; o > 0; o >>= 1) {
+            fue += __shfl_down_sync(0xffffffffu, fue, o);
+            fuv += __shfl_down_sync(0xffffffffu, fuv, o);
+        }
+        if ((lane & 15) == 0) sh.dred[(lane >> 4) * SEL_WARPS + warp] = x;
+        if (lane == 0) {
+            sh.fred[warp] = fue;
+            sh.fred[SEL_WARPS + warp] = fuv;
         }
     }
-    __syncthreads();
-    if (threadIdx.x < 2) {
-        sh.dred[threadIdx.x] = r;
-        sh.fred[threadIdx.x] = f;
+    odd = __syncthreads_or(odd);
+    UE = sh.fred[0];
+    UV = sh.fred[SEL_WARPS];
+    for (int w = 1; w < nw; ++w) {
+        UE += sh.fred[w];
+        UV += sh.fred[SEL_WARPS + w];
     }
-    if (threadIdx.x == 0) sh.odd = odd;
-    __syncthreads();
+    if (nw > 1) {
+        double r = 0;
+        if (threadIdx.x < 2)
+            for (int w = 0; w < nw; ++w) r += sh.dred[threadIdx.x * SEL_WARPS + w];
+        __syncthreads();
+        if (threadIdx.x < 2) sh.dred[threadIdx.x * SEL_WARPS] = r;
+        __syncthreads();
+    }
     V = sh.dred[0];
-    E = sh.dred[1];
+    E = sh.dred[SEL_WARPS];
+    return odd;
+}
+
+// One warp finds the boundary among n <= 32 candidates (sh.ck, sh.cq); sa, ca: sum and count
+// of the keys above them all.
+__device__ void rank_candidates(SelShared &sh, int n, bool by_sum, unsigned long long need,
+                                unsigned long long sa, unsigned int ca)
+{
+    const int lane = threadIdx.x & 31;
+    const unsigned long long k = lane < n ? sh.ck[lane] : 0, v = lane < n ? sh.cq[lane] : 0;
+    unsigned long long gt = 0, ge = 0;
+    unsigned int ngt = 0, nge = 0;
+    for (int j = 0; j < n; ++j) {
+        const unsigned long long kj = sh.ck[j], vj = sh.cq[j];
+        if (kj > k) {
+            gt += vj;
+            ++ngt;
+        }
+        if (kj >= k) {
+            ge += vj;
+            ++nge;
+        }
+    }
+    const unsigned long long from = by_sum ? sa : ca;
+    // (the largest or smallest key where `need` lies outside the total)
+    if (lane < n && (from + gt < need || ngt == 0) && (from + ge >= need || nge == (unsigned)n)) {
+        sh.bkey = k;
+        sh.qb = v;
+        sh.cnt_above = ca + ngt;
+        sh.sum_above = sa + (by_sum ? gt : 0);
+    }
 }
 
 // Boundary of a selection of the largest keys of one integral (err: keys as doubles >= 0,
@@ -136,7 +176,8 @@ __device__ void block_totals(double sv, double se, float fue, float fuv, bool od
 // itself start with bytes of sign and exponent that nearly all keys share, and the 64-bit
 // atomics of a whole integral then queue at one or two addresses (8 such passes were most
 // of k_select's time).  The boundary bucket is narrowed the same way until it holds at most
-// 32 keys, which one warp ranks.  All sums are integers: the result does not depend on the
+// 32 keys, which one warp ranks; an integral of at most 32 regions needs only that (every
+// round of a small look, and the first ones of any).  All sums are integers: the result does not depend on the
 // order of the threads.
 __device__ void boundary_select(const double *err, const unsigned long long *q, long long base, int R,
                                 bool by_sum, unsigned long long need, SelShared &sh,
@@ -144,6 +185,23 @@ __device__ void boundary_select(const double *err, const unsigned long long *q, 
                                 unsigned long long &sum_above, unsigned long long &qb)
 {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    if (R <= 32) {
+        if (tid < 32) {
+            if (lane < R) {
+                sh.ck[lane] = ekey(err, base + lane);
+                sh.cq[lane] = by_sum ? q[base + lane] : 1ull;
+            }
+            __syncwarp();
+            rank_candidates(sh, R, by_sum, need, 0, 0);
+        }
+        __syncthreads();
+        bkey = sh.bkey;
+        qb = sh.qb;
+        cnt_above = sh.cnt_above;
+        sum_above = sh.sum_above;
+        __syncthreads();
+        return;
+    }
     unsigned long long kmn = ~0ull, kmx = 0;
     for (int j = tid; j < R; j += SEL_BS) {
         const unsigned long long k = ekey(err, base + j);
@@ -256,31 +314,7 @@ __device__ void boundary_select(const double *err, const unsigned long long *q, 
                 }
             }
             __syncthreads();
-            if (tid < 32) {
-                const int n = min((int)sh.ncand, 32);
-                const unsigned long long k = lane < n ? sh.ck[lane] : 0, v = lane < n ? sh.cq[lane] : 0;
-                unsigned long long gt = 0, ge = 0;
-                unsigned int ngt = 0, nge = 0;
-                for (int j = 0; j < n; ++j) {
-                    const unsigned long long kj = sh.ck[j], vj = sh.cq[j];
-                    if (kj > k) {
-                        gt += vj;
-                        ++ngt;
-                    }
-                    if (kj >= k) {
-                        ge += vj;
-                        ++nge;
-                    }
-                }
-                const unsigned long long from = by_sum ? sa : ca;
-                // (the largest or smallest key where `need` lies outside the total)
-                if (lane < n && (from + gt < need || ngt == 0) && (from + ge >= need || nge == (unsigned)n)) {
-                    sh.bkey = k;
-                    sh.qb = v;
-                    sh.cnt_above = ca + ngt;
-                    sh.sum_above = sa + (by_sum ? gt : 0);
-                }
-            }
+            if (tid < 32) rank_candidates(sh, min((int)sh.ncand, 32), by_sum, need, sa, ca);
             __syncthreads();
             sa = sh.sum_above;
             ca = sh.cnt_above;
@@ -344,20 +378,21 @@ __global__ void __launch_bounds__(SEL_BS) k_select(const IntDesc *__restrict__ D
 {
     __shared__ SelShared sh;
     __shared__ int s_flag[4];  // fin, status, polish passes
-    __shared__ double s_tot[4];
-    __shared__ int s_cancel;
+    __shared__ double s_tot[2];
     // threshold guard (mixed precision): bound multiplier (gthr) and the value bounds' basis
-    const double gthr = H->mixed ? (double)H->thr_ratio : 0.0;
-    const double vr = (double)H->val_ratio;
+    const bool mixed = H->mixed;
+    const float gthr32 = mixed ? H->thr_ratio : 0.f, vr32 = H->val_ratio;
+    const bool guard = gthr32 > 0.f;
+    const double gthr = (double)gthr32, vr = (double)vr32;
     const int end = H->gbeg[NGROUPS];
     // a stop request: k_scan's (cancel or deadline), or a host cancel that arrived since
-    // (one read of the host-mapped word per block)
-    if (threadIdx.x == 0) {
+    // (one read of the host-mapped word per block, by a warp that is not waited for before
+    // the totals' barrier)
+    if (threadIdx.x == SEL_BS - 1) {
         int cz = H->cancel;
         if (!cz && H->cancel_word && *H->cancel_word) cz = 1;
-        s_cancel = cz;
+        sh.cancel = cz;
     }
-    __syncthreads();
     for (int i = H->gbeg[0] + blockIdx.x; i < end; i += gridDim.x) {
         if (pass == 1 && !S[i].defer) continue;  // block-uniform
         __syncthreads();
@@ -369,6 +404,9 @@ __global__ void __launch_bounds__(SEL_BS) k_select(const IntDesc *__restrict__ D
         const IntDesc &d = D[i];
         const long long base = d.base;
         const int R = S[i].nR;
+        const double rtol = d.rtol, err0 = S[i].err;
+        const unsigned long long neval = S[i].neval, max_eval = d.max_eval;
+        const int npts = d.npts;
         if (R == 0) {
             // fresh integral: its root region is this round's single work item (every warp has
             // to have read nR before it changes)
@@ -377,7 +415,7 @@ __global__ void __launch_bounds__(SEL_BS) k_select(const IntDesc *__restrict__ D
                 P.cand[base] = -1;
                 S[i].K = 1;
                 S[i].nR = 1;
-                S[i].neval = (unsigned long long)d.npts;
+                S[i].neval = (unsigned long long)npts;
             }
             __syncthreads();
             continue;
@@ -387,7 +425,7 @@ __global__ void __launch_bounds__(SEL_BS) k_select(const IntDesc *__restrict__ D
         // instructions of a pipe that issues one per 64 cycles, so it is first bounded in
         // FP32 from the operands' leading bits, relative to 2^-sref, and summed in FP64 only
         // where that does not settle the comparison.
-        const double eref = S[i].err > 0 ? S[i].err : P.err[base];
+        const double eref = __double_as_longlong(err0) > 0 ? err0 : P.err[base];
         const int sref = 1023 - (int)(((unsigned long long)__double_as_longlong(eref) >> 52) & 0x7ffu);
         double sv = 0, se = 0;
         float fue = 0.f, fuv = 0.f;
@@ -396,17 +434,43 @@ __global__ void __launch_bounds__(SEL_BS) k_select(const IntDesc *__restrict__ D
             const double v = P.val[base + j], e = P.err[base + j];
             sv += v;
             se += e;
-            if (gthr > 0.0) {
+            if (guard) {
                 fue = fmaf(f32_scaled(e, sref, odd), P.unc[base + j], fue);
                 fuv = fmaf(f32_scaled(fabs(v), sref, odd), P.uval[base + j], fuv);
             }
         }
         double V, E;
-        block_totals(sv, se, fue, fuv, odd, sh, V, E);
+        float fue_all, fuv_all;
+        odd = block_totals(sv, se, fue, fuv, odd, R, sh, V, E, fue_all, fuv_all);
+        // The selection's scalars, each by one thread of a warp of its own (a warp's FP64
+        // instruction costs the pipe the same for one lane as for 32, and all eight warps
+        // forming them would queue for it), beside thread 0's convergence test.
+        if (threadIdx.x == 32) {
+            const double sc = ddiv(1152921504606846976.0, E);  // fixed-point errors: floor(err * scale)
+            const double thr = fabs(V) * rtol * sc;
+            sh.scale = sc;
+            sh.qthr = thr >= 1.8e19 ? 0xFFFFFFFFFFFFFFFFull : (unsigned long long)thr;
+        } else if (threadIdx.x == 64) {
+            unsigned long long kc = (unsigned long long)R;
+            const unsigned long long twoNp = 2ull * (unsigned long long)npts;
+            if (max_eval > neval) {
+                const unsigned long long k = (max_eval - neval + twoNp - 1) / twoNp;
+                if (k < kc) kc = k;
+            }
+            sh.kcap = kc;
+            sh.tau_thr = H->tau_thr * fabs(V);
+            sh.tau_sel = tau_sel * fabs(V);
+        }
+        // the FP32 bound of the uncertainty each comparison below has, in units of 2^-sref:
+        // one that does not lie within 0.1% of the FP32 bound is settled by it, the others
+        // (and operands FP32 does not hold) take the FP64 sums
+        const float fV = (float)rtol * vr32 * fuv_all, fU = gthr32 * (fue_all + fV);
+        // 0: dist > bound, 1: dist <= bound, 2: not told apart
+        auto within = [&](float dist, float bound, bool odd) {
+            return odd || !(bound > 1e-30f) || !(bound < 1e30f) || !(fabsf(dist - bound) > 1e-3f * bound)
+                       ? 2 : (int)(dist <= bound);
+        };
         // FP64 totals of the uncertainty, formed on demand
-        const double f2 = ldexp(1.0, -sref);  // unit of the FP32 bounds
-        const double fUE = gthr * (double)sh.fred[0] * f2, fUV = gthr * vr * (double)sh.fred[1] * f2;
-        const bool fodd = sh.odd != 0 || !(fUE < 1e300) || !(fUV < 1e300);
         auto exact_unc = [&](double &UE, double &UV) {
             double sue = 0, suv = 0;
             for (int j = threadIdx.x; j < R; j += SEL_BS) {
@@ -417,19 +481,22 @@ __global__ void __launch_bounds__(SEL_BS) k_select(const IntDesc *__restrict__ D
             UV = gthr * vr * block_sum(suv, sh.dred);
         };
         if (threadIdx.x == 0) {
-            IntState st = S[i];
+            const auto expo = [](double x) { return ((unsigned long long)__double_as_longlong(x) >> 52) & 0x7ffu; };
+            const bool finite = expo(V) != 0x7ffu && expo(E) != 0x7ffu;
+            const double gate = fabs(V) * rtol;
+            const int rounds = S[i].rounds, cancel = sh.cancel;
             int fin = 0, status = ST_OK;
-            if (s_cancel) {
+            if (cancel) {
                 fin = 1;
-                status = s_cancel == 2 ? ST_DEADLINE : ST_CANCELLED;
-            } else if (!isfinite(V) || !isfinite(E)) {
+                status = cancel == 2 ? ST_DEADLINE : ST_CANCELLED;
+            } else if (!finite) {
                 fin = 1;
                 status = ST_NONFINITE;
-            } else if (d.max_eval && st.neval >= d.max_eval) {
+            } else if (max_eval && neval >= max_eval) {
                 fin = 1;
-            } else if (!(E > 0 && E > fabs(V) * d.rtol)) {
+            } else if (!(E > 0 && E > gate)) {
                 fin = 1;  // converged (src/converged.h:10-14 with reqAbsError = 0)
-            } else if (st.rounds >= H->max_rounds) {
+            } else if (rounds >= H->max_rounds) {
                 fin = 1;
                 status = ST_ROUNDS;
             }
@@ -437,17 +504,16 @@ __global__ void __launch_bounds__(SEL_BS) k_select(const IntDesc *__restrict__ D
             S[i].err = E;
             s_flag[0] = fin;
             s_flag[1] = status;
-            s_flag[2] = st.pad;  // polish passes so far
+            s_flag[2] = S[i].pad;  // polish passes so far
             s_tot[0] = V;
             s_tot[1] = E;
-            const bool tested = !s_cancel && isfinite(V) && isfinite(E) &&
-                                !(d.max_eval && st.neval >= d.max_eval);
             // the convergence test E <= rtol |V| decided within the FP32 uncertainty: 1 = yes,
             // 2 = the FP32 bound of the uncertainty does not tell
             s_flag[3] = 0;
-            if (gthr > 0.0 && tested) {
-                const double dist = fabs(E - fabs(V) * d.rtol), f = fUE + d.rtol * fUV;
-                s_flag[3] = fodd || (dist > 0.999 * f && dist < 1.001 * f) || !(f > 0.0) ? 2 : dist <= f;
+            if (guard && !cancel && finite && !(max_eval && neval >= max_eval)) {
+                bool od = odd;
+                const float dist = f32_scaled(fabs(E - gate), sref, od);
+                s_flag[3] = within(dist, fU, od);
             }
         }
         __syncthreads();
@@ -455,16 +521,16 @@ __global__ void __launch_bounds__(SEL_BS) k_select(const IntDesc *__restrict__ D
             double UE, UV;
             exact_unc(UE, UV);
             if (threadIdx.x == 0)
-                s_flag[3] = (UE + d.rtol * UV) > 0.0 &&
-                            fabs(s_tot[1] - fabs(s_tot[0]) * d.rtol) <= UE + d.rtol * UV;
+                s_flag[3] = (UE + rtol * UV) > 0.0 &&
+                            fabs(s_tot[1] - fabs(s_tot[0]) * rtol) <= UE + rtol * UV;
             __syncthreads();
         }
         if (s_flag[3]) {
-            const double margin = fabs(s_tot[1] - fabs(s_tot[0]) * d.rtol);
+            const double margin = fabs(s_tot[1] - fabs(s_tot[0]) * rtol);
             double ul = 0;
             for (int j = threadIdx.x; j < R; j += SEL_BS) {
                 const double kj = gthr * (P.err[base + j] * (double)P.unc[base + j] +
-                                         d.rtol * vr * fabs(P.val[base + j]) * (double)P.uval[base + j]);
+                                         rtol * vr * fabs(P.val[base + j]) * (double)P.uval[base + j]);
                 P.key[base + j] = kj;
                 ul += kj;
             }
@@ -477,7 +543,7 @@ __global__ void __launch_bounds__(SEL_BS) k_select(const IntDesc *__restrict__ D
             // If the regions' value bounds sum to more than tau_val |V|, re-evaluate in
             // FP64 the regions with the largest bounds until the rest is below half of it.
             bool polish = false;
-            if (H->mixed && tau_val > 0.0 && s_flag[1] == ST_OK && s_flag[2] < 2) {
+            if (mixed && tau_val > 0.0 && s_flag[1] == ST_OK && s_flag[2] < 2) {
                 const double Vt = s_tot[0];
                 double uloc = 0;
                 for (int j = threadIdx.x; j < R; j += SEL_BS) {
@@ -526,18 +592,8 @@ __global__ void __launch_bounds__(SEL_BS) k_select(const IntDesc *__restrict__ D
             __syncthreads();
             continue;
         }
-        V = s_tot[0];
-        E = s_tot[1];
-        const unsigned long long neval = S[i].neval;
-        const unsigned long long twoNp = 2ull * (unsigned long long)d.npts;
-        unsigned long long Kcap = (unsigned long long)R;
-        if (d.max_eval) {
-            unsigned long long left = d.max_eval - neval;  // > 0 here
-            unsigned long long kc = (left + twoNp - 1) / twoNp;
-            if (kc < Kcap) Kcap = kc;
-        }
-        // fixed-point errors: q = floor(err * 2^60 / E)
-        const double scale = 1152921504606846976.0 / E;  // 2^60 / E
+        const unsigned long long Kcap = sh.kcap;
+        const double scale = sh.scale;
         unsigned long long qs = 0;
         for (int j = threadIdx.x; j < R; j += SEL_BS) {
             const unsigned long long qq = floor_u64(P.err[base + j] * scale);
@@ -545,8 +601,7 @@ __global__ void __launch_bounds__(SEL_BS) k_select(const IntDesc *__restrict__ D
             qs += qq;
         }
         const unsigned long long Q = block_sum(qs, sh.ured);
-        const double thr = fabs(V) * d.rtol * scale;
-        const unsigned long long qthr = thr >= 1.8e19 ? 0xFFFFFFFFFFFFFFFFull : (unsigned long long)thr;
+        const unsigned long long qthr = sh.qthr;
         const unsigned long long need = Q > qthr ? Q - qthr : 0;
         // K_conv: smallest k >= 1 whose popped error sum reaches `need`
         unsigned long long Kconv;
@@ -567,41 +622,40 @@ __global__ void __launch_bounds__(SEL_BS) k_select(const IntDesc *__restrict__ D
             // the boundary, and rtol |V|), and the choice can matter (it moves a region of
             // error b, and neighbours only where the budget allows), re-evaluate the regions
             // carrying that uncertainty first.
-            const double b = __longlong_as_double((long long)bkey);
-            if (gthr > 0.0 && qb && Kconv <= Kcap && b > H->tau_thr * fabs(V)) {
+            if (guard && qb && Kconv <= Kcap && (long long)bkey > __double_as_longlong(sh.tau_thr)) {
                 const unsigned long long m_hi = sum_above + tneed * qb - need;  // < qb
                 const unsigned long long m_lo = qb - m_hi;
                 unsigned long long m = 0xFFFFFFFFFFFFFFFFull;
                 if (Kconv < Kcap && Kconv < (unsigned long long)R) m = m_hi;
                 if (Kconv > 1 && m_lo < m) m = m_lo;
                 if (m != 0xFFFFFFFFFFFFFFFFull) {
-                    const double m_abs = (double)m / scale;
-                    // the bound in FP32 first, as above
                     float fur = 0.f;
-                    bool od = false;
+                    bool od = odd;
                     for (int j = threadIdx.x; j < R; j += SEL_BS)
                         if (ekey(P.err, base + j) <= bkey)
                             fur = fmaf(f32_scaled(P.err[base + j], sref, od), P.unc[base + j], fur);
+                    const float m32 = (float)m * 8.67361738e-19f * f32_scaled(E, sref, od);  // m / scale
                     od = __syncthreads_or(od);
                     fur = block_sum(fur, sh.fred);
-                    const double f = gthr * (double)fur * f2 + d.rtol * fUV;
-                    double dlt = f;
-                    if (od || fodd || (m_abs > 0.999 * f && m_abs < 1.001 * f) || !(f > 0.0)) {
+                    int close = within(m32, gthr32 * (fur + fV), od);
+                    if (close == 2) {
                         double ur = 0, UE, UV;
                         for (int j = threadIdx.x; j < R; j += SEL_BS)
                             if (ekey(P.err, base + j) <= bkey)
                                 ur += P.err[base + j] * (double)P.unc[base + j];
                         ur = block_sum(ur, sh.dred);
                         exact_unc(UE, UV);
-                        dlt = gthr * ur + d.rtol * UV;
+                        const double dlt = gthr * ur + rtol * UV;
+                        close = dlt > 0.0 && (double)m / scale <= dlt;
                     }
-                    if (dlt > 0.0 && m_abs <= dlt) {
+                    if (close) {
+                        const double m_abs = (double)m / scale;
                         double ul = 0;
                         for (int j = threadIdx.x; j < R; j += SEL_BS) {
                             const double e = P.err[base + j];
                             const double kj =
                                 (ekey(P.err, base + j) <= bkey ? gthr * e * (double)P.unc[base + j] : 0.0) +
-                                d.rtol * gthr * vr * fabs(P.val[base + j]) * (double)P.uval[base + j];
+                                rtol * gthr * vr * fabs(P.val[base + j]) * (double)P.uval[base + j];
                             P.key[base + j] = kj;
                             ul += kj;
                         }
@@ -629,16 +683,14 @@ __global__ void __launch_bounds__(SEL_BS) k_select(const IntDesc *__restrict__ D
         // Mixed precision: if the boundary of this round's selection sits among regions
         // whose FP32-derived errors are uncertain (overlapping bounds), re-evaluate those
         // regions in FP64 first and select again next round.
-        if (H->mixed && K < (unsigned long long)R) {
-            const double b = __longlong_as_double((long long)bkey);
-            if (b > tau_sel * fabs(V)) {
+        if (mixed && K < (unsigned long long)R) {
+            if ((long long)bkey > __double_as_longlong(sh.tau_sel)) {
                 if (threadIdx.x == 0) sh.ubits = 0;
                 __syncthreads();
                 for (int j = threadIdx.x; j < R; j += SEL_BS)  // bounds are >= 0: order as integers
                     if (ekey(P.err, base + j) == bkey) atomicMax(&sh.ubits, __float_as_int(P.unc[base + j]));
                 __syncthreads();
                 const float ub = __int_as_float(sh.ubits);
-                const double blo = b * (1.0 - ub), bhi = b * (1.0 + ub);
                 // do the bounds of region j overlap the boundary's?  |key difference| 2^-52 is
                 // at most 2 |ln(e / b)|, and an overlap with bounds below 1/4 has |ln(e / b)| <=
                 // 2 (u + ub): what differs by more is told apart without FP64
@@ -646,7 +698,8 @@ __global__ void __launch_bounds__(SEL_BS) k_select(const IntDesc *__restrict__ D
                     const int dk = abs((int)((long long)(k >> 20) - (long long)(bkey >> 20)));
                     if (u < 0.25f && ub < 0.25f && (float)dk * 2.3283064e-10f > 4.1f * (u + ub) + 1e-6f)
                         return false;
-                    return e * (1.0 + u) >= blo && e * (1.0 - u) <= bhi;
+                    const double b = __longlong_as_double((long long)bkey);
+                    return e * (1.0 + u) >= b * (1.0 - ub) && e * (1.0 - u) <= b * (1.0 + ub);
                 };
                 bool some = false;
                 for (int j = threadIdx.x; j < R && !some; j += SEL_BS) {
@@ -717,7 +770,7 @@ __global__ void __launch_bounds__(SEL_BS) k_select(const IntDesc *__restrict__ D
                 const unsigned bs = __ballot_sync(0xffffffffu, sel);
                 if (sel) {
                     P.cand[base + pos + __popc(bs & lower)] = j;
-                    if (H->mixed && (P.split[base + j] & 0x80)) push_esc(H, P, pass, d.kind * 3 + d.term - 1, i, j);
+                    if (mixed && (P.split[base + j] & 0x80)) push_esc(H, P, pass, d.kind * 3 + d.term - 1, i, j);
                 }
                 pos += __popc(bs);
                 ties += __popc(be);
@@ -725,7 +778,7 @@ __global__ void __launch_bounds__(SEL_BS) k_select(const IntDesc *__restrict__ D
         }
         if (threadIdx.x == 0) {
             S[i].K = (int)K;
-            S[i].neval = neval + twoNp * K;
+            S[i].neval = neval + 2ull * (unsigned long long)npts * K;
             S[i].nR = R + (int)K;
             S[i].rounds += 1;
         }
@@ -738,27 +791,37 @@ __global__ void __launch_bounds__(1024) k_scan(IntState *__restrict__ S, long lo
                                                BatchHdr *H, cudaGraphConditionalHandle handle,
                                                int use_cond)
 {
-    __shared__ long long part[1024];
+    __shared__ long long part[32];
     const int beg = H->gbeg[0], n = H->gbeg[NGROUPS];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int per = (n - beg + blockDim.x - 1) / blockDim.x;
     const int b = beg + threadIdx.x * per, e = min(n, b + per);
     long long loc = 0;
     for (int i = b; i < e; ++i) loc += S[i].K;
-    part[threadIdx.x] = loc;
-    __syncthreads();
-    for (int o = 1; o < (int)blockDim.x; o <<= 1) {
-        long long t = threadIdx.x >= (unsigned)o ? part[threadIdx.x - o] : 0;
-        __syncthreads();
-        part[threadIdx.x] += t;
-        __syncthreads();
+    long long run = loc;  // inclusive sum over the threads
+    for (int o = 1; o < 32; o <<= 1) {
+        const long long t = __shfl_up_sync(0xffffffffu, run, o);
+        if (lane >= o) run += t;
     }
-    long long run = part[threadIdx.x] - loc;
+    if (lane == 31) part[warp] = run;
+    __syncthreads();
+    if (warp == 0) {
+        long long w = part[lane];
+        for (int o = 1; o < 32; o <<= 1) {
+            const long long t = __shfl_up_sync(0xffffffffu, w, o);
+            if (lane >= o) w += t;
+        }
+        part[lane] = w;
+    }
+    __syncthreads();
+    if (warp > 0) run += part[warp - 1];
+    run -= loc;
     for (int i = b; i < e; ++i) {
         woff[i] = run;
         run += S[i].K;
     }
     if (threadIdx.x == blockDim.x - 1) {
-        long long tot = part[blockDim.x - 1];
+        const long long tot = part[31];
         woff[n] = tot;
         H->total_work = tot;
         // Keep looping while there is work or a deferred FP64 re-evaluation.  The first stage's
