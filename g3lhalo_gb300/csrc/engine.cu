@@ -86,7 +86,7 @@ struct SelShared {
     unsigned long long ured[SEL_WARPS];
     float fred[2 * SEL_WARPS];
     int ired[2][SEL_WARPS];
-    int ubits, cancel;
+    int ubits;
     // set between the totals and the selection, each by one thread
     double scale;                    // 2^60 / E
     unsigned long long qthr, kcap;   // rtol |V| in units of 1 / scale; budget's region count
@@ -372,7 +372,14 @@ __device__ void escalate_keys(const IntDesc &d, IntState *S, const Pool &P, Batc
 // pass 0 selects for every live integral; pass 1 (mixed precision) selects again, in
 // the same round, for the integrals pass 0 deferred, once the FP64 re-evaluation of
 // their ambiguous boundary regions has run.
-__global__ void __launch_bounds__(SEL_BS) k_select(const IntDesc *__restrict__ D,
+//
+// An integral of few regions is latency: the reads, the FP64 scalars (each formed by one
+// warp), ~20 barriers.  One triplet at 30000 evaluations spends 14 us in a selection where it
+// spent 24 with all warps forming the scalars and every block, also those without an
+// integral, reading the host's cancel word first (call 2.05 -> 1.66 ms).  Blocks of 1024
+// threads for the large integrals of such calls are slower (1.66 -> 1.83 ms: their barriers),
+// and so are batched loads (more registers, fewer blocks).
+__global__ void __launch_bounds__(SEL_BS, 3) k_select(const IntDesc *__restrict__ D,
                                                    IntState *__restrict__ S, Pool P, BatchHdr *H,
                                                    double tau_sel, double tau_val, int pass)
 {
@@ -385,13 +392,13 @@ __global__ void __launch_bounds__(SEL_BS) k_select(const IntDesc *__restrict__ D
     const bool guard = gthr32 > 0.f;
     const double gthr = (double)gthr32, vr = (double)vr32;
     const int end = H->gbeg[NGROUPS];
-    // a stop request: k_scan's (cancel or deadline), or a host cancel that arrived since
-    // (one read of the host-mapped word per block, by a warp that is not waited for before
-    // the totals' barrier)
-    if (threadIdx.x == SEL_BS - 1) {
-        int cz = H->cancel;
-        if (!cz && H->cancel_word && *H->cancel_word) cz = 1;
-        sh.cancel = cz;
+    if (H->gbeg[0] + (int)blockIdx.x >= end) return;  // (before the read of host memory)
+    // a stop request: k_scan's (cancel or deadline), or a host cancel that arrived since (one
+    // read of the host-mapped word per block, not waited for before thread 0 needs it)
+    int stop = 0, host_stop = 0;
+    if (threadIdx.x == 0) {
+        stop = H->cancel;
+        if (H->cancel_word) host_stop = *H->cancel_word;
     }
     for (int i = H->gbeg[0] + blockIdx.x; i < end; i += gridDim.x) {
         if (pass == 1 && !S[i].defer) continue;  // block-uniform
@@ -484,7 +491,7 @@ __global__ void __launch_bounds__(SEL_BS) k_select(const IntDesc *__restrict__ D
             const auto expo = [](double x) { return ((unsigned long long)__double_as_longlong(x) >> 52) & 0x7ffu; };
             const bool finite = expo(V) != 0x7ffu && expo(E) != 0x7ffu;
             const double gate = fabs(V) * rtol;
-            const int rounds = S[i].rounds, cancel = sh.cancel;
+            const int rounds = S[i].rounds, cancel = stop ? stop : (host_stop ? 1 : 0);
             int fin = 0, status = ST_OK;
             if (cancel) {
                 fin = 1;
