@@ -716,6 +716,14 @@ struct Reeval {
     {
         return auxv(P) + (long long)P.rcap * AUX_MAX;
     }
+    __device__ static int ulist_cap(const Pool &P)
+    {
+        return P.rcap * (NCU + NCU3);
+    }
+    __device__ static uint32_t *ulist(const Pool &P)  // the stage's u_NFW tasks
+    {
+        return (uint32_t *)(mzv(P) + (long long)P.rcap * 3 * MZ_PAIRS * MZ_VALS);
+    }
     __device__ static double *mz(const Pool &P, int k, int mdim, uint32_t vv)
     {
         const int vm = (vv >> (3 * mdim)) & 7, vz = (vv >> (3 * (DIM - 1))) & 7;
@@ -730,6 +738,30 @@ struct Reeval {
         const int n = H->n_esc[stage][G] < cap ? H->n_esc[stage][G] : cap;
         return n < P.rcap ? n : P.rcap;
     }
+    // u_NFW tasks of m entries: [0, m NCU) the (l, m, z) combinations, then the k3 projections
+    static constexpr int NCU = ucache_nf(TERM) * UC_MAX, NCU3 = u3_nfun(TERM) * U3_MAX;
+    // Up to about a block of 64 tasks per SM the pass is one chain whatever the lanes do, and
+    // its tasks are taken as numbered (listing them costs a call of one triplet 1-2%).  From
+    // there on they are listed first (k_re_fill).
+    __device__ static bool u_listed(int m) { return m * (NCU + NCU3) > 64 * 128; }
+    // does the entry need combination j of function f (split only: those of the centre and one
+    // contender axis), and the k3 projection pr?
+    __device__ static bool need_uc(const Pool &P, const IntDesc &d, int2 ent, const ReTab<KIND, TERM> &tb,
+                                   int f, int j)
+    {
+        if (j >= tb.ucn[f]) return false;
+        if (ent.y >> 30) return true;
+        const uint32_t key = tb.ucl[f * UC_MAX + j];
+        const int vl = key & 7, vm = (key >> 3) & 7, vz = (key >> 6) & 7;
+        const unsigned cm = split_cmask(P, d, ent);
+        return (vl != 0) + (vm != 0) + (vz != 0) <= 1 &&
+               split_variant(cm, ucache_fun(KIND, TERM, f, 0), vl) &&
+               split_variant(cm, ucache_fun(KIND, TERM, f, 1), vm) && split_variant(cm, DIM - 1, vz);
+    }
+    __device__ static bool need_u3(const Pool &P, const IntDesc &d, int2 ent, int pr)
+    {
+        return (ent.y >> 30) || split_point(split_cmask(P, d, ent), pr, NAX);
+    }
     // coordinate of variant v of dimension dim of entry ent
     __device__ static double coord(const Pool &P, const IntDesc &d, int2 ent, int dim, int v)
     {
@@ -741,6 +773,45 @@ struct Reeval {
 
 __host__ __device__ constexpr long long warps_up(long long n) { return (n + 31) / 32 * 32; }
 
+// The u_NFW tasks are numbered over all entries alike, but a split-only entry needs a few of
+// them, and the FP64 pipe takes a warp's instruction in the same time for one lane as for 32
+// (11 of 32 were active in k_re_ucache, the largest of the passes).  So k_re_fill lists the
+// needed ones, packed over the whole queue, while its other blocks fill the slots: 220
+// triplets: 21 of 32 lanes, re-evaluations 22.5 -> 19.2 ms, call 49.1 -> 46.3 ms; 13 triplets
+// of two populations 5.3 -> 5.1 ms.  (A block listing its own share only leaves the device
+// uneven: 20.0-22.2 ms.  The same for the fill's own tasks gains nothing.)
+constexpr int RE_CHUNK = 1024;
+struct ReChunk {
+    int n, at;
+    uint16_t list[RE_CHUNK];
+};
+// chunk of a pass over `tasks` tasks by the whole grid, in units of a block's threads
+__device__ __forceinline__ int re_chunk_size(int tasks, int unit)
+{
+    const int c = tasks / (int)gridDim.x / unit * unit;
+    return c < unit ? unit : (c > RE_CHUNK ? RE_CHUNK : c);
+}
+// lists the needed tasks of [t0, t0 + size): their count
+template <class Need>
+__device__ __forceinline__ int re_gather(ReChunk &ck, int t0, int size, const Need &need)
+{
+    __syncthreads();
+    if (threadIdx.x == 0) ck.n = 0;
+    __syncthreads();
+    const int lane = threadIdx.x & 31;
+    for (int i0 = threadIdx.x - lane; i0 < size; i0 += blockDim.x) {
+        const int i = i0 + lane;
+        const bool on = i < size && need(t0 + i);
+        const unsigned b = __ballot_sync(0xffffffffu, on);
+        int at = 0;
+        if (lane == 0 && b) at = atomicAdd(&ck.n, __popc(b));
+        at = __shfl_sync(0xffffffffu, at, 0);
+        if (on) ck.list[at + __popc(b & ((1u << lane) - 1u))] = (uint16_t)i;
+    }
+    __syncthreads();
+    return ck.n;
+}
+
 template <int KIND, int TERM>
 __global__ void __launch_bounds__(128) k_re_fill(DevTables T, const IntDesc *__restrict__ D,
                                                  IntState *__restrict__ S, Pool P, BatchHdr *H,
@@ -748,6 +819,7 @@ __global__ void __launch_bounds__(128) k_re_fill(DevTables T, const IntDesc *__r
 {
     using R = Reeval<KIND, TERM>;
     using M = Model64<KIND, TERM>;
+    __shared__ ReChunk ck;
     // the second stage's queue of the previous round has been consumed
     if (stage == 0 && blockIdx.x == 0 && threadIdx.x == 0) H->n_esc[1][R::G] = 0;
     const int m = R::count(P, H, stage);
@@ -760,6 +832,32 @@ __global__ void __launch_bounds__(128) k_re_fill(DevTables T, const IntDesc *__r
     const long long b1 = warps_up((long long)m * NMS), b2 = b1 + (KIND == 0 ? b1 : 0);
     const long long nmz = warps_up((long long)m * NMZ), b3 = b2 + nmz, b4 = b3 + nmz;
     const long long tot = b4 + (long long)m * NLS;
+    // The u_NFW tasks of k_re_ucache, packed over the whole queue: listed by the other end of
+    // the grid, which has no task here in a round of few entries.
+    const int nu = R::u_listed(m) ? m * (R::NCU + R::NCU3) : 0;
+    const int usize = re_chunk_size(nu, 128);
+    const int ufirst = (int)(gridDim.x - 1 - blockIdx.x) * usize;
+    if (ufirst < nu) {
+        const ReTab<KIND, TERM> &tb =
+            *reinterpret_cast<const ReTab<KIND, TERM> *>(P.retab + R::G * RETAB_BYTES);
+        const auto need_u = [&](int t) {
+            const bool uc = t < m * R::NCU;
+            const int per = uc ? R::NCU : R::NCU3, t2 = uc ? t : t - m * R::NCU;
+            const int k = t2 / per, r = t2 - k * per;
+            if (k >= m) return false;
+            const int2 ent = Q[k];
+            return uc ? R::need_uc(P, D[ent.x], ent, tb, r / UC_MAX, r % UC_MAX)
+                      : R::need_u3(P, D[ent.x], ent, tb.u3list[r]);
+        };
+        uint32_t *U = R::ulist(P);
+        for (int t0 = ufirst; t0 < nu; t0 += (int)gridDim.x * usize) {
+            const int n = re_gather(ck, t0, usize, need_u);
+            if (threadIdx.x == 0) ck.at = atomicAdd(&H->n_ulist[R::G], n);
+            __syncthreads();
+            for (int u = threadIdx.x; u < n; u += blockDim.x)
+                if (ck.at + u < R::ulist_cap(P)) U[ck.at + u] = (uint32_t)(t0 + ck.list[u]);
+        }
+    }
     for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < tot;
          t += (long long)gridDim.x * blockDim.x) {
         if (t < b2) {
@@ -843,53 +941,47 @@ __global__ void __launch_bounds__(128) k_re_ucache(DevTables T, const IntDesc *_
     __shared__ double ex[3][64];
     const int m = R::count(P, H, stage);
     if (m == 0) return;
-    const long long b1 = warps_up((long long)m * NF * UC_MAX), nu = b1 + (long long)m * NU3 * U3_MAX;
+    const int b1 = m * R::NCU;
+    const bool listed = R::u_listed(m);
+    const int nu = listed ? min(H->n_ulist[R::G], R::ulist_cap(P)) : m * (R::NCU + R::NCU3);
     const long long a1 = warps_up((long long)m * R::NAUX);
     const long long na = a1 + (KIND == 0 ? (long long)m * TERM * NVAR : 0);
-    const long long nchunk = (nu + 63) / 64;
     // the auxiliary tasks start from the other end of the grid
     const long long first_aux = (long long)(gridDim.x - 1 - blockIdx.x) * blockDim.x;
-    if (blockIdx.x >= nchunk && first_aux >= na) return;  // no work here: skip the tables
+    if ((int)blockIdx.x * 64 >= nu && first_aux >= na) return;  // no work here: skip the tables
     const ReTab<KIND, TERM> &tb = load_retab<KIND, TERM>(P, tbuf);
     const int2 *Q = P.esc + H->esc_beg[R::G];
     Slot64 *SL = R::slots(P);
     double *UC = R::ucv(P), *U3C = R::u3v(P), *AX = R::auxv(P);
     const int part = threadIdx.x >> 6, q = threadIdx.x & 63;
-    for (long long c = blockIdx.x; c < nchunk; c += gridDim.x) {
-        const long long t = c * 64 + q;
+    const uint32_t *U = R::ulist(P);
+    const int tend = b1 + m * R::NCU3;
+    for (int u0 = (int)blockIdx.x * 64; u0 < nu; u0 += (int)gridDim.x * 64) {
         double kk = 1, r200 = 1, cc = 1, F = 1;
         double *out = nullptr;
+        const int t = u0 + q < nu ? (listed ? (int)U[u0 + q] : u0 + q) : tend;
         if (t < b1) {
-            const int k = (int)(t / (NF * UC_MAX)), r = (int)(t - (long long)k * NF * UC_MAX);
+            const int k = t / R::NCU, r = t - k * R::NCU;
             const int f = r / UC_MAX, j = r - f * UC_MAX;
-            if (k < m && j < tb.ucn[f]) {
-                const int2 ent = Q[k];
-                const IntDesc &d = D[ent.x];
+            const int2 ent = Q[k];
+            const IntDesc &d = D[ent.x];
+            if (listed || R::need_uc(P, d, ent, tb, f, j)) {
                 const uint32_t key = tb.ucl[f * UC_MAX + j];
                 const int vl = key & 7, vm = (key >> 3) & 7, vz = (key >> 6) & 7;
                 const int dl = ucache_fun(KIND, TERM, f, 0), dm = ucache_fun(KIND, TERM, f, 1);
-                bool need = true;
-                if (!(ent.y >> 30)) {  // combinations of the centre and one contender axis
-                    const unsigned cm = split_cmask(P, d, ent);
-                    need = (vl != 0) + (vm != 0) + (vz != 0) <= 1 && split_variant(cm, dl, vl) &&
-                           split_variant(cm, dm, vm) && split_variant(cm, ZD, vz);
-                }
-                if (need) {
-                    const Slot64 *base = SL + (long long)k * R::NS;
-                    M::ucached_args(T, d, f, base[dl * NVAR + vl], base[dm * NVAR + vm],
-                                    base[ZD * NVAR + vz],
-                                    R::mz(P, k, dm, ((uint32_t)vm << (3 * dm)) | ((uint32_t)vz << (3 * ZD))),
-                                    kk, r200, cc, F);
-                    out = UC + ((long long)k * UC_NF_MAX + f) * UC_MAX + j;
-                }
+                const Slot64 *base = SL + (long long)k * R::NS;
+                M::ucached_args(T, d, f, base[dl * NVAR + vl], base[dm * NVAR + vm], base[ZD * NVAR + vz],
+                                R::mz(P, k, dm, ((uint32_t)vm << (3 * dm)) | ((uint32_t)vz << (3 * ZD))),
+                                kk, r200, cc, F);
+                out = UC + ((long long)k * UC_NF_MAX + f) * UC_MAX + j;
             }
-        } else if (t < nu) {
-            const long long t2 = t - b1;
-            const int k = (int)(t2 / (NU3 * U3_MAX)), r = (int)(t2 - (long long)k * NU3 * U3_MAX);
-            const int f = r / U3_MAX, j = r - f * U3_MAX;
-            const int pr = tb.u3list[f * U3_MAX + j];  // every projection index is used (93)
+        } else if (t < tend) {
+            const int t2 = t - b1;
+            const int k = t2 / R::NCU3, r = t2 - k * R::NCU3;
             const int2 ent = Q[k];
-            if ((ent.y >> 30) || split_point(split_cmask(P, D[ent.x], ent), pr, R::NAX)) {
+            const int pr = tb.u3list[r];  // every projection index is used (93)
+            if (listed || R::need_u3(P, D[ent.x], ent, pr)) {
+                const int f = r / U3_MAX, j = r - f * U3_MAX;
                 const uint32_t vv = tb.sdesc[pr];
                 const Slot64 *base = SL + (long long)k * R::NS;
                 const Slot64 *sp[R::DIM];
@@ -1001,6 +1093,7 @@ __global__ void __launch_bounds__(128) k_re_finish(DevTables T, const IntDesc *_
     __shared__ __align__(16) unsigned char tbuf[sizeof(ReTab<KIND, TERM>)];
     __shared__ double vals[R::NP];
     const int m = R::count(P, H, stage);
+    if (blockIdx.x == 0 && threadIdx.x == 0) H->n_ulist[R::G] = 0;  // consumed by k_re_ucache
     if ((int)blockIdx.x >= m) return;  // no work here: skip the tables
     const ReTab<KIND, TERM> &tb = load_retab<KIND, TERM>(P, tbuf);
     const int2 *Q = P.esc + H->esc_beg[R::G];

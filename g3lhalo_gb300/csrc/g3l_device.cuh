@@ -234,7 +234,8 @@ __host__ __device__ constexpr long long reeval_scratch_group_bytes(int rcap)
     return ((long long)rcap * MAX_DIM * NVAR * reeval_slot_bytes + 255) / 256 * 256 +
            (long long)rcap * UC_NF_MAX * UC_MAX * 8 +
            (long long)rcap * U3_NF_MAX * U3_MAX * 8 + (long long)rcap * AUX_MAX * 8 +
-           (long long)rcap * 3 * MZ_PAIRS * MZ_VALS * 8;
+           (long long)rcap * 3 * MZ_PAIRS * MZ_VALS * 8 +
+           ((long long)rcap * (UC_NF_MAX * UC_MAX + U3_NF_MAX * U3_MAX) * 4 + 255) / 256 * 256;
 }
 
 // Header of one refinement loop, kept in device memory so one instantiated graph serves any
@@ -260,6 +261,7 @@ struct BatchHdr {
     // the first and by the second selection pass; the second stage's reuse the storage of
     // the first, which has been consumed by then),
     int n_esc[2][NGROUPS];
+    int n_ulist[NGROUPS];        //   and of its list of u_NFW tasks (k_re_fill to k_re_ucache)
     int esc_cap[NGROUPS];        //   capacity (the group's pool slots)
     long long esc_beg[NGROUPS];  //   and first entry in Pool::esc
     unsigned long long escalated;// statistics: regions re-evaluated in FP64

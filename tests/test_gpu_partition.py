@@ -95,3 +95,23 @@ def test_tables_over_bin_counts(bins):
     for k in ("g", "w", "dwdz", "P_lin", "conc", "hmf", "b_h"):
         a, b = np.asarray(r[k]), np.asarray(o[k])
         assert (np.abs(a - b) <= 1e-11 * np.abs(b)).all(), k
+
+
+# FP64 re-evaluations: few entries' u_NFW tasks are taken as numbered, those of a longer queue
+# listed first; the batched kernel (G3L_REEVAL_CAP=0) evaluates every point on its own.
+@pytest.mark.parametrize("kind", [G.NNMAP, G.NMAPMAP])
+@pytest.mark.parametrize("step", [200, 40, 4])
+def test_reevaluation_of_short_and_long_queues(setup, kind, step, monkeypatch):
+    c, _ = setup
+    specs = [(kind, t, 0, 1 if kind == G.NNMAP else 0, tuple(th), 1e-4, 150_000)
+             for th in W.triplets_all()[7::step] for t in (1, 2, 3)]
+    a = c.eval(specs, G.MIXED)
+    assert c.stats()["escalated"] > 0
+    monkeypatch.setenv("G3L_REEVAL_CAP", "0")
+    c2 = G.Context(make_tables(Nz=64, Nm=128, Nk=256), clamp_k=True)
+    c2.set_hod(0, W.hod_default())
+    c2.set_hod(1, W.hod_second())
+    b = c2.eval(specs, G.MIXED)
+    for k in SAME:
+        assert np.array_equal(a[k], b[k]), k
+    c2.close()
