@@ -2,9 +2,10 @@
 //
 // A call to g3l_eval turns its integrals into per-integral descriptors (sorted
 // by kind and term so each rule-evaluation kernel sees one integrand), sizes
-// the region pools from the evaluation caps, and runs one CUDA graph:
-//   k_init -> WHILE(any work) { k_select -> k_scan -> k_eval per group }
-// The loop condition is set on the device by k_scan, so the host waits once,
+// the region pools from the evaluation caps, and runs one CUDA graph, in which
+// every kind and term present has a loop of its own, side by side:
+//   k_init -> WHILE(any work) { k_select -> k_scan -> k_eval }
+// The loop conditions are set on the device by k_scan, so the host waits once,
 // at the end of the call.
 #include <cuda_runtime.h>
 #include <nvtx3/nvToolsExt.h>
