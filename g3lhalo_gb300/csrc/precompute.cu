@@ -34,6 +34,7 @@
 #include "g3l_gpu.h"
 #include "host_internal.h"
 #include "idiv64.cuh"
+#include "pc_nodes.cuh"
 
 namespace g3l {
 namespace {
@@ -154,11 +155,10 @@ struct PcNode {
     double x[15], g[15];     // abscissae and k^2 T^2 k^ns there
 };
 constexpr int PC_CACHE_LOG2 = 15;  // 32768 nodes, 8.4 MB (L2-resident)
-constexpr int PC_PROBES = 16;
 
 struct PcCache {
     PcNode *node;
-    unsigned *state;  // 0 free, 1 being filled, 2 ready
+    unsigned *state;  // NODE_FREE, NODE_FILLING, NODE_READY
 };
 
 __device__ __forceinline__ unsigned ld_acquire(const unsigned *p)
@@ -172,33 +172,29 @@ __device__ __forceinline__ void st_release(unsigned *p, unsigned v)
     asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
 
-// Find node (c, hw): mode 2 = ready at the returned slot, 1 = claimed by this caller (to
-// be filled and published), 0 = evaluate without the table.
+// the table as node_find sees it, for the node with key (k0, k1)
+struct PcProbe {
+    const PcCache &C;
+    unsigned long long k0, k1;
+    __device__ __forceinline__ unsigned acquire(int ix) const { return ld_acquire(C.state + ix); }
+    __device__ __forceinline__ unsigned claim(int ix) const
+    {
+        return atomicCAS(C.state + ix, (unsigned)NODE_FREE, (unsigned)NODE_FILLING);
+    }
+    __device__ __forceinline__ bool match(int ix) const
+    {
+        return __double_as_longlong(__ldcg(&C.node[ix].c)) == (long long)k0 &&
+               __double_as_longlong(__ldcg(&C.node[ix].hw)) == (long long)k1;
+    }
+};
+
+// find node (c, hw): node_find's mode and slot
 __device__ int pc_find(const PcCache &C, double c, double hw, int &mode)
 {
-    const unsigned long long k0 = (unsigned long long)__double_as_longlong(c);
-    const unsigned long long k1 = (unsigned long long)__double_as_longlong(hw);
-    unsigned ix = (unsigned)(((k0 * 0x9E3779B97F4A7C15ull) ^ (k1 * 0xC2B2AE3D27D4EB4Full)) >>
-                             (64 - PC_CACHE_LOG2));
-    for (int p = 0; p < PC_PROBES; ++p, ix = (ix + 1) & ((1u << PC_CACHE_LOG2) - 1)) {
-        unsigned st = ld_acquire(C.state + ix);
-        if (st == 0) {
-            st = atomicCAS(C.state + ix, 0u, 1u);
-            if (st == 0) {
-                mode = 1;
-                return (int)ix;
-            }
-        }
-        if (st == 1) break;  // being filled, perhaps by this node's first visitor
-        const double nc = __ldcg(&C.node[ix].c), nh = __ldcg(&C.node[ix].hw);
-        if (st == 2 && __double_as_longlong(nc) == (long long)k0 &&
-            __double_as_longlong(nh) == (long long)k1) {
-            mode = 2;
-            return (int)ix;
-        }
-    }
-    mode = 0;
-    return -1;
+    const PcProbe T{C, (unsigned long long)__double_as_longlong(c), (unsigned long long)__double_as_longlong(hw)};
+    const unsigned ix = (unsigned)(((T.k0 * 0x9E3779B97F4A7C15ull) ^ (T.k1 * 0xC2B2AE3D27D4EB4Full)) >>
+                                   (64 - PC_CACHE_LOG2));
+    return node_find(T, ix, (1u << PC_CACHE_LOG2) - 1, mode);
 }
 
 // lane hl < 15 stores its abscissa and factor of claimed slot ix; the caller publishes the
@@ -346,7 +342,7 @@ __global__ void __launch_bounds__(64) k_pc_warm(const PkDev *__restrict__ Pp, do
         pc_store(C, ix, c, hw, hl, x, k_factor(P, x));
     }
     __syncwarp();
-    if (mode == 1 && hl == 0) st_release(C.state + ix, 2u);
+    if (mode == 1 && hl == 0) st_release(C.state + ix, NODE_READY);
 }
 
 struct Heap {
@@ -730,7 +726,7 @@ struct PcEval {
                     f = k_integrand(t, x, g, amp);
                 }
                 __syncwarp();
-                if (hl == 0 && mode == 1) st_release(C.state + ix, 2u);
+                if (hl == 0 && mode == 1) st_release(C.state + ix, NODE_READY);
             }
             double v, e;
             rule_gk15_hw(f, hl, hw, v, e);
