@@ -41,4 +41,16 @@ __host__ __device__ __forceinline__ int node_find(Table &C, unsigned ix, unsigne
     return -1;
 }
 
+// Lane 0 of a half-warp has looked a node up; its other lanes take over the finding (every
+// lane of the warp calls).  Lanes: bcast(v), lane 0's v; sync(), a barrier of the warp that
+// orders memory.
+#pragma nv_exec_check_disable
+template <class Lanes>
+__host__ __device__ __forceinline__ void node_share(const Lanes &L, int &mode, int &ix)
+{
+    mode = L.bcast(mode);
+    ix = L.bcast(ix);
+    L.sync();  // lane 0's acquire load then comes before every lane's reads of the node
+}
+
 }  // namespace g3l

@@ -197,6 +197,12 @@ __device__ int pc_find(const PcCache &C, double c, double hw, int &mode)
     return node_find(T, ix, (1u << PC_CACHE_LOG2) - 1, mode);
 }
 
+// the half-warps of a warp as node_share sees them
+struct PcLanes {
+    __device__ __forceinline__ int bcast(int v) const { return __shfl_sync(0xffffffffu, v, 0, 16); }
+    __device__ __forceinline__ void sync() const { __syncwarp(); }
+};
+
 // lane hl < 15 stores its abscissa and factor of claimed slot ix; the caller publishes the
 // slot (st_release) after a __syncwarp
 __device__ __forceinline__ void pc_store(const PcCache &C, int ix, double c, double hw, int hl,
@@ -335,8 +341,7 @@ __global__ void __launch_bounds__(64) k_pc_warm(const PkDev *__restrict__ Pp, do
     const double hw = ldexp(0.5 * hi, -d), c = (2 * k + 1) * hw;
     int mode = 0, ix = -1;
     if (live && hl == 0) ix = pc_find(C, c, hw, mode);
-    mode = __shfl_sync(0xffffffffu, mode, 0, 16);
-    ix = __shfl_sync(0xffffffffu, ix, 0, 16);
+    node_share(PcLanes{}, mode, ix);
     if (mode == 1 && hl < 15) {
         const double x = gk_point(c, hw, hl);
         pc_store(C, ix, c, hw, hl, x, k_factor(P, x));
@@ -711,8 +716,7 @@ struct PcEval {
             } else {
                 int mode = 0, ix = -1;
                 if (live && hl == 0) ix = pc_find(C, c, hw, mode);
-                mode = __shfl_sync(0xffffffffu, mode, 0, 16);
-                ix = __shfl_sync(0xffffffffu, ix, 0, 16);
+                node_share(PcLanes{}, mode, ix);
                 if (on) {
                     double x, g;
                     if (mode == 2) {

@@ -3,7 +3,10 @@
 // 1, or prints "ok" and exits 0.
 #include <cstdio>
 #include <cstdlib>
+#include <thread>
 #include <vector>
+
+#include <pthread.h>
 
 #include "pc_nodes.cuh"
 
@@ -44,6 +47,73 @@ struct Table {
     }
 };
 
+// A warp of 32 threads.  seen[lane]: the slots whose publication the lane's reads are ordered
+// behind, a bit each; a broadcast moves a value and orders nothing, a barrier makes what any
+// lane is ordered behind hold for all.
+struct Warp {
+    pthread_barrier_t bar;
+    int val[32];
+    unsigned seen[32] = {};
+    Warp() { pthread_barrier_init(&bar, nullptr, 32); }
+    ~Warp() { pthread_barrier_destroy(&bar); }
+    void wait() { pthread_barrier_wait(&bar); }
+};
+struct Lanes {
+    Warp &w;
+    int lane;
+    int bcast(int v) const
+    {
+        w.val[lane] = v;
+        w.wait();
+        const int r = w.val[lane & 16];
+        w.wait();
+        return r;
+    }
+    void sync() const
+    {
+        unsigned all = 0;
+        w.wait();
+        for (unsigned s : w.seen) all |= s;
+        w.wait();
+        w.seen[lane] = all;
+        w.wait();
+    }
+};
+struct LaneTable {  // slots 3 and 9 are ready, the nodes of the first and the second half-warp
+    Warp &w;
+    int lane, want;
+    unsigned acquire(int ix) const
+    {
+        w.seen[lane] |= 1u << ix;
+        return NODE_READY;
+    }
+    unsigned claim(int) const { return NODE_READY; }
+    bool match(int ix) const { return ix == want; }
+};
+
+static void warp_reads_nodes()
+{
+    Warp w;
+    std::vector<std::thread> lanes;
+    bool ordered[32];
+    int slot[32], modes[32];
+    for (int lane = 0; lane < 32; ++lane)
+        lanes.emplace_back([&, lane] {
+            const LaneTable T{w, lane, lane < 16 ? 3 : 9};
+            int mode = 0, ix = -1;
+            if ((lane & 15) == 0) ix = node_find(T, 2, 31, mode);
+            node_share(Lanes{w, lane}, mode, ix);
+            slot[lane] = ix;
+            modes[lane] = mode;
+            ordered[lane] = ix >= 0 && ((w.seen[lane] >> ix) & 1u);
+        });
+    for (auto &t : lanes) t.join();
+    for (int lane = 0; lane < 32; ++lane) {
+        check(modes[lane] == 2 && slot[lane] == (lane < 16 ? 3 : 9), "lanes take over lane 0's finding");
+        check(ordered[lane], "a lane reads a node that only lane 0 is ordered behind");
+    }
+}
+
 int main()
 {
     int mode;
@@ -83,6 +153,7 @@ int main()
         for (int i = 0; i < PC_PROBES; ++i) t.state[i] = NODE_READY;
         check(node_find(t, 0, 31, mode) == -1 && mode == 0 && t.matches == PC_PROBES, "probe run exhausted");
     }
+    warp_reads_nodes();
     std::printf("ok\n");
     return 0;
 }
