@@ -21,10 +21,10 @@
 
 #include "g3l_device.cuh"
 #include "idiv64.cuh"
+#include "sel_bound.cuh"
 
 namespace g3l {
 
-constexpr int SEL_BS = 256;
 constexpr int SEL_WARPS = SEL_BS / 32;
 constexpr int SEL_BUCKETS = 1024;  // histogram of one selection pass (a multiple of SEL_BS)
 constexpr int SEL_PER = SEL_BUCKETS / SEL_BS;
@@ -50,17 +50,6 @@ __device__ T block_sum(T v, T *sh)
     r = sh[0];
     __syncthreads();
     return r;
-}
-
-// x 2^s as FP32, truncated (x >= 0); odd is set where x does not fit
-__device__ __forceinline__ float f32_scaled(double x, int s, bool &odd)
-{
-    const unsigned long long u = (unsigned long long)__double_as_longlong(x);
-    const int e = (int)((u >> 52) & 0x7ffu) - 1023 + s;
-    if (u == 0) return 0.f;
-    if (e < -126 || e > 60) odd = true;
-    const unsigned m = (unsigned)(u >> 29) & 0x7fffffu;
-    return e < -126 ? 0.f : __uint_as_float(((unsigned)min(e, 60) + 127u) << 23 | m);
 }
 
 // floor(t) of t >= 0, all ones from 1.8e19 on, by integer operations (an FP64 compare and
@@ -469,14 +458,9 @@ __global__ void __launch_bounds__(SEL_BS, 3) k_select(const IntDesc *__restrict_
             sh.tau_sel = tau_sel * fabs(V);
         }
         // the FP32 bound of the uncertainty each comparison below has, in units of 2^-sref:
-        // one that does not lie within 0.1% of the FP32 bound is settled by it, the others
-        // (and operands FP32 does not hold) take the FP64 sums
+        // one whose margin is clear of the FP32 bound's own rounding (f32_within) is settled by
+        // it, the others (and operands FP32 does not hold) take the FP64 sums
         const float fV = (float)rtol * vr32 * fuv_all, fU = gthr32 * (fue_all + fV);
-        // 0: dist > bound, 1: dist <= bound, 2: not told apart
-        auto within = [&](float dist, float bound, bool odd) {
-            return odd || !(bound > 1e-30f) || !(bound < 1e30f) || !(fabsf(dist - bound) > 1e-3f * bound)
-                       ? 2 : (int)(dist <= bound);
-        };
         // FP64 totals of the uncertainty, formed on demand
         auto exact_unc = [&](double &UE, double &UV) {
             double sue = 0, suv = 0;
@@ -520,7 +504,7 @@ __global__ void __launch_bounds__(SEL_BS, 3) k_select(const IntDesc *__restrict_
             if (guard && !cancel && finite && !(max_eval && neval >= max_eval)) {
                 bool od = odd;
                 const float dist = f32_scaled(fabs(E - gate), sref, od);
-                s_flag[3] = within(dist, fU, od);
+                s_flag[3] = f32_within(dist, fU, R, od);
             }
         }
         __syncthreads();
@@ -644,7 +628,7 @@ __global__ void __launch_bounds__(SEL_BS, 3) k_select(const IntDesc *__restrict_
                     const float m32 = (float)m * 8.67361738e-19f * f32_scaled(E, sref, od);  // m / scale
                     od = __syncthreads_or(od);
                     fur = block_sum(fur, sh.fred);
-                    int close = within(m32, gthr32 * (fur + fV), od);
+                    int close = f32_within(m32, gthr32 * (fur + fV), R, od);
                     if (close == 2) {
                         double ur = 0, UE, UV;
                         for (int j = threadIdx.x; j < R; j += SEL_BS)
