@@ -17,7 +17,7 @@ __host__ __device__ __forceinline__ float f32_scaled(double x, int s, bool &odd)
     const uint64_t u = bits_of(x);
     const int e = (int)((u >> 52) & 0x7ffu) - 1023 + s;
     if (u == 0) return 0.f;
-    if (e < -126 || e > 60) odd = true;
+    if (e < -126 || e > 60 || (u >> 52) == 0) odd = true;  // out of range, or a subnormal x
     const uint32_t m = (uint32_t)(u >> 29) & 0x7fffffu;
     return e < -126 ? 0.f : f32_of_bits((uint32_t)((e < 60 ? e : 60) + 127) << 23 | m);
 }

@@ -54,8 +54,22 @@ static void one(int pat, long long R)
     }
 }
 
+// f32_scaled: what it does not flag is x 2^s, cut to 24 bits
+static void scaled()
+{
+    const double x[] = {4.9406564584124654e-324, 1e-320, 1e-310, 2.2250738585072009e-308,
+                        2.2250738585072014e-308, 1e-300, 1e-100, 1.0, 1.5, 1e18, 1e300};
+    for (double v : x)
+        for (int s = -1100; s <= 1100; ++s) {
+            bool odd = false;
+            const double got = f32_scaled(v, s, odd), want = std::ldexp(v, s);
+            if (!odd && !(got <= want && got >= want * (1 - std::ldexp(1.0, -23)))) ++wrong;
+        }
+}
+
 int main()
 {
+    scaled();
     const long long R[] = {1, 31, 257, 4099, 100003, 1ll << 20, 1ll << 22, (1ll << 23) + 5, 1ll << 24, 1ll << 26};
     for (long long r : R)
         for (int pat = 0; pat < 4; ++pat) one(pat, r);
