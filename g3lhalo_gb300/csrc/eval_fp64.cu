@@ -740,10 +740,8 @@ struct Reeval {
     }
     // u_NFW tasks of m entries: [0, m NCU) the (l, m, z) combinations, then the k3 projections
     static constexpr int NCU = ucache_nf(TERM) * UC_MAX, NCU3 = u3_nfun(TERM) * U3_MAX;
-    // Up to about a block of 64 tasks per SM the pass is one chain whatever the lanes do, and
-    // its tasks are taken as numbered (listing them costs a call of one triplet 1-2%).  From
-    // there on they are listed first (k_re_fill).
-    __device__ static bool u_listed(int m) { return m * (NCU + NCU3) > 64 * 128; }
+    // are they listed first (ULIST_MIN)?
+    __device__ static bool u_listed(const Pool &P, int m) { return m * (NCU + NCU3) > P.ulist_min; }
     // does the entry need combination j of function f (split only: those of the centre and one
     // contender axis), and the k3 projection pr?
     __device__ static bool need_uc(const Pool &P, const IntDesc &d, int2 ent, const ReTab<KIND, TERM> &tb,
@@ -834,7 +832,7 @@ __global__ void __launch_bounds__(128) k_re_fill(DevTables T, const IntDesc *__r
     const long long tot = b4 + (long long)m * NLS;
     // The u_NFW tasks of k_re_ucache, packed over the whole queue: listed by the other end of
     // the grid, which has no task here in a round of few entries.
-    const int nu = R::u_listed(m) ? m * (R::NCU + R::NCU3) : 0;
+    const int nu = R::u_listed(P, m) ? m * (R::NCU + R::NCU3) : 0;
     const int usize = re_chunk_size(nu, 128);
     const int ufirst = (int)(gridDim.x - 1 - blockIdx.x) * usize;
     if (ufirst < nu) {
@@ -942,7 +940,7 @@ __global__ void __launch_bounds__(128) k_re_ucache(DevTables T, const IntDesc *_
     const int m = R::count(P, H, stage);
     if (m == 0) return;
     const int b1 = m * R::NCU;
-    const bool listed = R::u_listed(m);
+    const bool listed = R::u_listed(P, m);
     const int nu = listed ? min(H->n_ulist[R::G], R::ulist_cap(P)) : m * (R::NCU + R::NCU3);
     const long long a1 = warps_up((long long)m * R::NAUX);
     const long long na = a1 + (KIND == 0 ? (long long)m * TERM * NVAR : 0);

@@ -123,11 +123,16 @@ struct Pool {
     unsigned char *rscr;
     long long rscr_group;   // bytes per group
     int rcap;
+    int ulist_min;          // u_NFW tasks of a queue beyond which they are listed (k_re_fill)
     // the point tables of the re-evaluation passes, RETAB_BYTES per group (built once per
     // context by k_re_tables)
     const unsigned char *retab;
 };
 constexpr int RETAB_BYTES = 4096;
+// Up to about a block of 64 u_NFW tasks per SM the pass that evaluates them is one chain
+// whatever its lanes do, and they are taken as numbered (listing them costs a call of one
+// triplet 1-2%); from there on they are listed first (220 triplets 49.1 -> 46.3 ms).
+constexpr int ULIST_MIN = 64 * 128;
 
 // u_NFW at k3 = |l1 + l2| / w with one halo mass does not depend on the other mass
 // dimensions (2- and 3-halo terms), so the rule points that differ only there share it:

@@ -94,6 +94,18 @@ int reeval_cap(int n_integrals)
     return (int)std::min<long long>(std::max<long long>(4ll * n_integrals, 8192), 524288);
 }
 
+// G3L_REEVAL_LIST=<n> (read as above): u_NFW tasks of a queue beyond which they are listed, in
+// place of ULIST_MIN, so that tests can hold the two forms of the pass against each other
+// (0: always listed, 2147483647: never).
+int reeval_list_min()
+{
+    if (const char *e = std::getenv("G3L_REEVAL_LIST")) {
+        const long long v = std::atoll(e);
+        if (v >= 0) return (int)std::min<long long>(v, 0x7fffffff);
+    }
+    return ULIST_MIN;
+}
+
 struct Workspace {
     size_t pool_cap = 0;
     int n_cap = 0;
@@ -362,6 +374,7 @@ int alloc_workspace(Workspace &W, int ncap, size_t pcap, const unsigned char *re
     st |= dalloc(&W.P.key, pcap);
     st |= dalloc(&W.P.esc, pcap);
     W.P.rcap = reeval_cap(ncap);
+    W.P.ulist_min = reeval_list_min();
     W.P.rscr_group = reeval_scratch_group_bytes(W.P.rcap);
     st |= dalloc(&W.P.rscr, (size_t)(NGROUPS * W.P.rscr_group));
     st |= dalloc(&W.D, (size_t)ncap);
@@ -2335,6 +2348,7 @@ int eval_static_locked(g3l_ctx *c, const g3l_integral *items, int n, int precisi
     a.P.rscr = base + L.rscr;
     a.P.retab = c->retab_d;
     a.P.rcap = kStaticReevalCap;
+    a.P.ulist_min = ULIST_MIN;
     a.P.rscr_group = reeval_scratch_group_bytes(kStaticReevalCap);
     a.P.stride = (long long)pool;
     a.handle = 0;
