@@ -219,20 +219,20 @@ static __device__ __noinline__ float u_nfw32(float kr, float c, float small_arg,
             a2e = e;
         }
     }
-    // which product of a pair is fused is written out: left to the compiler it changes with
-    // the code around it, and with it the last bit
+    // which products are fused is written out: left to the compiler it can change with the
+    // code around it, and with it the last bit
     float N;
     if (a2 < 4.f) {
         const float dS = a2a - a1a;
         const float dC = lnopc + (a2b - a1b);
         N = fmaf(s1, dS, c1 * dC) - __fdividef(sk, a2);
     } else if (a1 >= 4.f) {
-        N = a1b - a2b * ck + a2e * sk;  // g(a1) - g(a2) cos(kr) + (f(a2) - 1/a2) sin(kr)
+        N = fmaf(a2e, sk, fmaf(-a2b, ck, a1b));  // g(a1) - g(a2) cos(kr) + (f(a2) - 1/a2) sin(kr)
     } else {
         const float f2 = a2a, g2 = a2b;
         const float s2 = fmaf(s1, ck, c1 * sk);  // sin(a1 + a1 c)
         const float c2 = fmaf(c1, ck, -(s1 * sk));
-        const float Si2 = HALF_PI_F - f2 * c2 - g2 * s2;
+        const float Si2 = fmaf(-g2, s2, fmaf(-f2, c2, HALF_PI_F));
         const float Ci2 = fmaf(f2, s2, -(g2 * c2));
         const float Si1 = a1a;
         const float Ci1 = GAMMA_F + __logf(a1) + a1b;
