@@ -476,9 +476,9 @@ __device__ inline void aux_tables(const uint32_t *sdesc, uint8_t *auxrep, uint8_
 // Point tables of a group's kernels: the point codes, the (l, m, z)
 // combinations of the cached u_NFW (ucache_tables) and the projections of the k3 u_NFW
 // (u3_tables) and of the auxiliary functions (aux_tables).  The same for every launch, so
-// k_re_tables builds them once per context into P.retab and each block copies what it needs
-// to shared memory (building them per block cost more than the cached work saves).
-// The members up to ucidx are all that the FP32 rule kernels read.
+// k_re_tables builds them once per context into P.retab and each block copies its group's
+// to shared memory (building them per block cost more than the cached work saves).  The
+// FP32 rule kernels read all of it, as the FP64 ones.
 template <int KIND, int TERM>
 struct ReTab {
     static constexpr int DIM = TERM + 4, NP = rule_points(DIM), NF = ucache_nf(TERM);
@@ -494,15 +494,13 @@ struct ReTab {
 };
 
 // copy group (KIND, TERM)'s tables to shared memory buf (every thread calls it)
-// (its first `bytes` bytes)
 template <int KIND, int TERM>
-__device__ inline const ReTab<KIND, TERM> &load_retab(const Pool &P, unsigned char *buf,
-                                                      int bytes = (int)sizeof(ReTab<KIND, TERM>))
+__device__ inline const ReTab<KIND, TERM> &load_retab(const Pool &P, unsigned char *buf)
 {
     using RT = ReTab<KIND, TERM>;
     const uint32_t *src =
         reinterpret_cast<const uint32_t *>(P.retab + (KIND * 3 + TERM - 1) * RETAB_BYTES);
-    for (int i = threadIdx.x; i < (bytes + 3) / 4; i += blockDim.x)
+    for (int i = threadIdx.x; i < (int)(sizeof(RT) / 4); i += blockDim.x)
         reinterpret_cast<uint32_t *>(buf)[i] = __ldg(src + i);
     __syncthreads();
     return *reinterpret_cast<const RT *>(buf);

@@ -34,7 +34,6 @@
 
 namespace g3l {
 void *eval64_kernel(int kind, int term);
-void *reeval64_kernel(int kind, int term);
 void *reeval_phase_kernel(int kind, int term, int phase);
 cudaError_t build_reeval_tables(unsigned char *out, cudaStream_t s);
 void *evalmx_kernel_k0(int term, int variant);
@@ -80,11 +79,12 @@ int dalloc(T **p, size_t n)
 }
 
 // FP64 re-evaluation entries per group and round that take the device-wide passes
-// (7.9 kB of scratch each): 4 per integral, between 8192 (65 MB per group) and 524288
-// (4.2 GB per group); further entries take the batched kernel k_reeval64, which
+// (9.2 kB of scratch each): 4 per integral, between 8192 (75 MB per group) and 524288
+// (4.8 GB per group); further entries take the batched kernel k_reeval64, which
 // evaluates every point on its own.  G3L_REEVAL_CAP=<n> (read when a workspace is
 // allocated) sets the count instead: 0 sends every entry through the batched kernel, so
 // that tests can hold the passes' cached values against it.
+static_assert(reeval_scratch_group_bytes(8192) == 8192ll * 9216, "re-evaluation scratch per entry");
 int reeval_cap(int n_integrals)
 {
     if (const char *e = std::getenv("G3L_REEVAL_CAP")) {

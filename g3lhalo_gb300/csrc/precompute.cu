@@ -1215,7 +1215,9 @@ void free_nbar_device(NbarDevice &W)
 }
 
 namespace {
-constexpr int kNbarChunk = 64;  // HOD vectors per launch (29 MB of factor tables)
+// HOD vectors per launch.  Their factor tables, (NBAR_NODES + 22 (Nm - 1)) x 15 x 8 bytes a
+// vector, stay allocated with the context: 29 MB at 128 mass bins, 58 MB at 300.
+constexpr int kNbarChunk = 64;
 constexpr int kNbarCapSmall = 1024;      // live regions of the first pass
 }  // namespace
 
