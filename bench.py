@@ -47,14 +47,14 @@ sys.path.insert(0, ROOT)
 METRIC = "NNMap evals/s (220 triplets,1h+2h+3h,rtol 1e-4) mixed vs FP64; p50/p99 ms"
 MAX_EVAL = 1_000_000
 RTOL = 1e-4
-# FP32 operations per integrand point of the NNMap 2-halo rule (algorithmic): the
-# integrand with its u_NFW calls de-duplicated within a point, counted by ncu as thread-
-# level fadd + fmul + 2 ffma on the kernel version that evaluated every u_NFW per point
-# (3.434e11 over 2.2005e8 points of the benchmark).  DRAM traffic per launch (read +
-# write): a launch of the kernel on the 110-triplet case (7.0 MB per ms of kernel
-# time), scaled by duration to the benchmark's mean launch (15.1 ms / 28 launches);
+# FP32 operations per integrand point of the NNMap 2-halo rule: what the kernel executes with
+# u_NFW, P_lin and the aperture filter shared by the points of a work item, counted by ncu as
+# thread-level fadd + fmul + 2 ffma (8.318e9 over the 1.334e7 points of three rounds of the
+# 110-triplet case; a kernel that evaluated every u_NFW per point took 1561).  DRAM traffic
+# per launch (read + write): a launch of the kernel on the 110-triplet case (7.0 MB per ms of
+# kernel time), scaled by duration to the benchmark's mean launch (15.1 ms / 28 launches);
 # profiles/k_evalmx_nnmap2h.md.
-FLOPS_PER_POINT = {"nnmap_2h": 1561.0}
+FLOPS_PER_POINT = {"nnmap_2h": 624.0}
 DRAM_BYTES_PER_LAUNCH = {"nnmap_2h": 3.8e6}
 # Pipe utilisation (% of peak while the SMs are active) of the dominant kernels, from one
 # ncu capture each (profiles/k_evalmx_nnmap2h.md, profiles/k_re_ucache_nnmap.md,
@@ -62,7 +62,7 @@ DRAM_BYTES_PER_LAUNCH = {"nnmap_2h": 3.8e6}
 PIPES_NCU = {
     "k_evalmx<NNMap,2h> (FP32 rule)": {"fma": 37.5, "alu": 38.9, "xu_mufu": 6.5, "fp64": 9.0,
                                        "warps_active": 34.0},
-    "k_re_ucache<NNMap,2h> (FP64 re-evaluation, u_NFW)": {"fp64": 72.0},
+    "k_re_ucache<NNMap,2h> (FP64 re-evaluation, u_NFW)": {"fp64": 78.0, "warps_active": 38.9},
     "k_nbar (n_bar integrals)": {"fp64": 33.5},
     "k_pc_integrate (table precompute)": {"fp64": 81.2, "fma": 4.0, "xu_mufu": 0.2},
 }
